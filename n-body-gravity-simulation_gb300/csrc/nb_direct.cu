@@ -21,12 +21,14 @@
 //    scaled by G in FP64.
 //    The tensor cores stay idle: a softened 1/r^3 sum is not a contraction.
 //
-//  * direct_fp64_kernel -- the 1e-12 path: the same tiling in FP64.
+//  * direct_fp64_pairs_kernel -- the 1e-12 path: an FP64 sum over unordered
+//    pairs of 32-body tiles (direct_fp64_row_kernel, a warp per body, for small n).
 //
-// Grid: x = i-blocks of BLOCK*IPT bodies, y = j-segments.  The j-split keeps
+// Grid of the mixed kernel: x = i-blocks of BLOCK*IPT bodies, y = j-segments.  The j-split keeps
 // all 152 SMs busy at small N (the reference runs 4 CTAs at N = 1024) and the
 // segment count is chosen to fill whole waves.
 #include "nb_internal.h"
+#include "nb_fp64pair.cuh"
 #include "nb_pair.cuh"
 
 #include <algorithm>
@@ -146,80 +148,218 @@ __global__ void combine_mixed_kernel(const float *__restrict__ psum,
     az[i] = G * ((double)hi[2] + (double)lo[2]);
 }
 
-template <int BLOCK, int IPT, bool ZERO_SOFT>
-__global__ void __launch_bounds__(BLOCK)
-direct_fp64_kernel(const double *__restrict__ x, const double *__restrict__ y,
-                   const double *__restrict__ z, const double *__restrict__ m, int n,
-                   double eps2, int seg_len, double *__restrict__ part)
+// ---------------------------------------------------------------- FP64
+// Small systems: one warp sums a body's whole row, lanes striding over j, and
+// reduces it with shuffles, so no partial sums and no second launch.  Bound by
+// the latency of a few dependent FP64 operations (8.1 us at n = 100; one-warp
+// CTAs of 32 bodies walking all j took 77 us there).  Up to 512 bodies: beyond,
+// its 16 FP64 operations per ordered pair cost more than the pairs kernel's 10
+// and a combine.
+template <bool ZERO_SOFT>
+__global__ void __launch_bounds__(32)
+direct_fp64_row_kernel(const double *__restrict__ x, const double *__restrict__ y,
+                       const double *__restrict__ z, const double *__restrict__ m, int n,
+                       double eps2, double G, double *__restrict__ ax, double *__restrict__ ay,
+                       double *__restrict__ az)
 {
-    __shared__ double4_32a sh[BLOCK];
-    const int tid = threadIdx.x;
-    const int ibase = blockIdx.x * (BLOCK * IPT);
-    double xi[IPT], yi[IPT], zi[IPT], ax[IPT], ay[IPT], az[IPT];
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = ibase + k * BLOCK + tid;
-        xi[k] = (i < n) ? x[i] : 0.0;
-        yi[k] = (i < n) ? y[i] : 0.0;
-        zi[k] = (i < n) ? z[i] : 0.0;
-        ax[k] = ay[k] = az[k] = 0.0;
-    }
-    const int j0 = blockIdx.y * seg_len;
-    const int j1 = min(n, j0 + seg_len);
-    for (int t0 = j0; t0 < j1; t0 += BLOCK) {
-        const int j = t0 + tid;
-        double4_32a b = make_double4_32a(1.0e150, 1.0e150, 1.0e150, 0.0);
-        if (j < j1) b = make_double4_32a(x[j], y[j], z[j], m[j]);
-        __syncthreads();
-        sh[tid] = b;
-        __syncthreads();
+    const int i = blockIdx.x;
+    const double xi = x[i], yi = y[i], zi = z[i];
+    double a[3] = {0.0, 0.0, 0.0};
 #pragma unroll 2
-        for (int jj = 0; jj < BLOCK; ++jj) {
-            const double4_32a B = sh[jj];
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) {
-                const double dx = B.x - xi[k];
-                const double dy = B.y - yi[k];
-                const double dz = B.z - zi[k];
-                const double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2)));
-                double inv = rsqrt(r2);
-                if (ZERO_SOFT) inv = (r2 > 0.0) ? inv : 0.0;
-                const double s = B.w * inv * inv * inv;
-                ax[k] = fma(dx, s, ax[k]);
-                ay[k] = fma(dy, s, ay[k]);
-                az[k] = fma(dz, s, az[k]);
-            }
-        }
+    for (int j = threadIdx.x; j < n; j += 32) {
+        const double dx = x[j] - xi, dy = y[j] - yi, dz = z[j] - zi;
+        const double s = m[j] * inv_cube<ZERO_SOFT>(fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
+        a[0] = fma(dx, s, a[0]);
+        a[1] = fma(dy, s, a[1]);
+        a[2] = fma(dz, s, a[2]);
     }
-    const size_t plane = (size_t)n;
-    const size_t base = (size_t)blockIdx.y * 3 * plane;
 #pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = ibase + k * BLOCK + tid;
-        if (i < n) {
-            part[base + i] = ax[k];
-            part[base + plane + i] = ay[k];
-            part[base + 2 * plane + i] = az[k];
-        }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
+    if (threadIdx.x == 0) {
+        ax[i] = G * a[0];
+        ay[i] = G * a[1];
+        az[i] = G * a[2];
     }
 }
 
-__global__ void combine_fp64_kernel(const double *__restrict__ part, int n, int segments,
-                                    double G, double *__restrict__ ax, double *__restrict__ ay,
-                                    double *__restrict__ az)
+// One step of a tile pair: the lane's i-body and the j-body it holds now.  The
+// pair's r^-3 serves both bodies: 20 FP64 operations for two interactions,
+// where a sum over ordered pairs spends 16 on each.
+struct Fp64Body {
+    double x, y, z, m;
+};
+template <bool ZERO_SOFT, bool BOTH>
+__device__ __forceinline__ void fp64_pair(const Fp64Body &bi, const Fp64Body &bj, double eps2,
+                                          bool valid, double (&ai)[3], double (&aj)[3])
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t plane = (size_t)n;
-    double a[3] = {0.0, 0.0, 0.0};
-    for (int s = 0; s < segments; ++s) {
-        const size_t base = (size_t)s * 3 * plane;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) a[c] += part[base + c * plane + i];
+    const double dx = bj.x - bi.x, dy = bj.y - bi.y, dz = bj.z - bi.z;
+    double q = inv_cube<ZERO_SOFT>(fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
+    q = valid ? q : 0.0;
+    const double si = bj.m * q;
+    ai[0] = fma(dx, si, ai[0]);
+    ai[1] = fma(dy, si, ai[1]);
+    ai[2] = fma(dz, si, ai[2]);
+    if (BOTH) {
+        const double sj = -(bi.m * q);
+        aj[0] = fma(dx, sj, aj[0]);
+        aj[1] = fma(dy, sj, aj[1]);
+        aj[2] = fma(dz, sj, aj[2]);
     }
-    ax[i] = G * a[0];
-    ay[i] = G * a[1];
-    az[i] = G * a[2];
+}
+
+__device__ __forceinline__ Fp64Body fp64_load(const double *__restrict__ x,
+                                              const double *__restrict__ y,
+                                              const double *__restrict__ z,
+                                              const double *__restrict__ m, int n, int i)
+{
+    if (i >= n) return Fp64Body{0.0, 0.0, 0.0, 0.0};
+    return Fp64Body{x[i], y[i], z[i], m[i]};
+}
+
+__device__ __forceinline__ Fp64Body fp64_rotate(const Fp64Body &b, int src)
+{
+    return Fp64Body{__shfl_sync(0xffffffffu, b.x, src), __shfl_sync(0xffffffffu, b.y, src),
+                    __shfl_sync(0xffffffffu, b.z, src), __shfl_sync(0xffffffffu, b.m, src)};
+}
+
+// One CTA = one block pair of diagonal p (blocks of 32 T bodies).  A warp holds
+// body l of an i-tile in lane l; the bodies of a j-tile and their sums rotate
+// through the lanes by shuffles, so at step s lane l meets body (l + s) mod 32
+// and adds to both sums: no partial of the j side leaves the registers before
+// its tile is done.  The i-tile's sums stay in registers over the second block,
+// the second block's in shared memory over the first; each is written once, to
+// the plane of its (diagonal, side).  Small systems (T == 1) split the 32
+// rotations of their one tile pair over the WARPS warps of the CTA.
+// Bound by the FP64 pipe: 86 % busy at n = 10,000, 1.98 ms for 5.0e7 pairs (the
+// sum over ordered pairs: 3.63 ms); 28 us at n = 1024 (57).
+template <bool ZERO_SOFT, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS)
+direct_fp64_pairs_kernel(const double *__restrict__ x, const double *__restrict__ y,
+                         const double *__restrict__ z, const double *__restrict__ m, int n,
+                         double eps2, int blocks, int T, int p0, int np,
+                         double *__restrict__ part)
+{
+    extern __shared__ double sums[];  // [WARPS][3][32 T] of the j side, [WARPS][3][32] of the i side
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, next = (lane + 1) & 31;
+    const int a = blockIdx.x % blocks, dp = blockIdx.x / blocks, p = p0 + dp;
+    if (!pair_first(p, a, blocks)) return;
+    const int b = (a + p) % blocks;
+    const int width = 32 * T;
+    const int a0 = a * width, b0 = b * width;
+    const int ta = min(T, (n - a0 + 31) / 32), tb = min(T, (n - b0 + 31) / 32);
+    double *jsum = sums + (size_t)w * 3 * width;
+    double *isum = sums + (size_t)WARPS * 3 * width;  // used when WARPS > 1
+    for (int k = lane; k < 3 * width; k += 32) jsum[k] = 0.0;
+    __syncwarp();
+    const size_t plane = 3 * (size_t)n;
+    double *pa = part + (size_t)dp * plane;
+    double *pb = part + (size_t)(np + dp) * plane;
+    for (int u = 0; u < ta; ++u) {
+        const int i = a0 + 32 * u + lane;
+        const Fp64Body bi = fp64_load(x, y, z, m, n, i);
+        double ai[3] = {0.0, 0.0, 0.0};
+        for (int v = p == 0 ? u : 0; v < tb; ++v) {
+            const bool self = p == 0 && u == v;
+            // the steps of this warp; a tile with itself needs 1 .. 16, the
+            // last of which meets every pair from both sides
+            const int steps = self ? 16 : 32, s0 = steps * w / WARPS + self,
+                      s1 = steps * (w + 1) / WARPS + self;
+            const int j0 = b0 + 32 * v;
+            Fp64Body bj = fp64_load(x, y, z, m, n, j0 + ((lane + s0) & 31));
+            double aj[3] = {0.0, 0.0, 0.0};
+            for (int s = s0; s < s1; ++s) {
+                const bool valid = i < n && j0 + ((lane + s) & 31) < n;
+                if (self && s == 16)
+                    fp64_pair<ZERO_SOFT, false>(bi, bj, eps2, valid, ai, aj);
+                else
+                    fp64_pair<ZERO_SOFT, true>(bi, bj, eps2, valid, ai, aj);
+                bj = fp64_rotate(bj, next);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) aj[c] = __shfl_sync(0xffffffffu, aj[c], next);
+            }
+            // the sums lane l holds now belong to body (l + s1) mod 32
+            const int at = 32 * v + ((lane + s1) & 31);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) jsum[c * width + at] += aj[c];
+            __syncwarp();
+        }
+        if (WARPS == 1) {
+            if (i < n)
+#pragma unroll
+                for (int c = 0; c < 3; ++c)  // within a block: what the tile took as a j-tile too
+                    pa[(size_t)c * n + i] =
+                        p == 0 ? ai[c] + jsum[c * width + 32 * u + lane] : ai[c];
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) isum[(w * 3 + c) * 32 + lane] = ai[c];
+        }
+    }
+    if (WARPS == 1) {
+        if (p == 0) return;
+        for (int v = 0; v < tb; ++v) {
+            const int j = b0 + 32 * v + lane;
+            if (j < n)
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    pb[(size_t)c * n + j] = jsum[c * width + 32 * v + lane];
+        }
+        return;
+    }
+    // T == 1: warp c (mod WARPS) adds the warps' sums of component c in order
+    __syncthreads();
+    for (int c = w; c < 3; c += WARPS) {
+        double si = 0.0, sj = 0.0;
+#pragma unroll
+        for (int k = 0; k < WARPS; ++k) {
+            si += isum[(k * 3 + c) * 32 + lane];
+            sj += sums[(k * 3 + c) * 32 + lane];
+        }
+        if (a0 + lane < n) pa[(size_t)c * n + a0 + lane] = p == 0 ? si + sj : si;
+        if (p > 0 && b0 + lane < n) pb[(size_t)c * n + b0 + lane] = sj;
+    }
+}
+
+// a_i = G * the sum of body i's planes in a fixed order: 8 bodies per block, 32
+// groups of planes in strides, each group's sum in order, then a fixed tree.
+// Large systems take their diagonals in several passes (add: a already holds
+// the earlier passes' sums, not yet scaled; last: scale by G).
+__global__ void __launch_bounds__(256)
+combine_fp64_kernel(const double *__restrict__ part, int n, int blocks, int width, int p0, int np,
+                    bool add, bool last, double G, double *__restrict__ ax,
+                    double *__restrict__ ay, double *__restrict__ az)
+{
+    __shared__ double sh[8][3][8];
+    const int body = threadIdx.x & 7, g = threadIdx.x >> 3;
+    const int i = blockIdx.x * 8 + body;
+    double s[3] = {0.0, 0.0, 0.0};
+    if (i < n) {
+        const int blk = i / width;
+#pragma unroll 4
+        for (int k = g; k < 2 * np; k += 32) {
+            const int p = p0 + (k < np ? k : k - np);
+            const bool use = k < np ? pair_first(p, blk, blocks) : pair_second(p, blk, blocks);
+            const double *src = part + (size_t)k * 3 * n + i;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) s[c] += use ? src[(size_t)c * n] : 0.0;
+        }
+    }
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+    if ((threadIdx.x & 31) < 8)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) sh[threadIdx.x >> 5][c][body] = s[c];
+    __syncthreads();
+    if (threadIdx.x >= 24 || i >= n) return;  // threads 8 c + body finish component c
+    const int c = threadIdx.x >> 3;
+    double *out = c == 0 ? ax : (c == 1 ? ay : az);
+    double t = ((sh[0][c][body] + sh[1][c][body]) + (sh[2][c][body] + sh[3][c][body])) +
+               ((sh[4][c][body] + sh[5][c][body]) + (sh[6][c][body] + sh[7][c][body]));
+    if (add) t = out[i] + t;
+    out[i] = last ? G * t : t;
 }
 
 __global__ void split_kernel(const double *__restrict__ x, const double *__restrict__ y,
@@ -269,9 +409,8 @@ int resident_ctas(const void *fn)
 
 constexpr int kMixBlock = 256;
 constexpr int kMixIpt = 4;
-constexpr int kF64Block = 128;
-constexpr int kF64Ipt = 2;
-constexpr int kF64SmallMax = 8192;  // largest N of the one-warp FP64 shape
+constexpr int kF64RowMax = 512;  // largest N of the one-warp-per-body FP64 kernel
+constexpr size_t kF64PlaneBytes = (size_t)512 << 20;  // FP64 partial planes per pass
 
 // Tile shapes of the mixed kernel the autotuner chooses from: threads per CTA
 // x i-bodies per thread.  More i-bodies per thread amortise the two
@@ -494,47 +633,76 @@ nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, doub
     return NB_OK;
 }
 
-template <int B, int I>
-static nb_status direct_fp64_shape(const double *x, const double *y, const double *z,
-                                   const double *m, int n, double G, double eps2, double *ax,
-                                   double *ay, double *az, DevBuf &partials, cudaStream_t st,
-                                   const KernelTimer *timer)
+// Tiles of 32 bodies per block of the FP64 block-pair sum: as many as leave 12
+// warps per SM (fewer partial planes), which fill the FP64 pipes evenly.  A
+// function of n and the SM count alone, so the bits of a result are too.
+static int fp64_tiles(int n)
 {
-    const int per_cta = B * I;
-    const int iblocks = (n + per_cta - 1) / per_cta;
-    const int tiles = (n + B - 1) / B;
-    static const int slots = resident_ctas<B, I>((const void *)direct_fp64_kernel<B, I, false>);
-    int segs = pick_segments(iblocks, tiles, slots);
-    const int seg_tiles = (tiles + segs - 1) / segs;
-    segs = (tiles + seg_tiles - 1) / seg_tiles;
-    NB_TRY(partials.reserve(sizeof(double) * 3 * (size_t)n * segs));
-    double *part = partials.as<double>();
-    dim3 grid(iblocks, segs);
-    const int seg_len = seg_tiles * B;
-    if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
-    if (eps2 > 0.0)
-        direct_fp64_kernel<B, I, false><<<grid, B, 0, st>>>(x, y, z, m, n, eps2, seg_len, part);
-    else
-        direct_fp64_kernel<B, I, true><<<grid, B, 0, st>>>(x, y, z, m, n, 0.0, seg_len, part);
-    NB_LAUNCH_CHECK();
-    if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
-    combine_fp64_kernel<<<(n + 255) / 256, 256, 0, st>>>(part, n, segs, G, ax, ay, az);
-    NB_LAUNCH_CHECK();
-    return NB_OK;
+    auto block_pairs = [&](int T) {
+        const long M = (n + 32 * T - 1) / (32 * T);
+        return M * (M + 1) / 2;
+    };
+    int T = 1;
+    while (T < 8 && block_pairs(2 * T) >= 12 * device_props().num_sms) T *= 2;
+    return T;
 }
 
-// Small systems take one-warp CTAs with 32-body j-tiles, so that up to
-// (N/32)^2 CTAs share the FP64 work (N = 1024 with the large shape fills only
-// 32 CTAs); large systems take 128 x 2.
+template <bool ZERO_SOFT>
+static void launch_fp64_pairs(const double *x, const double *y, const double *z, const double *m,
+                              int n, double eps2, int blocks, int T, int p0, int np, double *part,
+                              cudaStream_t st)
+{
+    const unsigned grid = (unsigned)blocks * (unsigned)np;
+    // one tile pair per CTA: four warps share it, so that 1024 bodies still
+    // give each SM 14 warps
+    if (T == 1)
+        direct_fp64_pairs_kernel<ZERO_SOFT, 4><<<grid, 128, sizeof(double) * 96 * 8, st>>>(
+            x, y, z, m, n, eps2, blocks, T, p0, np, part);
+    else
+        direct_fp64_pairs_kernel<ZERO_SOFT, 1><<<grid, 32, sizeof(double) * 96 * (size_t)T, st>>>(
+            x, y, z, m, n, eps2, blocks, T, p0, np, part);
+}
+
 nb_status direct_fp64(const double *x, const double *y, const double *z, const double *m, int n,
                       double G, double eps2, double *ax, double *ay, double *az,
                       DevBuf &partials, cudaStream_t st, const KernelTimer *timer)
 {
     if (n <= 0) return NB_OK;
-    if (n <= kF64SmallMax)
-        return direct_fp64_shape<32, 1>(x, y, z, m, n, G, eps2, ax, ay, az, partials, st, timer);
-    return direct_fp64_shape<kF64Block, kF64Ipt>(x, y, z, m, n, G, eps2, ax, ay, az, partials,
-                                                 st, timer);
+    if (n <= kF64RowMax) {
+        if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
+        if (eps2 > 0.0)
+            direct_fp64_row_kernel<false><<<n, 32, 0, st>>>(x, y, z, m, n, eps2, G, ax, ay, az);
+        else
+            direct_fp64_row_kernel<true><<<n, 32, 0, st>>>(x, y, z, m, n, 0.0, G, ax, ay, az);
+        NB_LAUNCH_CHECK();
+        if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
+        return NB_OK;
+    }
+    const int T = fp64_tiles(n);
+    const int blocks = (n + 32 * T - 1) / (32 * T);
+    const int diagonals = blocks / 2 + 1;
+    // planes of 3 n doubles, two per diagonal; bounded by taking the diagonals
+    // in passes
+    const size_t per_diagonal = sizeof(double) * 6 * (size_t)n;
+    const int pass = (int)std::min<size_t>(
+        diagonals, std::max<size_t>(1, kF64PlaneBytes / per_diagonal));
+    NB_TRY(partials.reserve(per_diagonal * pass));
+    double *part = partials.as<double>();
+    if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
+    for (int p0 = 0; p0 < diagonals; p0 += pass) {
+        const int np = std::min(pass, diagonals - p0);
+        if (eps2 > 0.0)
+            launch_fp64_pairs<false>(x, y, z, m, n, eps2, blocks, T, p0, np, part, st);
+        else
+            launch_fp64_pairs<true>(x, y, z, m, n, 0.0, blocks, T, p0, np, part, st);
+        NB_LAUNCH_CHECK();
+        const bool last = p0 + np == diagonals;
+        if (last && timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
+        combine_fp64_kernel<<<(n + 7) / 8, 256, 0, st>>>(part, n, blocks, 32 * T, p0, np, p0 > 0,
+                                                         last, G, ax, ay, az);
+        NB_LAUNCH_CHECK();
+    }
+    return NB_OK;
 }
 
 } // namespace nb
