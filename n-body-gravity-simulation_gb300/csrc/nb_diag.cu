@@ -6,11 +6,11 @@
 //   - per-body sums (kinetic energy, angular momentum, centre of mass, linear
 //     momentum, mass): one HBM-bound pass (56 B per body), block partials in a
 //     fixed tree order, then one block that adds the partials in index order;
-//   - potential energy: an O(N^2) FP64 pass (one thread per body i, j-tiles in
-//     shared memory, j in index order) that returns per-body sums
-//     sum_{j != i} m_j / r_ij, unsoftened and softened, reduced like the above.
+//   - potential energy: an O(N^2 / 2) FP64 pass over unordered pairs, unsoftened
+//     and softened together, reduced like the above.
 // All reductions have a fixed order, so results do not depend on scheduling.
 #include "nb_internal.h"
+#include "nb_fp64pair.cuh"
 
 #include <algorithm>
 
@@ -68,68 +68,100 @@ body_sums_kernel(const double *__restrict__ x, const double *__restrict__ y,
         for (int c = 0; c < kNSum; ++c) part[blockIdx.x * kNSum + c] = acc[c];
 }
 
-// Per-body potential sums: pu[i] = sum_{j!=i} m_j / r_ij,
-// ps[i] = sum_{j!=i} m_j / sqrt(r_ij^2 + eps2).
-__global__ void __launch_bounds__(kRed)
-potential_rows_kernel(const double *__restrict__ x, const double *__restrict__ y,
-                      const double *__restrict__ z, const double *__restrict__ m, int n,
-                      double eps2, double *__restrict__ pu, double *__restrict__ ps)
+// Potential sums over unordered pairs, unsoftened and softened: the warp of
+// block pair (p, a) holds 32 bodies of the first block in its lanes and rotates
+// the tiles of the second through them (the schedule of nb_fp64pair.cuh), so
+// each pair is met once.  Per pair 19 FP64 operations (13 without softening,
+// where the two sums are equal); the seed's integer work is free beside them.
+// Warps take block pairs in strides of the grid, a fixed assignment:
+// part[2 w], part[2 w + 1] = warp w's sums.  One-warp CTAs: with four warps a
+// CTA's slowest warp holds the others' places (8.31 ms instead of 7.70 at
+// n = 20,000).  Bound by the FP64 pipe, 84 % busy (the per-body rows that this
+// replaces, each pair met twice with a square root and a division a term: 56.2).
+template <bool SOFT>
+__global__ void __launch_bounds__(32)
+potential_pairs_kernel(const double *__restrict__ x, const double *__restrict__ y,
+                       const double *__restrict__ z, const double *__restrict__ m, int n,
+                       double eps2, int blocks, int T, long items, double *__restrict__ part)
 {
-    __shared__ double4_32a sh[kRed];
-    const int i = blockIdx.x * kRed + threadIdx.x;
-    const double xi = i < n ? x[i] : 0.0, yi = i < n ? y[i] : 0.0, zi = i < n ? z[i] : 0.0;
-    double su = 0.0, ss = 0.0;
-    for (int t0 = 0; t0 < n; t0 += kRed) {
-        const int j = t0 + threadIdx.x;
-        __syncthreads();
-        sh[threadIdx.x] = j < n ? make_double4_32a(x[j], y[j], z[j], m[j])
-                                : make_double4_32a(0.0, 0.0, 0.0, 0.0);
-        __syncthreads();
-        const int lim = min(kRed, n - t0);
-        for (int jj = 0; jj < lim; ++jj) {
-            if (t0 + jj == i) continue;
-            const double4_32a B = sh[jj];
-            const double dx = B.x - xi, dy = B.y - yi, dz = B.z - zi;
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            su += B.w / sqrt(r2);
-            ss += B.w / sqrt(r2 + eps2);
+    const int lane = threadIdx.x, next = (lane + 1) & 31;
+    const int width = 32 * T;
+    double tu = 0.0, ts = 0.0;
+    for (long it = blockIdx.x; it < items; it += gridDim.x) {
+        const int a = (int)(it % blocks), p = (int)(it / blocks);
+        if (!pair_first(p, a, blocks)) continue;
+        const int b = (a + p) % blocks;
+        const int ta = min(T, (n - a * width + 31) / 32), tb = min(T, (n - b * width + 31) / 32);
+        for (int u = 0; u < ta; ++u) {
+            const int i = a * width + 32 * u + lane;
+            const bool iv = i < n;
+            const double xi = iv ? x[i] : 0.0, yi = iv ? y[i] : 0.0, zi = iv ? z[i] : 0.0;
+            double su = 0.0, ss = 0.0;
+            for (int v = p == 0 ? u : 0; v < tb; ++v) {
+                const bool self = p == 0 && u == v;
+                const int j0 = b * width + 32 * v;
+                // a tile with itself: steps 1 .. 15 meet a pair once, step 16
+                // from both sides (the lower half of the lanes takes it)
+                const int s0 = self ? 1 : 0, s1 = self ? 17 : 32;
+                const int j = j0 + ((lane + s0) & 31);
+                double xj = j < n ? x[j] : 0.0, yj = j < n ? y[j] : 0.0, zj = j < n ? z[j] : 0.0,
+                       mj = j < n ? m[j] : 0.0;
+                for (int s = s0; s < s1; ++s) {
+                    const bool valid = iv && j0 + ((lane + s) & 31) < n &&
+                                       !(self && s == 16 && lane >= 16);
+                    const double dx = xj - xi, dy = yj - yi, dz = zj - zi;
+                    const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+                    const double qu = inv_sqrt(r2);
+                    su = fma(valid ? mj : 0.0, valid ? qu : 0.0, su);
+                    if (SOFT) {
+                        const double qs = inv_sqrt(r2 + eps2);
+                        ss = fma(valid ? mj : 0.0, valid ? qs : 0.0, ss);
+                    }
+                    xj = __shfl_sync(0xffffffffu, xj, next);
+                    yj = __shfl_sync(0xffffffffu, yj, next);
+                    zj = __shfl_sync(0xffffffffu, zj, next);
+                    mj = __shfl_sync(0xffffffffu, mj, next);
+                }
+            }
+            if (iv) {
+                const double mi = m[i];
+                tu = fma(mi, su, tu);
+                if (SOFT) ts = fma(mi, ss, ts);
+            }
         }
     }
-    if (i < n) {
-        pu[i] = su;
-        ps[i] = ss;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        tu += __shfl_xor_sync(0xffffffffu, tu, o);
+        ts += __shfl_xor_sync(0xffffffffu, ts, o);
+    }
+    if (lane == 0) {
+        part[2 * (size_t)blockIdx.x] = tu;
+        part[2 * (size_t)blockIdx.x + 1] = SOFT ? ts : tu;
     }
 }
 
-// Final pass: one block.  Adds the body-sum partials in block order and the
-// per-body potential terms m_i * row_i in index order (per thread, then a
-// fixed tree).
-__global__ void __launch_bounds__(kRed)
-finish_kernel(const double *__restrict__ part, int nparts, const double *__restrict__ m,
-              const double *__restrict__ pu, const double *__restrict__ ps, int n,
-              double *__restrict__ out)
+// Final pass, one block: warp c adds the partials of sum c (kNSum body sums,
+// then the two potential sums), lanes in strides and a fixed tree.
+__global__ void __launch_bounds__(32 * (kNSum + 2))
+finish_kernel(const double *__restrict__ part, int nparts, const double *__restrict__ pot,
+              int npot, double *__restrict__ out)
 {
-    __shared__ double sh[2 * kRed];
-    const int t = threadIdx.x;
-    if (t == 0) {
-        double s[kNSum];
-        for (int c = 0; c < kNSum; ++c) s[c] = 0.0;
-        for (int b = 0; b < nparts; ++b)
-            for (int c = 0; c < kNSum; ++c) s[c] += part[b * kNSum + c];
-        for (int c = 0; c < kNSum; ++c) out[c] = s[c];
-    }
-    double v[2] = {0.0, 0.0};
-    if (pu) {
-        for (int i = t; i < n; i += kRed) {
-            v[0] += m[i] * pu[i];
-            v[1] += m[i] * ps[i];
-        }
-    }
-    block_reduce<2>(v, sh);
-    if (t == 0) {
-        out[kNSum + 0] = v[0];
-        out[kNSum + 1] = v[1];
-    }
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool body = c < kNSum;
+    const double *src = body ? part + c : pot + (c - kNSum);
+    const int count = body ? nparts : npot, stride = body ? kNSum : 2;
+    // four running sums: the FP64 add latency, not the loads, sets the time
+    double r[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+    for (int k = lane; k < count; k += 128)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            r[u] += k + 32 * u < count ? src[(size_t)(k + 32 * u) * stride] : 0.0;
+    double s = (r[0] + r[1]) + (r[2] + r[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[c] = s;
 }
 
 // FP32 pipe rate probe: every thread runs kFmaRounds rounds of kFmaChains
@@ -190,17 +222,31 @@ nb_status diagnostics(const double *x, const double *y, const double *z, const d
 {
     if (n <= 0) return fail(NB_ERR_NOT_LOADED, "diagnostics: no bodies");
     const int nparts = std::min((n + kRed - 1) / kRed, 4 * device_props().num_sms);
-    const size_t bytes = sizeof(double) * ((size_t)nparts * kNSum + 2 * (size_t)n + 16);
+    // blocks of up to 8 tiles while the block pairs fill the FP64 pipes evenly
+    int T = 1;
+    auto block_pairs = [&](int t) {
+        const long M = (n + 32 * t - 1) / (32 * t);
+        return M * (M / 2 + 1);
+    };
+    while (T < 8 && block_pairs(2 * T) >= 12 * device_props().num_sms) T *= 2;
+    const int blocks = (n + 32 * T - 1) / (32 * T);
+    const long items = block_pairs(T);
+    const int npot = (int)std::min<long>(items, 32 * device_props().num_sms);
+    const size_t bytes = sizeof(double) * ((size_t)nparts * kNSum + 2 * (size_t)npot + 16);
     NB_TRY(scratch.reserve(bytes));
     double *part = scratch.as<double>();
-    double *pu = part + (size_t)nparts * kNSum;
-    double *ps = pu + n;
-    double *res = ps + n;
+    double *pot = part + (size_t)nparts * kNSum;
+    double *res = pot + 2 * (size_t)npot;
     body_sums_kernel<<<nparts, kRed, 0, st>>>(x, y, z, vx, vy, vz, m, n, part);
     NB_LAUNCH_CHECK();
-    potential_rows_kernel<<<(n + kRed - 1) / kRed, kRed, 0, st>>>(x, y, z, m, n, eps2, pu, ps);
+    if (eps2 > 0.0)
+        potential_pairs_kernel<true><<<npot, 32, 0, st>>>(x, y, z, m, n, eps2, blocks,
+                                                                     T, items, pot);
+    else
+        potential_pairs_kernel<false><<<npot, 32, 0, st>>>(x, y, z, m, n, 0.0, blocks,
+                                                                      T, items, pot);
     NB_LAUNCH_CHECK();
-    finish_kernel<<<1, kRed, 0, st>>>(part, nparts, m, pu, ps, n, res);
+    finish_kernel<<<1, 32 * (kNSum + 2), 0, st>>>(part, nparts, pot, npot, res);
     NB_LAUNCH_CHECK();
     double h[kNSum + 2];
     NB_CUDA_TRY(cudaMemcpyAsync(h, res, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -214,9 +260,8 @@ nb_status diagnostics(const double *x, const double *y, const double *z, const d
         out->center_of_mass[c] = h[4 + c] / h[10];
         out->momentum[c] = h[7 + c];
     }
-    // each unordered pair appears twice in sum_i m_i row_i
-    out->potential = -0.5 * G * h[kNSum + 0];
-    out->potential_softened = -0.5 * G * h[kNSum + 1];
+    out->potential = -G * h[kNSum + 0];
+    out->potential_softened = -G * h[kNSum + 1];
     out->total = out->kinetic + out->potential;
     out->total_softened = out->kinetic + out->potential_softened;
     return NB_OK;

@@ -47,3 +47,22 @@ def test_fp64_forces_of_extreme_scales(nb, oracle):
         sabs = oracle.forces_abs_sum(*p, m, 1.0, 0.0)
         d = np.sqrt(sum(((u - v) / sabs) ** 2 for u, v in zip(a, ref)))
         assert (d <= 664 * 2.0 ** -53).all(), (scale, d.max())
+
+
+@pytest.mark.parametrize("n", [1, 2, 33, 64, 65, 1000, 3500, 7001])
+@pytest.mark.parametrize("eps", [0.0, 0.02])
+def test_potential_at_tile_edges(nb, oracle, n, eps):
+    """Every unordered pair once: against a sum over ordered pairs in NumPy."""
+    x, y, z, vx, vy, vz, m = nb.plummer(max(n, 3), seed=n)
+    st = [c[:n].copy() for c in (x, y, z, vx, vy, vz, m * np.linspace(0.5, 2.0, len(m)))]
+    with nb.Sim(nb.Config(method=nb.DIRECT_FP64, G=1.5, softening=eps), capacity=n) as s:
+        s.load(*st)
+        d = s.diagnostics()
+    p, mm = np.stack(st[:3]), st[6]
+    want = [0.0, 0.0]
+    for i in range(n - 1):
+        r2 = ((p[:, i + 1:] - p[:, i:i + 1]) ** 2).sum(0)
+        for k, e2 in enumerate((0.0, eps * eps)):
+            want[k] -= 1.5 * mm[i] * (mm[i + 1:] / np.sqrt(r2 + e2)).sum()
+    for got, w in zip((d["potential"], d["potential_softened"]), want):
+        assert abs(got - w) <= (n + 64) * 2.0 ** -53 * abs(w)
