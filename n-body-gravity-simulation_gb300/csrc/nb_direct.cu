@@ -127,8 +127,13 @@ direct_mixed_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo
 }
 
 // a_i = G * sum_s (sum_s - comp_s), segments in index order, accumulated as a
-// double-single and scaled in FP64.
-__global__ void combine_mixed_kernel(const float *__restrict__ psum,
+// double-single and scaled in FP64.  Bound by the latency of its loads: those of
+// 16 segments go out before their ordered sums, and 32-body CTAs spread a
+// small system over the SMs (22.1 us at n = 1000 and 32 segments with one load
+// waiting for the last sum in 256-body CTAs; 7.8 us now).
+constexpr int kCombineBlock = 32;
+__global__ void __launch_bounds__(kCombineBlock)
+combine_mixed_kernel(const float *__restrict__ psum,
                                      const float *__restrict__ pcomp, int n, int segments,
                                      double G, double *__restrict__ ax,
                                      double *__restrict__ ay, double *__restrict__ az)
@@ -137,11 +142,21 @@ __global__ void combine_mixed_kernel(const float *__restrict__ psum,
     if (i >= n) return;
     const size_t plane = (size_t)n;
     float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
-    for (int s = 0; s < segments; ++s) {
-        const size_t base = (size_t)s * 3 * plane;
+    for (int s0 = 0; s0 < segments; s0 += 16) {
+        float t[16][3], q[16][3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-            ds_add_kahan(hi[c], lo[c], psum[base + c * plane + i], pcomp[base + c * plane + i]);
+        for (int u = 0; u < 16; ++u)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const size_t at = ((size_t)(s0 + u) * 3 + c) * plane + i;
+                t[u][c] = s0 + u < segments ? psum[at] : 0.f;
+                q[u][c] = s0 + u < segments ? pcomp[at] : 0.f;
+            }
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (s0 + u < segments)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) ds_add_kahan(hi[c], lo[c], t[u][c], q[u][c]);
     }
     ax[i] = G * ((double)hi[0] + (double)lo[0]);
     ay[i] = G * ((double)hi[1] + (double)lo[1]);
@@ -627,8 +642,8 @@ nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, doub
         return fail(NB_ERR_UNSUPPORTED, "direct_mixed: unsupported tile shape");
     NB_LAUNCH_CHECK();
     if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
-    combine_mixed_kernel<<<(n + 255) / 256, 256, 0, st>>>(psum, pcomp, n, p.segments, G, ax, ay,
-                                                         az);
+    combine_mixed_kernel<<<(n + kCombineBlock - 1) / kCombineBlock, kCombineBlock, 0, st>>>(
+        psum, pcomp, n, p.segments, G, ax, ay, az);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
@@ -805,8 +820,8 @@ extern "C" nb_status nb_direct_mixed_forces_noalloc(size_t n, const double *x, c
     if (!launch_mixed(p, st, hi, lo, ni, eps2, psum, pcomp))
         return fail(NB_ERR_UNSUPPORTED, "nb_direct_mixed_forces_noalloc: tile shape");
     NB_LAUNCH_CHECK();
-    combine_mixed_kernel<<<(ni + 255) / 256, 256, 0, st>>>(psum, pcomp, ni, p.segments, G, ax,
-                                                          ay, az);
+    combine_mixed_kernel<<<(ni + kCombineBlock - 1) / kCombineBlock, kCombineBlock, 0, st>>>(
+        psum, pcomp, ni, p.segments, G, ax, ay, az);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
