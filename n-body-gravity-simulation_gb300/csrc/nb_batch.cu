@@ -1,28 +1,24 @@
-// nb_batch.cu -- many independent systems of uneven N in one persistent launch.
+// nb_batch.cu -- many independent systems of uneven N in one launch.
 //
 // No reference counterpart: the reference simulates one system per process.
 // A batch holds the bodies of every system in one pool of FP64 planes
 // (x y z vx vy vz ax ay az m, 80 B/body) plus the float4 hi/lo mirror of the
-// mixed pair term (32 B/body).  A system is a descriptor {first, n, ipt}: its
-// bodies are pool slots [first, first + n).
+// mixed pair term (32 B/body).  A system is a descriptor (SysDesc): its bodies
+// are pool slots [first, first + n), in blocks of kBatchBlockBodies.
 //
-// Forces.  The work queue holds one item per (system, 32*ipt i-bodies); items
-// are ordered by cost, largest first.  A persistent kernel (a fixed grid of
-// resident CTAs) lets every warp take the next item with one atomicAdd and
-// sum its system's j-bodies in tiles of 32 staged in the warp's own slice of
-// shared memory: the same double-single / folded-Newton pair term as the
-// single-system kernel, evaluated on j-pairs in packed f32x2 arithmetic, and a
-// Kahan-compensated add after every tile.  Each item writes only its own
-// i-bodies' accelerations, after summing j in index order, so a system's
-// result does not depend on what else is in the batch or on which warp ran
-// which item: a system gives the same bits alone and in any mix.
-//
-// ipt (i-bodies per lane) is chosen per N bucket (powers of two) by an
-// autotuner that times the candidates on the batch's own systems.
+// Forces.  A work item is a pair of blocks of one system (or 32 rows of a small
+// one); the items are ordered by cost, largest first, one one-warp CTA each.  The
+// warp evaluates every unordered pair of the two blocks once (nb_tile.cuh),
+// keeping the second block's sums in shared memory, and writes one partial sum
+// (a Kahan pair) per body of either block to that body's plane of the (diagonal,
+// side); a
+// second launch adds each body's planes in order as a double-single.  A system's
+// partial sums depend on that system alone: it gives the same bits alone and in
+// any mix.
 #include "nb_internal.h"
 #include "nb_check.cuh"
 #include "nb_curve.cuh"
-#include "nb_pair.cuh"
+#include "nb_tile.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -30,144 +26,334 @@
 namespace nb {
 namespace {
 
-constexpr int kBatchBlock = 128;  // 4 warps
-constexpr int kBatchWarps = kBatchBlock / 32;
-// Systems of at least this many bodies take two i-chunks per warp item in the
-// sorted variant (a fixed rule of n, so that a system's item shapes -- and its
-// bits -- do not depend on the other systems of the batch).
-constexpr int kSortedIpt2Min = 2048;
+constexpr int kBatchTiles = kBatchBlockBodies / kTile;  // tiles per block
+// One-warp CTAs per SM.  16 leave 128 registers, with which a step's loads run
+// ahead of its arithmetic: 7.69 ms for two RK4 steps of the 1024-system ensemble,
+// 18 / 20 / 21 CTAs 7.71 / 7.80 / 7.92.  Four-warp CTAs that share the second
+// block's sums behind barriers: 8.06.
+constexpr int kBatchCtas = 16;
 
-template <int IPT, bool ZERO_SOFT>
-__device__ __forceinline__ void batch_item(const float4 *__restrict__ hi,
-                                           const float4 *__restrict__ lo, const SysDesc &sd,
-                                           int i0, float eps2, double G, double *__restrict__ ax,
-                                           double *__restrict__ ay, double *__restrict__ az,
-                                           PairTile &pt)
+// Bounding box of a 64-body tile of sorted bodies (the union of its two chunk
+// boxes, box[4 t .. 4 t + 3] = min, max, min, max; an empty chunk has an inverted
+// box) and its squared diameter.
+struct TileBox {
+    float4 mn, mx;
+    float diam2;
+};
+__device__ __forceinline__ TileBox tile_box(const float4 *__restrict__ box, int t)
 {
-    const int lane = threadIdx.x & 31;
-    // i-bodies negated and duplicated into f32x2 pairs
-    float2 nxh[IPT], nyh[IPT], nzh[IPT], nxl[IPT], nyl[IPT], nzl[IPT];
-    float sx[IPT], sy[IPT], sz[IPT], cx[IPT], cy[IPT], cz[IPT];
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = i0 + k * 32 + lane;
-        float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
-        if (i < sd.n) {
-            h = hi[sd.first + i];
-            l = lo[sd.first + i];
-        }
-        nxh[k] = dup2(-h.x); nyh[k] = dup2(-h.y); nzh[k] = dup2(-h.z);
-        nxl[k] = dup2(-l.x); nyl[k] = dup2(-l.y); nzl[k] = dup2(-l.z);
-        sx[k] = sy[k] = sz[k] = 0.f;
-        cx[k] = cy[k] = cz[k] = 0.f;
+    const float4 a = box[4 * (size_t)t], b = box[4 * (size_t)t + 1], c = box[4 * (size_t)t + 2],
+                 d = box[4 * (size_t)t + 3];
+    TileBox r;
+    r.mn = make_float4(fminf(a.x, c.x), fminf(a.y, c.y), fminf(a.z, c.z), 0.f);
+    r.mx = make_float4(fmaxf(b.x, d.x), fmaxf(b.y, d.y), fmaxf(b.z, d.z), 0.f);
+    const float dx = r.mx.x - r.mn.x, dy = r.mx.y - r.mn.y, dz = r.mx.z - r.mn.z;
+    r.diam2 = dx * dx + dy * dy + dz * dz;
+    return r;
+}
+
+// The row of 32 i-bodies [i0, i0 + 32) of a small system against all its
+// j-bodies in 32-body chunks (ordered pairs): one warp, no partial sums.
+// SORTED: the chunk's box centre is the origin of the staged coordinates, and by
+// the gap to the i-chunk's box (diameter D) a j-chunk takes the double-single
+// term, the plain FP32 one (D/8) or that without the Newton step (D/4).
+template <bool SORTED, bool ZERO_SOFT>
+__device__ __forceinline__ void batch_row(const float4 *__restrict__ hi,
+                                          const float4 *__restrict__ lo,
+                                          const float4 *__restrict__ box, const SysDesc &sd,
+                                          int i0, float eps2, double G,
+                                          const uint32_t *__restrict__ order,
+                                          double *__restrict__ ax, double *__restrict__ ay,
+                                          double *__restrict__ az, PairTile &sg, int total)
+{
+    const int lane = threadIdx.x & 31, i = i0 + lane;
+    const int nch = (sd.n + 31) / 32;
+    const float4 *cb = box + 4 * (size_t)sd.tile0;  // two chunk boxes per tile
+    float4 bmn = make_float4(0.f, 0.f, 0.f, 0.f), bmx = bmn;
+    if (SORTED) {
+        bmn = cb[2 * (i0 / 32)];
+        bmx = cb[2 * (i0 / 32) + 1];
     }
-    const float2 e2 = dup2(eps2);
-    for (int t0 = 0; t0 < sd.n; t0 += 32) {
-        const int j = t0 + lane;
-        float4 h = far_body(), l = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float diam2 = (bmx.x - bmn.x) * (bmx.x - bmn.x) + (bmx.y - bmn.y) * (bmx.y - bmn.y) +
+                        (bmx.z - bmn.z) * (bmx.z - bmn.z);
+    const float thr2 = kFarFactor2 * diam2, thr2v = kVeryFar2 * diam2;
+    const float cx = 0.5f * (bmn.x + bmx.x), cy = 0.5f * (bmn.y + bmx.y),
+                cz = 0.5f * (bmn.z + bmx.z);
+    float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
+    if (i < sd.n) {
+        h = hi[sd.first + i];
+        l = lo[sd.first + i];
+    }
+    float S[3] = {h.x, h.y, h.z}, E[3] = {l.x, l.y, l.z};
+    if (SORTED) {
+        rel_ds(h.x, l.x, cx, S[0], E[0]);
+        rel_ds(h.y, l.y, cy, S[1], E[1]);
+        rel_ds(h.z, l.z, cz, S[2], E[2]);
+    }
+    const float2 nsx = dup2(-S[0]), nsy = dup2(-S[1]), nsz = dup2(-S[2]);
+    const float2 nex = dup2(-E[0]), ney = dup2(-E[1]), nez = dup2(-E[2]), e2 = dup2(eps2);
+    float sx = 0.f, sy = 0.f, sz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;
+    for (int jc = 0; jc < nch; ++jc) {
+        bool far = false, vfar = false;
+        if (SORTED) {
+            const float4 jmn = cb[2 * jc], jmx = cb[2 * jc + 1];
+            const float gx = fmaxf(0.f, fmaxf(jmn.x - bmx.x, bmn.x - jmx.x));
+            const float gy = fmaxf(0.f, fmaxf(jmn.y - bmx.y, bmn.y - jmx.y));
+            const float gz = fmaxf(0.f, fmaxf(jmn.z - bmx.z, bmn.z - jmx.z));
+            const float gap2 = gx * gx + gy * gy + gz * gz;
+            far = gap2 > 0.f && gap2 >= thr2;
+            vfar = far && gap2 >= thr2v;
+        }
+        // lanes past the system stage a massless body far away: exactly 0
+        float T[3] = {1.0e18f, 1.0e18f, 1.0e18f}, U[3] = {0.f, 0.f, 0.f}, mj = 0.f;
+        const int j = 32 * jc + lane;
         if (j < sd.n) {
             h = hi[sd.first + j];
             l = lo[sd.first + j];
+            if (SORTED && far) {
+                T[0] = rel_s(h.x, l.x, cx);
+                T[1] = rel_s(h.y, l.y, cy);
+                T[2] = rel_s(h.z, l.z, cz);
+            } else if (SORTED) {
+                rel_ds(h.x, l.x, cx, T[0], U[0]);
+                rel_ds(h.y, l.y, cy, T[1], U[1]);
+                rel_ds(h.z, l.z, cz, T[2], U[2]);
+            } else {
+                T[0] = h.x; T[1] = h.y; T[2] = h.z;
+                U[0] = l.x; U[1] = l.y; U[2] = l.z;
+            }
+            mj = h.w;
         }
         __syncwarp();
-        pair_tile_put(pt, lane, h.x, h.y, h.z, h.w, l.x, l.y, l.z);
+        pair_tile_put(sg, lane, T[0], T[1], T[2], mj, U[0], U[1], U[2]);
         __syncwarp();
-        float2 ax_[IPT], ay_[IPT], az_[IPT];
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) ax_[k] = ay_[k] = az_[k] = dup2(0.f);
-#pragma unroll 2
-        for (int p = 0; p < 16; ++p) {
-            const JPair jp = pair_tile_get(pt, p);
-#pragma unroll
-            for (int k = 0; k < IPT; ++k)
-                pair_term2<ZERO_SOFT>(jp, nxh[k], nyh[k], nzh[k], nxl[k], nyl[k], nzl[k], e2,
-                                      ax_[k], ay_[k], az_[k]);
+        float2 fx = dup2(0.f), fy = dup2(0.f), fz = dup2(0.f);
+        if (vfar) {
+#pragma unroll 4
+            for (int p = 0; p < 16; ++p)
+                pair_term2_far<false>(pair_tile_get(sg, p), nsx, nsy, nsz, e2, fx, fy, fz);
+        } else if (far) {
+#pragma unroll 4
+            for (int p = 0; p < 16; ++p)
+                pair_term2_far<true>(pair_tile_get(sg, p), nsx, nsy, nsz, e2, fx, fy, fz);
+        } else {
+#pragma unroll 4
+            for (int p = 0; p < 16; ++p)
+                pair_term2<ZERO_SOFT>(pair_tile_get(sg, p), nsx, nsy, nsz, nex, ney, nez, e2, fx,
+                                      fy, fz);
         }
+        kahan_add(sx, qx, fx.x + fx.y);
+        kahan_add(sy, qy, fy.x + fy.y);
+        kahan_add(sz, qz, fz.x + fz.y);
+    }
+    if (i >= sd.n) return;
+    const int o = SORTED ? (int)order[sd.first + i] : sd.first + i;
+    if (!NB_IN_RANGE(o, total)) return;
+    ax[o] = G * ((double)sx - (double)qx);
+    ay[o] = G * ((double)sy - (double)qy);
+    az[o] = G * ((double)sz - (double)qz);
+}
+
+// SORTED: the bodies are in Hilbert order with one box per tile; coordinates are
+// staged relative to the i-tile's box centre, and a tile pair at least a
+// quarter of the larger box's diameter apart takes the plain FP32 term
+// (kVeryFar2: the bounds of nb_direct_sorted.cu hold for both sides), others the
+// double-single one.  Otherwise every pair takes the double-single term.
+// Bound by the FP32 pipe, 75 % busy: 0.82 ms for the 8.4e8 unordered pairs of the
+// 1024-system ensemble, where one warp per 32 or 64 rows took 1.11 ms.
+template <bool SORTED, bool ZERO_SOFT>
+__global__ void __launch_bounds__(32, kBatchCtas)
+batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
+                   const float4 *__restrict__ boxes, const SysDesc *__restrict__ sys,
+                   const PairItem *__restrict__ items, float eps2, float2 *__restrict__ part,
+                   double G, const uint32_t *__restrict__ order, double *__restrict__ ax,
+                   double *__restrict__ ay, double *__restrict__ az, int total, int num_tiles)
+{
+    __shared__ union {
+        TileJ tile;
+        PairTile chunk;
+    } stages;
+    __shared__ TileSums sums[kBatchTiles];  // of the second block's tiles
+    __shared__ TileSums isum;               // of the i-tile
+    const int lane = threadIdx.x;
+    const PairItem it = items[blockIdx.x];
+    const SysDesc sd = sys[it.sys];
+    if (!NB_IN_RANGE(sd.first, total) || !NB_IN_RANGE(sd.first + sd.n - 1, total) ||
+        !NB_IN_RANGE(sd.tile0 + (sd.n - 1) / kTile, num_tiles))
+        return;
+    if (it.p < 0) {  // a small system: 32 rows, straight to the result
+        batch_row<SORTED, ZERO_SOFT>(hi, lo, boxes, sd, 32 * it.a, eps2, G, order, ax, ay, az,
+                                     stages.chunk, total);
+        return;
+    }
+    TileJ &stage = stages.tile;
+    const bool within = it.p == 0;  // the block with itself
+    const int blk_b = (it.a + it.p) % sd.blocks;
+    const int tiles = (sd.n + kTile - 1) / kTile;
+    const int ti0 = it.a * kBatchTiles, tj0 = blk_b * kBatchTiles;
+    const int ta = min(kBatchTiles, tiles - ti0), tb = min(kBatchTiles, tiles - tj0);
+    const float2 e2 = dup2(eps2);
+    const size_t plane = (size_t)sd.n;
+    float2 *pa = part + sd.part0 + 3 * plane * it.p;
+    float2 *pb = part + sd.part0 + 3 * plane * (sd.blocks / 2 + it.p);
+    for (int v = 0; v < kBatchTiles; ++v) tile_sums_zero(sums[v], lane);
+
+    for (int u = 0; u < ta; ++u) {
+        TileI ti;
+        TileBox bi{};
+        float cx = 0.f, cy = 0.f, cz = 0.f;
+        if (SORTED) {
+            bi = tile_box(boxes, sd.tile0 + ti0 + u);
+            cx = 0.5f * (bi.mn.x + bi.mx.x);
+            cy = 0.5f * (bi.mn.y + bi.mx.y);
+            cz = 0.5f * (bi.mn.z + bi.mx.z);
+        }
+        tile_sums_zero(isum, lane);
+        const int i0 = (ti0 + u) * kTile + lane;
 #pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            kahan_add(sx[k], cx[k], ax_[k].x + ax_[k].y);
-            kahan_add(sy[k], cy[k], ay_[k].x + ay_[k].y);
-            kahan_add(sz[k], cz[k], az_[k].x + az_[k].y);
+        for (int k = 0; k < 2; ++k) {
+            const int i = i0 + 32 * k;
+            // a lane past the system holds a massless body far from every j-body
+            float S[3] = {-1.0e18f, -1.0e18f, -1.0e18f}, E[3] = {0.f, 0.f, 0.f}, mi = 0.f;
+            if (i < sd.n) {
+                const float4 h = hi[sd.first + i], l = lo[sd.first + i];
+                if (SORTED) {
+                    rel_ds(h.x, l.x, cx, S[0], E[0]);
+                    rel_ds(h.y, l.y, cy, S[1], E[1]);
+                    rel_ds(h.z, l.z, cz, S[2], E[2]);
+                } else {
+                    S[0] = h.x; S[1] = h.y; S[2] = h.z;
+                    E[0] = l.x; E[1] = l.y; E[2] = l.z;
+                }
+                mi = h.w;
+            }
+            tile_i_set(ti, k, S[0], S[1], S[2], E[0], E[1], E[2], mi);
+        }
+        for (int v = within ? u : 0; v < tb; ++v) {
+            const int tj = tj0 + v;
+            bool far = false;
+            if (SORTED) {
+                const TileBox bj = tile_box(boxes, sd.tile0 + tj);
+                const float gx = fmaxf(0.f, fmaxf(bj.mn.x - bi.mx.x, bi.mn.x - bj.mx.x));
+                const float gy = fmaxf(0.f, fmaxf(bj.mn.y - bi.mx.y, bi.mn.y - bj.mx.y));
+                const float gz = fmaxf(0.f, fmaxf(bj.mn.z - bi.mx.z, bi.mn.z - bj.mx.z));
+                const float gap2 = gx * gx + gy * gy + gz * gz;
+                far = gap2 > 0.f && gap2 >= kVeryFar2 * fmaxf(bi.diam2, bj.diam2);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int h2 = 0; h2 < 2; ++h2) {
+                const int j = tj * kTile + 32 * h2 + lane;
+                // lanes past the system stage a massless body far away: exactly 0
+                float S[3] = {1.0e18f, 1.0e18f, 1.0e18f}, E[3] = {0.f, 0.f, 0.f}, mj = 0.f;
+                if (j < sd.n) {
+                    const float4 h = hi[sd.first + j], l = lo[sd.first + j];
+                    if (SORTED) {
+                        rel_ds(h.x, l.x, cx, S[0], E[0]);
+                        rel_ds(h.y, l.y, cy, S[1], E[1]);
+                        rel_ds(h.z, l.z, cz, S[2], E[2]);
+                    } else {
+                        S[0] = h.x; S[1] = h.y; S[2] = h.z;
+                        E[0] = l.x; E[1] = l.y; E[2] = l.z;
+                    }
+                    mj = h.w;
+                }
+                tile_j_put(stage, lane, h2, S[0], S[1], S[2], E[0], E[1], E[2], mj);
+            }
+            __syncwarp();
+            if (within && u == v)
+                tile_self<ZERO_SOFT>(stage, lane, 0, 4, ti, e2, isum);
+            else if (far)
+                tile_pair<false, ZERO_SOFT>(stage, lane, 0, 4, ti, e2, isum, sums[v]);
+            else
+                tile_pair<true, ZERO_SOFT>(stage, lane, 0, 4, ti, e2, isum, sums[v]);
+        }
+        // the i-tile's partial sums; within a block with what it took as a j-tile
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            float2 t = isum.s[c][lane], e = isum.c[c][lane];
+            if (within) {
+                const float2 js = sums[u].s[c][lane], jc = sums[u].c[c][lane];
+                float2 r;
+                two_sum(t.x, js.x, t.x, r.x);
+                two_sum(t.y, js.y, t.y, r.y);
+                e = make_float2(r.x + (e.x + jc.x), r.y + (e.y + jc.y));
+            }
+            if (i0 < sd.n) pa[c * plane + i0] = make_float2(t.x, e.x);
+            if (i0 + 32 < sd.n) pa[c * plane + i0 + 32] = make_float2(t.y, e.y);
         }
     }
+    if (within) return;
+    for (int v = 0; v < tb; ++v) {
+        const int j = (tj0 + v) * kTile + lane;
 #pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = i0 + k * 32 + lane;
-        if (i < sd.n) {
-            ax[sd.first + i] = G * ((double)sx[k] - (double)cx[k]);
-            ay[sd.first + i] = G * ((double)sy[k] - (double)cy[k]);
-            az[sd.first + i] = G * ((double)sz[k] - (double)cz[k]);
+        for (int c = 0; c < 3; ++c) {
+            const float2 js = sums[v].s[c][lane], jc = sums[v].c[c][lane];
+            if (j < sd.n) pb[c * plane + j] = make_float2(js.x, jc.x);
+            if (j + 32 < sd.n) pb[c * plane + j + 32] = make_float2(js.y, jc.y);
         }
     }
 }
 
-template <bool ZERO_SOFT>
-__global__ void __launch_bounds__(kBatchBlock)
-batch_force_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
-                   const SysDesc *__restrict__ sys, const WorkItem *__restrict__ items,
-                   int num_items, int *__restrict__ counter, float eps2, double G,
-                   double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
-                   int total)
+// a = G * the sum of a body's planes in order (diagonal 0, 1, ... of the first
+// side, then 1, 2, ... of the second), as a double-single: one block per block
+// of bodies; order (sorted batches): the pool slot of a sorted body.
+__global__ void __launch_bounds__(kBatchBlockBodies)
+batch_combine_kernel(const float2 *__restrict__ part, const SysDesc *__restrict__ sys,
+                     const PairItem *__restrict__ items, const uint32_t *__restrict__ order,
+                     double G, double *__restrict__ ax, double *__restrict__ ay,
+                     double *__restrict__ az, int total)
 {
-    __shared__ PairTile tiles[kBatchWarps];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    while (true) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(counter, 1);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= num_items) break;
-        const WorkItem w = items[item];
-        const SysDesc sd = sys[w.sys];
-        if (!NB_IN_RANGE(sd.first, total) || !NB_IN_RANGE(sd.first + sd.n - 1, total)) continue;
-        switch (sd.ipt) {
-        case 1:
-            batch_item<1, ZERO_SOFT>(hi, lo, sd, w.i0, eps2, G, ax, ay, az,
-                                     tiles[warp]);
-            break;
-        case 2:
-            batch_item<2, ZERO_SOFT>(hi, lo, sd, w.i0, eps2, G, ax, ay, az,
-                                     tiles[warp]);
-            break;
-        default:
-            batch_item<4, ZERO_SOFT>(hi, lo, sd, w.i0, eps2, G, ax, ay, az,
-                                     tiles[warp]);
-            break;
+    const PairItem it = items[blockIdx.x];  // (system, block, 0)
+    const SysDesc sd = sys[it.sys];
+    const int i = it.a * kBatchBlockBodies + threadIdx.x;
+    if (i >= sd.n || !NB_IN_RANGE(sd.first + i, total)) return;
+    const size_t plane = (size_t)sd.n;
+    const float2 *src = part + sd.part0 + i;
+    const int half = sd.blocks / 2, planes = 2 * half + 1;
+    float s[3] = {0.f, 0.f, 0.f}, r[3] = {0.f, 0.f, 0.f};
+    for (int k0 = 0; k0 < planes; k0 += 4) {
+        float2 t[4][3];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k = k0 + u;
+            const bool use = k < planes && (k <= half ? pair_first(k, it.a, sd.blocks)
+                                                      : pair_second(k - half, it.a, sd.blocks));
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                t[u][c] = use ? src[(3 * (size_t)k + c) * plane] : dup2(0.f);
         }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) ds_add_kahan(s[c], r[c], t[u][c].x, -t[u][c].y);
     }
-}
-
-int batch_grid()
-{
-    // a function-local static: initialised once, thread-safe
-    static const int grid = [] {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, (const void *)batch_force_kernel<false>, kBatchBlock, 0);
-        return std::max(1, per_sm) * device_props().num_sms;
-    }();
-    return grid;
+    const int o = order ? (int)order[sd.first + i] : sd.first + i;
+    if (!NB_IN_RANGE(o, total)) return;
+    ax[o] = G * ((double)s[0] + (double)r[0]);
+    ay[o] = G * ((double)s[1] + (double)r[1]);
+    az[o] = G * ((double)s[2] + (double)r[2]);
 }
 
 // ---------------------------------------------------------------- sorted
 // The Hilbert-sorted variant (ensemble): every system's bodies are sorted
-// along a Hilbert curve through the cube around that system alone, so a
-// 32-body chunk of sorted bodies is spatially compact; a warp item is one
-// i-chunk, its box centre is the origin of its staged j-chunks, and j-chunks
-// far from its box take the plain FP32 term (see nb_direct_sorted.cu).  Every
-// quantity a system's result depends on -- its order, its centre, its chunk
-// boxes, each item's classification -- is computed from that system alone, so
-// a system still gives the same bits alone and in any mix.
+// along a Hilbert curve through the cube around that system alone, so a 64-body
+// tile of sorted bodies is spatially compact.  Every quantity a system's result
+// depends on -- its order, its centre, its tile boxes, each tile pair's
+// classification -- is computed from that system alone, so a system still
+// gives the same bits alone and in any mix.
 
-// body_sys[i] = s for the bodies of system s; chunk table entries (first
-// body, count) of its 32-body chunks.
+// body_sys[i] = s for the bodies of system s; tile table entries (first body,
+// count, system) of its 64-body tiles.
 __global__ void batch_layout_kernel(const SysDesc *__restrict__ sys, int *__restrict__ body_sys,
-                                    int2 *__restrict__ chunks)
+                                    int4 *__restrict__ tiles)
 {
     const SysDesc sd = sys[blockIdx.x];
     for (int i = threadIdx.x; i < sd.n; i += blockDim.x) body_sys[sd.first + i] = blockIdx.x;
-    const int nch = (sd.n + 31) / 32;
-    for (int c = threadIdx.x; c < nch; c += blockDim.x)
-        chunks[sd.chunk0 + c] = make_int2(sd.first + 32 * c, min(32, sd.n - 32 * c));
+    const int nt = (sd.n + kTile - 1) / kTile;
+    for (int c = threadIdx.x; c < nt; c += blockDim.x)
+        tiles[sd.tile0 + c] = make_int4(sd.first + kTile * c, min(kTile, sd.n - kTile * c),
+                                        blockIdx.x, 0);
 }
 
 // geom[s] = (centre x, y, z, side) of the cube around system s: one block per
@@ -245,234 +431,46 @@ batch_key_kernel(const double *__restrict__ x, const double *__restrict__ y,
 }
 
 // Sorted positions relative to their system's centre, split into hi/lo
-// (double-single) parts; mass in hi.w.
+// (double-single) parts, mass in hi.w, and the bounding box of every 32-body
+// chunk: one warp per chunk, two chunks per tile (an empty one gets an inverted
+// box).
 __global__ void __launch_bounds__(256)
 batch_split_sorted_kernel(const uint32_t *__restrict__ order, const double *__restrict__ x,
                           const double *__restrict__ y, const double *__restrict__ z,
-                          const double *__restrict__ m, const int *__restrict__ body_sys,
-                          const double4 *__restrict__ geom, int n, float4 *__restrict__ hi,
-                          float4 *__restrict__ lo)
+                          const double *__restrict__ m, const int4 *__restrict__ tiles,
+                          int num_tiles, const double4 *__restrict__ geom, int total,
+                          float4 *__restrict__ hi, float4 *__restrict__ lo,
+                          float4 *__restrict__ box)
 {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t o = order[i];
-    if (!NB_IN_RANGE(o, n)) return;
-    const double4 g = geom[body_sys[i]];
-    const double X = x[o] - g.x, Y = y[o] - g.y, Z = z[o] - g.z;
-    const float hx = __double2float_rn(X), hy = __double2float_rn(Y), hz = __double2float_rn(Z);
-    hi[i] = make_float4(hx, hy, hz, __double2float_rn(m[o]));
-    lo[i] = make_float4(__double2float_rn(X - (double)hx), __double2float_rn(Y - (double)hy),
-                        __double2float_rn(Z - (double)hz), 0.0f);
-}
-
-// Bounding box of every chunk (one warp per chunk): box[2g] = min, box[2g+1] = max.
-__global__ void batch_chunk_box_kernel(const float4 *__restrict__ hi,
-                                       const int2 *__restrict__ chunks, int num_chunks,
-                                       float4 *__restrict__ box)
-{
-    const int g = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    const int lane = threadIdx.x & 31;
-    if (g >= num_chunks) return;
-    const int2 ch = chunks[g];
-    const float4 p = hi[ch.x + (lane < ch.y ? lane : 0)];
-    float mn[3] = {p.x, p.y, p.z}, mx[3] = {p.x, p.y, p.z};
+    const int ch = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (ch >= 2 * num_tiles) return;
+    const int4 tl = tiles[ch >> 1];  // first body, count, system
+    const double4 g = geom[tl.z];
+    float mn[3] = {3.0e38f, 3.0e38f, 3.0e38f}, mx[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+    const int l = 32 * (ch & 1) + lane, i = tl.x + l;
+    const uint32_t o = l < tl.y ? order[i] : 0u;
+    if (l < tl.y && NB_IN_RANGE(o, total)) {
+        const double X = x[o] - g.x, Y = y[o] - g.y, Z = z[o] - g.z;
+        const float hx = __double2float_rn(X), hy = __double2float_rn(Y),
+                    hz = __double2float_rn(Z);
+        hi[i] = make_float4(hx, hy, hz, __double2float_rn(m[o]));
+        lo[i] = make_float4(__double2float_rn(X - (double)hx), __double2float_rn(Y - (double)hy),
+                            __double2float_rn(Z - (double)hz), 0.0f);
+        mn[0] = mx[0] = hx;
+        mn[1] = mx[1] = hy;
+        mn[2] = mx[2] = hz;
+    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int s = 16; s > 0; s >>= 1)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-            mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+        for (int c = 0; c < 3; ++c) {
+            mn[c] = fminf(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], s));
+            mx[c] = fmaxf(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], s));
         }
     if (lane == 0) {
-        box[2 * g] = make_float4(mn[0], mn[1], mn[2], 0.f);
-        box[2 * g + 1] = make_float4(mx[0], mx[1], mx[2], 0.f);
+        box[2 * (size_t)ch] = make_float4(mn[0], mn[1], mn[2], 0.f);
+        box[2 * (size_t)ch + 1] = make_float4(mx[0], mx[1], mx[2], 0.f);
     }
-}
-
-// One warp item = IPT consecutive 32-body i-chunks of a system (lane l holds
-// body l of each) against all its j-chunks.  The items's box (the union of its
-// i-chunk boxes, diameter D) is the origin of the staged j-chunks: near chunks
-// (closer than D/8) take the double-single term, far ones the plain FP32
-// term, very far ones (D/4) the plain term without the Newton step; each
-// chunk's 16 terms per accumulator lane are folded into Kahan sums.
-template <int IPT, bool ZERO_SOFT>
-__device__ __forceinline__ void batch_sorted_item(const float4 *__restrict__ hi,
-                                                  const float4 *__restrict__ lo,
-                                                  const float4 *__restrict__ box,
-                                                  const SysDesc &sd, int i0, float eps2,
-                                                  double G, const uint32_t *__restrict__ order,
-                                                  double *__restrict__ ax,
-                                                  double *__restrict__ ay,
-                                                  double *__restrict__ az, PairTile &sg,
-                                                  int total)
-{
-    const int lane = threadIdx.x & 31;
-    const int nch = (sd.n + 31) / 32;
-    const int ic0 = i0 / 32;
-    float4 bmn = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f);
-    float4 bmx = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.f);
-#pragma unroll
-    for (int k = 0; k < IPT; ++k)
-        if (ic0 + k < nch) {
-            const float4 a = box[2 * (sd.chunk0 + ic0 + k)], b = box[2 * (sd.chunk0 + ic0 + k) + 1];
-            bmn = make_float4(fminf(bmn.x, a.x), fminf(bmn.y, a.y), fminf(bmn.z, a.z), 0.f);
-            bmx = make_float4(fmaxf(bmx.x, b.x), fmaxf(bmx.y, b.y), fmaxf(bmx.z, b.z), 0.f);
-        }
-    const float diam2 = (bmx.x - bmn.x) * (bmx.x - bmn.x) + (bmx.y - bmn.y) * (bmx.y - bmn.y) +
-                        (bmx.z - bmn.z) * (bmx.z - bmn.z);
-    const float thr2 = kFarFactor2 * diam2, thr2v = kVeryFar2 * diam2;
-    const float cx = 0.5f * (bmn.x + bmx.x), cy = 0.5f * (bmn.y + bmx.y),
-                cz = 0.5f * (bmn.z + bmx.z);
-    float2 nsx[IPT], nsy[IPT], nsz[IPT], nex[IPT], ney[IPT], nez[IPT];
-    float sx[IPT], sy[IPT], sz[IPT], qx[IPT], qy[IPT], qz[IPT];
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = i0 + 32 * k + lane;
-        float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
-        if (i < sd.n) {
-            h = hi[sd.first + i];
-            l = lo[sd.first + i];
-        }
-        float S, E;
-        rel_ds(h.x, l.x, cx, S, E);
-        nsx[k] = dup2(-S);
-        nex[k] = dup2(-E);
-        rel_ds(h.y, l.y, cy, S, E);
-        nsy[k] = dup2(-S);
-        ney[k] = dup2(-E);
-        rel_ds(h.z, l.z, cz, S, E);
-        nsz[k] = dup2(-S);
-        nez[k] = dup2(-E);
-        sx[k] = sy[k] = sz[k] = qx[k] = qy[k] = qz[k] = 0.f;
-    }
-    const float2 e2 = dup2(eps2);
-    float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
-    bool valid = lane < sd.n;
-    if (valid) {
-        h = hi[sd.first + lane];
-        l = lo[sd.first + lane];
-    }
-    for (int jc = 0; jc < nch; ++jc) {
-        const float4 jmn = box[2 * (sd.chunk0 + jc)], jmx = box[2 * (sd.chunk0 + jc) + 1];
-        const float gx = fmaxf(0.f, fmaxf(jmn.x - bmx.x, bmn.x - jmx.x));
-        const float gy = fmaxf(0.f, fmaxf(jmn.y - bmx.y, bmn.y - jmx.y));
-        const float gz = fmaxf(0.f, fmaxf(jmn.z - bmx.z, bmn.z - jmx.z));
-        const float gap2 = gx * gx + gy * gy + gz * gz;
-        const bool far = gap2 > 0.f && gap2 >= thr2;
-        const bool vfar = far && gap2 >= thr2v;
-        // lanes past the system stage a massless body far away: exactly 0
-        float Sx = 1.0e18f, Sy = 1.0e18f, Sz = 1.0e18f, Ex = 0.f, Ey = 0.f, Ez = 0.f, mj = 0.f;
-        if (valid) {
-            if (far) {
-                Sx = rel_s(h.x, l.x, cx);
-                Sy = rel_s(h.y, l.y, cy);
-                Sz = rel_s(h.z, l.z, cz);
-            } else {
-                rel_ds(h.x, l.x, cx, Sx, Ex);
-                rel_ds(h.y, l.y, cy, Sy, Ey);
-                rel_ds(h.z, l.z, cz, Sz, Ez);
-            }
-            mj = h.w;
-        }
-        __syncwarp();
-        if (far)
-            pair_tile_put_hi(sg, lane, Sx, Sy, Sz, mj);
-        else
-            pair_tile_put(sg, lane, Sx, Sy, Sz, mj, Ex, Ey, Ez);
-        __syncwarp();
-        valid = (jc + 1) * 32 + lane < sd.n;
-        if (valid) {
-            h = hi[sd.first + (jc + 1) * 32 + lane];
-            l = lo[sd.first + (jc + 1) * 32 + lane];
-        }
-        float2 fx[IPT], fy[IPT], fz[IPT];
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) fx[k] = fy[k] = fz[k] = dup2(0.f);
-        if (vfar) {
-#pragma unroll 4
-            for (int p = 0; p < 16; ++p) {
-                const JPair j = pair_tile_get(sg, p);
-#pragma unroll
-                for (int k = 0; k < IPT; ++k)
-                    pair_term2_far<false>(j, nsx[k], nsy[k], nsz[k], e2, fx[k], fy[k], fz[k]);
-            }
-        } else if (far) {
-#pragma unroll 4
-            for (int p = 0; p < 16; ++p) {
-                const JPair j = pair_tile_get(sg, p);
-#pragma unroll
-                for (int k = 0; k < IPT; ++k)
-                    pair_term2_far<true>(j, nsx[k], nsy[k], nsz[k], e2, fx[k], fy[k], fz[k]);
-            }
-        } else {
-#pragma unroll 4
-            for (int p = 0; p < 16; ++p) {
-                const JPair j = pair_tile_get(sg, p);
-#pragma unroll
-                for (int k = 0; k < IPT; ++k)
-                    pair_term2<ZERO_SOFT>(j, nsx[k], nsy[k], nsz[k], nex[k], ney[k], nez[k], e2,
-                                          fx[k], fy[k], fz[k]);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            kahan_add(sx[k], qx[k], fx[k].x + fx[k].y);
-            kahan_add(sy[k], qy[k], fy[k].x + fy[k].y);
-            kahan_add(sz[k], qz[k], fz[k].x + fz[k].y);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = i0 + 32 * k + lane;
-        if (i < sd.n) {
-            const uint32_t o = order[sd.first + i];
-            if (!NB_IN_RANGE(o, total)) continue;
-            ax[o] = G * ((double)sx[k] - (double)qx[k]);
-            ay[o] = G * ((double)sy[k] - (double)qy[k]);
-            az[o] = G * ((double)sz[k] - (double)qz[k]);
-        }
-    }
-}
-
-template <bool ZERO_SOFT>
-__global__ void __launch_bounds__(kBatchBlock)
-batch_sorted_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
-                    const float4 *__restrict__ box, const SysDesc *__restrict__ sys,
-                    const WorkItem *__restrict__ items, int num_items, int *__restrict__ counter,
-                    float eps2, double G, const uint32_t *__restrict__ order,
-                    double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
-                    int total, int num_chunks)
-{
-    __shared__ PairTile tiles[kBatchWarps];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    while (true) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(counter, 1);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= num_items) break;
-        const WorkItem w = items[item];
-        const SysDesc sd = sys[w.sys];
-        if (!NB_IN_RANGE(sd.first, total) || !NB_IN_RANGE(sd.first + sd.n - 1, total) ||
-            !NB_IN_RANGE(sd.chunk0 + (sd.n - 1) / 32, num_chunks))
-            continue;
-        if (sd.ipt == 2)
-            batch_sorted_item<2, ZERO_SOFT>(hi, lo, box, sd, w.i0, eps2, G, order, ax, ay, az,
-                                            tiles[warp], total);
-        else
-            batch_sorted_item<1, ZERO_SOFT>(hi, lo, box, sd, w.i0, eps2, G, order, ax, ay, az,
-                                            tiles[warp], total);
-    }
-}
-
-int batch_sorted_grid()
-{
-    static const int grid = [] {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, (const void *)batch_sorted_kernel<false>, kBatchBlock, 0);
-        return std::max(1, per_sm) * device_props().num_sms;
-    }();
-    return grid;
 }
 
 } // namespace
@@ -484,71 +482,101 @@ int bucket_of(int n)
     return b;  // floor(log2(n))
 }
 
-void build_work_items(const std::vector<SysDesc> &sys, std::vector<WorkItem> &items)
+size_t batch_layout(std::vector<SysDesc> &sys, int *tiles)
 {
-    // largest cost first: an item costs ~ n_j * 32 ipt, the same for every
-    // full item of a system, so the systems are ordered (stably) by that cost
-    // and each contributes its items in order -- O(items), no per-item sort
-    std::vector<int> by_cost(sys.size());
-    for (int s = 0; s < (int)sys.size(); ++s) by_cost[s] = s;
-    std::stable_sort(by_cost.begin(), by_cost.end(), [&](int a, int b) {
-        return (long)sys[a].n * std::min(32 * sys[a].ipt, sys[a].n) >
-               (long)sys[b].n * std::min(32 * sys[b].ipt, sys[b].n);
-    });
-    items.clear();
-    for (int s : by_cost) {
-        const int per = 32 * sys[s].ipt;
-        for (int i0 = 0; i0 < sys[s].n; i0 += per) items.push_back(WorkItem{s, i0});
+    int t = 0;
+    long long pairs = 0;
+    for (SysDesc &s : sys) {
+        s.blocks = s.n < kBatchPairsMin ? 0 : (s.n + kBatchBlockBodies - 1) / kBatchBlockBodies;
+        s.tile0 = t;
+        s.part0 = pairs;
+        t += (s.n + kTile - 1) / kTile;
+        if (s.blocks) pairs += 3ll * s.n * (2 * (s.blocks / 2) + 1);
     }
+    *tiles = t;
+    return sizeof(float2) * (size_t)pairs;
 }
 
-nb_status batch_forces(const float4 *hi, const float4 *lo, const SysDesc *d_sys,
-                       const WorkItem *d_items, int num_items, int *d_counter, double G,
-                       double eps2, double *ax, double *ay, double *az, int total,
-                       cudaStream_t st, const KernelTimer *timer)
+void build_work_items(const std::vector<SysDesc> &sys, std::vector<PairItem> &items,
+                      int *num_blocks)
 {
-    if (num_items <= 0) return NB_OK;
-    NB_CUDA_TRY(cudaMemsetAsync(d_counter, 0, sizeof(int), st));
+    // first the (system, block, 0) list of the combine, then every item by
+    // cost, largest first, in units of a 64 x 64 tile pair (a stable counting
+    // sort: all full items of all systems cost the same; a row item is two
+    // tiles against half its system's, both directions apart)
+    constexpr int kMost = kBatchPairsMin / 16;
+    std::vector<PairItem> by_cost[kMost + 1];
+    items.clear();
+    for (int s = 0; s < (int)sys.size(); ++s) {
+        const int M = sys[s].blocks, tiles = (sys[s].n + kTile - 1) / kTile;
+        for (int r = 0; M == 0 && r * 32 < sys[s].n; ++r)
+            by_cost[std::min(kMost, (tiles + 1) / 2)].push_back(PairItem{s, r, -1});
+        if (M == 0) continue;
+        auto width = [&](int b) { return std::min(kBatchTiles, tiles - b * kBatchTiles); };
+        for (int p = 0; p <= M / 2; ++p)
+            for (int a = 0; a < M; ++a) {
+                if (p == 0) items.push_back(PairItem{s, a, 0});
+                if (!pair_first(p, a, M)) continue;
+                const int ta = width(a), tb = width((a + p) % M);
+                by_cost[p == 0 ? ta * (ta + 1) / 2 : ta * tb].push_back(PairItem{s, a, p});
+            }
+    }
+    *num_blocks = (int)items.size();
+    for (int c = kMost; c >= 0; --c) items.insert(items.end(), by_cost[c].begin(), by_cost[c].end());
+}
+
+static nb_status launch_batch(const float4 *hi, const float4 *lo, const float4 *boxes,
+                              const BatchQueue &q, double G, double eps2, const uint32_t *order,
+                              double *ax, double *ay, double *az, int total, int num_tiles,
+                              cudaStream_t st, const KernelTimer *timer)
+{
+    const PairItem *pairs = q.d_items + q.num_blocks;
+    const int num_pairs = q.num_items - q.num_blocks;
     if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
-    if (eps2 > 0.0)
-        batch_force_kernel<false><<<batch_grid(), kBatchBlock, 0, st>>>(
-            hi, lo, d_sys, d_items, num_items, d_counter, (float)eps2, G, ax, ay, az, total);
+    if (boxes && eps2 > 0.0)
+        batch_pairs_kernel<true, false><<<num_pairs, 32, 0, st>>>(
+            hi, lo, boxes, q.d_sys, pairs, (float)eps2, q.part, G, order, ax, ay, az, total, num_tiles);
+    else if (boxes)
+        batch_pairs_kernel<true, true><<<num_pairs, 32, 0, st>>>(
+            hi, lo, boxes, q.d_sys, pairs, 0.0f, q.part, G, order, ax, ay, az, total, num_tiles);
+    else if (eps2 > 0.0)
+        batch_pairs_kernel<false, false><<<num_pairs, 32, 0, st>>>(
+            hi, lo, boxes, q.d_sys, pairs, (float)eps2, q.part, G, order, ax, ay, az, total, num_tiles);
     else
-        batch_force_kernel<true><<<batch_grid(), kBatchBlock, 0, st>>>(
-            hi, lo, d_sys, d_items, num_items, d_counter, 0.0f, G, ax, ay, az, total);
+        batch_pairs_kernel<false, true><<<num_pairs, 32, 0, st>>>(
+            hi, lo, boxes, q.d_sys, pairs, 0.0f, q.part, G, order, ax, ay, az, total, num_tiles);
     NB_LAUNCH_CHECK();
     if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
+    if (q.num_blocks == 0) return NB_OK;  // small systems only: no partial sums
+    batch_combine_kernel<<<q.num_blocks, kBatchBlockBodies, 0, st>>>(
+        q.part, q.d_sys, q.d_items, order, G, ax, ay, az, total);
+    NB_LAUNCH_CHECK();
     return NB_OK;
 }
 
+nb_status batch_forces(const float4 *hi, const float4 *lo, const BatchQueue &q, double G,
+                       double eps2, double *ax, double *ay, double *az, int total,
+                       cudaStream_t st, const KernelTimer *timer)
+{
+    if (q.num_items <= 0) return NB_OK;
+    return launch_batch(hi, lo, nullptr, q, G, eps2, nullptr, ax, ay, az, total, q.num_tiles, st,
+                        timer);
+}
 
 void BatchSorted::release()
 {
     if (sorter) bh_destroy(sorter);
     sorter = nullptr;
     order = nullptr;
-    DevBuf *bufs[] = {&body_sys, &chunks, &geom, &boxes};
+    DevBuf *bufs[] = {&body_sys, &tiles, &geom, &boxes};
     for (DevBuf *b : bufs) b->release();
 }
 
-int batch_sorted_ipt(int n) { return n >= kSortedIpt2Min ? 2 : 1; }
-
-int batch_sorted_chunks(std::vector<SysDesc> &sys)
-{
-    int c = 0;
-    for (SysDesc &s : sys) {
-        s.ipt = batch_sorted_ipt(s.n);
-        s.chunk0 = c;
-        c += (s.n + 31) / 32;
-    }
-    return c;
-}
-
-nb_status batch_sorted_setup(BatchSorted &b, const SysDesc *d_sys, int num_sys, int num_chunks,
+nb_status batch_sorted_setup(BatchSorted &b, const SysDesc *d_sys, int num_sys, int num_tiles,
                              int total, cudaStream_t st)
 {
     b.num_sys = num_sys;
-    b.num_chunks = num_chunks;
+    b.num_tiles = num_tiles;
     b.total = total;
     int sys_bits = 1;
     while ((1 << sys_bits) < num_sys) ++sys_bits;
@@ -556,11 +584,11 @@ nb_status batch_sorted_setup(BatchSorted &b, const SysDesc *d_sys, int num_sys, 
     b.key_shift = 64 - key_bits;
     b.first_shift = b.key_shift / 8 * 8;
     NB_TRY(b.body_sys.reserve(sizeof(int) * (size_t)std::max(total, 1)));
-    NB_TRY(b.chunks.reserve(sizeof(int2) * (size_t)std::max(num_chunks, 1)));
+    NB_TRY(b.tiles.reserve(sizeof(int4) * (size_t)std::max(num_tiles, 1)));
     NB_TRY(b.geom.reserve(sizeof(double4) * (size_t)std::max(num_sys, 1)));
-    NB_TRY(b.boxes.reserve(sizeof(float4) * 2 * (size_t)std::max(num_chunks, 1)));
+    NB_TRY(b.boxes.reserve(sizeof(float4) * 4 * (size_t)std::max(num_tiles, 1)));
     if (!b.sorter) b.sorter = bh_create();
-    batch_layout_kernel<<<num_sys, 128, 0, st>>>(d_sys, b.body_sys.as<int>(), b.chunks.as<int2>());
+    batch_layout_kernel<<<num_sys, 128, 0, st>>>(d_sys, b.body_sys.as<int>(), b.tiles.as<int4>());
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
@@ -581,31 +609,17 @@ nb_status batch_sorted_sort(BatchSorted &b, const SysDesc *d_sys, const double *
 }
 
 nb_status batch_sorted_forces(BatchSorted &b, const double *x, const double *y, const double *z,
-                              const double *m, const SysDesc *d_sys, const WorkItem *d_items,
-                              int num_items, int *d_counter, double G, double eps2, float4 *hi,
-                              float4 *lo, double *ax, double *ay, double *az, cudaStream_t st,
-                              const KernelTimer *timer)
+                              const double *m, const BatchQueue &q, double G, double eps2,
+                              float4 *hi, float4 *lo, double *ax, double *ay, double *az,
+                              cudaStream_t st, const KernelTimer *timer)
 {
-    if (num_items <= 0) return NB_OK;
+    if (q.num_items <= 0) return NB_OK;
     if (!b.order) return fail(NB_ERR_NOT_LOADED, "sorted batch: no order (sort first)");
-    batch_split_sorted_kernel<<<(b.total + 255) / 256, 256, 0, st>>>(
-        b.order, x, y, z, m, b.body_sys.as<int>(), b.geom.as<double4>(), b.total, hi, lo);
+    batch_split_sorted_kernel<<<(2 * b.num_tiles + 7) / 8, 256, 0, st>>>(
+        b.order, x, y, z, m, b.tiles.as<int4>(), b.num_tiles, b.geom.as<double4>(), b.total, hi,
+        lo, b.boxes.as<float4>());
     NB_LAUNCH_CHECK();
-    batch_chunk_box_kernel<<<(b.num_chunks + 7) / 8, 256, 0, st>>>(
-        hi, b.chunks.as<int2>(), b.num_chunks, b.boxes.as<float4>());
-    NB_LAUNCH_CHECK();
-    NB_CUDA_TRY(cudaMemsetAsync(d_counter, 0, sizeof(int), st));
-    if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
-    if (eps2 > 0.0)
-        batch_sorted_kernel<false><<<batch_sorted_grid(), kBatchBlock, 0, st>>>(
-            hi, lo, b.boxes.as<float4>(), d_sys, d_items, num_items, d_counter, (float)eps2, G,
-            b.order, ax, ay, az, b.total, b.num_chunks);
-    else
-        batch_sorted_kernel<true><<<batch_sorted_grid(), kBatchBlock, 0, st>>>(
-            hi, lo, b.boxes.as<float4>(), d_sys, d_items, num_items, d_counter, 0.0f, G,
-            b.order, ax, ay, az, b.total, b.num_chunks);
-    NB_LAUNCH_CHECK();
-    if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
-    return NB_OK;
+    return launch_batch(hi, lo, b.boxes.as<float4>(), q, G, eps2, b.order, ax, ay, az, b.total,
+                        b.num_tiles, st, timer);
 }
 } // namespace nb

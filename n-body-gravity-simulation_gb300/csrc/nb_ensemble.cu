@@ -2,17 +2,16 @@
 //
 // Thousands of independent systems of uneven N advance together: the state of
 // all systems is concatenated (system order) in one set of FP64 planes; the
-// forces of every system come from one persistent launch over a per-system
-// work queue (nb_batch.cu); the per-body integrator updates run once over the
+// forces of every system come from one launch over a queue of block pairs
+// (nb_batch.cu); the per-body integrator updates run once over the
 // concatenation; the step loop is captured in a CUDA graph and replayed.
 //
 // By default the force launch is the Hilbert-sorted near/far variant: every
 // system is sorted along a Hilbert curve through its own cube at the start of
 // each nb_ensemble_step call and every kGraphChunk steps (between graph
 // replays, the same points whether or not the steps are replayed), and far
-// j-chunks of an i-chunk take the plain FP32 term.  NB_FLAG_MIXED_UNSORTED
-// selects the all-pairs double-single kernel, whose i-bodies per lane are
-// autotuned per N bucket before the first evaluation.
+// tile pairs take the plain FP32 term.  NB_FLAG_MIXED_UNSORTED selects the
+// double-single term for every pair.
 #include "nb_internal.h"
 
 #include <algorithm>
@@ -30,12 +29,12 @@ struct nb_ensemble {
     bool own_stream = false;
     bool loaded = false;
 
-    nb::DevBuf state, hi, lo, old_acc, rk4, d_sys, d_items, d_counter;
+    nb::DevBuf state, hi, lo, old_acc, rk4, d_sys, d_items, part;
     double *f[10] = {};
     std::vector<nb::SysDesc> sys;
-    int num_items = 0;
+    nb::BatchQueue queue;
     int ipt_bucket[32];
-    bool tuned = false;
+    bool ready = false;  // the work queue is uploaded
     bool forces_valid = false;
 
     // captured step loop
@@ -51,28 +50,30 @@ struct nb_ensemble {
 
     bool sorted = true;  // the Hilbert-sorted near/far force launch
     nb::BatchSorted sb;
-    int num_chunks = 0;
 };
 
 namespace nb {
 namespace {
 
 constexpr int kGraphChunk = 25;
-const int kIptCandidates[] = {1, 2, 4};
 
 nb_status upload_items(nb_ensemble *e)
 {
-    std::vector<WorkItem> items;
-    build_work_items(e->sys, items);
-    e->num_items = (int)items.size();
+    BatchQueue &q = e->queue;
+    const size_t bytes = batch_layout(e->sys, &q.num_tiles);
+    std::vector<PairItem> items;
+    build_work_items(e->sys, items, &q.num_blocks);
+    q.num_items = (int)items.size();
     NB_TRY(e->d_sys.reserve(sizeof(SysDesc) * e->sys.size()));
-    NB_TRY(e->d_items.reserve(sizeof(WorkItem) * std::max<size_t>(1, items.size())));
+    NB_TRY(e->d_items.reserve(sizeof(PairItem) * items.size()));
+    NB_TRY(e->part.reserve(bytes));
+    q.d_sys = e->d_sys.as<SysDesc>();
+    q.d_items = e->d_items.as<PairItem>();
+    q.part = e->part.as<float2>();
     NB_CUDA_TRY(cudaMemcpyAsync(e->d_sys.ptr, e->sys.data(), sizeof(SysDesc) * e->sys.size(),
                                 cudaMemcpyHostToDevice, e->stream));
-    if (!items.empty())
-        NB_CUDA_TRY(cudaMemcpyAsync(e->d_items.ptr, items.data(),
-                                    sizeof(WorkItem) * items.size(), cudaMemcpyHostToDevice,
-                                    e->stream));
+    NB_CUDA_TRY(cudaMemcpyAsync(e->d_items.ptr, items.data(), sizeof(PairItem) * items.size(),
+                                cudaMemcpyHostToDevice, e->stream));
     // the host vectors go out of scope: wait for the copies
     NB_CUDA_TRY(cudaStreamSynchronize(e->stream));
     return NB_OK;
@@ -95,68 +96,13 @@ nb_status ens_force(nb_ensemble *e, const double *px, const double *py, const do
 {
     const int n = (int)e->total;
     float4 *hi = e->hi.as<float4>(), *lo = e->lo.as<float4>();
+    const double eps2 = e->cfg.softening * e->cfg.softening;
     if (e->sorted)
-        return batch_sorted_forces(e->sb, px, py, pz, e->f[9], e->d_sys.as<SysDesc>(),
-                                   e->d_items.as<WorkItem>(), e->num_items,
-                                   e->d_counter.as<int>(), e->cfg.G,
-                                   e->cfg.softening * e->cfg.softening, hi, lo, ax, ay, az,
-                                   e->stream, ens_timer(e, capturing));
+        return batch_sorted_forces(e->sb, px, py, pz, e->f[9], e->queue, e->cfg.G, eps2, hi, lo,
+                                   ax, ay, az, e->stream, ens_timer(e, capturing));
     NB_TRY(split_positions(px, py, pz, e->f[9], n, hi, lo, e->stream));
-    const double eps2 = e->cfg.softening * e->cfg.softening;
-    return batch_forces(hi, lo, e->d_sys.as<SysDesc>(), e->d_items.as<WorkItem>(), e->num_items,
-                        e->d_counter.as<int>(), e->cfg.G, eps2, ax, ay, az, n, e->stream,
+    return batch_forces(hi, lo, e->queue, e->cfg.G, eps2, ax, ay, az, n, e->stream,
                         ens_timer(e, capturing));
-}
-
-// Times each candidate ipt on the systems of each N bucket and keeps the
-// fastest; then builds the full work queue.
-nb_status tune(nb_ensemble *e)
-{
-    const double eps2 = e->cfg.softening * e->cfg.softening;
-    const int n = (int)e->total;
-    float4 *hi = e->hi.as<float4>(), *lo = e->lo.as<float4>();
-    NB_TRY(split_positions(e->f[0], e->f[1], e->f[2], e->f[9], n, hi, lo, e->stream));
-    cudaEvent_t t0, t1;
-    NB_CUDA_TRY(cudaEventCreate(&t0));
-    NB_CUDA_TRY(cudaEventCreate(&t1));
-    std::vector<SysDesc> all = e->sys;
-    for (int b = 0; b < 32; ++b) {
-        std::vector<SysDesc> bs;
-        for (const SysDesc &s : all)
-            if (bucket_of(s.n) == b) bs.push_back(s);
-        if (bs.empty()) continue;
-        float best = 1e30f;
-        for (int ipt : kIptCandidates) {
-            for (SysDesc &s : bs) s.ipt = ipt;
-            e->sys = bs;
-            NB_TRY(upload_items(e));
-            // warm, then two timed launches into the real acceleration planes
-            NB_TRY(batch_forces(hi, lo, e->d_sys.as<SysDesc>(), e->d_items.as<WorkItem>(),
-                                e->num_items, e->d_counter.as<int>(), e->cfg.G, eps2, e->f[6],
-                                e->f[7], e->f[8], n, e->stream));
-            NB_CUDA_TRY(cudaEventRecord(t0, e->stream));
-            for (int r = 0; r < 2; ++r)
-                NB_TRY(batch_forces(hi, lo, e->d_sys.as<SysDesc>(), e->d_items.as<WorkItem>(),
-                                    e->num_items, e->d_counter.as<int>(), e->cfg.G, eps2,
-                                    e->f[6], e->f[7], e->f[8], n, e->stream));
-            NB_CUDA_TRY(cudaEventRecord(t1, e->stream));
-            NB_CUDA_TRY(cudaEventSynchronize(t1));
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, t0, t1);
-            if (ms < best) {
-                best = ms;
-                e->ipt_bucket[b] = ipt;
-            }
-        }
-    }
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
-    for (SysDesc &s : all) s.ipt = e->ipt_bucket[bucket_of(s.n)];
-    e->sys = all;
-    NB_TRY(upload_items(e));
-    e->tuned = true;
-    e->forces_valid = false;  // tuning overwrote the acceleration planes
-    return NB_OK;
 }
 
 nb_status step_direct(nb_ensemble *e, int integ, double dt, bool capturing)
@@ -172,14 +118,14 @@ nb_status step_direct(nb_ensemble *e, int integ, double dt, bool capturing)
     return integrate_step(integ, (int)e->total, dt, e->f, b, e->forces_valid, force, e->stream);
 }
 
-// The sorted path's tables (its shape is fixed: one 32-body i-chunk per item).
-nb_status setup_sorted(nb_ensemble *e)
+// Uploads the work queue and, for the sorted path, its tables.
+nb_status setup(nb_ensemble *e)
 {
-    for (const SysDesc &sd : e->sys) e->ipt_bucket[bucket_of(sd.n)] = sd.ipt;
     NB_TRY(upload_items(e));
-    NB_TRY(batch_sorted_setup(e->sb, e->d_sys.as<SysDesc>(), e->num_sys, e->num_chunks,
-                              (int)e->total, e->stream));
-    e->tuned = true;
+    if (e->sorted)
+        NB_TRY(batch_sorted_setup(e->sb, e->queue.d_sys, e->num_sys, e->queue.num_tiles,
+                                  (int)e->total, e->stream));
+    e->ready = true;
     return NB_OK;
 }
 
@@ -187,14 +133,14 @@ nb_status setup_sorted(nb_ensemble *e)
 nb_status sort_systems(nb_ensemble *e)
 {
     if (!e->sorted) return NB_OK;
-    return batch_sorted_sort(e->sb, e->d_sys.as<SysDesc>(), e->f[0], e->f[1], e->f[2],
+    return batch_sorted_sort(e->sb, e->queue.d_sys, e->f[0], e->f[1], e->f[2],
                              e->stream);
 }
 
 nb_status ready(nb_ensemble *e)
 {
     if (!e->loaded) return fail(NB_ERR_NOT_LOADED, "ensemble: nothing loaded");
-    if (!e->tuned) NB_TRY(e->sorted ? setup_sorted(e) : tune(e));
+    if (!e->ready) NB_TRY(setup(e));
     return NB_OK;
 }
 
@@ -226,7 +172,7 @@ nb_status nb_ensemble_create(const nb_config *cfg, int num_systems, const int *s
     e->sizes.assign(sizes, sizes + num_systems);
     e->total = total;
     e->ps = (total + 31) / 32 * 32;
-    for (int b = 0; b < 32; ++b) e->ipt_bucket[b] = 1;
+    for (int b = 0; b < 32; ++b) e->ipt_bucket[b] = 2;
     if (stream) {
         e->stream = static_cast<cudaStream_t>(stream);
     } else {
@@ -242,7 +188,6 @@ nb_status nb_ensemble_create(const nb_config *cfg, int num_systems, const int *s
     if (st == NB_OK) st = e->state.reserve(sizeof(double) * 10 * e->ps);
     if (st == NB_OK) st = e->hi.reserve(sizeof(float4) * e->ps);
     if (st == NB_OK) st = e->lo.reserve(sizeof(float4) * e->ps);
-    if (st == NB_OK) st = e->d_counter.reserve(sizeof(int));
     if (st != NB_OK) {
         nb_ensemble_destroy(e);
         return st;
@@ -251,11 +196,10 @@ nb_status nb_ensemble_create(const nb_config *cfg, int num_systems, const int *s
     size_t first = 0;
     e->sys.resize(num_systems);
     for (int s = 0; s < num_systems; ++s) {
-        e->sys[s] = SysDesc{(int)first, sizes[s], 1, 0};
+        e->sys[s] = SysDesc{(int)first, sizes[s], 0, 0, 0};
         first += sizes[s];
     }
     e->sorted = (cfg->flags & NB_FLAG_MIXED_UNSORTED) == 0;
-    if (e->sorted) e->num_chunks = batch_sorted_chunks(e->sys);
     *out = e;
     return NB_OK;
 }
@@ -270,7 +214,7 @@ nb_status nb_ensemble_destroy(nb_ensemble *e)
         cudaEventDestroy(t.stop);
     }
     nb::DevBuf *bufs[] = {&e->state, &e->hi, &e->lo, &e->old_acc, &e->rk4, &e->d_sys,
-                          &e->d_items, &e->d_counter};
+                          &e->d_items, &e->part};
     for (nb::DevBuf *b : bufs) b->release();
     e->sb.release();
     if (e->own_stream) cudaStreamDestroy(e->stream);
@@ -320,7 +264,7 @@ nb_status nb_ensemble_tune(nb_ensemble *e, int *ipt_by_bucket)
         cudaGraphExecDestroy(e->graph);
         e->graph = nullptr;
     }
-    NB_TRY(e->sorted ? setup_sorted(e) : tune(e));
+    NB_TRY(setup(e));
     if (ipt_by_bucket)
         for (int b = 0; b < 32; ++b) ipt_by_bucket[b] = e->ipt_bucket[b];
     return NB_OK;
@@ -421,7 +365,7 @@ nb_status nb_ensemble_info(nb_ensemble *e, nb_ensemble_info_t *info)
     double inter = 0.0;
     for (int n : e->sizes) inter += (double)n * (double)(n - 1);
     info->interactions_per_eval = inter;
-    info->work_items = e->num_items;
+    info->work_items = e->queue.num_items - e->queue.num_blocks;
     for (int b = 0; b < 32; ++b) info->ipt_by_bucket[b] = e->ipt_bucket[b];
     info->graph_launches = e->graph_launches;
     info->graph_steps = e->graph_steps;

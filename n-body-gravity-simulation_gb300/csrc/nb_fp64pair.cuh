@@ -1,6 +1,5 @@
 // nb_fp64pair.cuh -- FP64 building blocks of the all-pairs kernels: a reciprocal
-// square root seeded on the MUFU pipe, and the schedule of block pairs that
-// visits every unordered pair of bodies once.
+// square root seeded on the MUFU pipe.
 //
 // GB300 issues two FP64 lane operations per clock and SM, a 64th of its FP32
 // rate, so an FP64 all-pairs kernel is bound by the number of FP64 operations
@@ -60,20 +59,6 @@ __device__ __forceinline__ double inv_sqrt(double r2)
         return fma(y * e, fma(e, 0.375, 0.5), y);
     }
     return 1.0 / sqrt(r2);
-}
-
-// Block pairs.  n bodies in M blocks; diagonal p (0 <= p <= M / 2) pairs block A
-// with block (A + p) mod M for every A -- for an even M and p = M / 2 only for
-// A < M / 2 -- so each unordered block pair appears once and every block the
-// same number of times, once as the first and once as the second block of
-// each diagonal.
-__host__ __device__ __forceinline__ bool pair_first(int p, int a, int blocks)
-{
-    return 2 * p != blocks || 2 * a < blocks;
-}
-__host__ __device__ __forceinline__ bool pair_second(int p, int b, int blocks)
-{
-    return p > 0 && (2 * p != blocks || 2 * b >= blocks);
 }
 
 } // namespace nb

@@ -202,37 +202,61 @@ nb_status diagnostics(const double *x, const double *y, const double *z, const d
                       double eps2, DevBuf &scratch, cudaStream_t st, nb_diag *out);
 
 // ---------------------------------------------------------------- batches
-// A system of a batch: bodies [first, first + n) of the batch's pool, summed
-// with ipt i-bodies per lane.
+constexpr int kBatchBlockBodies = 256;  // four tiles of 64
+// Smallest system summed over unordered pairs; smaller ones by rows (ordered
+// pairs).  On the 1024-system ensemble (n log-uniform in [32, 4096], two RK4 steps)
+// a line at 512 / 1024 / 2048 / beyond every system measured 7.58 / 7.69 / 8.12 /
+// 9.15 ms.  It lies at 1024, not 512: in a system of a few hundred bodies one close
+// pair can carry a body's whole force, and the row sum is the order of rounding
+// that its trajectory has had.
+constexpr int kBatchPairsMin = 1024;
+// A system of a batch: bodies [first, first + n) of the batch's pool.
 struct SysDesc {
     int first;
     int n;
-    int ipt;
-    int chunk0;  // first 32-body chunk of the system (the sorted batch path)
+    int blocks;       // blocks of kBatchBlockBodies; 0: a small system, summed by rows
+    int tile0;        // first 64-body tile of the system
+    long long part0;  // its first entry of the partial planes
 };
-// One queue item: i-bodies [i0, i0 + 32 * ipt) of system `sys`.
-struct WorkItem {
+// One queue item: blocks a and (a + p) mod blocks of system `sys`; p < 0: the
+// rows of its 128 bodies from 128 a.
+struct PairItem {
     int sys;
-    int i0;
+    int a;
+    int p;
+};
+// The uploaded work of a set of systems: num_blocks (system, block, 0) entries
+// for the combine, then the items of the pair kernel; part: the partial planes.
+struct BatchQueue {
+    const SysDesc *d_sys = nullptr;
+    const PairItem *d_items = nullptr;
+    int num_blocks = 0, num_items = 0, num_tiles = 0;
+    float2 *part = nullptr;
 };
 int bucket_of(int n);  // floor(log2(n))
+// Sets every system's blocks, tile0 and part0; returns the bytes of the
+// partial planes and the tile count.
+size_t batch_layout(std::vector<SysDesc> &sys, int *tiles);
+// The combine's blocks, then the items of every system, largest cost first.
+void build_work_items(const std::vector<SysDesc> &sys, std::vector<PairItem> &items,
+                      int *num_blocks);
+// Mixed-precision forces of all systems of the queue.
+nb_status batch_forces(const float4 *hi, const float4 *lo, const BatchQueue &q, double G,
+                       double eps2, double *ax, double *ay, double *az, int total,
+                       cudaStream_t st, const KernelTimer *timer = nullptr);
+
 // Hilbert-sorted variant of the batched forces (nb_batch.cu): each system's
-// bodies are sorted along a Hilbert curve through its own cube; an item is one
-// or two 32-body i-chunks; j-chunks far from its box take the plain FP32 term.
-struct BHTree;
+// bodies are sorted along a Hilbert curve through its own cube; tile pairs far
+// apart take the plain FP32 term.
 struct BatchSorted {
     BHTree *sorter = nullptr;
-    DevBuf body_sys, chunks, geom, boxes;
+    DevBuf body_sys, tiles, geom, boxes;
     const uint32_t *order = nullptr;  // sorted index -> body (sorter-owned)
-    int num_sys = 0, num_chunks = 0, total = 0, key_shift = 0, first_shift = 0;
+    int num_sys = 0, num_tiles = 0, total = 0, key_shift = 0, first_shift = 0;
     void release();
 };
-// i-chunks per warp item of an n-body system in the sorted variant (1 or 2).
-int batch_sorted_ipt(int n);
-// Sets every system's ipt (batch_sorted_ipt) and chunk0; returns the chunk count.
-int batch_sorted_chunks(std::vector<SysDesc> &sys);
-// Device tables for the systems of d_sys (already uploaded with chunk0).
-nb_status batch_sorted_setup(BatchSorted &b, const SysDesc *d_sys, int num_sys, int num_chunks,
+// Device tables for the systems of d_sys (already uploaded with tile0).
+nb_status batch_sorted_setup(BatchSorted &b, const SysDesc *d_sys, int num_sys, int num_tiles,
                              int total, cudaStream_t st);
 // (Re)computes the order from the positions x, y, z.
 nb_status batch_sorted_sort(BatchSorted &b, const SysDesc *d_sys, const double *x,
@@ -240,18 +264,9 @@ nb_status batch_sorted_sort(BatchSorted &b, const SysDesc *d_sys, const double *
 // a = G sum_j ... for every body, in the order of the last sort (hi/lo are
 // scratch mirrors of total entries).
 nb_status batch_sorted_forces(BatchSorted &b, const double *x, const double *y, const double *z,
-                              const double *m, const SysDesc *d_sys, const WorkItem *d_items,
-                              int num_items, int *d_counter, double G, double eps2, float4 *hi,
-                              float4 *lo, double *ax, double *ay, double *az, cudaStream_t st,
-                              const KernelTimer *timer);
-
-// Items of every system, largest cost first.
-void build_work_items(const std::vector<SysDesc> &sys, std::vector<WorkItem> &items);
-// Mixed-precision forces of all systems of the queue (persistent kernel).
-nb_status batch_forces(const float4 *hi, const float4 *lo, const SysDesc *d_sys,
-                       const WorkItem *d_items, int num_items, int *d_counter, double G,
-                       double eps2, double *ax, double *ay, double *az, int total,
-                       cudaStream_t st, const KernelTimer *timer = nullptr);
+                              const double *m, const BatchQueue &q, double G, double eps2,
+                              float4 *hi, float4 *lo, double *ax, double *ay, double *az,
+                              cudaStream_t st, const KernelTimer *timer);
 
 // ---------------------------------------------------------------- Barnes-Hut
 struct BHTree;  // opaque, defined in nb_bh.cu

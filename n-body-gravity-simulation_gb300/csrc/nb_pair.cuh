@@ -349,4 +349,19 @@ __device__ __forceinline__ void pair_term2_far(const JPair &j, float2 nx, float2
     az = fma2(dz, s, az);
 }
 
+// ---------------------------------------------------------------- block pairs
+// The schedule of the sums over unordered pairs.  n bodies in M blocks; diagonal p (0 <= p <= M / 2) pairs block A
+// with block (A + p) mod M for every A -- for an even M and p = M / 2 only for
+// A < M / 2 -- so each unordered block pair appears once and every block the
+// same number of times, once as the first and once as the second block of
+// each diagonal.
+__host__ __device__ __forceinline__ bool pair_first(int p, int a, int blocks)
+{
+    return 2 * p != blocks || 2 * a < blocks;
+}
+__host__ __device__ __forceinline__ bool pair_second(int p, int b, int blocks)
+{
+    return p > 0 && (2 * p != blocks || 2 * b >= blocks);
+}
+
 } // namespace nb

@@ -7,7 +7,7 @@
 //   2. advances every running job by one leapfrog step:
 //      - direct jobs (n < direct_max_n) live in one body pool and advance
 //        together: one per-body kick-drift and kick over the pool and one
-//        persistent batched force launch over all of them (nb_batch.cu);
+//        batched force launch over all of them (nb_batch.cu);
 //      - Barnes-Hut jobs each own a simulation object and run on one of
 //        kBHStreams streams (the process should allow that many hardware
 //        queues: CUDA_DEVICE_MAX_CONNECTIONS >= 16), each stream's jobs issued
@@ -113,8 +113,6 @@ struct SlotAllocator {
     }
 };
 
-int default_ipt(int n) { return n < 1024 ? 1 : (n < 4096 ? 2 : 4); }
-
 double quantile(std::vector<double> v, double q)
 {
     if (v.empty()) return 0.0;
@@ -209,7 +207,12 @@ struct nb_server {
     cudaStream_t bh_streams[nb::kBHStreams] = {};
     nb::StreamPool pool_threads;  // issues the Barnes-Hut streams' steps
     size_t ps = 0;
-    nb::DevBuf pool, hi, lo, d_sys, d_items, d_counter, d_new_sys, d_new_items;
+    nb::DevBuf pool, hi, lo;
+    // the direct jobs' work queue, and that of the jobs admitted this tick
+    struct Queue {
+        nb::DevBuf d_sys, d_items, part;
+        nb::BatchQueue q;
+    } queue_all, queue_new;
     double *f[10] = {};
     nb::SlotAllocator slots;
     int64_t next_id = 1;
@@ -219,7 +222,6 @@ struct nb_server {
     size_t bh_bytes = 0;
     size_t peak_bytes = 0;
     bool items_dirty = true;
-    int num_items = 0;
     cudaEvent_t tick_start = nullptr, direct_done = nullptr;
     // statistics
     std::vector<double> step_ms, queue_ms;
@@ -235,20 +237,24 @@ namespace {
 
 size_t pool_bytes(const nb_server *s) { return s->pool.bytes + s->hi.bytes + s->lo.bytes; }
 
-nb_status upload_systems(nb_server *s, const std::vector<Job *> &jobs, DevBuf &d_sys,
-                         DevBuf &d_items, int *num_items)
+nb_status upload_systems(nb_server *s, const std::vector<Job *> &jobs, nb_server::Queue &to)
 {
     std::vector<SysDesc> sys;
-    for (Job *j : jobs) sys.push_back(SysDesc{(int)j->first, (int)j->n, default_ipt((int)j->n), 0});
-    std::vector<WorkItem> items;
-    build_work_items(sys, items);
-    *num_items = (int)items.size();
+    for (Job *j : jobs) sys.push_back(SysDesc{(int)j->first, (int)j->n, 0, 0, 0});
+    const size_t bytes = batch_layout(sys, &to.q.num_tiles);
+    std::vector<PairItem> items;
+    build_work_items(sys, items, &to.q.num_blocks);
+    to.q.num_items = (int)items.size();
     if (sys.empty()) return NB_OK;
-    NB_TRY(d_sys.reserve(sizeof(SysDesc) * sys.size()));
-    NB_TRY(d_items.reserve(sizeof(WorkItem) * items.size()));
-    NB_CUDA_TRY(cudaMemcpyAsync(d_sys.ptr, sys.data(), sizeof(SysDesc) * sys.size(),
+    NB_TRY(to.d_sys.reserve(sizeof(SysDesc) * sys.size()));
+    NB_TRY(to.d_items.reserve(sizeof(PairItem) * items.size()));
+    NB_TRY(to.part.reserve(bytes));
+    to.q.d_sys = to.d_sys.as<SysDesc>();
+    to.q.d_items = to.d_items.as<PairItem>();
+    to.q.part = to.part.as<float2>();
+    NB_CUDA_TRY(cudaMemcpyAsync(to.d_sys.ptr, sys.data(), sizeof(SysDesc) * sys.size(),
                                 cudaMemcpyHostToDevice, s->stream));
-    NB_CUDA_TRY(cudaMemcpyAsync(d_items.ptr, items.data(), sizeof(WorkItem) * items.size(),
+    NB_CUDA_TRY(cudaMemcpyAsync(to.d_items.ptr, items.data(), sizeof(PairItem) * items.size(),
                                 cudaMemcpyHostToDevice, s->stream));
     NB_CUDA_TRY(cudaStreamSynchronize(s->stream));
     return NB_OK;
@@ -417,7 +423,7 @@ nb_status tick(nb_server *s)
     const int hw = (int)s->slots.high_water;
     if (s->items_dirty) {
         const auto t_up = Clock::now();
-        NB_TRY(upload_systems(s, direct, s->d_sys, s->d_items, &s->num_items));
+        NB_TRY(upload_systems(s, direct, s->queue_all));
         s->items_dirty = false;
         s->upload_ms += ms_since(t_up);
     }
@@ -455,20 +461,17 @@ nb_status tick(nb_server *s)
         float4 *hi = s->hi.as<float4>(), *lo = s->lo.as<float4>();
         if (!new_direct.empty()) {
             // start-of-step force of the jobs admitted this tick
-            int nn = 0;
-            NB_TRY(upload_systems(s, new_direct, s->d_new_sys, s->d_new_items, &nn));
+            NB_TRY(upload_systems(s, new_direct, s->queue_new));
             NB_TRY(split_positions(s->f[0], s->f[1], s->f[2], s->f[9], hw, hi, lo, s->stream));
-            NB_TRY(batch_forces(hi, lo, s->d_new_sys.as<SysDesc>(), s->d_new_items.as<WorkItem>(),
-                                nn, s->d_counter.as<int>(), s->cfg.G, eps2, s->f[6], s->f[7],
+            NB_TRY(batch_forces(hi, lo, s->queue_new.q, s->cfg.G, eps2, s->f[6], s->f[7],
                                 s->f[8], hw, s->stream));
         }
         NB_TRY(kick_drift(NB_LEAPFROG, hw, dt, s->f[0], s->f[1], s->f[2], s->f[3], s->f[4],
                           s->f[5], s->f[6], s->f[7], s->f[8], nullptr, nullptr, nullptr,
                           s->stream));
         NB_TRY(split_positions(s->f[0], s->f[1], s->f[2], s->f[9], hw, hi, lo, s->stream));
-        NB_TRY(batch_forces(hi, lo, s->d_sys.as<SysDesc>(), s->d_items.as<WorkItem>(),
-                            s->num_items, s->d_counter.as<int>(), s->cfg.G, eps2, s->f[6],
-                            s->f[7], s->f[8], hw, s->stream));
+        NB_TRY(batch_forces(hi, lo, s->queue_all.q, s->cfg.G, eps2, s->f[6], s->f[7], s->f[8], hw,
+                            s->stream));
         NB_TRY(kick(NB_LEAPFROG, hw, dt, s->f[3], s->f[4], s->f[5], s->f[6], s->f[7], s->f[8],
                     nullptr, nullptr, nullptr, s->stream));
         NB_CUDA_TRY(cudaEventRecord(s->direct_done, s->stream));
@@ -551,7 +554,6 @@ nb_status nb_server_create(const nb_server_config *cfg, nb_server **out)
     if (st == NB_OK) st = s->pool.reserve(sizeof(double) * 10 * s->ps);
     if (st == NB_OK) st = s->hi.reserve(sizeof(float4) * s->ps);
     if (st == NB_OK) st = s->lo.reserve(sizeof(float4) * s->ps);
-    if (st == NB_OK) st = s->d_counter.reserve(sizeof(int));
     if (st == NB_OK) {
         e = cudaMemsetAsync(s->pool.ptr, 0, s->pool.bytes, s->stream);
         if (e != cudaSuccess) st = cuda_fail(e, "cudaMemsetAsync");
@@ -582,8 +584,9 @@ nb_status nb_server_destroy(nb_server *s)
         if (j->sim) nb_destroy(j->sim);
         if (j->step_done) cudaEventDestroy(j->step_done);
     }
-    DevBuf *bufs[] = {&s->pool, &s->hi, &s->lo, &s->d_sys, &s->d_items, &s->d_counter,
-                      &s->d_new_sys, &s->d_new_items};
+    DevBuf *bufs[] = {&s->pool, &s->hi, &s->lo, &s->queue_all.d_sys, &s->queue_all.d_items,
+                      &s->queue_all.part, &s->queue_new.d_sys, &s->queue_new.d_items,
+                      &s->queue_new.part};
     for (DevBuf *b : bufs) b->release();
     if (s->tick_start) cudaEventDestroy(s->tick_start);
     if (s->direct_done) cudaEventDestroy(s->direct_done);
