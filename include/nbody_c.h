@@ -118,11 +118,12 @@ typedef struct nb_config {
  * a warp-local origin, the closest pairs in double-single) and smaller ones the
  * all-pairs double-single kernel; these flags force one or the other.  The
  * sorted kernel also holds every body to |da| <= 1e-6 |a| without the
- * conditioning clause of the all-pairs kernel.  Both kernels time their CTA
- * shapes on the first evaluation of each N in a process and keep the fastest;
- * the j-segments and the bodies per warp (which set the summation order) are
- * fixed by N alone, so results are bit-identical within a process and between
- * processes on the same GPU model. */
+ * conditioning clause of the all-pairs kernel.  The all-pairs kernel times its
+ * CTA shapes on the first evaluation of each N in a process and keeps the
+ * fastest.  The order in which a body's terms are summed is fixed by N alone in
+ * both, so results are bit-identical within a process and between processes on
+ * the same GPU model.
+ */
 #define NB_FLAG_MIXED_SORTED 4
 #define NB_FLAG_MIXED_UNSORTED 8
 
@@ -260,11 +261,10 @@ nb_status nb_bh_read_nodes(nb_sim *sim, int max_nodes, int *depth, uint64_t *pre
  * concatenation, the step loop captured in a CUDA graph and replayed.  By
  * default every system is sorted along a Hilbert curve through its own cube
  * (at the start of each nb_ensemble_step call, every 25 steps within it, and
- * in nb_ensemble_compute_forces) and far 32-body chunks take the plain FP32
+ * in nb_ensemble_compute_forces) and far 64-body tiles take the plain FP32
  * pair term, as in the single-system sorted kernel; cfg->flags
- * NB_FLAG_MIXED_UNSORTED selects the all-pairs kernel, whose i-bodies per lane
- * are autotuned per N bucket on the loaded systems at the first evaluation (or
- * by nb_ensemble_tune).  Either way a system's result does not depend on the
+ * NB_FLAG_MIXED_UNSORTED selects the double-single term for every pair.  Either
+ * way a system's result does not depend on the
  * other systems of the ensemble. */
 typedef struct nb_ensemble nb_ensemble;
 

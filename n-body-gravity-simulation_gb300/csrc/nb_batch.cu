@@ -170,7 +170,10 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                    double *__restrict__ ay, double *__restrict__ az, int total, int num_tiles)
 {
     __shared__ union {
-        TileJ tile;
+        struct {
+            TileJ hi;
+            TileJLow lo;
+        } tile;
         PairTile chunk;
     } stages;
     __shared__ TileSums sums[kBatchTiles];  // of the second block's tiles
@@ -186,7 +189,8 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                                      stages.chunk, total);
         return;
     }
-    TileJ &stage = stages.tile;
+    TileJ &stage = stages.tile.hi;
+    TileJLow &low = stages.tile.lo;
     const bool within = it.p == 0;  // the block with itself
     const int blk_b = (it.a + it.p) % sd.blocks;
     const int tiles = (sd.n + kTile - 1) / kTile;
@@ -199,7 +203,8 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     for (int v = 0; v < kBatchTiles; ++v) tile_sums_zero(sums[v], lane);
 
     for (int u = 0; u < ta; ++u) {
-        TileI ti;
+        TileI<2> ti;
+        TileILow<2> tl;
         TileBox bi{};
         float cx = 0.f, cy = 0.f, cz = 0.f;
         if (SORTED) {
@@ -227,7 +232,8 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                 }
                 mi = h.w;
             }
-            tile_i_set(ti, k, S[0], S[1], S[2], E[0], E[1], E[2], mi);
+            tile_i_set(ti, k, S, mi);
+            tile_i_set_low(tl, k, E);
         }
         for (int v = within ? u : 0; v < tb; ++v) {
             const int tj = tj0 + v;
@@ -258,15 +264,18 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                     }
                     mj = h.w;
                 }
-                tile_j_put(stage, lane, h2, S[0], S[1], S[2], E[0], E[1], E[2], mj);
+                tile_j_put(stage, lane, h2, S, mj);
+                tile_j_put_low(low, lane, h2, E);
             }
             __syncwarp();
             if (within && u == v)
-                tile_self<ZERO_SOFT>(stage, lane, 0, 4, ti, e2, isum);
+                tile_self<ZERO_SOFT>(stage, &low, lane, ti, &tl, e2, isum);
             else if (far)
-                tile_pair<false, ZERO_SOFT>(stage, lane, 0, 4, ti, e2, isum, sums[v]);
+                tile_pair<kVeryFarTerm, false, ZERO_SOFT, 2>(stage, &low, lane, ti, &tl, e2, 0.f, 0.f, &isum,
+                                                      sums[v]);
             else
-                tile_pair<true, ZERO_SOFT>(stage, lane, 0, 4, ti, e2, isum, sums[v]);
+                tile_pair<kNearTerm, false, ZERO_SOFT, 2>(stage, &low, lane, ti, &tl, e2, 0.f, 0.f, &isum,
+                                                     sums[v]);
         }
         // the i-tile's partial sums; within a block with what it took as a j-tile
 #pragma unroll

@@ -1,33 +1,37 @@
 // nb_direct_sorted.cu -- the mixed-precision all-pairs sum over Hilbert-sorted
-// bodies with a near/far split decided per warp and per 32-body j-chunk, in
-// packed FP32x2 arithmetic.
+// bodies, in packed FP32x2 arithmetic: far 64-body tiles once for both bodies of
+// a pair, near ones as ordered pairs by 32-body j-chunk, the closest pairs in
+// double-single.
 //
 // Near/far.  The double-single displacement of the mixed pair term costs 6 of
 // its 21 FP32 operations and is needed only when a pair is close compared with
 // the distance of its bodies from the coordinate origin.  Here the origin
 // moves to each warp: bodies are sorted along a Hilbert curve (the Barnes-Hut
-// radix sort on Hilbert keys), so the 32*IPT consecutive bodies a warp owns are
+// radix sort on Hilbert keys), so the 64 consecutive bodies of a tile are
 // spatially compact.  The Hilbert curve never jumps between distant cells (the
-// Morton curve does at every cell boundary), so its warp and chunk boxes are
+// Morton curve does at every cell boundary), so its tile and chunk boxes are
 // smaller: on a 65,536-body Plummer sphere 5 % of the chunk pairs are near
-// instead of 11 %, and the kernel runs 4.7 % faster.  The warp takes the centre c of their bounding box as
-// origin and stages every j-chunk (32 consecutive sorted bodies, one per lane)
-// as a normalised double-single (S, E) of x - c.  A chunk whose bounding box
-// lies at least kFarFactor * D from the warp's box (D: the warp box diameter)
-// runs the plain FP32 term on S alone (15 FP32 operations + 1 MUFU), and a
-// chunk at least kVeryFar * D away drops the folded Newton step too (12 + 1); other
-// chunks take the full double-single term on S and E (21 + 1).  Decisions are
-// uniform over the warp (no divergence) and a warp stages its own chunks in its
-// own shared memory: no CTA-wide barrier.
+// instead of 11 %.
+//
+// direct_far_kernel takes the tile pairs that hold no close pair and lie at least
+// kFarFactor D apart (D: the smaller box's diameter; 97 % of them at
+// N = 65,536) over unordered pairs (nb_tile.cuh), relative to a tile's centre in
+// plain FP32; at kVeryFar of the larger diameter the folded Newton step is left
+// out too.  direct_near_kernel sums the others by row: a warp takes its tile's
+// centre c as the origin and stages each j-chunk as a normalised double-single
+// (S, E) of x - c, or S alone where the chunk's box is far or very far from its
+// own.  Decisions are uniform over a warp, and a warp stages its own tiles in
+// its own shared memory: no CTA-wide barrier.
+//
+// Measured at N = 65,536 (a velocity-Verlet step) and N = 400,003 (an
+// evaluation): 1.48 and 46.3 ms, where the row kernel over every j-chunk, each
+// pair evaluated twice, took 1.98 and 67 ms.
 //
 // Packed arithmetic.  sm_100-class SMs execute FP32 add, multiply and FMA on
 // register pairs (f32x2) at the FP32 pipe's lane rate but half the issue
-// slots.  The scalar kernels issue ~24 instructions per interaction for 21 FP32
-// operations and sit at the issue limit; here each thread evaluates two j at
-// once (a j-pair, staged side by side in shared memory) against IPT i-bodies
-// held as duplicated pairs, so the FP32 work issues as f32x2 and the FP32 pipe,
-// not issue, bounds the kernel.  Every lane of an f32x2 operation rounds like
-// its scalar counterpart.
+// slots: each thread evaluates two j at once (a j-pair, staged side by side in
+// shared memory) against i-bodies held as duplicated pairs.  Every lane of an
+// f32x2 operation rounds like its scalar counterpart.
 //
 // Error of a far term: S carries one FP32 rounding of x - c.  With
 // |xi - c| <= D/2, |xj - c| <= r + D/2 and the subtraction's own rounding, the
@@ -41,98 +45,74 @@
 // so their errors average out: on a 65,536-body Plummer sphere the far /
 // very-far factors (1/8, 1/4), (1/4, 1/4), (1/4, 1/2), (1/2, 1/2) and (1/2, 1)
 // give the same errors (largest relative 5e-7 where S_i / |a_i| <= 10, RMS
-// 2.5e-8), and (1/8, 1/4) the shortest kernel (2 % under (1/4, 1/2)).  Near terms keep the double-single
+// 2.5e-8), and (1/8, 1/4) the shortest kernel.  The bounds hold for both bodies of
+// a far pair: they are in units of r.  Near terms keep the double-single
 // displacement (absolute error ~2^-48 |x|) and the Newton step; every FP32
 // accumulator takes 16 terms before its Kahan-compensated add, and the
 // segments combine as a double-single.
 #include "nb_internal.h"
 #include "nb_check.cuh"
-#include "nb_pair.cuh"
+#include "nb_tile.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <map>
-#include <mutex>
 
 namespace nb {
 namespace {
 
 constexpr int kChunk = 32;             // j-chunk = one body per lane
-constexpr int kIpt = 2;                // 32-body i-chunks per warp (fixed: it sets the bits)
-constexpr int kExactWarps = 8;         // warps of exact_pairs_kernel per main-kernel warp
+constexpr int kIpt = kTile / kChunk;   // 32-body i-chunks per warp
+constexpr int kFarTiles = 4;           // tiles per block of the far kernel
+// Its one-warp CTAs per SM: 12 / 14 / 16 measured 1.53 / 1.47 / 1.47 ms a step.
+constexpr int kFarCtas = 16;
+constexpr size_t kFarPlaneBytes = (size_t)1 << 30;  // its partial planes per pass
+constexpr int kExactWarps = 8;         // warps of exact_pairs_kernel per tile
 constexpr int kExactRound = 64;        // left-out pairs evaluated per round and warp
 constexpr int kResortEvals = 8;        // force evaluations per re-sort
 constexpr bool kHilbertOrder = true;   // sort along the Hilbert curve (else Morton)
 
-// Positions in sorted order relative to the root centre, split into
-// double-single hi/lo parts (mass in hi.w), and the bounding box of the hi
-// positions of every 32-body chunk (a warp is a chunk: box[2t] = min,
-// box[2t+1] = max; lanes past n take the chunk's first body).  Blocks are
-// multiples of 32 threads.
-__global__ void split_sorted_kernel(const uint32_t *__restrict__ order,
-                                    const double *__restrict__ x, const double *__restrict__ y,
-                                    const double *__restrict__ z, const double *__restrict__ m,
-                                    int n, const double *__restrict__ centre,
-                                    float4 *__restrict__ hi, float4 *__restrict__ lo,
-                                    float4 *__restrict__ box)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int chunk = i / kChunk, lane = threadIdx.x & 31;
-    if (chunk * kChunk >= n) return;  // the whole warp is past n
-    float p[3] = {0.f, 0.f, 0.f};
-    const uint32_t o = i < n ? order[i] : 0u;
-    if (i < n && NB_IN_RANGE(o, n)) {
-        const double X = x[o] - centre[0], Y = y[o] - centre[1], Z = z[o] - centre[2];
-        const float hx = __double2float_rn(X), hy = __double2float_rn(Y),
-                    hz = __double2float_rn(Z);
-        const float hm = __double2float_rn(m[o]);
-        hi[i] = make_float4(hx, hy, hz, hm);
-        lo[i] = make_float4(__double2float_rn(X - (double)hx), __double2float_rn(Y - (double)hy),
-                            __double2float_rn(Z - (double)hz), __double2float_rn(m[o] - (double)hm));
-        p[0] = hx;
-        p[1] = hy;
-        p[2] = hz;
-    }
+// The mass of a tile whose bodies do not all have one (compares false).
+#define kNoMass __int_as_float(0x7fffffff)
+
+// A 64-body tile: its box, squared diameter, the mass of its bodies (kNoMass:
+// not all equal) and the squared left-out radius of its pairs.  Every product
+// and sum here and in the functions below is an explicit round-to-nearest
+// intrinsic: the kernels must take the same decisions bit for bit.
+struct TileGeom {
     float mn[3], mx[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float first = __shfl_sync(0xffffffffu, p[k], 0);
-        mn[k] = mx[k] = i < n ? p[k] : first;
-    }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], s));
-            mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], s));
-        }
-    if (lane == 0) {
-        box[2 * chunk] = make_float4(mn[0], mn[1], mn[2], 0.f);
-        box[2 * chunk + 1] = make_float4(mx[0], mx[1], mx[2], 0.f);
-    }
+    float diam2, mass, thr2x;
+};
+__device__ __forceinline__ float box_diam2(const float (&mn)[3], const float (&mx)[3])
+{
+    const float sx = __fsub_rn(mx[0], mn[0]), sy = __fsub_rn(mx[1], mn[1]),
+                sz = __fsub_rn(mx[2], mn[2]);
+    return __fmaf_rn(sz, sz, __fmaf_rn(sy, sy, __fmul_rn(sx, sx)));
 }
 
-// A warp's box (the union of its IPT chunk boxes), its centre (the origin of
-// every staged coordinate), and the squared thresholds of its near/far and
-// left-out decisions.  Every product and sum is an explicit round-to-nearest
-// intrinsic: direct_sorted_kernel and exact_pairs_kernel must take the same
-// decisions bit for bit.
-struct WarpGeom {
-    float bmn[3], bmx[3], c[3];
-    float thr2, thr2v, thr2x;
-};
-
-// The global cap of the left-out radius, squared: kExactSpacing times the
-// mean body spacing of the root cube, (side^3 / n)^(1/3).  A warp of sparse
-// bodies spread over a large box would otherwise get a radius that takes in
-// whole dense regions, whose terms are a tiny part of its bodies' sums.
-// per_n = kExactSpacing2 n^(-2/3), computed on the host.
-__device__ __forceinline__ float exact_cap2(const double *__restrict__ root, float per_n)
+// Pairs closer than R leave the FP32 sum and are evaluated in double-single by
+// exact_pairs_kernel (only chunks nearer than R can hold one):
+// R = min(kExact D, kExactSpacing s, the global cap), s the mean body spacing of
+// the tile's box, (V / 64)^(1/3) with every side padded by D / 16 so that a flat
+// box keeps its in-plane spacing.
+// The cap is kExactSpacing times the mean body spacing of the root cube,
+// (side^3 / n)^(1/3).  A tile of sparse bodies spread over a large box would
+// otherwise get a radius that takes in whole dense regions, whose terms are a
+// tiny part of its bodies' sums.  per_n = kExactSpacing2 n^(-2/3), computed on
+// the host.
+__device__ __forceinline__ float left_out_radius2(const float (&mn)[3], const float (&mx)[3],
+                                                  const double *__restrict__ root, float per_n)
 {
+    const float diam2 = box_diam2(mn, mx);
+    const float pad = __fmul_rn(0.0625f, sqrtf(diam2));
+    float vol = 1.0f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) vol = __fmul_rn(vol, __fadd_rn(__fsub_rn(mx[a], mn[a]), pad));
+    const float s2 = exp2f(__fmul_rn(0.6666667f, log2f(__fmul_rn(vol, 1.0f / kTile))));
     const float side = __double2float_rn(root[3]);
-    return __fmul_rn(__fmul_rn(side, side), per_n);
+    const float cap2 = __fmul_rn(__fmul_rn(side, side), per_n);
+    return fminf(fminf(__fmul_rn(kExact2, diam2), __fmul_rn(kExactSpacing2, s2)), cap2);
 }
 
 float exact_cap_per_n(int n)
@@ -140,78 +120,351 @@ float exact_cap_per_n(int n)
     return (float)((double)kExactSpacing2 / std::cbrt((double)n * (double)n));
 }
 
-template <int IPT>
-__device__ __forceinline__ WarpGeom warp_geometry(const float4 *__restrict__ box, int tile0,
-                                                  int nchunks, float far2, float cap2)
+// Positions in sorted order relative to the root centre, split into
+// double-single hi/lo parts (mass in hi.w); the bounding box of the hi positions
+// of every 32-body chunk (box[2c] = min, box[2c+1] = max; lanes past n take the
+// chunk's first body); and every 64-body tile's record (tile[2t] = min and mass,
+// tile[2t+1] = max and left-out radius).  A warp is a tile.
+__global__ void __launch_bounds__(128)
+split_sorted_kernel(const uint32_t *__restrict__ order, const double *__restrict__ x,
+                    const double *__restrict__ y, const double *__restrict__ z,
+                    const double *__restrict__ m, int n, const double *__restrict__ root,
+                    float cap_per_n, float4 *__restrict__ hi, float4 *__restrict__ lo,
+                    float4 *__restrict__ box, float4 *__restrict__ tile)
+{
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (t * kTile >= n) return;
+    float tmn[3] = {3.0e38f, 3.0e38f, 3.0e38f}, tmx[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+    float m0 = 0.f;
+    bool equal = true;
+#pragma unroll
+    for (int c = 0; c < kIpt; ++c) {
+        const int i = t * kTile + kChunk * c + lane;
+        if (i - lane >= n) break;  // the whole chunk is past n
+        float p[3] = {0.f, 0.f, 0.f}, hm = 0.f;
+        const uint32_t o = i < n ? order[i] : 0u;
+        if (i < n && NB_IN_RANGE(o, n)) {
+            const double X = x[o] - root[0], Y = y[o] - root[1], Z = z[o] - root[2];
+            p[0] = __double2float_rn(X);
+            p[1] = __double2float_rn(Y);
+            p[2] = __double2float_rn(Z);
+            hm = __double2float_rn(m[o]);
+            hi[i] = make_float4(p[0], p[1], p[2], hm);
+            lo[i] = make_float4(__double2float_rn(X - (double)p[0]),
+                                __double2float_rn(Y - (double)p[1]),
+                                __double2float_rn(Z - (double)p[2]),
+                                __double2float_rn(m[o] - (double)hm));
+        }
+        float mn[3], mx[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float first = __shfl_sync(0xffffffffu, p[k], 0);
+            mn[k] = mx[k] = i < n ? p[k] : first;
+        }
+        if (c == 0) m0 = __shfl_sync(0xffffffffu, hm, 0);
+        equal = equal && __all_sync(0xffffffffu, i >= n || hm == m0);
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], s));
+                mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], s));
+            }
+        if (lane == 0) {
+            box[2 * (kIpt * t + c)] = make_float4(mn[0], mn[1], mn[2], 0.f);
+            box[2 * (kIpt * t + c) + 1] = make_float4(mx[0], mx[1], mx[2], 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            tmn[k] = fminf(tmn[k], mn[k]);
+            tmx[k] = fmaxf(tmx[k], mx[k]);
+        }
+    }
+    if (lane == 0) {
+        tile[2 * t] = make_float4(tmn[0], tmn[1], tmn[2], equal ? m0 : kNoMass);
+        tile[2 * t + 1] = make_float4(tmx[0], tmx[1], tmx[2],
+                                      left_out_radius2(tmn, tmx, root, cap_per_n));
+    }
+}
+
+__device__ __forceinline__ TileGeom tile_geometry(const float4 *__restrict__ tile, int t)
+{
+    const float4 a = tile[2 * t], b = tile[2 * t + 1];
+    TileGeom g;
+    g.mn[0] = a.x; g.mn[1] = a.y; g.mn[2] = a.z;
+    g.mx[0] = b.x; g.mx[1] = b.y; g.mx[2] = b.z;
+    g.mass = a.w;
+    g.thr2x = b.w;
+    g.diam2 = box_diam2(g.mn, g.mx);
+    return g;
+}
+
+// Squared gap between two boxes, the same bits whichever is called first.
+__device__ __forceinline__ float box_gap2(const float (&amn)[3], const float (&amx)[3],
+                                          const float (&bmn)[3], const float (&bmx)[3])
+{
+    float g[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        g[a] = fmaxf(0.f, fmaxf(__fsub_rn(bmn[a], amx[a]), __fsub_rn(amn[a], bmx[a])));
+    return __fmaf_rn(g[2], g[2], __fmaf_rn(g[1], g[1], __fmul_rn(g[0], g[0])));
+}
+
+// Whether two tiles are direct_far_kernel's: an eighth of the smaller diameter
+// apart (a plain FP32 displacement relative to that tile's centre is enough) and
+// without left-out pairs on either side.  All other tile pairs are
+// direct_near_kernel's and exact_pairs_kernel's; a chunk of such a tile lies no
+// nearer than the tile, in these operations too, so neither kernel leaves out a
+// pair of the far tiles.
+__device__ __forceinline__ bool tiles_apart(const TileGeom &a, const TileGeom &b, float gap2)
+{
+    return gap2 > 0.f && gap2 >= __fmul_rn(kFarFactor2, fminf(a.diam2, b.diam2)) &&
+           gap2 >= fmaxf(a.thr2x, b.thr2x);
+}
+// Whether they are very far apart seen from both (a quarter of the larger
+// diameter): no Newton step.  Implies tiles_apart.
+__device__ __forceinline__ bool tiles_very_far(const TileGeom &a, const TileGeom &b, float gap2)
+{
+    return tiles_apart(a, b, gap2) && gap2 >= __fmul_rn(kVeryFar2, fmaxf(a.diam2, b.diam2));
+}
+
+// A warp's tile, its centre (the origin of every staged coordinate), and the
+// squared thresholds of its near/far decisions.
+struct WarpGeom {
+    TileGeom tile;
+    float c[3];
+    float thr2, thr2v;
+};
+
+__device__ __forceinline__ WarpGeom warp_geometry(const float4 *__restrict__ tiles, int t,
+                                                  float far2)
 {
     WarpGeom g;
+    g.tile = tile_geometry(tiles, t);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        g.bmn[a] = 3.0e38f;
-        g.bmx[a] = -3.0e38f;
-    }
-#pragma unroll
-    for (int k = 0; k < IPT; ++k)
-        if (tile0 + k < nchunks) {
-            const float4 a = box[2 * (tile0 + k)], b = box[2 * (tile0 + k) + 1];
-            g.bmn[0] = fminf(g.bmn[0], a.x); g.bmn[1] = fminf(g.bmn[1], a.y);
-            g.bmn[2] = fminf(g.bmn[2], a.z);
-            g.bmx[0] = fmaxf(g.bmx[0], b.x); g.bmx[1] = fmaxf(g.bmx[1], b.y);
-            g.bmx[2] = fmaxf(g.bmx[2], b.z);
-        }
-    float side[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        g.c[a] = __fmul_rn(0.5f, __fadd_rn(g.bmn[a], g.bmx[a]));
-        side[a] = __fsub_rn(g.bmx[a], g.bmn[a]);
-    }
-    const float diam2 = __fmaf_rn(side[2], side[2],
-                                  __fmaf_rn(side[1], side[1], __fmul_rn(side[0], side[0])));
-    g.thr2 = __fmul_rn(far2, diam2);        // far: double-single not needed
-    g.thr2v = __fmul_rn(kVeryFar2, diam2);  // very far: Newton step not needed
-    // Pairs closer than R leave the FP32 sum and are evaluated in double-single
-    // by exact_pairs_kernel (only chunks nearer than R can hold one):
-    // R = min(kExact D, kExactSpacing s, the global cap), s the mean body
-    // spacing of the warp's box, (V / 64)^(1/3) with every side padded by D / 16
-    // so that a flat box keeps its in-plane spacing.
-    const float pad = __fmul_rn(0.0625f, sqrtf(diam2));
-    const float vol = __fmul_rn(__fmul_rn(__fadd_rn(side[0], pad), __fadd_rn(side[1], pad)),
-                                __fadd_rn(side[2], pad));
-    const float s2 = exp2f(__fmul_rn(0.6666667f, log2f(__fmul_rn(vol, 1.0f / (32.0f * IPT)))));
-    g.thr2x = fminf(fminf(__fmul_rn(kExact2, diam2), __fmul_rn(kExactSpacing2, s2)), cap2);
+    for (int a = 0; a < 3; ++a) g.c[a] = __fmul_rn(0.5f, __fadd_rn(g.tile.mn[a], g.tile.mx[a]));
+    g.thr2 = __fmul_rn(far2, g.tile.diam2);        // far: double-single not needed
+    g.thr2v = __fmul_rn(kVeryFar2, g.tile.diam2);  // very far: Newton step not needed
     return g;
 }
 
 // Squared gap between the warp's box and a j-chunk's box.
 __device__ __forceinline__ float chunk_gap2(const WarpGeom &g, float4 jmn, float4 jmx)
 {
-    const float gx = fmaxf(0.f, fmaxf(__fsub_rn(jmn.x, g.bmx[0]), __fsub_rn(g.bmn[0], jmx.x)));
-    const float gy = fmaxf(0.f, fmaxf(__fsub_rn(jmn.y, g.bmx[1]), __fsub_rn(g.bmn[1], jmx.y)));
-    const float gz = fmaxf(0.f, fmaxf(__fsub_rn(jmn.z, g.bmx[2]), __fsub_rn(g.bmn[2], jmx.z)));
-    return __fmaf_rn(gz, gz, __fmaf_rn(gy, gy, __fmul_rn(gx, gx)));
+    const float mn[3] = {jmn.x, jmn.y, jmn.z}, mx[3] = {jmx.x, jmx.y, jmx.z};
+    return box_gap2(g.tile.mn, g.tile.mx, mn, mx);
 }
 
-// One warp = 32*IPT consecutive sorted i-bodies (chunks tile0 .. tile0+IPT-1,
-// lane l of chunk k holds body (tile0 + k) * 32 + l); blockIdx.y selects the
-// j-chunks [y * seg_chunks, (y + 1) * seg_chunks).  Writes per-segment Kahan
-// sums and compensations (sorted order).  Warps are independent: a warp whose
-// chunks are all past n returns at once.
-template <int WARPS, int IPT, bool ZERO_SOFT>
-__global__ void __launch_bounds__(WARPS * 32)
-direct_sorted_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
-                     const float4 *__restrict__ box, int n, int nchunks, float eps2,
-                     int seg_chunks, float *__restrict__ psum, float *__restrict__ pcomp,
-                     float far2, const double *__restrict__ root, float cap_per_n)
+// Stages the i-bodies (IPT chunks from i0) relative to c.
+template <int IPT>
+__device__ __forceinline__ void far_load_i(const float4 *__restrict__ hi,
+                                           const float4 *__restrict__ lo, int n, int i0,
+                                           const float (&c)[3], TileI<IPT> &ti)
 {
-    __shared__ PairTile stage[WARPS];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int tile0 = (blockIdx.x * WARPS + w) * IPT;
-    if (tile0 >= nchunks) return;
-    PairTile &sg = stage[w];
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        // lanes past n: massless and far from every j-body (r^-3 is exactly 0)
+        float S[3] = {-1.0e18f, -1.0e18f, -1.0e18f}, m = 0.f;
+        const int i = i0 + 32 * k + (int)threadIdx.x;
+        if (i < n) {
+            const float4 h = hi[i], l = lo[i];
+            S[0] = rel_s(h.x, l.x, c[0]);
+            S[1] = rel_s(h.y, l.y, c[1]);
+            S[2] = rel_s(h.z, l.z, c[2]);
+            m = h.w;
+        }
+        tile_i_set(ti, k, S, m);
+    }
+}
 
-    const WarpGeom gm = warp_geometry<IPT>(box, tile0, nchunks, far2, exact_cap2(root, cap_per_n));
+// Stages the j-tile from body j0 relative to c and adds its pairs with ti.
+// equal: the equal-mass loop, mi = the i-bodies' mass.
+template <int TERM, int IPT>
+__device__ __forceinline__ void far_tile_pair(const float4 *__restrict__ hi,
+                                              const float4 *__restrict__ lo, int n, int j0,
+                                              const float (&c)[3], const TileI<IPT> &ti, bool equal,
+                                              float mi, float2 e2, TileJ &stage, TileSums *isum,
+                                              TileSums &jsum)
+{
+    const int lane = threadIdx.x;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int j = j0 + 32 * k + lane;
+        float S[3] = {1.0e18f, 1.0e18f, 1.0e18f}, mj = 0.f;
+        if (j < n) {
+            const float4 h = hi[j], l = lo[j];
+            S[0] = rel_s(h.x, l.x, c[0]);
+            S[1] = rel_s(h.y, l.y, c[1]);
+            S[2] = rel_s(h.z, l.z, c[2]);
+            mj = h.w;
+        }
+        tile_j_put(stage, lane, k, S, mj);
+    }
+    __syncwarp();
+    if (equal)
+        tile_pair<TERM, true, false, IPT>(stage, nullptr, lane, ti, nullptr, e2, mi, stage.b[0].z,
+                                          isum, jsum);
+    else
+        tile_pair<TERM, false, false, IPT>(stage, nullptr, lane, ti, nullptr, e2, 0.f, 0.f, isum,
+                                           jsum);
+}
+
+// The pairs of far tiles, once for both bodies (nb_tile.cuh).  One warp = one
+// pair of 256-body blocks (a, a + p), the second block's sums in shared memory.
+// It takes two of the first block's tiles at a time (four i-bodies per lane)
+// against a tile of the second that both are very far from; they share an
+// origin, the centre of their common box, which has to be D / 8 or more from the
+// j-tile (D its diameter), the bound of a plain FP32 displacement.  Other far
+// tile pairs are met one by one, relative to the smaller tile's centre and with
+// the Newton step.
+// part: plane p - p0 holds the first side's sums of diagonal p, plane np + p - p0
+// the second's (one rounding of a Kahan pair: with 64 planes and more it adds
+// 2e-9 to an error of 3e-8).
+__global__ void __launch_bounds__(32, kFarCtas)
+direct_far_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
+                  const float4 *__restrict__ tile, int n, int tiles, float eps2, int blocks,
+                  int p0, int np, float *__restrict__ part)
+{
+    static_assert(kFarTiles == 4, "the lanes' tile-pair tests");
+    __shared__ TileJ stage;
+    __shared__ TileSums jsum[kFarTiles], isum[2];
+    const int lane = threadIdx.x;
+    const int a = blockIdx.x % blocks, dp = blockIdx.x / blocks, p = p0 + dp;
+    if (!pair_first(p, a, blocks)) return;
+    const int ti0 = a * kFarTiles, tj0 = (a + p) % blocks * kFarTiles;
+    const int ta = min(kFarTiles, tiles - ti0), tb = min(kFarTiles, tiles - tj0);
+    // lane 4 u + v decides the tile pair (u, v), lane 16 + 4 h + v tiles 2 h and
+    // 2 h + 1 together against v
+    bool far = false, equal = false;
+    {
+        const bool two = lane >= 16;
+        const int u = two ? (lane & 4) / 2 : lane / 4, v = lane & 3;
+        if (lane < 24 && u + two < ta && v < tb && (p > 0 || v > u + two)) {
+            TileGeom gi = tile_geometry(tile, ti0 + u);
+            const TileGeom gj = tile_geometry(tile, tj0 + v);
+            float gap2 = box_gap2(gi.mn, gi.mx, gj.mn, gj.mx);
+            if (two) {
+                const TileGeom g1 = tile_geometry(tile, ti0 + u + 1);
+                far = tiles_very_far(gi, gj, gap2) &&
+                      tiles_very_far(g1, gj, box_gap2(g1.mn, g1.mx, gj.mn, gj.mx));
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    gi.mn[d] = fminf(gi.mn[d], g1.mn[d]);
+                    gi.mx[d] = fmaxf(gi.mx[d], g1.mx[d]);
+                }
+                gap2 = box_gap2(gi.mn, gi.mx, gj.mn, gj.mx);
+                far = far && gap2 >= kFarFactor2 * box_diam2(gi.mn, gi.mx);
+                gi.mass = gi.mass == g1.mass ? gi.mass : kNoMass;
+            } else {
+                far = tiles_apart(gi, gj, gap2);
+            }
+            float span2 = 0.f;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const float s = fmaxf(gi.mx[d], gj.mx[d]) - fminf(gi.mn[d], gj.mn[d]);
+                span2 = fmaf(s, s, span2);
+            }
+            equal = far && gi.mass == gi.mass && gj.mass == gj.mass &&
+                    equal_range(gap2, span2, eps2);
+        }
+    }
+    const unsigned fars = __ballot_sync(0xffffffffu, far);
+    const unsigned equals = __ballot_sync(0xffffffffu, equal);
+    const float2 e2 = dup2(eps2);
+    for (int v = 0; v < kFarTiles; ++v) tile_sums_zero(jsum[v], lane);
+    const size_t plane = (size_t)n;
+    float *pa = part + 3 * plane * dp, *pb = part + 3 * plane * (np + dp);
+    for (int h = 0; 2 * h < ta; ++h) {
+        tile_sums_zero(isum[0], lane);
+        tile_sums_zero(isum[1], lane);
+        const unsigned both = fars >> (16 + 4 * h) & 15u;
+        if (both) {
+            const TileGeom g = tile_geometry(tile, ti0 + 2 * h),
+                           g1 = tile_geometry(tile, ti0 + 2 * h + 1);
+            float c[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                c[d] = 0.5f * (fminf(g.mn[d], g1.mn[d]) + fmaxf(g.mx[d], g1.mx[d]));
+            TileI<4> ti;
+            far_load_i(hi, lo, n, (ti0 + 2 * h) * kTile, c, ti);
+            for (int v = 0; v < tb; ++v)
+                if (both >> v & 1u)
+                    far_tile_pair<kVeryFarTerm>(hi, lo, n, (tj0 + v) * kTile, c, ti,
+                                                equals >> (16 + 4 * h + v) & 1u, g.mass, e2, stage,
+                                                isum, jsum[v]);
+        }
+#pragma unroll 1
+        for (int w = 0; w < 2; ++w) {
+            const int u = 2 * h + w;
+            const unsigned one = (fars >> (4 * u) & 15u) & ~both;
+#pragma unroll 1
+            for (int v = 0; v < tb; ++v) {
+                if (!(one >> v & 1u)) continue;
+                const TileGeom g = tile_geometry(tile, ti0 + u), gj = tile_geometry(tile, tj0 + v);
+                const bool mine = g.diam2 <= gj.diam2;
+                float c[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    c[d] = mine ? 0.5f * (g.mn[d] + g.mx[d]) : 0.5f * (gj.mn[d] + gj.mx[d]);
+                TileI<2> ti;
+                far_load_i(hi, lo, n, (ti0 + u) * kTile, c, ti);
+                far_tile_pair<kFarTerm>(hi, lo, n, (tj0 + v) * kTile, c, ti,
+                                        equals >> (4 * u + v) & 1u, g.mass, e2, stage, isum + w,
+                                        jsum[v]);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const int u = 2 * h + w, i = (ti0 + u) * kTile + lane;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                float2 t = isum[w].s[d][lane], e = isum[w].c[d][lane];
+                if (p == 0) {  // within a block: with what the tile took as a j-tile
+                    const float2 js = jsum[u].s[d][lane], jc = jsum[u].c[d][lane];
+                    float2 r;
+                    two_sum(t.x, js.x, t.x, r.x);
+                    two_sum(t.y, js.y, t.y, r.y);
+                    e = make_float2(r.x + (e.x + jc.x), r.y + (e.y + jc.y));
+                }
+                if (i < n) pa[d * plane + i] = t.x + e.x;
+                if (i + 32 < n) pa[d * plane + i + 32] = t.y + e.y;
+            }
+        }
+    }
+    if (p == 0) return;
+    for (int v = 0; v < tb; ++v) {
+        const int j = (tj0 + v) * kTile + lane;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float2 js = jsum[v].s[d][lane], jc = jsum[v].c[d][lane];
+            if (j < n) pb[d * plane + j] = js.x + jc.x;
+            if (j + 32 < n) pb[d * plane + j + 32] = js.y + jc.y;
+        }
+    }
+}
+
+// All other pairs, as ordered pairs.  One warp = one tile of i-bodies (lane l of
+// chunk k holds body 64 tile + 32 k + l) and the j-tiles t = y (mod segments)
+// that are not far from it, chunk by chunk.  Writes per-segment Kahan sums
+// and compensations (sorted order).
+template <bool ZERO_SOFT>
+__global__ void __launch_bounds__(32)
+direct_near_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
+                   const float4 *__restrict__ box, const float4 *__restrict__ tile, int n,
+                   int nchunks, float eps2, float *__restrict__ psum, float *__restrict__ pcomp,
+                   float far2)
+{
+    constexpr int IPT = kIpt;
+    __shared__ PairTile sg;
+    const int lane = threadIdx.x;
+    const int tile0 = blockIdx.x * IPT, seg = blockIdx.y, segments = gridDim.y;
+    const int tiles = (nchunks + 1) / 2;
+
+    const WarpGeom gm = warp_geometry(tile, blockIdx.x, far2);
     const float cx = gm.c[0], cy = gm.c[1], cz = gm.c[2];
-    const float thr2 = gm.thr2, thr2v = gm.thr2v, thr2x = gm.thr2x;
+    const float thr2 = gm.thr2, thr2v = gm.thr2v, thr2x = gm.tile.thr2x;
     const float thrx = __fadd_rn(thr2x, eps2);
 
     // i-bodies relative to c, negated and duplicated into pairs
@@ -242,16 +495,37 @@ direct_sorted_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ l
     }
     const float2 e2 = dup2(eps2);
 
-    const int jc0 = blockIdx.y * seg_chunks;
-    const int jc1 = min(nchunks, jc0 + seg_chunks);
+    // the next chunk of a tile that is not far, in increasing order (-1: none):
+    // the lanes test 32 of the segment's tiles at a time
+    unsigned todo = 0;
+    int scan = seg - 32 * segments, cur = -1;
+    auto next_chunk = [&]() {
+        if (cur >= 0 && !(cur & 1) && cur + 1 < nchunks) return ++cur;
+        while (!todo) {
+            scan += 32 * segments;
+            if (scan >= tiles) return cur = -1;
+            const int t = scan + lane * segments;
+            bool near = false;
+            if (t < tiles) {
+                const TileGeom gj = tile_geometry(tile, t);
+                near = !tiles_apart(gm.tile, gj, box_gap2(gm.tile.mn, gm.tile.mx, gj.mn, gj.mx));
+            }
+            todo = __ballot_sync(0xffffffffu, near);
+        }
+        const int b = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        return cur = 2 * (scan + b * segments);
+    };
+
+    int jc = next_chunk();
     // the lane's body of the next chunk, loaded one chunk ahead
     float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
-    bool valid = jc0 < jc1 && jc0 * kChunk + lane < n;
+    bool valid = jc >= 0 && jc * kChunk + lane < n;
     if (valid) {
-        h = hi[jc0 * kChunk + lane];
-        l = lo[jc0 * kChunk + lane];
+        h = hi[jc * kChunk + lane];
+        l = lo[jc * kChunk + lane];
     }
-    for (int jc = jc0; jc < jc1; ++jc) {
+    while (jc >= 0) {
         const float gap2 = chunk_gap2(gm, box[2 * jc], box[2 * jc + 1]);
         const bool far = gap2 > 0.f && gap2 >= thr2;
         const bool vfar = far && gap2 >= thr2v;
@@ -277,10 +551,11 @@ direct_sorted_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ l
         else
             pair_tile_put(sg, lane, Sx, Sy, Sz, mj, Ex, Ey, Ez);
         __syncwarp();
-        valid = jc + 1 < jc1 && (jc + 1) * kChunk + lane < n;
+        jc = next_chunk();
+        valid = jc >= 0 && jc * kChunk + lane < n;
         if (valid) {
-            h = hi[(jc + 1) * kChunk + lane];
-            l = lo[(jc + 1) * kChunk + lane];
+            h = hi[jc * kChunk + lane];
+            l = lo[jc * kChunk + lane];
         }
 
         if (vfar) {
@@ -333,7 +608,7 @@ direct_sorted_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ l
     }
 
     const size_t plane = (size_t)n;
-    const size_t base = (size_t)blockIdx.y * 3 * plane;
+    const size_t base = (size_t)seg * 3 * plane;
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
         const int i = (tile0 + k) * kChunk + lane;
@@ -348,29 +623,28 @@ direct_sorted_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ l
     }
 }
 
-// The pairs direct_sorted_kernel leaves out, in double-single.  It needs
+// The pairs direct_near_kernel leaves out, in double-single.  It needs
 // nothing from that kernel -- it takes the same decisions from the same data
-// -- so it runs beside it on a second stream.  One CTA per warp of the main
+// -- so it runs beside it on a second stream.  One CTA per warp of the near
 // kernel (the same i-chunks and geometry) and kExactWarps warps in it: warp w
-// takes the chunks jc = w (mod kExactWarps) that the main kernel tests for
+// takes the chunks jc = w (mod kExactWarps) that the near kernel tests for
 // left-out pairs (not far, nearer than R), in increasing order, skipping those
 // that no lane's i-body comes within R of.  For each it stages the chunk
-// exactly as the main kernel does, recomputes the same r^2 bits, and marks the
+// exactly as the near kernel does, recomputes the same r^2 bits, and marks the
 // left-out pairs of each lane (bit 2p + u of mk[k]: tile body 2p + u against
 // the lane's i-body k).  The marked pairs are evaluated one per lane,
 // whole-warp, in rounds of kExactRound, and every lane adds its own bodies'
 // terms into their double-single sums in increasing j; the warps' sums are
 // then added in warp order.  The result does not depend on timing.
 // ex[c n + i] = the FP64 value of body i's sum (sorted order), 0 if none.
-// At most 64 registers (four CTAs per SM): beside direct_sorted_kernel, whose
+// At most 64 registers (four CTAs per SM): beside direct_far_kernel, whose
 // one-warp CTAs fill the register file, a leaner CTA displaces fewer of them.
-template <int IPT>
 __global__ void __launch_bounds__(kExactWarps * 32, 4)
 exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
-                   const float4 *__restrict__ box, int n, int nchunks, float eps2, float far2,
-                   double eps2d, const double *__restrict__ root, float cap_per_n,
-                   double *__restrict__ ex)
+                   const float4 *__restrict__ box, const float4 *__restrict__ tile, int n,
+                   int nchunks, float eps2, float far2, double eps2d, double *__restrict__ ex)
 {
+    constexpr int IPT = kIpt;
     __shared__ PairTile stage[kExactWarps];
     __shared__ float ibody[IPT * 32][6];                      // (S, E) of x, y, z
     __shared__ uint16_t evt[kExactWarps][kExactRound];        // (k 32 + lane) << 5 | bit
@@ -381,8 +655,8 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     const int tile0 = wg * IPT;
     if (tile0 >= nchunks) return;  // the whole CTA
     PairTile &sg = stage[w];
-    const WarpGeom gm = warp_geometry<IPT>(box, tile0, nchunks, far2, exact_cap2(root, cap_per_n));
-    const float thrx = __fadd_rn(gm.thr2x, eps2);
+    const WarpGeom gm = warp_geometry(tile, wg, far2);
+    const float thrx = __fadd_rn(gm.tile.thr2x, eps2);
     const float2 e2 = dup2(eps2);
     const DS e2ds{__double2float_rn(eps2d),
                   __double2float_rn(eps2d - (double)__double2float_rn(eps2d))};
@@ -434,13 +708,13 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     // i-chunk of it) that holds a left-out pair: R grows by a slack far above
     // the FP32 roundings that separate the boxes (hi coordinates) from the
     // staged ones and the box distance from the pair's r^2 (softening included).
-    const float Rw = sqrtf(gm.thr2x);
+    const float Rw = sqrtf(gm.tile.thr2x);
     const float cmag = fmaxf(fabsf(gm.c[0]), fmaxf(fabsf(gm.c[1]), fabsf(gm.c[2])));
-    const float e2slack = 1e-6f * (gm.thr2x + eps2);
+    const float e2slack = 1e-6f * (gm.tile.thr2x + eps2);
 
     int scan = w;
     while (true) {
-        // the next chunk jc = w (mod kExactWarps) the main kernel tests, with
+        // the next chunk jc = w (mod kExactWarps) the near kernel tests, with
         // a lane whose bodies come within R of its box
         int jc = -1;
         while (scan < nchunks) {
@@ -451,7 +725,7 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                 jmn = box[2 * c];
                 jmx = box[2 * c + 1];
                 const float gap2 = chunk_gap2(gm, jmn, jmx);
-                t = !(gap2 > 0.f && gap2 >= gm.thr2) && gap2 < gm.thr2x;
+                t = !(gap2 > 0.f && gap2 >= gm.thr2) && gap2 < gm.tile.thr2x;
             }
             uint32_t cand = __ballot_sync(0xffffffffu, t);
             while (cand) {
@@ -506,7 +780,7 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
             }
         }
 
-        // stage the chunk as the main kernel's near path does
+        // stage the chunk as the near kernel does
         const int b = jc * kChunk + lane;
         float Sx = 1.0e18f, Sy = 1.0e18f, Sz = 1.0e18f, Ex = 0.f, Ey = 0.f, Ez = 0.f, mj = 0.f,
               ml = 0.f;
@@ -523,7 +797,7 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
         pair_tile_put_mlo(sg, lane, ml);
         __syncwarp();
 
-        // the left-out pairs: the main kernel's r^2 test, same operands
+        // the left-out pairs: the near kernel's r^2 test, same operands
         uint32_t mk[IPT];
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
@@ -627,133 +901,71 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     }
 }
 
-// a[order[i]] = G * (sum_s (sum_s - comp_s) + ex_i) for sorted body i: a
-// double-single sum over the segments, plus the left-out pairs (ex: none when
-// NULL), scaled in FP64.
-__global__ void combine_sorted_kernel(const float *__restrict__ psum,
-                                      const float *__restrict__ pcomp, int n, int segments,
-                                      double G, const uint32_t *__restrict__ order,
-                                      const double *__restrict__ ex, double *__restrict__ ax,
-                                      double *__restrict__ ay, double *__restrict__ az)
+// Body i's sum over the planes of np diagonals from p0, as a double-single: 32
+// bodies per block, 8 groups of planes in strides (each group's sum in order,
+// its loads ahead of it), then the groups in order.  acc: the sums of the earlier
+// passes (first: none yet), written back unless this is the last pass, which
+// adds the near segments (sum - comp; in strides too) and the left-out pairs:
+// a[order[i]] = G * (far + near + ex_i), scaled in FP64.  Bound by memory: one
+// thread per body had too few loads in flight (66 us at n = 65,536, 205 MB).
+constexpr int kCombineGroups = 8;
+__global__ void __launch_bounds__(32 * kCombineGroups)
+combine_sorted_kernel(const float *__restrict__ part, int blocks, int p0, int np, bool first,
+                      bool last, float *__restrict__ acc, const float *__restrict__ psum,
+                      const float *__restrict__ pcomp, int n, int segments, double G,
+                      const uint32_t *__restrict__ order, const double *__restrict__ ex,
+                      double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    __shared__ float2 sh[kCombineGroups][3][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
     const size_t plane = (size_t)n;
+    const int blk = i / (kFarTiles * kTile);
     float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
-    // the loads of several segments go out before their (ordered) sums
-#pragma unroll 8
-    for (int s = 0; s < segments; ++s) {
-        const size_t base = (size_t)s * 3 * plane;
+    if (i < n) {
+        for (int k0 = g; k0 < 2 * np; k0 += 8 * kCombineGroups) {
+            float t[8][3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-            ds_add_kahan(hi[c], lo[c], psum[base + c * plane + i], pcomp[base + c * plane + i]);
+            for (int u = 0; u < 8; ++u) {
+                const int k = k0 + u * kCombineGroups;
+                const bool use = k < np ? pair_first(p0 + k, blk, blocks)
+                                        : k < 2 * np && pair_second(p0 + k - np, blk, blocks);
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    t[u][c] = use ? part[((size_t)k * 3 + c) * plane + i] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) ds_add_kahan(hi[c], lo[c], t[u][c], 0.f);
+        }
+        for (int s = g; last && s < segments; s += kCombineGroups)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const size_t at = ((size_t)s * 3 + c) * plane + i;
+                ds_add_kahan(hi[c], lo[c], psum[at], pcomp[at]);
+            }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sh[g][c][lane] = make_float2(hi[c], lo[c]);
+    __syncthreads();
+    if (g >= 3 || i >= n) return;  // warp c finishes component c
+    const int c = g;
+    float2 s = first ? make_float2(0.f, 0.f)
+                     : make_float2(acc[c * plane + i], acc[(3 + c) * plane + i]);
+#pragma unroll
+    for (int k = 0; k < kCombineGroups; ++k)
+        ds_add_kahan(s.x, s.y, sh[k][c][lane].x, -sh[k][c][lane].y);
+    if (!last) {
+        acc[c * plane + i] = s.x;
+        acc[(3 + c) * plane + i] = s.y;
+        return;
     }
     const uint32_t o = order[i];
     if (!NB_IN_RANGE(o, n)) return;
-    double a[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-        a[c] = ((double)hi[c] + (double)lo[c]) + (ex ? ex[c * plane + i] : 0.0);
-    ax[o] = G * a[0];
-    ay[o] = G * a[1];
-    az[o] = G * a[2];
+    double *out = c == 0 ? ax : (c == 1 ? ay : az);
+    out[o] = G * (((double)s.x + (double)s.y) + ex[c * plane + i]);
 }
-
-// CTA shapes the autotuner times: warps per CTA x 32-body chunks per warp.
-// Warps stage their own j-chunks, so the CTA size matters only for
-// scheduling: with one- or two-warp CTAs a slow warp (many near chunks) holds
-// fewer idle warp slots until its CTA retires (1.2 % faster at N = 65,536).
-// Chunks per warp (the warp's box, hence its near/far decisions and origin)
-// and the j-segments (sorted_plan_for_shape) are the same for every shape, so
-// the timed choice never changes the bits of a result.
-struct SortedShape {
-    int warps, ipt;
-};
-constexpr SortedShape kSortedShapes[] = {{4, kIpt}, {8, kIpt}, {2, kIpt}, {1, kIpt}};
-constexpr int kNumSortedShapes = sizeof(kSortedShapes) / sizeof(kSortedShapes[0]);
-
-template <int W, int I>
-int sorted_slots()
-{
-    static const int slots = [] {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, (const void *)direct_sorted_kernel<W, I, false>, W * 32, 0);
-        return std::max(1, per_sm) * device_props().num_sms;
-    }();
-    return slots;
-}
-
-int sorted_slots_for(int warps, int ipt)
-{
-    if (warps == 4 && ipt == 2) return sorted_slots<4, 2>();
-    if (warps == 8 && ipt == 2) return sorted_slots<8, 2>();
-    if (warps == 2 && ipt == 2) return sorted_slots<2, 2>();
-    if (warps == 1 && ipt == 2) return sorted_slots<1, 2>();
-    return 0;
-}
-
-template <int W, int I>
-void launch_sorted_shape(dim3 grid, cudaStream_t st, const float4 *hi, const float4 *lo,
-                         const float4 *box, int n, double eps2, int seg_chunks, float *psum,
-                         float *pcomp, const double *root)
-{
-    const int nchunks = (n + kChunk - 1) / kChunk;
-    if (eps2 > 0.0)
-        direct_sorted_kernel<W, I, false><<<grid, W * 32, 0, st>>>(
-            hi, lo, box, n, nchunks, (float)eps2, seg_chunks, psum, pcomp, kFarFactor2, root,
-            exact_cap_per_n(n));
-    else
-        direct_sorted_kernel<W, I, true><<<grid, W * 32, 0, st>>>(
-            hi, lo, box, n, nchunks, 0.0f, seg_chunks, psum, pcomp, kFarFactor2, root,
-            exact_cap_per_n(n));
-}
-
-// DirectPlan fields here: block = threads per CTA (32 * warps), ipt = chunks
-// per warp, seg_tiles = j-chunks per segment.
-bool launch_sorted(const DirectPlan &p, cudaStream_t st, const float4 *hi, const float4 *lo,
-                   const float4 *box, int n, double eps2, float *psum, float *pcomp,
-                   const double *root)
-{
-    const int warps = p.block / 32;
-    const int nchunks = (n + kChunk - 1) / kChunk;
-    const int per_cta = warps * p.ipt;
-    const dim3 grid((nchunks + per_cta - 1) / per_cta, p.segments);
-    if (warps == 4 && p.ipt == 2)
-        launch_sorted_shape<4, 2>(grid, st, hi, lo, box, n, eps2, p.seg_tiles, psum, pcomp,
-                                  root);
-    else if (warps == 8 && p.ipt == 2)
-        launch_sorted_shape<8, 2>(grid, st, hi, lo, box, n, eps2, p.seg_tiles, psum, pcomp,
-                                  root);
-    else if (warps == 2 && p.ipt == 2)
-        launch_sorted_shape<2, 2>(grid, st, hi, lo, box, n, eps2, p.seg_tiles, psum, pcomp,
-                                  root);
-    else if (warps == 1 && p.ipt == 2)
-        launch_sorted_shape<1, 2>(grid, st, hi, lo, box, n, eps2, p.seg_tiles, psum, pcomp,
-                                  root);
-    else
-        return false;
-    return true;
-}
-
-// The j-split is modelled on one-warp CTAs of two chunks for every shape
-// (segments of at least 8 chunks, 256 j), so it depends on n alone.
-DirectPlan sorted_plan_for_shape(int n, int warps, int ipt)
-{
-    DirectPlan p;
-    p.block = warps * 32;
-    p.ipt = ipt;
-    const int nchunks = (n + kChunk - 1) / kChunk;
-    const int iblocks = (nchunks + 1) / 2;
-    const int units = std::max(1, nchunks / 8);
-    const int s = direct_pick_segments(iblocks, units, sorted_slots_for(1, 2));
-    p.seg_tiles = (nchunks + s - 1) / s;
-    p.segments = (nchunks + p.seg_tiles - 1) / p.seg_tiles;
-    return p;
-}
-
-std::mutex g_sorted_mutex;
-std::map<int, DirectPlan> g_sorted_tuned;
 
 } // namespace
 
@@ -763,7 +975,10 @@ void SortedBuffers::release()
     lo.release();
     partials.release();
     boxes.release();
+    tiles.release();
     exact.release();
+    far.release();
+    acc.release();
     if (side) cudaStreamDestroy(side);
     if (fork) cudaEventDestroy(fork);
     if (join) cudaEventDestroy(join);
@@ -787,30 +1002,21 @@ bool direct_sorted_enabled(int n, int flags)
     return on && n >= kSortedMinBodies;
 }
 
-// Warps of the main kernel (one per kIpt i-chunks).
-static int sorted_warps(int n) { return ((n + kChunk - 1) / kChunk + kIpt - 1) / kIpt; }
+// The near kernel's j-split: about 10,000 warps (16 per SM and four waves),
+// at most 32 segments (4,000 warps: 1.93 ms a step instead of 1.48 at N = 65,536,
+// the longest rows alone at the end; 20,000: the same).  A function of n alone.
+static int near_segments(int tiles) { return std::min(32, std::max(2, 10000 / tiles)); }
 
-static nb_status run_sorted(const DirectPlan &p, const float4 *hi, const float4 *lo, int n,
-                            double eps2, SortedBuffers &b, cudaStream_t st, float **psum_out)
-{
-    NB_TRY(b.partials.reserve(sizeof(float) * 6 * (size_t)n * p.segments));
-    float *psum = b.partials.as<float>();
-    float *pcomp = psum + 3 * (size_t)n * p.segments;
-    if (!launch_sorted(p, st, hi, lo, b.boxes.as<float4>(), n, eps2, psum, pcomp, b.centre))
-        return fail(NB_ERR_UNSUPPORTED, "direct_mixed_sorted: unsupported tile shape");
-    NB_LAUNCH_CHECK();
-    *psum_out = psum;
-    return NB_OK;
-}
-
-// The left-out pairs, into b.exact (3 n doubles), on b.side: the kernel
-// waits for the staging on st (fork) and st waits for it before the combine
-// (join).  The side stream has the highest priority, so the exact CTAs start
-// at once and their longest chains run while the main kernel fills the GPU.
-static nb_status launch_exact_pairs(const float4 *hi, const float4 *lo, int n, double eps2,
-                                    SortedBuffers &b, cudaStream_t st)
+// The near kernel's ordered pairs (into b.partials) and the left-out ones (into
+// b.exact, 3 n doubles), on b.side: it waits for the staging on st (fork) and st
+// waits for it before the combine (join).  The side stream has the highest
+// priority, so the exact CTAs start at once and their longest chains run while
+// the far kernel fills the GPU.
+static nb_status launch_side(const float4 *hi, const float4 *lo, int n, int segments, double eps2,
+                             SortedBuffers &b, cudaStream_t st)
 {
     NB_TRY(b.exact.reserve(sizeof(double) * 3 * (size_t)n));
+    NB_TRY(b.partials.reserve(sizeof(float) * 6 * (size_t)n * segments));
     if (!b.side) {
         int least = 0, greatest = 0;
         NB_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -820,61 +1026,22 @@ static nb_status launch_exact_pairs(const float4 *hi, const float4 *lo, int n, d
     }
     NB_CUDA_TRY(cudaEventRecord(b.fork, st));
     NB_CUDA_TRY(cudaStreamWaitEvent(b.side, b.fork, 0));
-    const int nchunks = (n + kChunk - 1) / kChunk;
-    exact_pairs_kernel<kIpt><<<sorted_warps(n), kExactWarps * 32, 0, b.side>>>(
-        hi, lo, b.boxes.as<float4>(), n, nchunks, eps2 > 0.0 ? (float)eps2 : 0.0f, kFarFactor2,
-        eps2 > 0.0 ? eps2 : 0.0, b.centre, exact_cap_per_n(n), b.exact.as<double>());
+    const int nchunks = (n + kChunk - 1) / kChunk, tiles = (nchunks + 1) / 2;
+    const float4 *box = b.boxes.as<float4>(), *tile = b.tiles.as<float4>();
+    exact_pairs_kernel<<<tiles, kExactWarps * 32, 0, b.side>>>(
+        hi, lo, box, tile, n, nchunks, eps2 > 0.0 ? (float)eps2 : 0.0f, kFarFactor2,
+        eps2 > 0.0 ? eps2 : 0.0, b.exact.as<double>());
+    NB_LAUNCH_CHECK();
+    float *psum = b.partials.as<float>(), *pcomp = psum + 3 * (size_t)n * segments;
+    const dim3 grid(tiles, segments);
+    if (eps2 > 0.0)
+        direct_near_kernel<false><<<grid, 32, 0, b.side>>>(hi, lo, box, tile, n, nchunks,
+                                                           (float)eps2, psum, pcomp, kFarFactor2);
+    else
+        direct_near_kernel<true><<<grid, 32, 0, b.side>>>(hi, lo, box, tile, n, nchunks, 0.0f,
+                                                          psum, pcomp, kFarFactor2);
     NB_LAUNCH_CHECK();
     NB_CUDA_TRY(cudaEventRecord(b.join, b.side));
-    return NB_OK;
-}
-
-// Times every CTA shape, kernel and combine together (the combine writes the
-// real outputs, which the evaluation then overwrites), and records the
-// fastest plan for this n.
-static nb_status autotune_sorted(const float4 *hi, const float4 *lo, int n, double eps2,
-                                 double G, const uint32_t *order, double *ax, double *ay,
-                                 double *az, SortedBuffers &b, cudaStream_t st, DirectPlan *best)
-{
-    cudaEvent_t e0, e1;
-    NB_CUDA_TRY(cudaEventCreate(&e0));
-    NB_CUDA_TRY(cudaEventCreate(&e1));
-    float best_ms = 1e30f;
-    // Above 2^18 bodies every shape is timed on all i-bodies against the first
-    // 512 j-chunks only (one segment): an evaluation there takes 0.1 s and more.
-    const bool probe = n > (1 << 18);
-    for (int k = 0; k < kNumSortedShapes; ++k) {
-        const DirectPlan p = sorted_plan_for_shape(n, kSortedShapes[k].warps, kSortedShapes[k].ipt);
-        {
-            DirectPlan t = p;
-            if (probe) {
-                t.segments = 1;
-                t.seg_tiles = std::min(p.seg_tiles * p.segments, 512);
-            }
-            float *psum = nullptr;
-            NB_TRY(run_sorted(t, hi, lo, n, eps2, b, st, &psum));
-            cudaEventRecord(e0, st);
-            for (int r = 0; r < 2; ++r) {
-                NB_TRY(run_sorted(t, hi, lo, n, eps2, b, st, &psum));
-                combine_sorted_kernel<<<(n + 255) / 256, 256, 0, st>>>(
-                    psum, psum + 3 * (size_t)n * t.segments, n, t.segments, G, order, nullptr,
-                    ax, ay, az);
-                NB_LAUNCH_CHECK();
-            }
-            cudaEventRecord(e1, st);
-            NB_CUDA_TRY(cudaEventSynchronize(e1));
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            if (ms < best_ms) {
-                best_ms = ms;
-                *best = p;
-            }
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    std::lock_guard<std::mutex> lock(g_sorted_mutex);
-    g_sorted_tuned[n] = *best;
     return NB_OK;
 }
 
@@ -902,33 +1069,40 @@ nb_status direct_mixed_sorted(const double *x, const double *y, const double *z,
     NB_TRY(b.lo.reserve(sizeof(float4) * (size_t)n));
     NB_TRY(b.boxes.reserve(sizeof(float4) * 2 * (size_t)nchunks));
     float4 *hi = b.hi.as<float4>(), *lo = b.lo.as<float4>();
-    split_sorted_kernel<<<(n + 255) / 256, 256, 0, st>>>(order, x, y, z, m, n, centre, hi, lo,
-                                                         b.boxes.as<float4>());
+    const int tiles = (nchunks + 1) / 2;
+    NB_TRY(b.tiles.reserve(sizeof(float4) * 2 * (size_t)tiles));
+    split_sorted_kernel<<<(tiles + 3) / 4, 128, 0, st>>>(order, x, y, z, m, n, centre,
+                                                         exact_cap_per_n(n), hi, lo,
+                                                         b.boxes.as<float4>(),
+                                                         b.tiles.as<float4>());
     NB_LAUNCH_CHECK();
-    DirectPlan p;
-    bool tuned;
-    {
-        std::lock_guard<std::mutex> lock(g_sorted_mutex);
-        auto it = g_sorted_tuned.find(n);
-        tuned = it != g_sorted_tuned.end();
-        if (tuned) p = it->second;
-    }
-    if (!tuned) {
-        const char *e = std::getenv("NB_AUTOTUNE");
-        if (!(e && std::strcmp(e, "0") == 0))
-            NB_TRY(autotune_sorted(hi, lo, n, eps2, G, order, ax, ay, az, b, st, &p));
-        else p = sorted_plan_for_shape(n, 1, 2);
-    }
-    NB_TRY(launch_exact_pairs(hi, lo, n, eps2, b, st));
+    const int segments = near_segments(tiles);
+    const int blocks = (tiles + kFarTiles - 1) / kFarTiles, diagonals = blocks / 2 + 1;
+    // the diagonals in passes whose planes stay within kFarPlaneBytes
+    const size_t per_diagonal = sizeof(float) * 6 * (size_t)n;
+    const int pass = (int)std::min<size_t>(diagonals,
+                                           std::max<size_t>(1, kFarPlaneBytes / per_diagonal));
+    NB_TRY(b.far.reserve(per_diagonal * pass));
+    NB_TRY(b.acc.reserve(sizeof(float) * 6 * (size_t)n));
     if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
-    float *psum = nullptr;
-    NB_TRY(run_sorted(p, hi, lo, n, eps2, b, st, &psum));
-    if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
-    float *pcomp = psum + 3 * (size_t)n * p.segments;
-    NB_CUDA_TRY(cudaStreamWaitEvent(st, b.join, 0));
-    combine_sorted_kernel<<<(n + 255) / 256, 256, 0, st>>>(psum, pcomp, n, p.segments, G, order,
-                                                          b.exact.as<double>(), ax, ay, az);
-    NB_LAUNCH_CHECK();
+    NB_TRY(launch_side(hi, lo, n, segments, eps2, b, st));
+    float *psum = b.partials.as<float>(), *pcomp = psum + 3 * (size_t)n * segments;
+    for (int p0 = 0; p0 < diagonals; p0 += pass) {
+        const int np = std::min(pass, diagonals - p0);
+        direct_far_kernel<<<(unsigned)blocks * (unsigned)np, 32, 0, st>>>(
+            hi, lo, b.tiles.as<float4>(), n, tiles, eps2 > 0.0 ? (float)eps2 : 0.0f, blocks, p0, np,
+            b.far.as<float>());
+        NB_LAUNCH_CHECK();
+        const bool last = p0 + np == diagonals;
+        if (last) {
+            NB_CUDA_TRY(cudaStreamWaitEvent(st, b.join, 0));
+            if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
+        }
+        combine_sorted_kernel<<<(n + 31) / 32, 32 * kCombineGroups, 0, st>>>(
+            b.far.as<float>(), blocks, p0, np, p0 == 0, last, b.acc.as<float>(), psum, pcomp, n,
+            segments, G, order, b.exact.as<double>(), ax, ay, az);
+        NB_LAUNCH_CHECK();
+    }
     return NB_OK;
 }
 

@@ -120,9 +120,10 @@ constexpr float kExactSpacing2 = 0.5625f;   // kExactSpacing = 3/4
 // Hilbert-sorted near/far variant of the mixed path (nb_direct_sorted.cu).
 struct BHTree;
 struct SortedBuffers {
-    DevBuf hi, lo, partials, boxes;
+    DevBuf hi, lo, partials, boxes, tiles;
     DevBuf exact;  // the left-out pairs' sums, 3 n doubles (sorted order)
-    cudaStream_t side = nullptr;              // the exact-pair kernel's stream
+    DevBuf far, acc;  // the far kernel's partial planes, and their sums between passes
+    cudaStream_t side = nullptr;              // the near and exact-pair kernels' stream
     cudaEvent_t fork = nullptr, join = nullptr;
     BHTree *sorter = nullptr;
     // The sort order is a performance device only (near/far decisions use

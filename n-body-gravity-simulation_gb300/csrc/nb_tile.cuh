@@ -1,21 +1,33 @@
-// nb_tile.cuh -- the mixed-precision pair term over unordered pairs: 64 x 64
-// body tiles whose j side rotates through the lanes of a warp.
+// nb_tile.cuh -- the mixed-precision pair term over unordered pairs: tiles of
+// 64 j-bodies that rotate through the lanes of a warp.
 //
 // A sum over ordered pairs evaluates a pair's displacement, r^2 and r^-3 twice,
-// once for each body.  Here a warp holds a tile of 64 i-bodies (two per lane)
-// and meets a tile of 64 j-bodies, two at a time as an f32x2 pair: at step s
-// lane l meets j-bodies (l + s) mod 32 and 32 + (l + s) mod 32, adds the pair
-// terms to its own bodies' sums in registers and to the j-bodies' running sums,
-// which move one lane down per step by shuffles.  Per unordered pair the far
-// term costs 17 FP32 lane operations and the near one 26, where ordered pairs
-// cost 2 x 12 and 2 x 21; two MUFU operations become one.  The FP32 pipe bounds the
-// loop (34 packed operations, 68 cycles, per step against 50 issue slots).
+// once for each body.  Here a warp holds IPT i-bodies per lane (tiles of 64) and
+// meets a tile of 64 j-bodies, two at a time as an f32x2 pair: at step s lane l
+// meets j-bodies (l + s) mod 32 and 32 + (l + s) mod 32, adds the pair terms to its
+// own bodies' sums in registers and to the j-bodies' running sums, which move one
+// lane down per step by shuffles.  Per unordered pair the far term costs 17 FP32
+// lane operations and the near one 26, where ordered pairs cost 2 x 12 and
+// 2 x 21; two MUFU operations become one.
+//
+// What bounds the loop is dispatch, not the FP32 pipe alone.  Measured on GB300
+// in cycles per warp instruction and SM quarter: a packed operation 2, but 3 when
+// its three operands are all different registers; a MUFU, a shuffle and a
+// shared-memory load 2 each; an integer operation about 0.6.  Four far pairs per
+// lane took 110 cycles with two i-bodies per lane, 96 with four (half the
+// shuffles and loads per pair, and tiles staged twice over so that no index
+// wraps), 84 when the masses leave the loop (below).
+//
+// Equal masses.  Where all bodies of the i-tiles have one mass and all of the
+// j-tile one (as in most N-body set-ups), the loop sums r^-3 d alone and each
+// fold multiplies by the mass: 14 operations per far pair instead of 17, 23 per
+// near one instead of 26.
 //
 // Rounding is as in the sums over ordered pairs: 16 terms per f32x2 lane in
 // plain FP32, then a Kahan-compensated add -- after every 16 steps on the i side
-// (one term per lane and step) and every 8 on the j side (two).  The Kahan pairs
-// live in shared memory (the registers they would take cost more), the j side's
-// indexed by the j-body the lane holds then.
+// (one term per lane and step) and every 32 / (2 IPT) on the j side (IPT terms).
+// The Kahan pairs live in shared memory (the registers they would take cost
+// more), the j side's indexed by the j-body the lane holds then.
 #pragma once
 
 #include "nb_pair.cuh"
@@ -24,12 +36,15 @@ namespace nb {
 
 constexpr int kTile = 64;  // bodies per tile
 
-// A staged j-tile: index l holds bodies l and 32 + l side by side.
+// A staged j-tile: index l (and 32 + l, a copy) holds bodies l and 32 + l side
+// by side.
 struct TileJ {
-    float4 a[32];  // (x_l, x_32+l, y_l, y_32+l)
-    float4 b[32];  // (z_l, z_32+l, m_l, m_32+l)
-    float4 c[32];  // low parts of x and y
-    float2 d[32];  // low parts of z
+    float4 a[64];  // (x_l, x_32+l, y_l, y_32+l)
+    float4 b[64];  // (z_l, z_32+l, m_l, m_32+l)
+};
+struct TileJLow {
+    float4 c[64];  // low parts of x and y
+    float2 d[64];  // low parts of z
 };
 
 // Sums of a tile, one f32x2 per component and index (bodies l and 32 + l): Kahan
@@ -38,12 +53,15 @@ struct TileSums {
     float2 s[3][32], c[3][32];
 };
 
-// The warp's i-tile: body 32 k + lane in k = 0, 1, coordinates negated and
-// duplicated.
+// The warp's i-bodies, coordinates negated and duplicated: body 32 k + lane.
+template <int IPT>
 struct TileI {
-    float2 nx[2], ny[2], nz[2];     // high parts
-    float2 ex[2], ey[2], ez[2];     // low parts
-    float2 nm[2];                   // negated mass
+    float2 nx[IPT], ny[IPT], nz[IPT];
+    float2 nm[IPT];  // negated mass
+};
+template <int IPT>
+struct TileILow {
+    float2 ex[IPT], ey[IPT], ez[IPT];
 };
 
 __device__ __forceinline__ void tile_sums_zero(TileSums &t, int lane)
@@ -52,28 +70,40 @@ __device__ __forceinline__ void tile_sums_zero(TileSums &t, int lane)
     for (int c = 0; c < 3; ++c) t.s[c][lane] = t.c[c][lane] = dup2(0.f);
 }
 
-__device__ __forceinline__ void tile_i_set(TileI &t, int k, float x, float y, float z, float xl,
-                                           float yl, float zl, float m)
+template <int IPT>
+__device__ __forceinline__ void tile_i_set(TileI<IPT> &t, int k, const float (&S)[3], float m)
 {
-    t.nx[k] = dup2(-x); t.ny[k] = dup2(-y); t.nz[k] = dup2(-z);
-    t.ex[k] = dup2(-xl); t.ey[k] = dup2(-yl); t.ez[k] = dup2(-zl);
+    t.nx[k] = dup2(-S[0]); t.ny[k] = dup2(-S[1]); t.nz[k] = dup2(-S[2]);
     t.nm[k] = dup2(-m);
+}
+template <int IPT>
+__device__ __forceinline__ void tile_i_set_low(TileILow<IPT> &t, int k, const float (&E)[3])
+{
+    t.ex[k] = dup2(-E[0]); t.ey[k] = dup2(-E[1]); t.ez[k] = dup2(-E[2]);
 }
 
 // Lane `lane` stages body 32 k + lane of a j-tile (between two __syncwarp).
-__device__ __forceinline__ void tile_j_put(TileJ &t, int lane, int k, float x, float y, float z,
-                                           float xl, float yl, float zl, float m)
+__device__ __forceinline__ void tile_j_put(TileJ &t, int lane, int k, const float (&S)[3], float m)
 {
-    float *a = reinterpret_cast<float *>(&t.a[lane]) + k;
-    float *b = reinterpret_cast<float *>(&t.b[lane]) + k;
-    float *c = reinterpret_cast<float *>(&t.c[lane]) + k;
-    a[0] = x;
-    a[2] = y;
-    b[0] = z;
-    b[2] = m;
-    c[0] = xl;
-    c[2] = yl;
-    reinterpret_cast<float *>(&t.d[lane])[k] = zl;
+#pragma unroll
+    for (int r = 0; r < 64; r += 32) {
+        float *a = reinterpret_cast<float *>(&t.a[lane + r]) + k;
+        float *b = reinterpret_cast<float *>(&t.b[lane + r]) + k;
+        a[0] = S[0];
+        a[2] = S[1];
+        b[0] = S[2];
+        b[2] = m;
+    }
+}
+__device__ __forceinline__ void tile_j_put_low(TileJLow &t, int lane, int k, const float (&E)[3])
+{
+#pragma unroll
+    for (int r = 0; r < 64; r += 32) {
+        float *c = reinterpret_cast<float *>(&t.c[lane + r]) + k;
+        c[0] = E[0];
+        c[2] = E[1];
+        reinterpret_cast<float *>(&t.d[lane + r])[k] = E[2];
+    }
 }
 
 // (sum, negated compensation) += t, four packed additions.
@@ -86,31 +116,37 @@ __device__ __forceinline__ void kahan_add2(float2 &s, float2 &nc, float2 t)
     s = u;
 }
 
-// One step: the lane's two i-bodies against the staged j-pair idx.  NEAR takes the
-// double-single displacement and the folded Newton step (pair_term2), else the
-// plain FP32 term (pair_term2_far<false>).  BOTH = false adds to the i side
-// only.  The scale m r^-3 is built as (m y) y^2 for each side, not from a shared
-// y^3, so that lengths of 1e13 and more (y^3 below FP32's range) still work.
-template <bool NEAR, bool ZERO_SOFT, bool BOTH>
-__device__ __forceinline__ void tile_step(const TileJ &t, int idx, const TileI &ti, float2 e2,
-                                          float2 (&fi)[2][3], float2 (&fj)[3])
+// How a pair is evaluated: the plain FP32 term (pair_term2_far<false>), that with
+// the folded Newton step (pair_term2_far<true>), or the double-single
+// displacement and the Newton step (pair_term2).
+enum TileTerm { kVeryFarTerm, kFarTerm, kNearTerm };
+
+// One step: the lane's i-bodies against the staged j-pair idx.  BOTH = false adds to the i side
+// only.  EQUAL: fi and fj receive r^-3 d without the masses, and y^3 must be in
+// FP32's range (equal_range); otherwise the scale is built as (m y) y^2 for each
+// side, so that lengths of 1e13 and more (y^3 below FP32's range) still work.
+template <int TERM, bool EQUAL, bool ZERO_SOFT, bool BOTH, int IPT>
+__device__ __forceinline__ void tile_step(const TileJ &t, const TileJLow *low, int idx,
+                                          const TileI<IPT> &ti, const TileILow<IPT> *lo, float2 e2,
+                                          float2 (&fi)[IPT][3], float2 (&fj)[3])
 {
+    constexpr bool NEAR = TERM == kNearTerm;
     const float4 A = t.a[idx], B = t.b[idx];
     float4 C = make_float4(0.f, 0.f, 0.f, 0.f);
     float2 D = make_float2(0.f, 0.f);
     if (NEAR) {
-        C = t.c[idx];
-        D = t.d[idx];
+        C = low->c[idx];
+        D = low->d[idx];
     }
     const float2 jx = make_float2(A.x, A.y), jy = make_float2(A.z, A.w),
                  jz = make_float2(B.x, B.y), jm = make_float2(B.z, B.w);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < IPT; ++k) {
         float2 dx = add2(jx, ti.nx[k]), dy = add2(jy, ti.ny[k]), dz = add2(jz, ti.nz[k]);
         if (NEAR) {
-            dx = add2(dx, add2(make_float2(C.x, C.y), ti.ex[k]));
-            dy = add2(dy, add2(make_float2(C.z, C.w), ti.ey[k]));
-            dz = add2(dz, add2(D, ti.ez[k]));
+            dx = add2(dx, add2(make_float2(C.x, C.y), lo->ex[k]));
+            dy = add2(dy, add2(make_float2(C.z, C.w), lo->ey[k]));
+            dz = add2(dz, add2(D, lo->ez[k]));
         }
         const float2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, e2)));
         float2 inv = make_float2(rsqrt_mufu(r2.x), rsqrt_mufu(r2.y));
@@ -119,13 +155,13 @@ __device__ __forceinline__ void tile_step(const TileJ &t, int idx, const TileI &
             inv.y = r2.y > 0.f ? inv.y : 0.f;
         }
         float2 w = mul2(inv, inv);
-        if (NEAR) w = mul2(w, fma2(dup2(-1.5f), mul2(r2, w), dup2(2.5f)));
-        const float2 si = mul2(mul2(jm, inv), w);
+        if (TERM != kVeryFarTerm) w = mul2(w, fma2(dup2(-1.5f), mul2(r2, w), dup2(2.5f)));
+        const float2 si = EQUAL ? mul2(inv, w) : mul2(mul2(jm, inv), w);
         fi[k][0] = fma2(dx, si, fi[k][0]);
         fi[k][1] = fma2(dy, si, fi[k][1]);
         fi[k][2] = fma2(dz, si, fi[k][2]);
         if (BOTH) {
-            const float2 sj = mul2(mul2(ti.nm[k], inv), w);
+            const float2 sj = EQUAL ? si : mul2(mul2(ti.nm[k], inv), w);
             fj[0] = fma2(dx, sj, fj[0]);
             fj[1] = fma2(dy, sj, fj[1]);
             fj[2] = fma2(dz, sj, fj[2]);
@@ -133,52 +169,61 @@ __device__ __forceinline__ void tile_step(const TileJ &t, int idx, const TileI &
     }
 }
 
-__device__ __forceinline__ void tile_fold_i(TileSums &is, int lane, float2 (&fi)[2][3])
+template <bool EQUAL, int IPT>
+__device__ __forceinline__ void tile_fold_i(TileSums *is, int lane, float2 (&fi)[IPT][3], float mj)
 {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        kahan_add2(is.s[c][lane], is.c[c][lane],
-                   make_float2(fi[0][c].x + fi[0][c].y, fi[1][c].x + fi[1][c].y));
-        fi[0][c] = fi[1][c] = dup2(0.f);
-    }
+    for (int h = 0; h < IPT / 2; ++h)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 t = make_float2(fi[2 * h][c].x + fi[2 * h][c].y,
+                                         fi[2 * h + 1][c].x + fi[2 * h + 1][c].y);
+            kahan_add2(is[h].s[c][lane], is[h].c[c][lane], EQUAL ? mul2(t, dup2(mj)) : t);
+            fi[2 * h][c] = fi[2 * h + 1][c] = dup2(0.f);
+        }
 }
 
-// Steps [8 g0, 8 g1) of the i-tile against a staged j-tile (g1 = 4: the whole
-// pair of tiles).  is, js: the sums of either side, this warp's alone.
-template <bool NEAR, bool ZERO_SOFT>
-__device__ __forceinline__ void tile_pair(const TileJ &t, int lane, int g0, int g1, const TileI &ti,
-                                          float2 e2, TileSums &is, TileSums &js)
+// The i-bodies against a staged j-tile, both sides.  is[h]: the sums of the
+// lane's bodies 2 h and 2 h + 1; js: those of the j-tile; this warp's alone
+// meanwhile.  EQUAL: mi, mj = the masses of the i- and the j-bodies.
+template <int TERM, bool EQUAL, bool ZERO_SOFT, int IPT>
+__device__ __forceinline__ void tile_pair(const TileJ &t, const TileJLow *low, int lane,
+                                          const TileI<IPT> &ti, const TileILow<IPT> *lo, float2 e2,
+                                          float mi, float mj, TileSums *is, TileSums &js)
 {
+    constexpr int kRun = 16 / IPT;  // steps per j-side fold
     const int next = (lane + 1) & 31;
-    float2 fi[2][3];
+    float2 fi[IPT][3];
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < IPT; ++k)
 #pragma unroll
         for (int c = 0; c < 3; ++c) fi[k][c] = dup2(0.f);
 #pragma unroll 1
-    for (int g = g0; g < g1; ++g) {
+    for (int g = 0; g < 32; g += kRun) {
         float2 fj[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            tile_step<NEAR, ZERO_SOFT, true>(t, (lane + 8 * g + u) & 31, ti, e2, fi, fj);
-            if (u < 7)
+        for (int u = 0; u < kRun; ++u) {
+            tile_step<TERM, EQUAL, ZERO_SOFT, true, IPT>(t, low, lane + g + u, ti, lo, e2, fi, fj);
+            if (u < kRun - 1)
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
                     fj[c] = make_float2(__shfl_sync(0xffffffffu, fj[c].x, next),
                                         __shfl_sync(0xffffffffu, fj[c].y, next));
         }
-        const int idx = (lane + 8 * g + 7) & 31;
+        const int idx = (lane + g + kRun - 1) & 31;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) kahan_add2(js.s[c][idx], js.c[c][idx], fj[c]);
-        if ((g & 1) || g + 1 == g1) tile_fold_i(is, lane, fi);
-        __syncwarp();  // the next group's fold takes other lanes' entries
+        for (int c = 0; c < 3; ++c)
+            kahan_add2(js.s[c][idx], js.c[c][idx], EQUAL ? mul2(fj[c], dup2(-mi)) : fj[c]);
+        if (((g + kRun) & 15) == 0) tile_fold_i<EQUAL, IPT>(is, lane, fi, mj);
+        __syncwarp();  // the next run's fold takes other lanes' entries
     }
 }
 
 // A tile with itself (staged in t): every ordered pair, the i side only.
 template <bool ZERO_SOFT>
-__device__ __forceinline__ void tile_self(const TileJ &t, int lane, int g0, int g1, const TileI &ti,
-                                          float2 e2, TileSums &is)
+__device__ __forceinline__ void tile_self(const TileJ &t, const TileJLow *low, int lane,
+                                          const TileI<2> &ti, const TileILow<2> *lo, float2 e2,
+                                          TileSums &is)
 {
     float2 fi[2][3], none[3];
 #pragma unroll
@@ -186,12 +231,19 @@ __device__ __forceinline__ void tile_self(const TileJ &t, int lane, int g0, int 
 #pragma unroll
         for (int c = 0; c < 3; ++c) fi[k][c] = dup2(0.f);
 #pragma unroll 1
-    for (int g = g0; g < g1; ++g) {
+    for (int g = 0; g < 32; g += 8) {
 #pragma unroll 4
         for (int u = 0; u < 8; ++u)
-            tile_step<true, ZERO_SOFT, false>(t, (lane + 8 * g + u) & 31, ti, e2, fi, none);
-        if ((g & 1) || g + 1 == g1) tile_fold_i(is, lane, fi);
+            tile_step<kNearTerm, false, ZERO_SOFT, false, 2>(t, low, lane + g + u, ti, lo, e2, fi, none);
+        if (g & 8) tile_fold_i<false, 2>(&is, lane, fi, 0.f);
     }
+}
+
+// Whether r^-3 of pairs at least sqrt(gap2 + eps2) and at most sqrt(span2 + eps2)
+// apart is well inside FP32's normal range (r in [1e-11, 1e11]).
+__device__ __forceinline__ bool equal_range(float gap2, float span2, float eps2)
+{
+    return gap2 + eps2 >= 1e-22f && span2 + eps2 <= 1e22f;
 }
 
 } // namespace nb
