@@ -27,19 +27,28 @@ namespace nb {
 namespace {
 
 constexpr int kBatchTiles = kBatchBlockBodies / kTile;  // tiles per block
-// One-warp CTAs per SM.  16 leave 128 registers, with which a step's loads run
-// ahead of its arithmetic: 7.69 ms for two RK4 steps of the 1024-system ensemble,
-// 18 / 20 / 21 CTAs 7.71 / 7.80 / 7.92.  Four-warp CTAs that share the second
-// block's sums behind barriers: 8.06.
+// One-warp CTAs per SM: 10 / 12 (166 registers) / 14 / 16 (128) measured 7.27 /
+// 7.27 / 7.16 / 7.17 ms for two RK4 steps of the 1024-system ensemble.
 constexpr int kBatchCtas = 16;
 
 // Bounding box of a 64-body tile of sorted bodies (the union of its two chunk
 // boxes, box[4 t .. 4 t + 3] = min, max, min, max; an empty chunk has an inverted
-// box) and its squared diameter.
+// box), or of two tiles; diam2: its squared diameter.
 struct TileBox {
     float4 mn, mx;
-    float diam2;
+    __device__ float diam2() const
+    {
+        const float dx = mx.x - mn.x, dy = mx.y - mn.y, dz = mx.z - mn.z;
+        return dx * dx + dy * dy + dz * dz;
+    }
 };
+__device__ __forceinline__ TileBox box_union(const TileBox &a, const TileBox &b)
+{
+    return TileBox{make_float4(fminf(a.mn.x, b.mn.x), fminf(a.mn.y, b.mn.y),
+                               fminf(a.mn.z, b.mn.z), 0.f),
+                   make_float4(fmaxf(a.mx.x, b.mx.x), fmaxf(a.mx.y, b.mx.y),
+                               fmaxf(a.mx.z, b.mx.z), 0.f)};
+}
 __device__ __forceinline__ TileBox tile_box(const float4 *__restrict__ box, int t)
 {
     const float4 a = box[4 * (size_t)t], b = box[4 * (size_t)t + 1], c = box[4 * (size_t)t + 2],
@@ -47,8 +56,6 @@ __device__ __forceinline__ TileBox tile_box(const float4 *__restrict__ box, int 
     TileBox r;
     r.mn = make_float4(fminf(a.x, c.x), fminf(a.y, c.y), fminf(a.z, c.z), 0.f);
     r.mx = make_float4(fmaxf(b.x, d.x), fmaxf(b.y, d.y), fmaxf(b.z, d.z), 0.f);
-    const float dx = r.mx.x - r.mn.x, dy = r.mx.y - r.mn.y, dz = r.mx.z - r.mn.z;
-    r.diam2 = dx * dx + dy * dy + dz * dz;
     return r;
 }
 
@@ -154,13 +161,87 @@ __device__ __forceinline__ void batch_row(const float4 *__restrict__ hi,
     az[o] = G * ((double)sz - (double)qz);
 }
 
+// A body relative to c as a normalised double-single (SORTED), or as it is.
+template <bool SORTED>
+__device__ __forceinline__ void batch_relative(const float4 h, const float4 l, const float (&c)[3],
+                                               float (&S)[3], float (&E)[3], float &m)
+{
+    if (SORTED) {
+        rel_ds(h.x, l.x, c[0], S[0], E[0]);
+        rel_ds(h.y, l.y, c[1], S[1], E[1]);
+        rel_ds(h.z, l.z, c[2], S[2], E[2]);
+    } else {
+        S[0] = h.x; S[1] = h.y; S[2] = h.z;
+        E[0] = l.x; E[1] = l.y; E[2] = l.z;
+    }
+    m = h.w;
+}
+// Coordinates whose differences stay within equal_range's farthest pair.
+__device__ __forceinline__ bool batch_in_span(const float (&S)[3])
+{
+    return fmaxf(fabsf(S[0]), fmaxf(fabsf(S[1]), fabsf(S[2]))) <= 2.5e10f;
+}
+
+// Loads IPT chunks of i-bodies from body i0 of the system, relative to c.  Returns
+// whether they all have one mass, mass, and coordinates within equal_range's
+// span; lanes past the system hold massless bodies far from every j-body.
+template <bool SORTED, int IPT>
+__device__ __forceinline__ bool batch_load_i(const float4 *__restrict__ hi,
+                                             const float4 *__restrict__ lo, const SysDesc &sd,
+                                             int i0, const float (&c)[3], TileI<IPT> &ti,
+                                             TileILow<IPT> &tl, float &mass)
+{
+    bool equal = true;
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const int i = i0 + 32 * k + (int)threadIdx.x;
+        float S[3] = {-1.0e18f, -1.0e18f, -1.0e18f}, E[3] = {0.f, 0.f, 0.f}, m = 0.f;
+        if (i < sd.n) batch_relative<SORTED>(hi[sd.first + i], lo[sd.first + i], c, S, E, m);
+        if (k == 0) mass = __shfl_sync(0xffffffffu, m, 0);
+        equal = equal && (i >= sd.n || (m == mass && batch_in_span(S)));
+        tile_i_set(ti, k, S, m);
+        tile_i_set_low(tl, k, E);
+    }
+    return __all_sync(0xffffffffu, equal);
+}
+
+// Stages the j-tile from body j0 of the system relative to c; returns as
+// batch_load_i.
+template <bool SORTED>
+__device__ __forceinline__ bool batch_stage_j(const float4 *__restrict__ hi,
+                                              const float4 *__restrict__ lo, const SysDesc &sd,
+                                              int j0, const float (&c)[3], TileJ &stage,
+                                              TileJLow &low, float &mass)
+{
+    const int lane = threadIdx.x;
+    bool equal = true;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int j = j0 + 32 * k + lane;
+        // lanes past the system stage a massless body far away: exactly 0
+        float S[3] = {1.0e18f, 1.0e18f, 1.0e18f}, E[3] = {0.f, 0.f, 0.f}, m = 0.f;
+        if (j < sd.n) batch_relative<SORTED>(hi[sd.first + j], lo[sd.first + j], c, S, E, m);
+        if (k == 0) mass = __shfl_sync(0xffffffffu, m, 0);
+        equal = equal && (j >= sd.n || (m == mass && batch_in_span(S)));
+        tile_j_put(stage, lane, k, S, m);
+        tile_j_put_low(low, lane, k, E);
+    }
+    equal = __all_sync(0xffffffffu, equal);
+    __syncwarp();
+    return equal;
+}
+
 // SORTED: the bodies are in Hilbert order with one box per tile; coordinates are
-// staged relative to the i-tile's box centre, and a tile pair at least a
-// quarter of the larger box's diameter apart takes the plain FP32 term
-// (kVeryFar2: the bounds of nb_direct_sorted.cu hold for both sides), others the
-// double-single one.  Otherwise every pair takes the double-single term.
-// Bound by the FP32 pipe, 75 % busy: 0.82 ms for the 8.4e8 unordered pairs of the
-// 1024-system ensemble, where one warp per 32 or 64 rows took 1.11 ms.
+// staged relative to the centre of the i-tiles' box, and a j-tile an eighth of
+// that box's diameter or more away takes the plain FP32 displacement (the bound of
+// nb_direct_sorted.cu, for both sides), others the double-single one.
+// Otherwise every pair takes the double-single term.  Two i-tiles at a time (four
+// bodies per lane), but a tile against itself and its neighbour in the pair one
+// by one.  Bound by dispatch (nb_tile.cuh): two RK4 steps of the 1024-system
+// ensemble (8.4e8 unordered pairs an evaluation) take 7.17 ms, with one i-tile at
+// a time and the masses in the loop 7.78, with a row of 32 or 64 bodies per warp
+// over ordered pairs 9.92.
 template <bool SORTED, bool ZERO_SOFT>
 __global__ void __launch_bounds__(32, kBatchCtas)
 batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
@@ -177,7 +258,7 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
         PairTile chunk;
     } stages;
     __shared__ TileSums sums[kBatchTiles];  // of the second block's tiles
-    __shared__ TileSums isum;               // of the i-tile
+    __shared__ TileSums isum[2];            // of the two i-tiles
     const int lane = threadIdx.x;
     const PairItem it = items[blockIdx.x];
     const SysDesc sd = sys[it.sys];
@@ -197,109 +278,105 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     const int ti0 = it.a * kBatchTiles, tj0 = blk_b * kBatchTiles;
     const int ta = min(kBatchTiles, tiles - ti0), tb = min(kBatchTiles, tiles - tj0);
     const float2 e2 = dup2(eps2);
+    const bool soft = eps2 >= 1e-22f;  // equal_range's nearest pair
     const size_t plane = (size_t)sd.n;
     float2 *pa = part + sd.part0 + 3 * plane * it.p;
     float2 *pb = part + sd.part0 + 3 * plane * (sd.blocks / 2 + it.p);
     for (int v = 0; v < kBatchTiles; ++v) tile_sums_zero(sums[v], lane);
 
-    for (int u = 0; u < ta; ++u) {
-        TileI<2> ti;
-        TileILow<2> tl;
+    for (int u0 = 0; u0 < ta; u0 += 2) {
+        tile_sums_zero(isum[0], lane);
+        tile_sums_zero(isum[1], lane);
+        const bool two = u0 + 1 < ta;
         TileBox bi{};
-        float cx = 0.f, cy = 0.f, cz = 0.f;
+        float c[3] = {0.f, 0.f, 0.f};
         if (SORTED) {
-            bi = tile_box(boxes, sd.tile0 + ti0 + u);
-            cx = 0.5f * (bi.mn.x + bi.mx.x);
-            cy = 0.5f * (bi.mn.y + bi.mx.y);
-            cz = 0.5f * (bi.mn.z + bi.mx.z);
+            bi = tile_box(boxes, sd.tile0 + ti0 + u0);
+            if (two) bi = box_union(bi, tile_box(boxes, sd.tile0 + ti0 + u0 + 1));
+            c[0] = 0.5f * (bi.mn.x + bi.mx.x);
+            c[1] = 0.5f * (bi.mn.y + bi.mx.y);
+            c[2] = 0.5f * (bi.mn.z + bi.mx.z);
         }
-        tile_sums_zero(isum, lane);
-        const int i0 = (ti0 + u) * kTile + lane;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int i = i0 + 32 * k;
-            // a lane past the system holds a massless body far from every j-body
-            float S[3] = {-1.0e18f, -1.0e18f, -1.0e18f}, E[3] = {0.f, 0.f, 0.f}, mi = 0.f;
-            if (i < sd.n) {
-                const float4 h = hi[sd.first + i], l = lo[sd.first + i];
+        if (two && (!within || u0 + 2 < tb)) {
+            TileI<4> ti;
+            TileILow<4> tl;
+            float mi, mj;
+            const bool ei = batch_load_i<SORTED>(hi, lo, sd, (ti0 + u0) * kTile, c, ti, tl, mi);
+            for (int v = within ? u0 + 2 : 0; v < tb; ++v) {
+                bool far = false;
                 if (SORTED) {
-                    rel_ds(h.x, l.x, cx, S[0], E[0]);
-                    rel_ds(h.y, l.y, cy, S[1], E[1]);
-                    rel_ds(h.z, l.z, cz, S[2], E[2]);
-                } else {
-                    S[0] = h.x; S[1] = h.y; S[2] = h.z;
-                    E[0] = l.x; E[1] = l.y; E[2] = l.z;
+                    const TileBox bj = tile_box(boxes, sd.tile0 + tj0 + v);
+                    const float gx = fmaxf(0.f, fmaxf(bj.mn.x - bi.mx.x, bi.mn.x - bj.mx.x));
+                    const float gy = fmaxf(0.f, fmaxf(bj.mn.y - bi.mx.y, bi.mn.y - bj.mx.y));
+                    const float gz = fmaxf(0.f, fmaxf(bj.mn.z - bi.mx.z, bi.mn.z - bj.mx.z));
+                    const float gap2 = gx * gx + gy * gy + gz * gz;
+                    far = gap2 > 0.f && gap2 >= kFarFactor2 * bi.diam2();
                 }
-                mi = h.w;
+                const bool equal = batch_stage_j<SORTED>(hi, lo, sd, (tj0 + v) * kTile, c, stage,
+                                                         low, mj) && ei && soft;
+                if (far && equal)
+                    tile_pair<kFarTerm, true, ZERO_SOFT, 4>(stage, &low, lane, ti, &tl, e2, mi, mj,
+                                                            isum, sums[v]);
+                else if (far)
+                    tile_pair<kFarTerm, false, ZERO_SOFT, 4>(stage, &low, lane, ti, &tl, e2, 0.f,
+                                                             0.f, isum, sums[v]);
+                else if (equal)
+                    tile_pair<kNearTerm, true, ZERO_SOFT, 4>(stage, &low, lane, ti, &tl, e2, mi,
+                                                             mj, isum, sums[v]);
+                else
+                    tile_pair<kNearTerm, false, ZERO_SOFT, 4>(stage, &low, lane, ti, &tl, e2, 0.f,
+                                                              0.f, isum, sums[v]);
             }
-            tile_i_set(ti, k, S, mi);
-            tile_i_set_low(tl, k, E);
         }
-        for (int v = within ? u : 0; v < tb; ++v) {
-            const int tj = tj0 + v;
-            bool far = false;
-            if (SORTED) {
-                const TileBox bj = tile_box(boxes, sd.tile0 + tj);
-                const float gx = fmaxf(0.f, fmaxf(bj.mn.x - bi.mx.x, bi.mn.x - bj.mx.x));
-                const float gy = fmaxf(0.f, fmaxf(bj.mn.y - bi.mx.y, bi.mn.y - bj.mx.y));
-                const float gz = fmaxf(0.f, fmaxf(bj.mn.z - bi.mx.z, bi.mn.z - bj.mx.z));
-                const float gap2 = gx * gx + gy * gy + gz * gz;
-                far = gap2 > 0.f && gap2 >= kVeryFar2 * fmaxf(bi.diam2, bj.diam2);
+        // one tile at a time: within the block the pair's own tiles, else the
+        // last tile of an odd number
+        for (int u = u0; u < u0 + 1 + two; ++u) {
+            if (two && !within) break;
+            TileI<2> ti;
+            TileILow<2> tl;
+            float mi, mj;
+            const bool ei = batch_load_i<SORTED>(hi, lo, sd, (ti0 + u) * kTile, c, ti, tl, mi);
+            const int v1 = two ? u0 + 2 : tb;
+            for (int v = within ? u : 0; v < v1; ++v) {
+                const bool equal = batch_stage_j<SORTED>(hi, lo, sd, (tj0 + v) * kTile, c, stage,
+                                                         low, mj) && ei && soft;
+                if (within && u == v)
+                    tile_self<ZERO_SOFT>(stage, &low, lane, ti, &tl, e2, isum[u - u0]);
+                else if (equal)
+                    tile_pair<kNearTerm, true, ZERO_SOFT, 2>(stage, &low, lane, ti, &tl, e2, mi,
+                                                             mj, isum + (u - u0), sums[v]);
+                else
+                    tile_pair<kNearTerm, false, ZERO_SOFT, 2>(stage, &low, lane, ti, &tl, e2, 0.f,
+                                                              0.f, isum + (u - u0), sums[v]);
             }
-            __syncwarp();
+        }
+        __syncwarp();
+        // the i-tiles' partial sums; within a block with what they took as j-tiles
+        for (int w = 0; w < 1 + two; ++w) {
+            const int i = (ti0 + u0 + w) * kTile + lane;
 #pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {
-                const int j = tj * kTile + 32 * h2 + lane;
-                // lanes past the system stage a massless body far away: exactly 0
-                float S[3] = {1.0e18f, 1.0e18f, 1.0e18f}, E[3] = {0.f, 0.f, 0.f}, mj = 0.f;
-                if (j < sd.n) {
-                    const float4 h = hi[sd.first + j], l = lo[sd.first + j];
-                    if (SORTED) {
-                        rel_ds(h.x, l.x, cx, S[0], E[0]);
-                        rel_ds(h.y, l.y, cy, S[1], E[1]);
-                        rel_ds(h.z, l.z, cz, S[2], E[2]);
-                    } else {
-                        S[0] = h.x; S[1] = h.y; S[2] = h.z;
-                        E[0] = l.x; E[1] = l.y; E[2] = l.z;
-                    }
-                    mj = h.w;
+            for (int d = 0; d < 3; ++d) {
+                float2 t = isum[w].s[d][lane], e = isum[w].c[d][lane];
+                if (within) {
+                    const float2 js = sums[u0 + w].s[d][lane], jc = sums[u0 + w].c[d][lane];
+                    float2 r;
+                    two_sum(t.x, js.x, t.x, r.x);
+                    two_sum(t.y, js.y, t.y, r.y);
+                    e = make_float2(r.x + (e.x + jc.x), r.y + (e.y + jc.y));
                 }
-                tile_j_put(stage, lane, h2, S, mj);
-                tile_j_put_low(low, lane, h2, E);
+                if (i < sd.n) pa[d * plane + i] = make_float2(t.x, e.x);
+                if (i + 32 < sd.n) pa[d * plane + i + 32] = make_float2(t.y, e.y);
             }
-            __syncwarp();
-            if (within && u == v)
-                tile_self<ZERO_SOFT>(stage, &low, lane, ti, &tl, e2, isum);
-            else if (far)
-                tile_pair<kVeryFarTerm, false, ZERO_SOFT, 2>(stage, &low, lane, ti, &tl, e2, 0.f, 0.f, &isum,
-                                                      sums[v]);
-            else
-                tile_pair<kNearTerm, false, ZERO_SOFT, 2>(stage, &low, lane, ti, &tl, e2, 0.f, 0.f, &isum,
-                                                     sums[v]);
-        }
-        // the i-tile's partial sums; within a block with what it took as a j-tile
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            float2 t = isum.s[c][lane], e = isum.c[c][lane];
-            if (within) {
-                const float2 js = sums[u].s[c][lane], jc = sums[u].c[c][lane];
-                float2 r;
-                two_sum(t.x, js.x, t.x, r.x);
-                two_sum(t.y, js.y, t.y, r.y);
-                e = make_float2(r.x + (e.x + jc.x), r.y + (e.y + jc.y));
-            }
-            if (i0 < sd.n) pa[c * plane + i0] = make_float2(t.x, e.x);
-            if (i0 + 32 < sd.n) pa[c * plane + i0 + 32] = make_float2(t.y, e.y);
         }
     }
     if (within) return;
     for (int v = 0; v < tb; ++v) {
         const int j = (tj0 + v) * kTile + lane;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const float2 js = sums[v].s[c][lane], jc = sums[v].c[c][lane];
-            if (j < sd.n) pb[c * plane + j] = make_float2(js.x, jc.x);
-            if (j + 32 < sd.n) pb[c * plane + j + 32] = make_float2(js.y, jc.y);
+        for (int d = 0; d < 3; ++d) {
+            const float2 js = sums[v].s[d][lane], jc = sums[v].c[d][lane];
+            if (j < sd.n) pb[d * plane + j] = make_float2(js.x, jc.x);
+            if (j + 32 < sd.n) pb[d * plane + j + 32] = make_float2(js.y, jc.y);
         }
     }
 }

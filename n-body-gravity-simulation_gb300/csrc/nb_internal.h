@@ -207,7 +207,7 @@ constexpr int kBatchBlockBodies = 256;  // four tiles of 64
 // Smallest system summed over unordered pairs; smaller ones by rows (ordered
 // pairs).  On the 1024-system ensemble (n log-uniform in [32, 4096], two RK4 steps)
 // a line at 512 / 1024 / 2048 / beyond every system measured 7.58 / 7.69 / 8.12 /
-// 9.15 ms.  It lies at 1024, not 512: in a system of a few hundred bodies one close
+// 9.15 ms (one i-tile at a time).  It lies at 1024, not 512: in a system of a few hundred bodies one close
 // pair can carry a body's whole force, and the row sum is the order of rounding
 // that its trajectory has had.
 constexpr int kBatchPairsMin = 1024;

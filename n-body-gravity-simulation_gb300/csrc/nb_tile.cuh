@@ -155,7 +155,12 @@ __device__ __forceinline__ void tile_step(const TileJ &t, const TileJLow *low, i
             inv.y = r2.y > 0.f ? inv.y : 0.f;
         }
         float2 w = mul2(inv, inv);
-        if (TERM != kVeryFarTerm) w = mul2(w, fma2(dup2(-1.5f), mul2(r2, w), dup2(2.5f)));
+        if (TERM != kVeryFarTerm) {
+            // the residual by one FMA (pair_scale rounds the product r2 w, of size
+            // one, first): the same operations, a third of the scale's error
+            const float2 d = fma2(r2, w, dup2(-1.f));
+            w = fma2(w, mul2(d, dup2(-1.5f)), w);
+        }
         const float2 si = EQUAL ? mul2(inv, w) : mul2(mul2(jm, inv), w);
         fi[k][0] = fma2(dx, si, fi[k][0]);
         fi[k][1] = fma2(dy, si, fi[k][1]);
