@@ -625,10 +625,10 @@ direct_near_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
 
 // The pairs direct_near_kernel leaves out, in double-single.  It needs
 // nothing from that kernel -- it takes the same decisions from the same data
-// -- so it runs beside it on a second stream.  One CTA per warp of the near
-// kernel (the same i-chunks and geometry) and kExactWarps warps in it: warp w
-// takes the chunks jc = w (mod kExactWarps) that the near kernel tests for
-// left-out pairs (not far, nearer than R), in increasing order, skipping those
+// -- so it runs beside it on a second stream.  S CTAs per tile (the same i-chunks
+// and geometry) and kExactWarps warps in each: warp w
+// of share y of S takes the chunks jc = kExactWarps y + w (mod kExactWarps S)
+// that the near kernel tests for left-out pairs (not far, nearer than R), in increasing order, skipping those
 // that no lane's i-body comes within R of.  For each it stages the chunk
 // exactly as the near kernel does, recomputes the same r^2 bits, and marks the
 // left-out pairs of each lane (bit 2p + u of mk[k]: tile body 2p + u against
@@ -636,7 +636,7 @@ direct_near_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
 // whole-warp, in rounds of kExactRound, and every lane adds its own bodies'
 // terms into their double-single sums in increasing j; the warps' sums are
 // then added in warp order.  The result does not depend on timing.
-// ex[c n + i] = the FP64 value of body i's sum (sorted order), 0 if none.
+// ex[(3 y + c) n + i] = the FP64 value of body i's sum (sorted order), 0 if none.
 // At most 64 registers (four CTAs per SM): beside direct_far_kernel, whose
 // one-warp CTAs fill the register file, a leaner CTA displaces fewer of them.
 __global__ void __launch_bounds__(kExactWarps * 32, 4)
@@ -652,6 +652,7 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     __shared__ float red[kExactWarps][IPT * 32][6];           // the warps' sums
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int wg = blockIdx.x;
+    const int stride = kExactWarps * gridDim.y;  // candidate chunks: every stride-th
     const int tile0 = wg * IPT;
     if (tile0 >= nchunks) return;  // the whole CTA
     PairTile &sg = stage[w];
@@ -712,13 +713,13 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     const float cmag = fmaxf(fabsf(gm.c[0]), fmaxf(fabsf(gm.c[1]), fabsf(gm.c[2])));
     const float e2slack = 1e-6f * (gm.tile.thr2x + eps2);
 
-    int scan = w;
+    int scan = kExactWarps * blockIdx.y + w;
     while (true) {
-        // the next chunk jc = w (mod kExactWarps) the near kernel tests, with
+        // the next chunk of this warp's that the near kernel tests, with
         // a lane whose bodies come within R of its box
         int jc = -1;
         while (scan < nchunks) {
-            const int c = scan + kExactWarps * lane;
+            const int c = scan + stride * lane;
             bool t = false;
             float4 jmn = make_float4(0.f, 0.f, 0.f, 0.f), jmx = jmn;
             if (c < nchunks) {
@@ -746,15 +747,15 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                                                      fmaxf(fabsf(bz0), fabsf(bz1))));
                 const float Re = Rw + 1e-6f * mag;
                 if (__any_sync(0xffffffffu, gx * gx + gy * gy + gz * gz <= Re * Re + e2slack)) {
-                    jc = scan + kExactWarps * src;
+                    jc = scan + stride * src;
                     break;
                 }
             }
             if (jc >= 0) {
-                scan = jc + kExactWarps;
+                scan = jc + stride;
                 break;
             }
-            scan += 32 * kExactWarps;
+            scan += 32 * stride;
         }
         if (jc < 0) break;
 
@@ -897,7 +898,7 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
         if (i < n)
 #pragma unroll
             for (int a = 0; a < 3; ++a)
-                ex[(size_t)a * n + i] = (double)sum[a].hi + (double)sum[a].lo;
+                ex[(size_t)(3 * blockIdx.y + a) * n + i] = (double)sum[a].hi + (double)sum[a].lo;
     }
 }
 
@@ -914,7 +915,8 @@ combine_sorted_kernel(const float *__restrict__ part, int blocks, int p0, int np
                       bool last, float *__restrict__ acc, const float *__restrict__ psum,
                       const float *__restrict__ pcomp, int n, int segments, double G,
                       const uint32_t *__restrict__ order, const double *__restrict__ ex,
-                      double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az)
+                      int shares, double *__restrict__ ax, double *__restrict__ ay,
+                      double *__restrict__ az)
 {
     __shared__ float2 sh[kCombineGroups][3][32];
     const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -963,8 +965,10 @@ combine_sorted_kernel(const float *__restrict__ part, int blocks, int p0, int np
     }
     const uint32_t o = order[i];
     if (!NB_IN_RANGE(o, n)) return;
+    double left_out = ex[c * plane + i];
+    for (int k = 1; k < shares; ++k) left_out += ex[(3 * (size_t)k + c) * plane + i];
     double *out = c == 0 ? ax : (c == 1 ? ay : az);
-    out[o] = G * (((double)s.x + (double)s.y) + ex[c * plane + i]);
+    out[o] = G * (((double)s.x + (double)s.y) + left_out);
 }
 
 } // namespace
@@ -979,11 +983,14 @@ void SortedBuffers::release()
     exact.release();
     far.release();
     acc.release();
-    if (side) cudaStreamDestroy(side);
     if (fork) cudaEventDestroy(fork);
-    if (join) cudaEventDestroy(join);
-    side = nullptr;
-    fork = join = nullptr;
+    fork = nullptr;
+    for (int k = 0; k < 2; ++k) {
+        if (side[k]) cudaStreamDestroy(side[k]);
+        if (join[k]) cudaEventDestroy(join[k]);
+        side[k] = nullptr;
+        join[k] = nullptr;
+    }
     if (sorter) bh_destroy(sorter);
     sorter = nullptr;
     order = nullptr;
@@ -1007,41 +1014,50 @@ bool direct_sorted_enabled(int n, int flags)
 // the longest rows alone at the end; 20,000: the same).  A function of n alone.
 static int near_segments(int tiles) { return std::min(32, std::max(2, 10000 / tiles)); }
 
-// The near kernel's ordered pairs (into b.partials) and the left-out ones (into
-// b.exact, 3 n doubles), on b.side: it waits for the staging on st (fork) and st
-// waits for it before the combine (join).  The side stream has the highest
-// priority, so the exact CTAs start at once and their longest chains run while
-// the far kernel fills the GPU.
+// CTAs per tile of the exact kernel: about 1,000 CTAs, so that a tile with many
+// left-out pairs is shared out where the tiles are few (at N = 16,384 one CTA
+// per tile took 175 us, longer than all the other pairs).
+static int exact_shares(int tiles) { return std::min(8, std::max(1, 1024 / tiles)); }
+
+// The left-out pairs (into b.exact, 3 n doubles per share) and the near kernel's
+// ordered pairs (into b.partials), each on a side stream: both wait for the
+// staging on st (fork) and st waits for them before the combine (join).  The side
+// streams have the highest priority, so their CTAs start at once and the longest
+// chains run while the far kernel fills the GPU.
 static nb_status launch_side(const float4 *hi, const float4 *lo, int n, int segments, double eps2,
                              SortedBuffers &b, cudaStream_t st)
 {
-    NB_TRY(b.exact.reserve(sizeof(double) * 3 * (size_t)n));
-    NB_TRY(b.partials.reserve(sizeof(float) * 6 * (size_t)n * segments));
-    if (!b.side) {
-        int least = 0, greatest = 0;
-        NB_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        NB_CUDA_TRY(cudaStreamCreateWithPriority(&b.side, cudaStreamNonBlocking, greatest));
-        NB_CUDA_TRY(cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming));
-        NB_CUDA_TRY(cudaEventCreateWithFlags(&b.join, cudaEventDisableTiming));
-    }
-    NB_CUDA_TRY(cudaEventRecord(b.fork, st));
-    NB_CUDA_TRY(cudaStreamWaitEvent(b.side, b.fork, 0));
     const int nchunks = (n + kChunk - 1) / kChunk, tiles = (nchunks + 1) / 2;
+    const int shares = exact_shares(tiles);
+    NB_TRY(b.exact.reserve(sizeof(double) * 3 * (size_t)n * shares));
+    NB_TRY(b.partials.reserve(sizeof(float) * 6 * (size_t)n * segments));
+    int least = 0, greatest = 0;
+    if (!b.fork) {
+        NB_CUDA_TRY(cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming));
+    }
+    for (int k = 0; k < 2; ++k)
+        if (!b.side[k]) {
+            NB_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+            NB_CUDA_TRY(cudaEventCreateWithFlags(&b.join[k], cudaEventDisableTiming));
+            NB_CUDA_TRY(cudaStreamCreateWithPriority(&b.side[k], cudaStreamNonBlocking, greatest));
+        }
+    NB_CUDA_TRY(cudaEventRecord(b.fork, st));
+    for (int k = 0; k < 2; ++k) NB_CUDA_TRY(cudaStreamWaitEvent(b.side[k], b.fork, 0));
     const float4 *box = b.boxes.as<float4>(), *tile = b.tiles.as<float4>();
-    exact_pairs_kernel<<<tiles, kExactWarps * 32, 0, b.side>>>(
+    exact_pairs_kernel<<<dim3(tiles, shares), kExactWarps * 32, 0, b.side[0]>>>(
         hi, lo, box, tile, n, nchunks, eps2 > 0.0 ? (float)eps2 : 0.0f, kFarFactor2,
         eps2 > 0.0 ? eps2 : 0.0, b.exact.as<double>());
     NB_LAUNCH_CHECK();
     float *psum = b.partials.as<float>(), *pcomp = psum + 3 * (size_t)n * segments;
     const dim3 grid(tiles, segments);
     if (eps2 > 0.0)
-        direct_near_kernel<false><<<grid, 32, 0, b.side>>>(hi, lo, box, tile, n, nchunks,
-                                                           (float)eps2, psum, pcomp, kFarFactor2);
+        direct_near_kernel<false><<<grid, 32, 0, b.side[1]>>>(
+            hi, lo, box, tile, n, nchunks, (float)eps2, psum, pcomp, kFarFactor2);
     else
-        direct_near_kernel<true><<<grid, 32, 0, b.side>>>(hi, lo, box, tile, n, nchunks, 0.0f,
-                                                          psum, pcomp, kFarFactor2);
+        direct_near_kernel<true><<<grid, 32, 0, b.side[1]>>>(hi, lo, box, tile, n, nchunks, 0.0f,
+                                                             psum, pcomp, kFarFactor2);
     NB_LAUNCH_CHECK();
-    NB_CUDA_TRY(cudaEventRecord(b.join, b.side));
+    for (int k = 0; k < 2; ++k) NB_CUDA_TRY(cudaEventRecord(b.join[k], b.side[k]));
     return NB_OK;
 }
 
@@ -1095,12 +1111,12 @@ nb_status direct_mixed_sorted(const double *x, const double *y, const double *z,
         NB_LAUNCH_CHECK();
         const bool last = p0 + np == diagonals;
         if (last) {
-            NB_CUDA_TRY(cudaStreamWaitEvent(st, b.join, 0));
+            for (int k = 0; k < 2; ++k) NB_CUDA_TRY(cudaStreamWaitEvent(st, b.join[k], 0));
             if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
         }
         combine_sorted_kernel<<<(n + 31) / 32, 32 * kCombineGroups, 0, st>>>(
             b.far.as<float>(), blocks, p0, np, p0 == 0, last, b.acc.as<float>(), psum, pcomp, n,
-            segments, G, order, b.exact.as<double>(), ax, ay, az);
+            segments, G, order, b.exact.as<double>(), exact_shares(tiles), ax, ay, az);
         NB_LAUNCH_CHECK();
     }
     return NB_OK;

@@ -121,10 +121,10 @@ constexpr float kExactSpacing2 = 0.5625f;   // kExactSpacing = 3/4
 struct BHTree;
 struct SortedBuffers {
     DevBuf hi, lo, partials, boxes, tiles;
-    DevBuf exact;  // the left-out pairs' sums, 3 n doubles (sorted order)
+    DevBuf exact;  // the left-out pairs' sums, 3 n doubles per share (sorted order)
     DevBuf far, acc;  // the far kernel's partial planes, and their sums between passes
-    cudaStream_t side = nullptr;              // the near and exact-pair kernels' stream
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t side[2] = {};  // the exact-pair and near kernels' streams
+    cudaEvent_t fork = nullptr, join[2] = {};
     BHTree *sorter = nullptr;
     // The sort order is a performance device only (near/far decisions use
     // the current chunk boxes, any order gives results within tolerance), so
