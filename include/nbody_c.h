@@ -118,12 +118,9 @@ typedef struct nb_config {
  * a warp-local origin, the closest pairs in double-single) and smaller ones the
  * all-pairs double-single kernel; these flags force one or the other.  The
  * sorted kernel also holds every body to |da| <= 1e-6 |a| without the
- * conditioning clause of the all-pairs kernel.  The all-pairs kernel times its
- * CTA shapes on the first evaluation of each N in a process and keeps the
- * fastest.  The order in which a body's terms are summed is fixed by N alone in
- * both, so results are bit-identical within a process and between processes on
- * the same GPU model.
- */
+ * conditioning clause of the all-pairs kernel.  The order in which a body's
+ * terms are summed is fixed by N alone in both, so results are bit-identical
+ * within a process and between processes on the same GPU model. */
 #define NB_FLAG_MIXED_SORTED 4
 #define NB_FLAG_MIXED_UNSORTED 8
 
@@ -449,12 +446,10 @@ nb_status nb_checkpoint_load(nb_sim *sim, const char *path);
  * (split, all-pairs sum, combine) from caller-owned DEVICE arrays x, y, z, m
  * into caller-owned DEVICE arrays ax, ay, az, on `stream` (NULL = legacy
  * default stream), asynchronously.  It never runs the Hilbert-sorted kernel
- * that NB_DIRECT_MIXED uses from 16,384 bodies, never autotunes, and caps its
- * j-split to fit its scratch, so it agrees with NB_DIRECT_MIXED to the
- * mixed-path tolerance; its bits equal those of an NB_DIRECT_MIXED evaluation
- * only when both run the same plan (the all-pairs kernel with autotuning off,
- * NB_AUTOTUNE=0, and n small enough that the j-split is not capped, about
- * n < 150,000).  It allocates nothing: its scratch is one 16 MiB array in the
+ * that NB_DIRECT_MIXED uses from 16,384 bodies nor the unordered-pairs one it uses
+ * from 4096, and caps its j-split to fit its scratch, so it agrees with
+ * NB_DIRECT_MIXED to the mixed-path tolerance; below 4096 bodies its bits equal
+ * those of an NB_DIRECT_MIXED evaluation.  It allocates nothing: its scratch is one 16 MiB array in the
  * library's device memory, present on every device that loads the library
  * until the process exits, which limits n to 262144 (larger n returns
  * NB_ERR_CAPACITY).  The first call on each device looks up that array's

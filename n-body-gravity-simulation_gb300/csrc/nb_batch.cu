@@ -161,77 +161,6 @@ __device__ __forceinline__ void batch_row(const float4 *__restrict__ hi,
     az[o] = G * ((double)sz - (double)qz);
 }
 
-// A body relative to c as a normalised double-single (SORTED), or as it is.
-template <bool SORTED>
-__device__ __forceinline__ void batch_relative(const float4 h, const float4 l, const float (&c)[3],
-                                               float (&S)[3], float (&E)[3], float &m)
-{
-    if (SORTED) {
-        rel_ds(h.x, l.x, c[0], S[0], E[0]);
-        rel_ds(h.y, l.y, c[1], S[1], E[1]);
-        rel_ds(h.z, l.z, c[2], S[2], E[2]);
-    } else {
-        S[0] = h.x; S[1] = h.y; S[2] = h.z;
-        E[0] = l.x; E[1] = l.y; E[2] = l.z;
-    }
-    m = h.w;
-}
-// Coordinates whose differences stay within equal_range's farthest pair.
-__device__ __forceinline__ bool batch_in_span(const float (&S)[3])
-{
-    return fmaxf(fabsf(S[0]), fmaxf(fabsf(S[1]), fabsf(S[2]))) <= 2.5e10f;
-}
-
-// Loads IPT chunks of i-bodies from body i0 of the system, relative to c.  Returns
-// whether they all have one mass, mass, and coordinates within equal_range's
-// span; lanes past the system hold massless bodies far from every j-body.
-template <bool SORTED, int IPT>
-__device__ __forceinline__ bool batch_load_i(const float4 *__restrict__ hi,
-                                             const float4 *__restrict__ lo, const SysDesc &sd,
-                                             int i0, const float (&c)[3], TileI<IPT> &ti,
-                                             TileILow<IPT> &tl, float &mass)
-{
-    bool equal = true;
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = i0 + 32 * k + (int)threadIdx.x;
-        float S[3] = {-1.0e18f, -1.0e18f, -1.0e18f}, E[3] = {0.f, 0.f, 0.f}, m = 0.f;
-        if (i < sd.n) batch_relative<SORTED>(hi[sd.first + i], lo[sd.first + i], c, S, E, m);
-        if (k == 0) mass = __shfl_sync(0xffffffffu, m, 0);
-        equal = equal && (i >= sd.n || (m == mass && batch_in_span(S)));
-        tile_i_set(ti, k, S, m);
-        tile_i_set_low(tl, k, E);
-    }
-    return __all_sync(0xffffffffu, equal);
-}
-
-// Stages the j-tile from body j0 of the system relative to c; returns as
-// batch_load_i.
-template <bool SORTED>
-__device__ __forceinline__ bool batch_stage_j(const float4 *__restrict__ hi,
-                                              const float4 *__restrict__ lo, const SysDesc &sd,
-                                              int j0, const float (&c)[3], TileJ &stage,
-                                              TileJLow &low, float &mass)
-{
-    const int lane = threadIdx.x;
-    bool equal = true;
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int j = j0 + 32 * k + lane;
-        // lanes past the system stage a massless body far away: exactly 0
-        float S[3] = {1.0e18f, 1.0e18f, 1.0e18f}, E[3] = {0.f, 0.f, 0.f}, m = 0.f;
-        if (j < sd.n) batch_relative<SORTED>(hi[sd.first + j], lo[sd.first + j], c, S, E, m);
-        if (k == 0) mass = __shfl_sync(0xffffffffu, m, 0);
-        equal = equal && (j >= sd.n || (m == mass && batch_in_span(S)));
-        tile_j_put(stage, lane, k, S, m);
-        tile_j_put_low(low, lane, k, E);
-    }
-    equal = __all_sync(0xffffffffu, equal);
-    __syncwarp();
-    return equal;
-}
-
 // SORTED: the bodies are in Hilbert order with one box per tile; coordinates are
 // staged relative to the centre of the i-tiles' box, and a j-tile an eighth of
 // that box's diameter or more away takes the plain FP32 displacement (the bound of
@@ -277,6 +206,7 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     const int tiles = (sd.n + kTile - 1) / kTile;
     const int ti0 = it.a * kBatchTiles, tj0 = blk_b * kBatchTiles;
     const int ta = min(kBatchTiles, tiles - ti0), tb = min(kBatchTiles, tiles - tj0);
+    const float4 *bhi = hi + sd.first, *blo = lo + sd.first;
     const float2 e2 = dup2(eps2);
     const bool soft = eps2 >= 1e-22f;  // equal_range's nearest pair
     const size_t plane = (size_t)sd.n;
@@ -301,7 +231,7 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
             TileI<4> ti;
             TileILow<4> tl;
             float mi, mj;
-            const bool ei = batch_load_i<SORTED>(hi, lo, sd, (ti0 + u0) * kTile, c, ti, tl, mi);
+            const bool ei = tile_load_i<SORTED>(bhi, blo, sd.n, (ti0 + u0) * kTile, c, ti, tl, mi);
             for (int v = within ? u0 + 2 : 0; v < tb; ++v) {
                 bool far = false;
                 if (SORTED) {
@@ -312,8 +242,8 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                     const float gap2 = gx * gx + gy * gy + gz * gz;
                     far = gap2 > 0.f && gap2 >= kFarFactor2 * bi.diam2();
                 }
-                const bool equal = batch_stage_j<SORTED>(hi, lo, sd, (tj0 + v) * kTile, c, stage,
-                                                         low, mj) && ei && soft;
+                const bool equal = tile_stage_j<SORTED>(bhi, blo, sd.n, (tj0 + v) * kTile, c,
+                                                        stage, low, mj) && ei && soft;
                 if (far && equal)
                     tile_pair<kFarTerm, true, ZERO_SOFT, 4>(stage, &low, lane, ti, &tl, e2, mi, mj,
                                                             isum, sums[v]);
@@ -335,11 +265,11 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
             TileI<2> ti;
             TileILow<2> tl;
             float mi, mj;
-            const bool ei = batch_load_i<SORTED>(hi, lo, sd, (ti0 + u) * kTile, c, ti, tl, mi);
+            const bool ei = tile_load_i<SORTED>(bhi, blo, sd.n, (ti0 + u) * kTile, c, ti, tl, mi);
             const int v1 = two ? u0 + 2 : tb;
             for (int v = within ? u : 0; v < v1; ++v) {
-                const bool equal = batch_stage_j<SORTED>(hi, lo, sd, (tj0 + v) * kTile, c, stage,
-                                                         low, mj) && ei && soft;
+                const bool equal = tile_stage_j<SORTED>(bhi, blo, sd.n, (tj0 + v) * kTile, c,
+                                                        stage, low, mj) && ei && soft;
                 if (within && u == v)
                     tile_self<ZERO_SOFT>(stage, &low, lane, ti, &tl, e2, isum[u - u0]);
                 else if (equal)

@@ -3,7 +3,8 @@
 // Replaces computeAccelerationNaiveKernel (CUDA/src/force_calculator_naive.cu:4-59,
 // one FP64 thread per body, 256-body tiles, ceil(N/256) CTAs).  Two kernels:
 //
-//  * direct_mixed_kernel -- the production path.  Each body is held as a float4
+//  * direct_mixed_kernel -- the mixed path of small systems and of the no-allocation
+//    entry point.  Each body is held as a float4
 //    "hi" (x, y, z, m) plus a float4 "lo" (x - hi, ...): a double-single copy of
 //    its FP64 position.  The pair displacement is formed as
 //    (xj_hi - xi_hi) + (xj_lo - xi_lo), which is exact to FP32 rounding for close
@@ -21,6 +22,9 @@
 //    scaled by G in FP64.
 //    The tensor cores stay idle: a softened 1/r^3 sum is not a contraction.
 //
+//  * direct_mixed_pairs_kernel -- the same term over unordered pairs from 4096
+//    bodies (below 16,384, where the Hilbert-sorted path takes over).
+//
 //  * direct_fp64_pairs_kernel -- the 1e-12 path: an FP64 sum over unordered
 //    pairs of 32-body tiles (direct_fp64_row_kernel, a warp per body, for small n).
 //
@@ -29,13 +33,12 @@
 // segment count is chosen to fill whole waves.
 #include "nb_internal.h"
 #include "nb_fp64pair.cuh"
-#include "nb_pair.cuh"
+#include "nb_tile.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <string>
 
@@ -161,6 +164,152 @@ combine_mixed_kernel(const float *__restrict__ psum,
     ax[i] = G * ((double)hi[0] + (double)lo[0]);
     ay[i] = G * ((double)hi[1] + (double)lo[1]);
     az[i] = G * ((double)hi[2] + (double)lo[2]);
+}
+
+// ---------------------------------------------------------------- mixed, unordered pairs
+// From kMixedPairsMin bodies every unordered pair is evaluated once (nb_tile.cuh)
+// over pairs of 256-body blocks: diagonal p pairs block a with a + p.  A one-warp
+// CTA takes an eighth of a block pair's 4 x 4 tiles: two i-tiles (four bodies per
+// lane) against one j-tile, whose sums it keeps in shared memory.  A body has
+// kPairV planes of Kahan pairs per diagonal from its block as the first, kPairH
+// as the second; the combine adds them in order.
+// Bound by dispatch (nb_tile.cuh), below 8,000 bodies by how evenly the CTAs fill
+// the SMs.  An evaluation at n = 5,003 / 8,000 / 16,383 takes 29 / 46 / 140 us;
+// one CTA per block pair (fewer planes) 51 / 54 / 150, the ordered-pairs kernel
+// 40 / 73 / 200.
+constexpr int kPairTiles = 4;
+constexpr int kPairBlock = kPairTiles * kTile;
+constexpr int kPairH = kPairTiles / 2, kPairV = kPairTiles;
+
+template <bool ZERO_SOFT>
+__global__ void __launch_bounds__(32, 16)
+direct_mixed_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo, int n,
+                          float eps2, int blocks, int p0, int np, float2 *__restrict__ part)
+{
+    __shared__ TileJ stage;
+    __shared__ TileJLow low;
+    __shared__ TileSums jsum, isum[2];
+    const int lane = threadIdx.x;
+    const int share = blockIdx.x % (kPairH * kPairV), item = blockIdx.x / (kPairH * kPairV);
+    const int a = item % blocks, dp = item / blocks, p = p0 + dp;
+    if (!pair_first(p, a, blocks)) return;
+    const int h = share / kPairV, v = share % kPairV, u = 2 * h;
+    const int tiles = (n + kTile - 1) / kTile;
+    const int ti0 = a * kPairTiles, tj0 = (a + p) % blocks * kPairTiles;
+    const int ta = min(kPairTiles, tiles - ti0), tb = min(kPairTiles, tiles - tj0);
+    const bool two = u + 1 < ta;
+    const float2 e2 = dup2(eps2);
+    const float c[3] = {0.f, 0.f, 0.f};
+    const bool soft = eps2 >= 1e-22f;  // equal_range's nearest pair
+    tile_sums_zero(jsum, lane);
+    tile_sums_zero(isum[0], lane);
+    tile_sums_zero(isum[1], lane);
+    // within a block: the j-tiles after the pair's own two, and with the last of
+    // those (own) the pair's tiles against themselves and each other
+    const int own = p == 0 ? u + two : -1;
+    float mi, mj;
+    if (two && v > own && v < tb) {
+        TileI<4> ti;
+        TileILow<4> tl;
+        const bool ei = tile_load_i<false>(hi, lo, n, (ti0 + u) * kTile, c, ti, tl, mi);
+        if (tile_stage_j<false>(hi, lo, n, (tj0 + v) * kTile, c, stage, low, mj) && ei && soft)
+            tile_pair<kNearTerm, true, ZERO_SOFT, 4>(stage, &low, lane, ti, &tl, e2, mi, mj, isum,
+                                                     jsum);
+        else
+            tile_pair<kNearTerm, false, ZERO_SOFT, 4>(stage, &low, lane, ti, &tl, e2, 0.f, 0.f,
+                                                      isum, jsum);
+    } else if (u < ta && v < tb && (p == 0 ? v == own : !two)) {
+        // one i-tile at a time: the pair's own (within), or the last of an odd number
+        for (int w = 0; w < 1 + two; ++w) {
+            TileI<2> ti;
+            TileILow<2> tl;
+            const bool ei = tile_load_i<false>(hi, lo, n, (ti0 + u + w) * kTile, c, ti, tl, mi);
+            for (int t = p == 0 ? u + w : v; t <= v; ++t) {
+                const bool equal =
+                    tile_stage_j<false>(hi, lo, n, (tj0 + t) * kTile, c, stage, low, mj) && ei &&
+                    soft;
+                if (p == 0 && t == u + w)
+                    tile_self<ZERO_SOFT>(stage, &low, lane, ti, &tl, e2, isum[w]);
+                else if (equal)
+                    tile_pair<kNearTerm, true, ZERO_SOFT, 2>(stage, &low, lane, ti, &tl, e2, mi,
+                                                             mj, isum + w, jsum);
+                else
+                    tile_pair<kNearTerm, false, ZERO_SOFT, 2>(stage, &low, lane, ti, &tl, e2, 0.f,
+                                                              0.f, isum + w, jsum);
+            }
+        }
+    }
+    __syncwarp();
+    // a share without pairs writes zeros: the combine reads every plane
+    const size_t plane = 3 * (size_t)n;
+    float2 *pa = part + (size_t)(dp * kPairV + v) * plane;
+    float2 *pb = part + (size_t)(np * kPairV + dp * kPairH + h) * plane;
+    for (int w = 0; w < 3; ++w) {
+        if (w < 2 ? u + w >= ta : v >= tb) continue;
+        float2 *out = w < 2 ? pa : pb;
+        const int i = (w < 2 ? ti0 + u + w : tj0 + v) * kTile + lane;
+        const TileSums &sum = w < 2 ? isum[w] : jsum;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float2 t = sum.s[d][lane], e = sum.c[d][lane];
+            if (i < n) out[(size_t)d * n + i] = make_float2(t.x, e.x);
+            if (i + 32 < n) out[(size_t)d * n + i + 32] = make_float2(t.y, e.y);
+        }
+    }
+}
+
+// a_i = G * the sum of body i's planes as a double-single: 32 bodies per block, 8
+// groups of planes in strides (their loads ahead of the ordered sums), then the
+// groups in order.  acc: the sums of earlier passes over the diagonals (first:
+// none yet), written back unless this is the last.
+constexpr int kPairGroups = 8;
+__global__ void __launch_bounds__(32 * kPairGroups)
+combine_mixed_pairs_kernel(const float2 *__restrict__ part, int n, int blocks, int p0, int np,
+                           bool first, bool last, float *__restrict__ acc, double G,
+                           double *__restrict__ ax, double *__restrict__ ay,
+                           double *__restrict__ az)
+{
+    constexpr int H = kPairH, V = kPairV;
+    __shared__ float2 sh[kPairGroups][3][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
+    if (i < n) {
+        const int blk = i / kPairBlock, planes = np * (V + H);
+        for (int k0 = g; k0 < planes; k0 += 4 * kPairGroups) {
+            float2 t[4][3];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int k = k0 + u * kPairGroups, q = k - np * V;
+                const bool use =
+                    q < 0 ? pair_first(p0 + k / V, blk, blocks)
+                          : k < planes && (p0 + q / H == 0 || pair_second(p0 + q / H, blk, blocks));
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    t[u][c] = use ? part[((size_t)k * 3 + c) * n + i] : dup2(0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) ds_add_kahan(hi[c], lo[c], t[u][c].x, -t[u][c].y);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sh[g][c][lane] = make_float2(hi[c], lo[c]);
+    __syncthreads();
+    if (g >= 3 || i >= n) return;  // warp c finishes component c
+    const int c = g;
+    float2 s = first ? dup2(0.f) : make_float2(acc[(size_t)c * n + i], acc[(size_t)(3 + c) * n + i]);
+#pragma unroll
+    for (int k = 0; k < kPairGroups; ++k)
+        ds_add_kahan(s.x, s.y, sh[k][c][lane].x, -sh[k][c][lane].y);
+    if (!last) {
+        acc[(size_t)c * n + i] = s.x;
+        acc[(size_t)(3 + c) * n + i] = s.y;
+        return;
+    }
+    double *out = c == 0 ? ax : (c == 1 ? ay : az);
+    out[i] = G * ((double)s.x + (double)s.y);
 }
 
 // ---------------------------------------------------------------- FP64
@@ -424,19 +573,12 @@ int resident_ctas(const void *fn)
 
 constexpr int kMixBlock = 256;
 constexpr int kMixIpt = 4;
+// Smallest system the mixed path sums over unordered pairs: an evaluation takes
+// 24.8 us there and 28.9 with ordered pairs at n = 4,000, 24.7 and 22.7 at 3,000.
+constexpr int kMixedPairsMin = 4096;
+constexpr size_t kPairPlaneBytes = (size_t)512 << 20;  // partial planes per pass
 constexpr int kF64RowMax = 512;  // largest N of the one-warp-per-body FP64 kernel
 constexpr size_t kF64PlaneBytes = (size_t)512 << 20;  // FP64 partial planes per pass
-
-// Tile shapes of the mixed kernel the autotuner chooses from: threads per CTA
-// x i-bodies per thread.  More i-bodies per thread amortise the two
-// broadcast shared-memory loads of a j-body and add independent work per
-// warp; fewer keep more warps resident.
-struct MixShape {
-    int block, ipt;
-};
-constexpr MixShape kMixShapes[] = {{256, 4}, {128, 2}, {128, 4}, {256, 2}, {64, 4},
-                                    {32, 1}, {32, 2}};
-constexpr int kNumMixShapes = sizeof(kMixShapes) / sizeof(kMixShapes[0]);
 
 template <int B, int I>
 int mix_slots()
@@ -447,11 +589,7 @@ int mix_slots()
 
 int mix_slots_for(int block, int ipt)
 {
-    if (block == 256 && ipt == 4) return mix_slots<256, 4>();
-    if (block == 128 && ipt == 2) return mix_slots<128, 2>();
-    if (block == 128 && ipt == 4) return mix_slots<128, 4>();
-    if (block == 256 && ipt == 2) return mix_slots<256, 2>();
-    if (block == 64 && ipt == 4) return mix_slots<64, 4>();
+    if (block == kMixBlock && ipt == kMixIpt) return mix_slots<kMixBlock, kMixIpt>();
     if (block == 32 && ipt == 1) return mix_slots<32, 1>();
     if (block == 32 && ipt == 2) return mix_slots<32, 2>();
     return 0;
@@ -476,16 +614,8 @@ bool launch_mixed(const DirectPlan &p, cudaStream_t st, const float4 *hi, const 
     const int per_cta = p.block * p.ipt;
     dim3 grid((n + per_cta - 1) / per_cta, p.segments);
     const int seg_len = p.seg_tiles * p.block;
-    if (p.block == 256 && p.ipt == 4)
-        launch_mixed_shape<256, 4>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
-    else if (p.block == 128 && p.ipt == 2)
-        launch_mixed_shape<128, 2>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
-    else if (p.block == 128 && p.ipt == 4)
-        launch_mixed_shape<128, 4>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
-    else if (p.block == 256 && p.ipt == 2)
-        launch_mixed_shape<256, 2>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
-    else if (p.block == 64 && p.ipt == 4)
-        launch_mixed_shape<64, 4>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
+    if (p.block == kMixBlock && p.ipt == kMixIpt)
+        launch_mixed_shape<kMixBlock, kMixIpt>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
     else if (p.block == 32 && p.ipt == 1)
         launch_mixed_shape<32, 1>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
     else if (p.block == 32 && p.ipt == 2)
@@ -495,7 +625,7 @@ bool launch_mixed(const DirectPlan &p, cudaStream_t st, const float4 *hi, const 
     return true;
 }
 
-DirectPlan plan_for_shape_model(int n, int block, int ipt)
+DirectPlan plan_for_shape(int n, int block, int ipt)
 {
     DirectPlan p;
     p.block = block;
@@ -509,101 +639,14 @@ DirectPlan plan_for_shape_model(int n, int block, int ipt)
     return p;
 }
 
-// The j-segment length of n bodies: that of the default shape (one-warp CTAs
-// below 4096 bodies, kMixBlock x kMixIpt above).  A body's summation order
-// depends only on the segment boundaries (every shape sums each segment in
-// 32-body tiles from its start), so fixing them per n makes every tile shape
-// give the same bits and the autotuner's timed choice cannot change a result.
-int mixed_segment_length(int n)
-{
-    const DirectPlan d = n < 4096 ? plan_for_shape_model(n, 32, n < 2048 ? 1 : 2)
-                                  : plan_for_shape_model(n, kMixBlock, kMixIpt);
-    return d.seg_tiles * d.block;
-}
-
-DirectPlan plan_for_shape(int n, int block, int ipt)
-{
-    DirectPlan p;
-    p.block = block;
-    p.ipt = ipt;
-    const int seg_len = mixed_segment_length(n);  // a multiple of every block size below it
-    p.seg_tiles = std::max(1, seg_len / block);
-    p.segments = std::max(1, (n + seg_len - 1) / seg_len);
-    return p;
-}
-
-// Autotuned plans by body count (the tuner times every shape on the caller's
-// own bodies at the first evaluation of each N; NB_AUTOTUNE=0 disables it).
-std::mutex g_tune_mutex;
-std::map<int, DirectPlan> g_tuned;
-
-bool autotune_enabled()
-{
-    static const bool on = [] {
-        const char *e = std::getenv("NB_AUTOTUNE");
-        return !(e && std::strcmp(e, "0") == 0);
-    }();
-    return on;
-}
-
 } // namespace
 
-int direct_pick_segments(int iblocks, int tiles, int slots)
-{
-    return pick_segments(iblocks, tiles, slots);
-}
-
+// The ordered-pairs kernel's shape: one-warp CTAs, as many as the j-split allows,
+// for small systems; kMixBlock x kMixIpt above (the no-allocation entry point).
 DirectPlan direct_mixed_plan(int n)
 {
-    {
-        std::lock_guard<std::mutex> lock(g_tune_mutex);
-        auto it = g_tuned.find(n);
-        if (it != g_tuned.end()) return it->second;
-    }
-    // small systems (not tuned): one-warp CTAs, as many as the j-split allows
     if (n < 4096) return plan_for_shape(n, 32, n < 2048 ? 1 : 2);
     return plan_for_shape(n, kMixBlock, kMixIpt);
-}
-
-// Times every tile shape on the given bodies (two launches each after one
-// warm-up, CUDA events on `st`) and records the fastest for this n.
-static nb_status autotune_mixed(const float4 *hi, const float4 *lo, int n, double eps2,
-                                DevBuf &partials, cudaStream_t st, DirectPlan *best)
-{
-    DirectPlan plans[kNumMixShapes];
-    size_t need = 0;
-    for (int k = 0; k < kNumMixShapes; ++k) {
-        plans[k] = plan_for_shape(n, kMixShapes[k].block, kMixShapes[k].ipt);
-        need = std::max(need, sizeof(float) * 6 * (size_t)n * plans[k].segments);
-    }
-    NB_TRY(partials.reserve(need));
-    cudaEvent_t e0, e1;
-    NB_CUDA_TRY(cudaEventCreate(&e0));
-    NB_CUDA_TRY(cudaEventCreate(&e1));
-    float best_ms = 1e30f;
-    *best = plans[0];
-    for (int k = 0; k < kNumMixShapes; ++k) {
-        float *psum = partials.as<float>();
-        float *pcomp = psum + 3 * (size_t)n * plans[k].segments;
-        launch_mixed(plans[k], st, hi, lo, n, eps2, psum, pcomp);
-        NB_LAUNCH_CHECK();
-        cudaEventRecord(e0, st);
-        for (int r = 0; r < 2; ++r) launch_mixed(plans[k], st, hi, lo, n, eps2, psum, pcomp);
-        cudaEventRecord(e1, st);
-        NB_LAUNCH_CHECK();
-        NB_CUDA_TRY(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_ms) {
-            best_ms = ms;
-            *best = plans[k];
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    std::lock_guard<std::mutex> lock(g_tune_mutex);
-    g_tuned[n] = *best;
-    return NB_OK;
 }
 
 nb_status split_positions(const double *x, const double *y, const double *z, const double *m,
@@ -615,25 +658,47 @@ nb_status split_positions(const double *x, const double *y, const double *z, con
     return NB_OK;
 }
 
+static nb_status direct_mixed_pairs(const float4 *hi, const float4 *lo, int n, double G,
+                                    double eps2, double *ax, double *ay, double *az,
+                                    DevBuf &partials, cudaStream_t st, const KernelTimer *timer)
+{
+    const int blocks = (n + kPairBlock - 1) / kPairBlock, diagonals = blocks / 2 + 1;
+    // planes of 3 n Kahan pairs, the diagonals in passes whose planes stay
+    // within kPairPlaneBytes; behind them the sums between passes
+    const size_t per_diagonal = sizeof(float2) * 3 * (size_t)n * (kPairH + kPairV);
+    const int pass = (int)std::min<size_t>(diagonals,
+                                           std::max<size_t>(1, kPairPlaneBytes / per_diagonal));
+    NB_TRY(partials.reserve(per_diagonal * pass + sizeof(float) * 6 * (size_t)n));
+    float2 *part = partials.as<float2>();
+    float *acc = reinterpret_cast<float *>(part + per_diagonal / sizeof(float2) * pass);
+    if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
+    for (int p0 = 0; p0 < diagonals; p0 += pass) {
+        const int np = std::min(pass, diagonals - p0);
+        const unsigned grid = (unsigned)blocks * (unsigned)np * (kPairH * kPairV);
+        if (eps2 > 0.0)
+            direct_mixed_pairs_kernel<false><<<grid, 32, 0, st>>>(hi, lo, n, (float)eps2, blocks,
+                                                                  p0, np, part);
+        else
+            direct_mixed_pairs_kernel<true><<<grid, 32, 0, st>>>(hi, lo, n, 0.0f, blocks, p0, np,
+                                                                 part);
+        NB_LAUNCH_CHECK();
+        const bool last = p0 + np == diagonals;
+        if (last && timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
+        combine_mixed_pairs_kernel<<<(n + 31) / 32, 32 * kPairGroups, 0, st>>>(
+            part, n, blocks, p0, np, p0 == 0, last, acc, G, ax, ay, az);
+        NB_LAUNCH_CHECK();
+    }
+    return NB_OK;
+}
+
 nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, double eps2,
                        double *ax, double *ay, double *az, DevBuf &partials, cudaStream_t st,
-                       const KernelTimer *timer, const DirectPlan *plan_override)
+                       const KernelTimer *timer)
 {
     if (n <= 0) return NB_OK;
-    DirectPlan p;
-    if (plan_override) {
-        p = *plan_override;
-    } else {
-        bool tuned;
-        {
-            std::lock_guard<std::mutex> lock(g_tune_mutex);
-            tuned = g_tuned.count(n) != 0;
-        }
-        if (!tuned && autotune_enabled() && n >= 4096)
-            NB_TRY(autotune_mixed(hi, lo, n, eps2, partials, st, &p));
-        else
-            p = direct_mixed_plan(n);
-    }
+    if (n >= kMixedPairsMin)
+        return direct_mixed_pairs(hi, lo, n, G, eps2, ax, ay, az, partials, st, timer);
+    const DirectPlan p = direct_mixed_plan(n);
     NB_TRY(partials.reserve(sizeof(float) * 6 * (size_t)n * p.segments));
     float *psum = partials.as<float>();
     float *pcomp = psum + 3 * (size_t)n * p.segments;

@@ -98,11 +98,7 @@ struct DirectPlan {
 // (x_lo, y_lo, z_lo, 0) of every body.  Writes G * sum into ax/ay/az (FP64).
 nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, double eps2,
                        double *ax, double *ay, double *az, DevBuf &partials,
-                       cudaStream_t st, const KernelTimer *timer = nullptr,
-                       const DirectPlan *plan_override = nullptr);
-DirectPlan direct_mixed_plan(int n);
-// j-split count filling whole waves of `slots` resident CTAs.
-int direct_pick_segments(int iblocks, int tiles, int slots);
+                       cudaStream_t st, const KernelTimer *timer = nullptr);
 
 // Thresholds of the sorted near/far kernels as (gap / D)^2, D the diameter of
 // a warp's i-box: a j-chunk at least D/8 away takes the plain FP32 term, one

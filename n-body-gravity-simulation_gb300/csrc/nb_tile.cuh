@@ -251,4 +251,75 @@ __device__ __forceinline__ bool equal_range(float gap2, float span2, float eps2)
     return gap2 + eps2 >= 1e-22f && span2 + eps2 <= 1e22f;
 }
 
+// A body relative to c as a normalised double-single (RELATIVE), or as it is.
+template <bool RELATIVE>
+__device__ __forceinline__ void tile_relative(const float4 h, const float4 l, const float (&c)[3],
+                                               float (&S)[3], float (&E)[3], float &m)
+{
+    if (RELATIVE) {
+        rel_ds(h.x, l.x, c[0], S[0], E[0]);
+        rel_ds(h.y, l.y, c[1], S[1], E[1]);
+        rel_ds(h.z, l.z, c[2], S[2], E[2]);
+    } else {
+        S[0] = h.x; S[1] = h.y; S[2] = h.z;
+        E[0] = l.x; E[1] = l.y; E[2] = l.z;
+    }
+    m = h.w;
+}
+// Coordinates whose differences stay within equal_range's farthest pair.
+__device__ __forceinline__ bool tile_in_span(const float (&S)[3])
+{
+    return fmaxf(fabsf(S[0]), fmaxf(fabsf(S[1]), fabsf(S[2]))) <= 2.5e10f;
+}
+
+// Loads IPT chunks of i-bodies from body i0 of n, relative to c.  Returns
+// whether they all have one mass, mass, and coordinates within equal_range's
+// span; lanes past n hold massless bodies far from every j-body.
+template <bool RELATIVE, int IPT>
+__device__ __forceinline__ bool tile_load_i(const float4 *__restrict__ hi,
+                                             const float4 *__restrict__ lo, int n, int i0,
+                                             const float (&c)[3], TileI<IPT> &ti,
+                                             TileILow<IPT> &tl, float &mass)
+{
+    bool equal = true;
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const int i = i0 + 32 * k + (int)threadIdx.x;
+        float S[3] = {-1.0e18f, -1.0e18f, -1.0e18f}, E[3] = {0.f, 0.f, 0.f}, m = 0.f;
+        if (i < n) tile_relative<RELATIVE>(hi[i], lo[i], c, S, E, m);
+        if (k == 0) mass = __shfl_sync(0xffffffffu, m, 0);
+        equal = equal && (i >= n || (m == mass && tile_in_span(S)));
+        tile_i_set(ti, k, S, m);
+        tile_i_set_low(tl, k, E);
+    }
+    return __all_sync(0xffffffffu, equal);
+}
+
+// Stages the j-tile from body j0 of n relative to c; returns as
+// tile_load_i.
+template <bool RELATIVE>
+__device__ __forceinline__ bool tile_stage_j(const float4 *__restrict__ hi,
+                                              const float4 *__restrict__ lo, int n, int j0,
+                                              const float (&c)[3], TileJ &stage,
+                                              TileJLow &low, float &mass)
+{
+    const int lane = threadIdx.x;
+    bool equal = true;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int j = j0 + 32 * k + lane;
+        // lanes past n stage a massless body far away: exactly 0
+        float S[3] = {1.0e18f, 1.0e18f, 1.0e18f}, E[3] = {0.f, 0.f, 0.f}, m = 0.f;
+        if (j < n) tile_relative<RELATIVE>(hi[j], lo[j], c, S, E, m);
+        if (k == 0) mass = __shfl_sync(0xffffffffu, m, 0);
+        equal = equal && (j >= n || (m == mass && tile_in_span(S)));
+        tile_j_put(stage, lane, k, S, m);
+        tile_j_put_low(low, lane, k, E);
+    }
+    equal = __all_sync(0xffffffffu, equal);
+    __syncwarp();
+    return equal;
+}
+
 } // namespace nb
