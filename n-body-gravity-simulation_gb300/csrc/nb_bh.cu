@@ -30,15 +30,15 @@
 // from FP64 prefix sums of (m, m x, m y, m z) over the sorted bodies (positions
 // relative to the root centre), so no level-by-level pass is needed.
 //
-// Walk.  One warp walks for 64 consecutive sorted bodies, two per lane.  At
-// each node every body applies the reference's opening test (open when size^2
-// >= theta^2 d^2 to the COM, or when the node holds the body); the warp opens
-// the node if any body does (so each body gets a refinement of its own walk,
+// Walk.  One CTA walks for 64 consecutive sorted bodies, two per lane of each of
+// its warps.  At each node every body applies the reference's opening test (open
+// when size^2 >= theta^2 d^2 to the COM, or when the node holds the body); the
+// node is opened if any body does (so each body gets a refinement of its own walk,
 // never a coarser one).  The children of every node are stored together (a
-// group): the warp reads a group in one round trip, adds the monopoles of the
-// children no body opens and the bodies of opened leaves, and pushes the
-// groups of opened internal children on its stack, which holds the deepest
-// tree's groups.  The stackless preorder walk over skip pointers finds the
+// group): a warp decides the nodes of four groups at once, lists the monopoles of
+// the nodes no body opens and the bodies of opened leaves for evaluation, and
+// pushes the groups of opened internal nodes on the CTA's stack, which holds the
+// deepest tree's groups.  The stackless preorder walk over skip pointers finds the
 // same interactions (NB_BH_WALK=preorder).  Accelerations are scattered back
 // to the original order in FP64, multiplied by G.
 #include "nb_internal.h"
@@ -1262,22 +1262,230 @@ group_kernel(const BHNode *__restrict__ nodes, const int *__restrict__ total,
     }
 }
 
-// A depth-first walk over groups keeps, per level of its current path, at most
-// 7 groups of unvisited siblings, plus the at most 8 groups the last group
-// pushed; groups lie at levels 0 .. kMaxLevels.
-constexpr int kGroupBlock = 32;  // threads of a group-walk CTA
-constexpr int kWalkWarps = kGroupBlock / 32;
-constexpr int kGroupStack = 8 * (kMaxLevels + 1);
+// ------------------------------------------------------------ group walk
+// One CTA walks for 64 NP consecutive sorted bodies, 2 NP per lane of each of its
+// W warps.  A warp decides 32 nodes at a time, one per lane, and only then
+// computes.  In each round
+//   - warp w takes the groups w, W + w, 2 W + w, 3 W + w below the top of the
+//     CTA's stack, and every lane loads one node's record;
+//   - a lane closes its node when no body can open it, or opens it when some
+//     body must, by the bounding boxes of the 32-body chunks; the few nodes in
+//     between are tested against every body, two nodes at a time.  The distances
+//     to a box are computed as those to a body are, operation by operation, so
+//     rounding keeps their order and the decisions are those of testing every
+//     body;
+//   - closed nodes and the bodies of opened leaves are appended to the warp's
+//     list in shared memory, two side by side, and the groups of opened internal
+//     nodes go onto the stack; a long enough list is evaluated as f32x2 pairs of
+//     list entries.
+// The interactions are those of walk2_kernel; only their order differs, and it is
+// a function of the tree, n and W alone.
+//
+// Bound by dispatch.  Testing each node by all bodies, one round trip to memory
+// per group, took 2.32 ms at N = 2^20 (theta 0.5), 3.67 ms at N = 100,000 under
+// the reference's opening rule (ten warps per SM, each a serial walk, the longest
+// five times the mean); this takes 1.73 ms with one warp per walk and 0.55 ms with
+// sixteen.  Of the 1.73 ms, about 1.2 are the 15.5 dispatch cycles per interaction
+// of the evaluation, the rest the decisions (2,600 nodes per walk, a fifth of them
+// undecided).
+//
+// Stack bound: the groups pushed by one round (at most 32 W) are children of
+// nodes at or below the lowest level of the groups it took, so the lowest
+// levels of the rounds on the stack strictly increase: 32 W per level.
+constexpr int kWalkWarps = 16;                     // at most
+constexpr int kWalkStack = 32 * (kMaxLevels + 1);  // per warp
+constexpr int kListPairs = 32;                     // list capacity: 64 entries
+constexpr int kListFlush = 2 * kListPairs - 32;    // evaluate from here on
 
-// The walk of walk2_kernel (64 NP bodies per warp, 2 NP per lane as packed
-// pairs; the same opening rule, decided for the whole warp) over child groups:
-// one round trip to memory brings a group's records into the warp's shared
-// memory, and the warp then tests the children one after the other, adding
-// the monopoles of the children no body opens, summing opened leaves' bodies,
-// and pushing the groups of opened internal children onto its stack.  The
-// interactions are those of walk2_kernel; only their order differs.
+// Lists of one warp; entry e lies in half e & 1 of pair e >> 1.
+struct WalkList {
+    float4 a[kListPairs];  // (x_0, x_1, y_0, y_1)
+    float4 b[kListPairs];  // (z_0, z_1, m_0, m_1)
+};
+struct WalkQuads {
+    float4 q[kListPairs][3];  // (xx, yy), (zz, xy), (xz, yz) of both entries
+};
+// Shared memory of a CTA: W of these, then its stack of W * kWalkStack groups
+// (int first records, then unsigned char record counts).
+template <bool QUAD>
+struct WalkShared {
+    float4 test[32];  // (com, size2) of the batch's nodes
+    float4 side[32];  // their parents' centres (DIR)
+    WalkList list;
+};
+template <>
+struct WalkShared<true> : WalkShared<false> {
+    WalkList bodies;  // leaf bodies apart: they have no quadrupole
+    WalkQuads quads;
+};
+template <bool QUAD>
+constexpr size_t walk_shared_bytes(int warps)
+{
+    return warps * (sizeof(WalkShared<QUAD>) + kWalkStack * (sizeof(int) + 1));
+}
+
+__device__ __forceinline__ void list_put(WalkList &l, int e, float x, float y, float z, float m)
+{
+    float *a = reinterpret_cast<float *>(&l.a[e >> 1]) + (e & 1);
+    float *b = reinterpret_cast<float *>(&l.b[e >> 1]) + (e & 1);
+    a[0] = x;
+    a[2] = y;
+    b[0] = z;
+    b[2] = m;
+}
+
+// The lane's K bodies, negated and duplicated, and their sums (over the even
+// and the odd list entries).
+template <int K>
+struct WalkBodies {
+    float2 nx[K], ny[K], nz[K];
+    float2 fx[K], fy[K], fz[K];
+};
+
+// Pairs [0, pairs) of a list, pairs a multiple of 4.
+template <bool ZERO_SOFT, bool QUAD, int K>
+__device__ __forceinline__ void list_eval(const WalkList &l, const WalkQuads *quads, int pairs,
+                                          float2 e2, WalkBodies<K> &wb)
+{
+#pragma unroll 4
+    for (int p = 0; p < pairs; ++p) {
+        const float4 A = l.a[p], B = l.b[p];
+        float2 qxx, qyy, qzz, qxy, qxz, qyz;
+        if (QUAD) {
+            const float4 Q0 = quads->q[p][0], Q1 = quads->q[p][1], Q2 = quads->q[p][2];
+            qxx = make_float2(Q0.x, Q0.y); qyy = make_float2(Q0.z, Q0.w);
+            qzz = make_float2(Q1.x, Q1.y); qxy = make_float2(Q1.z, Q1.w);
+            qxz = make_float2(Q2.x, Q2.y); qyz = make_float2(Q2.z, Q2.w);
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const float2 dx = add2(make_float2(A.x, A.y), wb.nx[k]);
+            const float2 dy = add2(make_float2(A.z, A.w), wb.ny[k]);
+            const float2 dz = add2(make_float2(B.x, B.y), wb.nz[k]);
+            const float2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, e2)));
+            float2 inv = make_float2(rsqrt_mufu(r2.x), rsqrt_mufu(r2.y));
+            if (ZERO_SOFT) {
+                inv.x = r2.x > 0.f ? inv.x : 0.f;
+                inv.y = r2.y > 0.f ? inv.y : 0.f;
+            }
+            const float2 inv2 = mul2(inv, inv);
+            const float2 s = mul2(mul2(make_float2(B.z, B.w), inv), inv2);
+            wb.fx[k] = fma2(dx, s, wb.fx[k]);
+            wb.fy[k] = fma2(dy, s, wb.fy[k]);
+            wb.fz[k] = fma2(dz, s, wb.fz[k]);
+            if (QUAD) {
+                const float2 qx = fma2(qxx, dx, fma2(qxy, dy, mul2(qxz, dz)));
+                const float2 qy = fma2(qxy, dx, fma2(qyy, dy, mul2(qyz, dz)));
+                const float2 qz = fma2(qxz, dx, fma2(qyz, dy, mul2(qzz, dz)));
+                const float2 rqr = fma2(dx, qx, fma2(dy, qy, mul2(dz, qz)));
+                const float2 inv5 = mul2(mul2(inv, inv2), inv2);
+                const float2 f = mul2(mul2(dup2(2.5f), rqr), inv2);
+                wb.fx[k] = fma2(inv5, fma2(f, dx, make_float2(-qx.x, -qx.y)), wb.fx[k]);
+                wb.fy[k] = fma2(inv5, fma2(f, dy, make_float2(-qy.x, -qy.y)), wb.fy[k]);
+                wb.fz[k] = fma2(inv5, fma2(f, dz, make_float2(-qz.x, -qz.y)), wb.fz[k]);
+            }
+        }
+    }
+}
+
+// Evaluates the list down to its last 0 .. 7 entries, which move to the front;
+// all: those too (padded with massless far bodies).
+template <bool ZERO_SOFT, bool QUAD, int K>
+__device__ __forceinline__ int list_flush(WalkList &l, WalkQuads *quads, int count, bool all,
+                                          float2 e2, WalkBodies<K> &wb)
+{
+    const int lane = threadIdx.x & 31;
+    const int full = all ? (count + 7) & ~7 : count & ~7, rest = all ? 0 : count - full;
+    if (all && count + lane < full) {
+        list_put(l, count + lane, 1.0e18f, 1.0e18f, 1.0e18f, 0.f);
+        if (QUAD)
+            for (int c = 0; c < 6; ++c)
+                reinterpret_cast<float *>(&quads->q[(count + lane) >> 1][c >> 1])
+                    [2 * (c & 1) + ((count + lane) & 1)] = 0.f;
+    }
+    __syncwarp();
+    list_eval<ZERO_SOFT, QUAD, K>(l, quads, full / 2, e2, wb);
+    __syncwarp();
+    if (full > 0 && lane < (rest + 1) / 2) {  // full is even: whole pairs move
+        l.a[lane] = l.a[full / 2 + lane];
+        l.b[lane] = l.b[full / 2 + lane];
+        if (QUAD)
+            for (int c = 0; c < 3; ++c) quads->q[lane][c] = quads->q[full / 2 + lane][c];
+    }
+    __syncwarp();
+    return rest;
+}
+
+__device__ __forceinline__ float warp_min(float v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float warp_max(float v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// The boxes of the CTA's 32-body chunks.
+template <int K>
+struct WalkBoxes {
+    float mn[K][3], mx[K][3];
+};
+// Bounds of the squared distance from a point to the nearest body: the distance
+// to the nearest box, and that to the farthest point of the nearest face of a
+// box (on each face of a box lies one of its bodies).
+template <int K>
+__device__ __forceinline__ void box_distances(const WalkBoxes<K> &b, const float (&c)[3],
+                                              float &least, float &most)
+{
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        float out[3], face[3], far[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float lo = b.mn[k][d] - c[d], hi = c[d] - b.mx[k][d];
+            out[d] = fmaxf(0.f, fmaxf(lo, hi));
+            face[d] = fminf(fabsf(lo), fabsf(hi));
+            far[d] = fmaxf(fabsf(lo), fabsf(hi));
+        }
+        const float near2 = fmaf(out[2], out[2], fmaf(out[1], out[1], out[0] * out[0]));
+        const float xy = fmaf(far[1], far[1], far[0] * far[0]);
+        const float fx = fmaf(far[2], far[2], fmaf(far[1], far[1], face[0] * face[0]));
+        const float fy = fmaf(far[2], far[2], fmaf(face[1], face[1], far[0] * far[0]));
+        const float fz = fmaf(face[2], face[2], xy);
+        const float face2 = fminf(fx, fminf(fy, fz));
+        least = k == 0 ? near2 : fminf(least, near2);
+        most = k == 0 ? face2 : fminf(most, face2);
+    }
+}
+// toward_body for the CTA's bodies by their boxes: whether some body may lie on
+// the node's side of its parent's centre, and whether all of a chunk's do.
+template <int K>
+__device__ __forceinline__ void toward_boxes(const WalkBoxes<K> &b, float4 pc, bool &some,
+                                             bool &all)
+{
+    const int oct = __float_as_int(pc.w);
+    const float p[3] = {pc.x, pc.y, pc.z};
+    some = all = false;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        bool may = oct < 8, must = oct < 8;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const bool high = (oct >> d & 1) != 0;
+            may = may && (high ? b.mx[k][d] >= p[d] : b.mn[k][d] < p[d]);
+            must = must && (high ? b.mn[k][d] >= p[d] : b.mx[k][d] < p[d]);
+        }
+        some = some || may;
+        all = all || must;
+    }
+}
+
 template <bool ZERO_SOFT, bool QUAD, int NP, bool DIR>
-__global__ void __launch_bounds__(kGroupBlock)
+__global__ void __maxnreg__(QUAD || NP > 1 ? 128 : DIR ? 64 : 80)
 group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restrict__ gnk,
                   const int *__restrict__ total, const float4 *__restrict__ body,
                   const uint32_t *__restrict__ order, int n, float theta2, float eps2, double G,
@@ -1285,155 +1493,241 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
                   BHStats *__restrict__ stats, const float4 *__restrict__ gquad,
                   const float4 *__restrict__ gpcen)
 {
-    __shared__ BHGNode s_rec[kWalkWarps][8];
-    __shared__ float4 s_quad[kWalkWarps][QUAD ? 16 : 1];
-    __shared__ float4 s_pc[kWalkWarps][DIR ? 8 : 1];
-    __shared__ int2 s_stack[kWalkWarps][kGroupStack];
-    constexpr int kPer = 64 * NP;  // bodies per warp
+    extern __shared__ __align__(16) unsigned char walk_shared[];
+    using Shared = WalkShared<QUAD>;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
+    __shared__ int s_push[kWalkWarps];  // groups pushed in this round
+    Shared &sh = reinterpret_cast<Shared *>(walk_shared)[w];
+    int *s_first = reinterpret_cast<int *>(reinterpret_cast<Shared *>(walk_shared) + W);
+    unsigned char *s_kids = reinterpret_cast<unsigned char *>(s_first + W * kWalkStack);
+    constexpr int K = 2 * NP;
     const int num_nodes = *total;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int w0 = ((blockIdx.x * kGroupBlock + threadIdx.x) >> 5) * kPer;
-    if (w0 >= n) return;  // whole warp past the end
-    const int wend = min(n, w0 + kPer);  // the warp's bodies: [w0, wend)
-    int ia[NP], ib[NP];
-    bool va[NP], vb[NP];
-    float2 npx[NP], npy[NP], npz[NP], fx[NP], fy[NP], fz[NP];
+    const int w0 = blockIdx.x * 32 * K;
+    const int wend = min(n, w0 + 32 * K);  // the CTA's bodies: [w0, wend)
+    const float2 e2 = dup2(eps2);
+
+    WalkBodies<K> wb;
+    WalkBoxes<K> box;
+    float p[K][3];
 #pragma unroll
-    for (int k = 0; k < NP; ++k) {
-        ia[k] = w0 + 64 * k + lane;
-        ib[k] = ia[k] + 32;
-        va[k] = ia[k] < n;
-        vb[k] = ib[k] < n;
+    for (int k = 0; k < K; ++k) {
         // a slot past n walks with body w0: its tests repeat that body's
-        const float4 pa = body[va[k] ? ia[k] : w0], pb = body[vb[k] ? ib[k] : w0];
-        npx[k] = make_float2(-pa.x, -pb.x);
-        npy[k] = make_float2(-pa.y, -pb.y);
-        npz[k] = make_float2(-pa.z, -pb.z);
-        fx[k] = fy[k] = fz[k] = dup2(0.f);
+        const int i = w0 + 32 * k + lane;
+        const float4 q = body[i < n ? i : w0];
+        p[k][0] = q.x; p[k][1] = q.y; p[k][2] = q.z;
+        wb.nx[k] = dup2(-q.x); wb.ny[k] = dup2(-q.y); wb.nz[k] = dup2(-q.z);
+        wb.fx[k] = wb.fy[k] = wb.fz[k] = dup2(0.f);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            box.mn[k][d] = warp_min(p[k][d]);
+            box.mx[k][d] = warp_max(p[k][d]);
+        }
     }
-    const float2 e2 = dup2(eps2), t2 = dup2(theta2);
+
     unsigned m2p = 0, p2p = 0;
+    int count = 0, bcount = 0;  // list entries (bcount: the body list, QUAD only)
     int sp = 1;
-    if (lane == 0) s_stack[w][0] = make_int2(0, 1);
+    if (threadIdx.x == 0) {
+        s_first[0] = 0;
+        s_kids[0] = 1;
+    }
     while (sp > 0) {
-        __syncwarp();
-        const int2 g = s_stack[w][--sp];
-        if (!NB_IN_RANGE(g.x + g.y - 1, num_nodes)) break;
-        int mynk = 0;
-        if (lane < g.y) {
-            s_rec[w][lane] = gnodes[g.x + lane];
-            mynk = gnk[g.x + lane];
-            if (DIR) s_pc[w][lane] = gpcen[g.x + lane];
+        __syncthreads();
+        // one node per lane: child lane & 7 of the warp's group lane >> 3
+        const int e = sp - 1 - (w + W * (lane >> 3));
+        const int kids = e >= 0 ? s_kids[e] : 0;
+        const bool have = (lane & 7) < kids;
+        const int id = have ? s_first[e] + (lane & 7) : 0;
+        sp = max(0, sp - 4 * W);
+        const BHGNode nd = gnodes[NB_IN_RANGE(id, num_nodes) ? id : 0];
+        const float c[3] = {nd.com_mass.x, nd.com_mass.y, nd.com_mass.z};
+        float least, most;
+        box_distances(box, c, least, most);
+        // a node that holds one of the CTA's bodies is opened (each body's own cell)
+        bool open = nd.first < wend && nd.first + nd.count > w0;
+        open = open || nd.size2 >= theta2 * most;
+        bool closed = !open && nd.size2 < theta2 * least;
+        float4 pc = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (DIR) {
+            pc = gpcen[id];
+            bool some, all;
+            toward_boxes(box, pc, some, all);
+            open = open || all;
+            closed = closed && !some;
         }
-        if (QUAD && lane < 2 * g.y) s_quad[w][lane] = gquad[2 * g.x + lane];
-        __syncwarp();
-        for (int c = 0; c < g.y; ++c) {
-            const BHGNode nd = s_rec[w][c];
-            const float4 pc = DIR ? s_pc[w][c] : make_float4(0.f, 0.f, 0.f, 0.f);
-            float2 dx[NP], dy[NP], dz[NP], d2[NP];
-            // a node that holds one of the warp's bodies is opened (each body's
-            // own cell); the others by the opening test of any body
-            bool open = nd.first < wend && nd.first + nd.count > w0;
+        // the undecided ones by every body
+        unsigned undecided = __ballot_sync(0xffffffffu, have && !open && !closed);
+        if (undecided) {
+            sh.test[lane] = make_float4(c[0], c[1], c[2], nd.size2);
+            if (DIR) sh.side[lane] = pc;
+            __syncwarp();
+            while (undecided) {  // two at a time
+                const int q0 = __ffs(undecided) - 1;
+                undecided &= undecided - 1u;
+                const int q1 = undecided ? __ffs(undecided) - 1 : q0;
+                undecided &= undecided - 1u;
+                const float4 t0 = sh.test[q0], t1 = sh.test[q1];
+                bool any0 = false, any1 = false;
 #pragma unroll
-            for (int k = 0; k < NP; ++k) {
-                dx[k] = add2(dup2(nd.com_mass.x), npx[k]);
-                dy[k] = add2(dup2(nd.com_mass.y), npy[k]);
-                dz[k] = add2(dup2(nd.com_mass.z), npz[k]);
-                d2[k] = fma2(dz[k], dz[k], fma2(dy[k], dy[k], mul2(dx[k], dx[k])));
-                const float2 td2 = mul2(t2, d2[k]);
-                open = open | (nd.size2 >= td2.x) | (nd.size2 >= td2.y);
-                if (DIR)
-                    open = open | toward_body(pc, -npx[k].x, -npy[k].x, -npz[k].x) |
-                           toward_body(pc, -npx[k].y, -npy[k].y, -npz[k].y);
+                for (int k = 0; k < K; ++k) {
+                    const float dx0 = t0.x - p[k][0], dx1 = t1.x - p[k][0];
+                    const float dy0 = t0.y - p[k][1], dy1 = t1.y - p[k][1];
+                    const float dz0 = t0.z - p[k][2], dz1 = t1.z - p[k][2];
+                    any0 |= t0.w >= theta2 * fmaf(dz0, dz0, fmaf(dy0, dy0, dx0 * dx0));
+                    any1 |= t1.w >= theta2 * fmaf(dz1, dz1, fmaf(dy1, dy1, dx1 * dx1));
+                }
+                if (DIR) {
+                    const float4 c0 = sh.side[q0], c1 = sh.side[q1];
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        any0 |= toward_body(c0, p[k][0], p[k][1], p[k][2]);
+                        any1 |= toward_body(c1, p[k][0], p[k][1], p[k][2]);
+                    }
+                }
+                any0 = __any_sync(0xffffffffu, any0);
+                any1 = __any_sync(0xffffffffu, any1);
+                if (lane == q0) open = any0;
+                if (lane == q1) open = any1;
             }
-            if (__any_sync(0xffffffffu, open)) {
-                if (nd.kids >= 0) {  // internal: its children's group, later
-                    const int nk = __shfl_sync(0xffffffffu, mynk, c);
-                    if (NB_IN_RANGE(sp, kGroupStack) && sp < kGroupStack) {
-                        if (lane == 0) s_stack[w][sp] = make_int2(nd.kids, nk);
-                        ++sp;
-                    }
-                    continue;
-                }
-                const int e = NB_IN_RANGE(nd.first, n) && NB_IN_RANGE(nd.first + nd.count - 1, n)
-                                  ? nd.first + nd.count
-                                  : nd.first;
-#pragma unroll 2
-                for (int b = nd.first; b < e; ++b) {
-                    const float4 q = body[b];
+            __syncwarp();
+        }
+
+        // push the groups of the opened internal nodes
+        const bool inner = have && open && nd.kids >= 0;
+        const unsigned push = __ballot_sync(0xffffffffu, inner);
+        const unsigned below = (1u << lane) - 1u;
+        int top = sp;
+        if (W > 1) {
+            if (lane == 0) s_push[w] = __popc(push);
+            __syncthreads();  // every warp has read its groups, too
+            for (int v = 0; v < W; ++v) {
+                if (v < w) top += s_push[v];
+                sp += s_push[v];
+            }
+        } else {
+            __syncwarp();
+            sp += __popc(push);
+        }
+        if (inner) {
+            const int to = top + __popc(push & below);
+            if (NB_IN_RANGE(to, W * kWalkStack)) {
+                s_first[to] = nd.kids;
+                s_kids[to] = gnk[id];
+            }
+        }
+
+        // closed nodes to the list
+        const bool add = have && !open;
+        const unsigned adds = __ballot_sync(0xffffffffu, add);
+        if (add) {
+            const int to = count + __popc(adds & below);
+            list_put(sh.list, to, c[0], c[1], c[2], nd.com_mass.w);
+            if constexpr (QUAD) {
+                const float4 q0 = gquad[2 * id], q1 = gquad[2 * id + 1];
+                const float v[6] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
 #pragma unroll
-                    for (int k = 0; k < NP; ++k) {
-                        const float2 rx = add2(dup2(q.x), npx[k]);
-                        const float2 ry = add2(dup2(q.y), npy[k]);
-                        const float2 rz = add2(dup2(q.z), npz[k]);
-                        const float2 r2 = fma2(rz, rz, fma2(ry, ry, fma2(rx, rx, e2)));
-                        float2 inv = make_float2(rsqrt_mufu(r2.x), rsqrt_mufu(r2.y));
-                        if (ZERO_SOFT) {
-                            inv.x = r2.x > 0.f ? inv.x : 0.f;
-                            inv.y = r2.y > 0.f ? inv.y : 0.f;
-                        }
-                        const float2 s = mul2(mul2(dup2(q.w), inv), mul2(inv, inv));
-                        fx[k] = fma2(rx, s, fx[k]);
-                        fy[k] = fma2(ry, s, fy[k]);
-                        fz[k] = fma2(rz, s, fz[k]);
-                    }
-                }
-                p2p += nd.count;
+                for (int d = 0; d < 6; ++d)
+                    reinterpret_cast<float *>(&sh.quads.q[to >> 1][d >> 1])
+                        [2 * (d & 1) + (to & 1)] = v[d];
+            }
+        }
+        count += __popc(adds);
+        m2p += __popc(adds);
+        if constexpr (QUAD) {
+            if (count >= kListFlush)
+                count = list_flush<ZERO_SOFT, true, K>(sh.list, &sh.quads, count, false, e2, wb);
+        } else if (count >= kListFlush) {
+            count = list_flush<ZERO_SOFT, false, K>(sh.list, nullptr, count, false, e2, wb);
+        }
+
+        // the bodies of opened leaves: entry t of the batch's leaf bodies lies in
+        // the leaf whose range of the running count holds t
+        const int lc = have && open && nd.kids < 0 ? nd.count : 0;
+        int lincl = lc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, lincl, o);
+            if (lane >= o) lincl += t;
+        }
+        const int leaf_bodies = __shfl_sync(0xffffffffu, lincl, 31);
+        p2p += leaf_bodies;
+        for (int t0 = 0; t0 < leaf_bodies; t0 += 32) {
+            const int t = t0 + lane;
+            int leaf = 0;  // the number of lanes whose running count is at most t
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int v = __shfl_sync(0xffffffffu, lincl, leaf + o - 1);
+                if (v <= t) leaf += o;
+            }
+            const int b0 = __shfl_sync(0xffffffffu, nd.first + lc - lincl, leaf & 31);
+            const bool put = t < leaf_bodies;
+            WalkList *list = &sh.list;
+            int at = count;
+            if constexpr (QUAD) {
+                list = &sh.bodies;
+                at = bcount;
+            }
+            if (put && NB_IN_RANGE(b0 + t, n)) {
+                const float4 q = body[b0 + t];
+                list_put(*list, at + lane, q.x, q.y, q.z, q.w);
+            }
+            const int got = min(32, leaf_bodies - t0);
+            if constexpr (QUAD) {
+                bcount += got;
+                if (bcount >= kListFlush)
+                    bcount = list_flush<ZERO_SOFT, false, K>(sh.bodies, nullptr, bcount, false, e2,
+                                                          wb);
             } else {
-                float4 q0, q1;
-                if (QUAD) {
-                    q0 = s_quad[w][2 * c];
-                    q1 = s_quad[w][2 * c + 1];
-                }
-#pragma unroll
-                for (int k = 0; k < NP; ++k) {
-                    const float2 r2 = add2(d2[k], e2);
-                    const float2 inv = make_float2(rsqrt_mufu(r2.x), rsqrt_mufu(r2.y));
-                    const float2 inv2 = mul2(inv, inv);
-                    const float2 s = mul2(mul2(dup2(nd.com_mass.w), inv), inv2);
-                    fx[k] = fma2(dx[k], s, fx[k]);
-                    fy[k] = fma2(dy[k], s, fy[k]);
-                    fz[k] = fma2(dz[k], s, fz[k]);
-                    if (QUAD) {
-                        const float2 qx = fma2(dup2(q0.x), dx[k],
-                                               fma2(dup2(q0.w), dy[k], mul2(dup2(q1.x), dz[k])));
-                        const float2 qy = fma2(dup2(q0.w), dx[k],
-                                               fma2(dup2(q0.y), dy[k], mul2(dup2(q1.y), dz[k])));
-                        const float2 qz = fma2(dup2(q1.x), dx[k],
-                                               fma2(dup2(q1.y), dy[k], mul2(dup2(q0.z), dz[k])));
-                        const float2 rqr = fma2(dx[k], qx, fma2(dy[k], qy, mul2(dz[k], qz)));
-                        const float2 inv5 = mul2(mul2(inv, inv2), inv2);
-                        const float2 f = mul2(mul2(dup2(2.5f), rqr), inv2);
-                        fx[k] = fma2(inv5, fma2(f, dx[k], make_float2(-qx.x, -qx.y)), fx[k]);
-                        fy[k] = fma2(inv5, fma2(f, dy[k], make_float2(-qy.x, -qy.y)), fy[k]);
-                        fz[k] = fma2(inv5, fma2(f, dz[k], make_float2(-qz.x, -qz.y)), fz[k]);
-                    }
-                }
-                ++m2p;
+                count += got;
+                if (count >= kListFlush)
+                    count = list_flush<ZERO_SOFT, false, K>(sh.list, nullptr, count, false, e2, wb);
             }
         }
+        __syncwarp();
     }
-    unsigned nv = 0;
-#pragma unroll
-    for (int k = 0; k < NP; ++k) {
-        if (va[k]) {
-            const uint32_t o = order[ia[k]];
-            ax[o] = G * (double)fx[k].x;
-            ay[o] = G * (double)fy[k].x;
-            az[o] = G * (double)fz[k].x;
-        }
-        if (vb[k]) {
-            const uint32_t o = order[ib[k]];
-            ax[o] = G * (double)fx[k].y;
-            ay[o] = G * (double)fy[k].y;
-            az[o] = G * (double)fz[k].y;
-        }
-        nv += __popc(__ballot_sync(0xffffffffu, va[k])) + __popc(__ballot_sync(0xffffffffu, vb[k]));
+    if constexpr (QUAD) {
+        list_flush<ZERO_SOFT, true, K>(sh.list, &sh.quads, count, true, e2, wb);
+        list_flush<ZERO_SOFT, false, K>(sh.bodies, nullptr, bcount, true, e2, wb);
+    } else {
+        list_flush<ZERO_SOFT, false, K>(sh.list, nullptr, count, true, e2, wb);
     }
+
     if (lane == 0) {
-        atomicAdd(&stats->m2p, (unsigned long long)m2p * nv);
-        atomicAdd(&stats->p2p, (unsigned long long)p2p * nv);
-        atomicAdd(&stats->total, (unsigned long long)(m2p + p2p) * nv);
+        const unsigned long long nv = wend - w0;
+        atomicAdd(&stats->m2p, m2p * nv);
+        atomicAdd(&stats->p2p, p2p * nv);
+        atomicAdd(&stats->total, (m2p + p2p) * nv);
+    }
+    double f[K][3];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        f[k][0] = (double)wb.fx[k].x + (double)wb.fx[k].y;
+        f[k][1] = (double)wb.fy[k].x + (double)wb.fy[k].y;
+        f[k][2] = (double)wb.fz[k].x + (double)wb.fz[k].y;
+    }
+    if (W > 1) {
+        __syncthreads();  // every warp is done with its lists
+        double *part = reinterpret_cast<double *>(walk_shared);  // [W][3 K][32]
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) part[(w * 3 * K + 3 * k + d) * 32 + lane] = f[k][d];
+        __syncthreads();
+        if (w > 0) return;
+        for (int v = 1; v < W; ++v)
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) f[k][d] += part[(v * 3 * K + 3 * k + d) * 32 + lane];
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = w0 + 32 * k + lane;
+        if (i >= n) continue;
+        const uint32_t o = order[i];
+        ax[o] = G * f[k][0];
+        ay[o] = G * f[k][1];
+        az[o] = G * f[k][2];
     }
 }
 
@@ -1660,7 +1954,34 @@ nb_status bh_hilbert_order(BHTree *t, const double *x, const double *y, const do
     return NB_OK;
 }
 
-// Packed body pairs per lane of the walk (0: the one-body-per-lane walk);
+// Warps that share the walk of one CTA's bodies: doubled while there are no more
+// than 110 per SM, up to 8.  Fewer CTAs than fill the chip leave it to the longest
+// walks, which more warps shorten; with enough CTAs the rounds' barriers and the
+// shorter lists only cost.  A whole force evaluation took, with 1 / 2 / 4 / 8 / 16
+// warps (theta 0.5, disk galaxy), in us:
+//   n =    16,384    501 /  402 /  335 /  303 /  300
+//   n =   100,000    598 /  511 /  463 /  459 /  522
+//   n =   262,144    999 /  928 /  881 /  913 / 1111
+//   n =   524,288   1380 / 1347 / 1364 / 1479 / 1887
+//   n = 1,048,576   2368 / 2395 / 2501 / 2725 / 3606
+// The reference's rule opens far more for some bodies than for others (the longest
+// walk at n = 100,000 has 20,270 interactions, the mean 3,891), so three times as
+// many, up to 16:
+//   n =   100,000   3141 / 1925 / 1196 /  922 /  830
+//   n =   400,000   7618 / 4921 / 3417 / 2928 / 3036
+// Quadrupoles hold more registers, so half as many:
+//   n =   100,000    766 /  726 /  665 /  685 /  806
+//   n =   500,000   2132 / 2169 / 2324 / 2666 / 3400
+template <bool Q, bool D>
+int walk_warps(int ctas)
+{
+    const long sought = (Q ? 55L : 110L) * (D ? 3 : 1) * device_props().num_sms;
+    int w = 1;
+    while (w < (D ? kWalkWarps : kWalkWarps / 2) && 2L * w * ctas <= sought) w *= 2;
+    return w;
+}
+
+// Body pairs per lane of the walk (0: the one-body-per-lane preorder walk);
 // NB_BH_WALK_PAIRS overrides the default.
 int walk_pairs()
 {
@@ -1690,14 +2011,14 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
         const BHGNode *gn = t->gnodes.as<BHGNode>();
         const unsigned char *gk = t->gnk.as<unsigned char>();
         const float4 *gq = t->gquad.as<float4>(), *gp = t->gpcen.as<float4>();
-        if (np == 2)
-            group_walk_kernel<ZS, Q, 2, D><<<div_up(n, 4 * kGroupBlock), kGroupBlock, 0, st>>>(
-                gn, gk, d_total(t), t->body.as<float4>(), t->order, n, theta2, eps2, G, ax, ay,
-                az, t->stats.as<BHStats>(), gq, gp);
-        else
-            group_walk_kernel<ZS, Q, 1, D><<<div_up(n, 2 * kGroupBlock), kGroupBlock, 0, st>>>(
-                gn, gk, d_total(t), t->body.as<float4>(), t->order, n, theta2, eps2, G, ax, ay,
-                az, t->stats.as<BHStats>(), gq, gp);
+        const int ctas = div_up(n, 64 * np), warps = walk_warps<Q, D>(ctas);
+        auto *kernel = np == 2 ? group_walk_kernel<ZS, Q, 2, D> : group_walk_kernel<ZS, Q, 1, D>;
+        const size_t shared = walk_shared_bytes<Q>(warps);
+        if (shared > 48 * 1024 - 256)
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        kernel<<<ctas, 32 * warps, shared, st>>>(
+            gn, gk, d_total(t), t->body.as<float4>(), t->order, n, theta2, eps2, G, ax, ay, az,
+            t->stats.as<BHStats>(), gq, gp);
     } else if (np == 2)
         walk2_kernel<ZS, Q, 2, D><<<div_up(n, 4 * kWalkBlock), kWalkBlock, 0, st>>>(
             t->nodes.as<BHNode>(), d_total(t), t->body.as<float4>(), t->order, n, theta2,
