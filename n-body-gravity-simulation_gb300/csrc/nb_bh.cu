@@ -72,7 +72,9 @@ struct BHRoot {
     double off[kMaxLevels];         // child-centre offset below depth l: size * 2^-(l+2)
     float size2[kMaxLevels + 1];    // squared side of a depth-d cell (opening test)
     int levels;                     // depths the root may split into (<= 21)
-    int pad;
+    float margin;                   // encode_kernel: distance from a grid line, in cells
+    double scale;                   // 2^21 / size
+    double lo[3], lo_scaled[3];     // the cube's lower corner, and that times scale
 };
 
 // A leaf is the node whose skip pointer is the next node (no subtree).
@@ -94,7 +96,7 @@ struct BHStats {
 // ------------------------------------------------------------ bounding box
 __global__ void __launch_bounds__(256)
 bbox_partial_kernel(const double *__restrict__ x, const double *__restrict__ y,
-                    const double *__restrict__ z, int n, double *__restrict__ part)
+                    const double *__restrict__ z, int n, long long *__restrict__ part)
 {
     constexpr long long kMax = 0x7fffffffffffffffll, kMin = -kMax - 1;
     __shared__ long long sh[6][8];
@@ -140,62 +142,85 @@ bbox_partial_kernel(const double *__restrict__ x, const double *__restrict__ y,
         const int c = threadIdx.x;
         long long r = sh[c][0];
         for (int w = 1; w < 8; ++w) r = c < 3 ? min(r, sh[c][w]) : max(r, sh[c][w]);
-        // a block that saw only NaN (or nothing) reports the neutral value
-        const bool empty = r == (c < 3 ? kMax : kMin);
-        part[blockIdx.x * 6 + c] = empty ? (c < 3 ? 1e308 : -1e308) : key_value(r);
+        part[blockIdx.x * 6 + c] = r;  // the neutral key if it saw only NaN (or nothing)
     }
 }
 
-// One block: reduce the partials, then thread 0 derives the root cube by the
+// One block: reduce the partials' keys, then one warp derives the root cube by the
 // CPU tree's rule (force_calculator_barnes_hut_optimized.cpp:112-124,
-// std::max(a,b) = a<b?b:a).  Min and max are exact, so the order of the
-// reduction does not matter.
+// std::max(a,b) = a<b?b:a), a lane per level: halving is exact, so size * 2^-l is
+// the side after l halvings.  Min and max are exact, so the order of the
+// reduction does not matter.  What encode_kernel's blocks share of the cube is
+// derived here, once.  Latency alone: FP64 min/max in shared memory and one thread
+// for the 21 levels took 10.4 us.
 __global__ void __launch_bounds__(256)
-bbox_final_kernel(const double *__restrict__ part, int nparts, BHRoot *root)
+bbox_final_kernel(const long long *__restrict__ part, int nparts, BHRoot *root)
 {
-    __shared__ double sh[6][256];
-    double v[6] = {1e308, 1e308, 1e308, -1e308, -1e308, -1e308};
-    for (int b = threadIdx.x; b < nparts; b += 256) {
-        for (int k = 0; k < 3; ++k) v[k] = fmin(v[k], part[b * 6 + k]);
-        for (int k = 3; k < 6; ++k) v[k] = fmax(v[k], part[b * 6 + k]);
-    }
-    for (int k = 0; k < 6; ++k) sh[k][threadIdx.x] = v[k];
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            for (int k = 0; k < 3; ++k)
-                sh[k][threadIdx.x] = fmin(sh[k][threadIdx.x], sh[k][threadIdx.x + w]);
-            for (int k = 3; k < 6; ++k)
-                sh[k][threadIdx.x] = fmax(sh[k][threadIdx.x], sh[k][threadIdx.x + w]);
+    __shared__ long long sh[6][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long v[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = order_key(k < 3 ? 1e308 : -1e308, 0);
+    for (int b = threadIdx.x; b < nparts; b += 256)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            v[k] = min(v[k], part[b * 6 + k]);
+            v[k + 3] = max(v[k + 3], part[b * 6 + k + 3]);
         }
-        __syncthreads();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            v[k] = min(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+            v[k + 3] = max(v[k + 3], __shfl_xor_sync(0xffffffffu, v[k + 3], o));
+        }
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) sh[k][warp] = v[k];
+    __syncthreads();
+    if (warp > 0) return;
+    double e[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        long long r = sh[k][0];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) r = k < 3 ? min(r, sh[k][w]) : max(r, sh[k][w]);
+        e[k] = key_value(r);
     }
-    if (threadIdx.x != 0) return;
-    for (int k = 0; k < 6; ++k) v[k] = sh[k][0];
-    const double ex = v[3] - v[0], ey = v[4] - v[1], ez = v[5] - v[2];
+    const double ex = e[3] - e[0], ey = e[4] - e[1], ez = e[5] - e[2];
     const double eyz = (ey < ez) ? ez : ey;
-    double size = ((ex < eyz) ? eyz : ex) + 1e-9;
-    root->cx = (v[0] + v[3]) / 2;
-    root->cy = (v[1] + v[4]) / 2;
-    root->cz = (v[2] + v[5]) / 2;
+    const double size = ((ex < eyz) ? eyz : ex) + 1e-9;
+    if (lane <= kMaxLevels) {
+        const double side = size * double_of((long long)(1023 - lane) << 52);
+        root->size2[lane] = (float)(side * side);
+        if (lane < kMaxLevels) root->off[lane] = side / 4.0;
+        // levels: halvings until the half falls below 1e-9
+        const bool splits = lane < kMaxLevels && !(side / 2.0 < 1e-9);
+        const unsigned vote = __ballot_sync((2u << kMaxLevels) - 1u, splits);
+        if (lane == 0) root->levels = __ffs(~vote) - 1;
+    }
+    const double scale = 2097152.0 / size;
+    double cmax = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double c = (e[k] + e[k + 3]) / 2, lo = c - size / 2;
+        cmax = fmax(cmax, fabs(c));
+        if (lane == k) {
+            (&root->cx)[k] = c;
+            root->lo[k] = lo;
+            root->lo_scaled[k] = lo * scale;
+        }
+    }
+    if (lane != 0) return;
     root->size = size;
-    int lv = 0;
-    double s = size;
-    while (lv < kMaxLevels) {
-        const double half = s / 2.0;
-        if (half < 1e-9) break;
-        s = half;
-        ++lv;
-    }
-    root->levels = lv;
-    s = size;
-    for (int l = 0; l < kMaxLevels; ++l) {
-        root->size2[l] = (float)(s * s);
-        const double half = s / 2.0;
-        root->off[l] = half / 2.0;
-        s = half;
-    }
-    root->size2[kMaxLevels] = (float)(s * s);
+    root->scale = scale;
+    // Running centres accumulate at most 21 roundings of half an ulp of
+    // |centre| <= cmax + size; the fast index adds a few more roundings
+    // (of |p| * scale and of lo * scale: 2^-52 (cmax + size) scale each).
+    // Positions farther than this from every grid line index exactly.
+    const double u_c = ldexp(1.0, ilogb(cmax + size) - 52);
+    const double u_s = ldexp(1.0, ilogb(size) - 52);
+    root->margin = (float)((32.0 * u_c + 4.0 * u_s) * scale + 1e-6);
 }
 
 // ------------------------------------------------------------ Morton encode
@@ -221,37 +246,16 @@ encode_kernel(const double *__restrict__ x, const double *__restrict__ y,
               const double *__restrict__ z, int n, const BHRoot *__restrict__ root,
               uint64_t *__restrict__ keys, uint32_t *__restrict__ vals)
 {
-    __shared__ double off[kMaxLevels];
-    __shared__ double c0[3], lo_scaled[3], scale;
-    __shared__ float margin;
-    __shared__ int levels;
-    if (threadIdx.x < kMaxLevels) off[threadIdx.x] = root->off[threadIdx.x];
-    if (threadIdx.x == 0) {
-        c0[0] = root->cx; c0[1] = root->cy; c0[2] = root->cz;
-        levels = root->levels;
-        const double size = root->size;
-        scale = 2097152.0 / size;
-        double cmax = 0.0;
-        for (int k = 0; k < 3; ++k) {
-            lo_scaled[k] = (c0[k] - size / 2) * scale;
-            cmax = fmax(cmax, fabs(c0[k]));
-        }
-        // Running centres accumulate at most 21 roundings of half an ulp of
-        // |centre| <= cmax + size; the fast index adds a few more roundings
-        // (of |p| * scale and of lo * scale: 2^-52 (cmax + size) scale each).
-        // Positions farther than this from every grid line index exactly.
-        const double u_c = ldexp(1.0, ilogb(cmax + size) - 52);
-        const double u_s = ldexp(1.0, ilogb(size) - 52);
-        margin = (float)((32.0 * u_c + 4.0 * u_s) * scale + 1e-6);
-    }
-    __syncthreads();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
+    const double scale = root->scale;
+    const float margin = root->margin;
+    const int levels = root->levels;
     const double px = x[i], py = y[i], pz = z[i];
     uint64_t qx, qy, qz;
-    const bool okx = grid_index(px, lo_scaled[0], scale, margin, &qx);
-    const bool oky = grid_index(py, lo_scaled[1], scale, margin, &qy);
-    const bool okz = grid_index(pz, lo_scaled[2], scale, margin, &qz);
+    const bool okx = grid_index(px, root->lo_scaled[0], scale, margin, &qx);
+    const bool oky = grid_index(py, root->lo_scaled[1], scale, margin, &qy);
+    const bool okz = grid_index(pz, root->lo_scaled[2], scale, margin, &qz);
     if (okx && oky && okz) {
         uint64_t code = (spread21(qx) << 2) | (spread21(qy) << 1) | spread21(qz);
         const int drop = 3 * (kMaxLevels - levels);  // digits below the split limit are 0
@@ -262,14 +266,14 @@ encode_kernel(const double *__restrict__ x, const double *__restrict__ y,
         return;
     }
     // Exact path: the CPU tree's own comparisons and child-centre additions.
-    double cx = c0[0], cy = c0[1], cz = c0[2];
+    double cx = root->cx, cy = root->cy, cz = root->cz;
     uint64_t code = 0;
     for (int l = 0; l < kMaxLevels; ++l) {
         uint64_t d = 0;
         if (l < levels) {
             const bool bx = px >= cx, by = py >= cy, bz = pz >= cz;
             d = ((uint64_t)bx << 2) | ((uint64_t)by << 1) | (uint64_t)bz;
-            const double o = off[l];
+            const double o = root->off[l];
             cx = __dadd_rn(cx, bx ? o : -o);
             cy = __dadd_rn(cy, by ? o : -o);
             cz = __dadd_rn(cz, bz ? o : -o);
@@ -290,12 +294,12 @@ hilbert_kernel(const double *__restrict__ x, const double *__restrict__ y,
 {
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
-    const double size = root->size, scale = 1024.0 / size;
-    const double p[3] = {x[i], y[i], z[i]}, c[3] = {root->cx, root->cy, root->cz};
+    const double scale = root->scale * (1.0 / 2048);  // 1024 / size
+    const double p[3] = {x[i], y[i], z[i]};
     uint32_t g[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double f = floor((p[k] - (c[k] - size / 2)) * scale);
+        const double f = floor((p[k] - root->lo[k]) * scale);
         g[k] = (uint32_t)fmin(fmax(f, 0.0), 1023.0);
     }
     keys[i] = (uint64_t)hilbert_index30(g[0], g[1], g[2]) << 33;
@@ -452,7 +456,7 @@ constexpr int kSortFusedTiles = 64;
 
 __global__ void __launch_bounds__(256)
 radix_hist_kernel(const uint64_t *__restrict__ keys, int n, int shift, int *__restrict__ counts,
-                  int num_tiles)
+                  int digit_stride, int tile_stride)
 {
     __shared__ int h[kSortWarps][256];
     const int warp = threadIdx.x >> 5;
@@ -466,7 +470,7 @@ radix_hist_kernel(const uint64_t *__restrict__ keys, int n, int shift, int *__re
     __syncthreads();
     int c = 0;
     for (int w = 0; w < kSortWarps; ++w) c += h[w][threadIdx.x];
-    counts[threadIdx.x * num_tiles + blockIdx.x] = c;
+    counts[threadIdx.x * digit_stride + blockIdx.x * tile_stride] = c;
 }
 
 // Stable scatter of one 8-bit digit.  Warp w of the block ranks keys
@@ -495,14 +499,26 @@ radix_scatter_kernel(const uint64_t *__restrict__ kin, const uint32_t *__restric
     __shared__ uint64_t skey[kSortTile];
     __shared__ uint32_t sval[kSortTile];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile0 = blockIdx.x * kSortTile;
+    const int base = tile0 + warp * 32 * kSortRounds;
+    uint64_t key[kSortRounds];
+    uint32_t val[kSortRounds];
+    int rank[kSortRounds], dig[kSortRounds];
+    // every load before the first barrier: one round trip to memory, not one per round
+#pragma unroll
+    for (int r = 0; r < kSortRounds; ++r) {
+        const int idx = base + r * 32 + lane;
+        key[r] = idx < n ? kin[idx] : 0ull;
+        val[r] = idx < n ? vin[idx] : 0u;
+    }
     for (int k = threadIdx.x; k < kSortWarps * 256; k += 256) (&wh[0][0])[k] = 0;
     if (offsets) {
         toff[threadIdx.x] = offsets[threadIdx.x * num_tiles + blockIdx.x];
     } else {
-        const int *row = counts + threadIdx.x * num_tiles;
         int before = 0, all = 0;
+#pragma unroll 16
         for (int tl = 0; tl < num_tiles; ++tl) {
-            const int c = row[tl];
+            const int c = counts[tl * 256 + threadIdx.x];
             all += c;
             if (tl < (int)blockIdx.x) before += c;
         }
@@ -510,17 +526,9 @@ radix_scatter_kernel(const uint64_t *__restrict__ kin, const uint32_t *__restric
         toff[threadIdx.x] = block_exclusive<int, kSortWarps>(all, dsum, &keys) + before;
     }
     __syncthreads();
-    const int tile0 = blockIdx.x * kSortTile;
-    const int base = tile0 + warp * 32 * kSortRounds;
-    uint64_t key[kSortRounds];
-    uint32_t val[kSortRounds];
-    int rank[kSortRounds], dig[kSortRounds];
 #pragma unroll
     for (int r = 0; r < kSortRounds; ++r) {
-        const int idx = base + r * 32 + lane;
-        const bool valid = idx < n;
-        key[r] = valid ? kin[idx] : 0ull;
-        val[r] = valid ? vin[idx] : 0u;
+        const bool valid = base + r * 32 + lane < n;
         const int d = valid ? (int)((key[r] >> shift) & 0xFF) : -1;
         const unsigned peers = __match_any_sync(0xffffffffu, d);
         const int before = __popc(peers & ((1u << lane) - 1u));
@@ -575,9 +583,9 @@ radix_scatter_kernel(const uint64_t *__restrict__ kin, const uint32_t *__restric
         kout[pos] = k;
         vout[pos] = sval[j];
         if (next_counts)
-            atomicAdd(&next_counts[(int)((k >> (shift + 8)) & 0xFF) * num_tiles + pos / kSortTile], 1);
+            atomicAdd(&next_counts[pos / kSortTile * 256 + (int)((k >> (shift + 8)) & 0xFF)], 1);
     }
-    if (zero_counts) zero_counts[threadIdx.x * num_tiles + blockIdx.x] = 0;
+    if (zero_counts) zero_counts[blockIdx.x * 256 + threadIdx.x] = 0;
 }
 
 // ------------------------------------------------------------ gather
@@ -614,14 +622,14 @@ gather2_kernel(const uint32_t *__restrict__ order, const double *__restrict__ x,
     mb[i] = D4{mm * rx * rz, mm * ry * rz, 0.0, 0.0};
 }
 
-// ------------------------------------------------------------ tree build
-// First index after i whose depth-d prefix differs from code[i]'s (galloping).
-__device__ __forceinline__ int cell_end(const uint64_t *__restrict__ c, int n, int i, int d)
+// One past the last body of the depth-d cell that contains bodies i .. from - 1.
+__device__ __forceinline__ int cell_end(const uint64_t *__restrict__ c, int n, int i, int d,
+                                        int from)
 {
     if (d == 0) return n;
     const int sh = 63 - 3 * d;
     const uint64_t p = c[i] >> sh;
-    int lo = i, hi, step = 1;
+    int lo = from - 1, hi, step = from - i;
     while (true) {
         hi = lo + step;
         if (hi >= n) {
@@ -665,6 +673,13 @@ __device__ __forceinline__ int cell_start(const uint64_t *__restrict__ c, int i,
     return hi;
 }
 
+// The depth down to which two codes lie in the same cell.
+__device__ __forceinline__ int common_levels(uint64_t a, uint64_t b)
+{
+    const uint64_t x = a ^ b;
+    return (x == 0 ? 63 : __clzll((long long)x) - 1) / 3;
+}
+
 // Depth of the first node starting at body i and the length of its chain
 // (0 when no node starts at i); pstart[i]: the first body of that node's
 // parent cell (when i starts a chain below the root).
@@ -678,27 +693,21 @@ chain_kernel(const uint64_t *__restrict__ c, int n, int cap, const BHRoot *__res
     int a = 0, L = 0;
     bool starts = true;
     if (i > 0) {
-        const uint64_t x = c[i] ^ c[i - 1];
-        const int common = x == 0 ? 63 : (__clzll((long long)x) - 1);
-        const int s = min(common / 3, levels);
+        const int s = min(common_levels(c[i], c[i - 1]), levels);
         if (s >= levels) {
             starts = false;
         } else {
             a = s + 1;
             const int ps = cell_start(c, i, s);
-            const int pc = cell_end(c, n, i, s) - ps;
-            starts = pc > cap;
+            starts = cap < n - ps && common_levels(c[ps + cap], c[i]) >= s;  // more than cap
             pstart[i] = ps;
         }
     }
     if (starts) {
-        int d = a;
-        while (true) {
-            const int cnt = cell_end(c, n, i, d) - i;
-            ++L;
-            if (cnt > cap && d < levels) ++d;
-            else break;
-        }
+        // the first depth from a on at which the cell holds cap bodies at most: body
+        // i + cap is in body i's cells down to the depth their codes share
+        const int t = cap < n - i ? common_levels(c[i], c[i + cap]) : -1;
+        L = min(levels, max(a, t + 1)) - a + 1;
     }
     chain_len[i] = L;
     chain_depth[i] = a;
@@ -757,23 +766,20 @@ node_kernel(const uint64_t *__restrict__ c, int n, int cap, const BHRoot *__rest
             BHStats *__restrict__ stats, int node_cap)
 {
     const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= n) return;
-    const int L = chain_len[i];
-    if (L == 0) return;
-    const int levels = root->levels;
-    const int a = chain_depth[i];
-    const int id0 = offsets[i];
-    int leaves = 0, maxd = 0;
-    for (int k = 0; k < L; ++k) {
+    const int L = i < n ? chain_len[i] : 0;
+    const int a = L > 0 ? chain_depth[i] : 0;
+    const int id0 = L > 0 ? offsets[i] : 0;
+    const D4 before = L > 0 ? P[i] : D4{0.0, 0.0, 0.0, 0.0};
+    int end = i + 1;
+    for (int k = L - 1; k >= 0; --k) {  // deepest first: each cell holds the one before
         const int d = a + k;
-        const int cnt = cell_end(c, n, i, d) - i;
-        const bool leaf = !(cnt > cap && d < levels);
-        if (!NB_IN_RANGE(id0 + k, node_cap) || !NB_IN_RANGE(i + cnt, n + 1)) break;
+        end = cell_end(c, n, i, d, end);
+        if (!NB_IN_RANGE(id0 + k, node_cap) || !NB_IN_RANGE(end, n + 1)) break;
         BHNode nd;
-        nd.com_mass = monopole(P[i], P[i + cnt]);
+        nd.com_mass = monopole(before, P[end]);
         nd.first = i;
-        nd.count = cnt;
-        nd.skip = offsets[i + cnt];
+        nd.count = end - i;
+        nd.skip = offsets[end];
         nd.size2 = root->size2[d];
         nodes[id0 + k] = nd;
         node_depth[id0 + k] = (unsigned char)d;
@@ -788,11 +794,14 @@ node_kernel(const uint64_t *__restrict__ c, int n, int cap, const BHRoot *__rest
             octant[id0 + k] = (unsigned char)oct;
             if (NB_IN_RANGE(par, node_cap)) kidflag[(size_t)par * 8 + oct] = 1;
         }
-        leaves += leaf;
-        maxd = max(maxd, d);
     }
-    if (leaves) atomicAdd(&stats->leaves, leaves);
-    atomicMax(&stats->max_depth, maxd);
+    // every chain ends in a leaf
+    const unsigned leaves = __popc(__ballot_sync(0xffffffffu, L > 0));
+    const int deepest = __reduce_max_sync(0xffffffffu, L > 0 ? a + L - 1 : 0);
+    if ((threadIdx.x & 31) == 0 && leaves > 0) {
+        atomicAdd(&stats->leaves, (int)leaves);
+        atomicMax(&stats->max_depth, deepest);
+    }
 }
 
 // Parent centres and octants of every node (parent_centre), for the walk
@@ -1643,6 +1652,7 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
         // the bodies of opened leaves: entry t of the batch's leaf bodies lies in
         // the leaf whose range of the running count holds t
         const int lc = have && open && nd.kids < 0 ? nd.count : 0;
+        if (!__any_sync(0xffffffffu, lc > 0)) continue;
         int lincl = lc;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1866,7 +1876,8 @@ static nb_status radix_passes(BHTree *t, int n, int first_shift, cudaStream_t st
         const bool last = shift + 8 >= 64;
         int *cur = fused ? cnt[p % 3] : cnt[0];
         if (!fused || p == 0) {
-            radix_hist_kernel<<<num_tiles, 256, 0, st>>>(kin, n, shift, cur, num_tiles);
+            radix_hist_kernel<<<num_tiles, 256, 0, st>>>(kin, n, shift, cur, direct ? 1 : num_tiles,
+                                                         direct ? 256 : 1);
             NB_LAUNCH_CHECK();
         }
         if (!direct) NB_TRY(scan_exclusive<int>(cur, 256 * num_tiles, digit_off, t->scan_tmp, st));
@@ -1890,14 +1901,14 @@ static nb_status morton_sort(BHTree *t, const double *x, const double *y, const 
                              int n, int first_shift, cudaStream_t st, bool hilbert = false)
 {
     const int nparts = std::min(div_up(n, 1024), 4 * device_props().num_sms);
-    NB_TRY(t->part.reserve(sizeof(double) * 6 * nparts));
+    NB_TRY(t->part.reserve(sizeof(long long) * 6 * nparts));
     NB_TRY(t->root.reserve(sizeof(BHRoot)));
     NB_TRY(reserve_sort(t, n));
     BHRoot *root = t->root.as<BHRoot>();
 
-    bbox_partial_kernel<<<nparts, 256, 0, st>>>(x, y, z, n, t->part.as<double>());
+    bbox_partial_kernel<<<nparts, 256, 0, st>>>(x, y, z, n, t->part.as<long long>());
     NB_LAUNCH_CHECK();
-    bbox_final_kernel<<<1, 256, 0, st>>>(t->part.as<double>(), nparts, root);
+    bbox_final_kernel<<<1, 256, 0, st>>>(t->part.as<long long>(), nparts, root);
     NB_LAUNCH_CHECK();
     if (hilbert)
         hilbert_kernel<<<div_up(n, 256), 256, 0, st>>>(x, y, z, n, root, t->keys0.as<uint64_t>(),
