@@ -33,6 +33,7 @@
 // segment count is chosen to fill whole waves.
 #include "nb_internal.h"
 #include "nb_fp64pair.cuh"
+#include "nb_after.cuh"
 #include "nb_tile.cuh"
 
 #include <algorithm>
@@ -129,41 +130,54 @@ direct_mixed_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo
     }
 }
 
-// a_i = G * sum_s (sum_s - comp_s), segments in index order, accumulated as a
-// double-single and scaled in FP64.  Bound by the latency of its loads: those of
-// 16 segments go out before their ordered sums, and 32-body CTAs spread a
-// small system over the SMs (22.1 us at n = 1000 and 32 segments with one load
-// waiting for the last sum in 256-body CTAs; 7.8 us now).
-constexpr int kCombineBlock = 32;
-__global__ void __launch_bounds__(kCombineBlock)
+// a_i = G * sum_s (sum_s - comp_s) as a double-single scaled in FP64: 32 bodies per
+// block, 8 groups of segments in strides (their loads ahead of the ordered sums),
+// then the groups in order.  Bound by the latency of those loads and sums: 22.1 us
+// at n = 1000 and 32 segments with one load waiting for the last sum in 256-body
+// CTAs, 6.9 with one warp per 32 bodies and 16 segments' loads at once, 6.2 now.
+constexpr int kCombineGroups = 8;
+__global__ void __launch_bounds__(32 * kCombineGroups)
 combine_mixed_kernel(const float *__restrict__ psum,
                                      const float *__restrict__ pcomp, int n, int segments,
                                      double G, double *__restrict__ ax,
-                                     double *__restrict__ ay, double *__restrict__ az)
+                                     double *__restrict__ ay, double *__restrict__ az,
+                                     const AfterForce after)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    __shared__ float2 sh[kCombineGroups][3][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
     const size_t plane = (size_t)n;
     float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
-    for (int s0 = 0; s0 < segments; s0 += 16) {
-        float t[16][3], q[16][3];
+    if (i < n)
+        for (int s0 = g; s0 < segments; s0 += 4 * kCombineGroups) {
+            float t[4][3], q[4][3];
 #pragma unroll
-        for (int u = 0; u < 16; ++u)
+            for (int u = 0; u < 4; ++u)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const size_t at = ((size_t)(s0 + u) * 3 + c) * plane + i;
-                t[u][c] = s0 + u < segments ? psum[at] : 0.f;
-                q[u][c] = s0 + u < segments ? pcomp[at] : 0.f;
-            }
+                for (int c = 0; c < 3; ++c) {
+                    const int s = s0 + u * kCombineGroups;
+                    const size_t at = ((size_t)s * 3 + c) * plane + i;
+                    t[u][c] = s < segments ? psum[at] : 0.f;
+                    q[u][c] = s < segments ? pcomp[at] : 0.f;
+                }
 #pragma unroll
-        for (int u = 0; u < 16; ++u)
-            if (s0 + u < segments)
+            for (int u = 0; u < 4; ++u)
 #pragma unroll
                 for (int c = 0; c < 3; ++c) ds_add_kahan(hi[c], lo[c], t[u][c], q[u][c]);
-    }
-    ax[i] = G * ((double)hi[0] + (double)lo[0]);
-    ay[i] = G * ((double)hi[1] + (double)lo[1]);
-    az[i] = G * ((double)hi[2] + (double)lo[2]);
+        }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sh[g][c][lane] = make_float2(hi[c], lo[c]);
+    __syncthreads();
+    if (g >= 3 || i >= n) return;  // warp c finishes component c
+    const int c = g;
+    float2 s = dup2(0.f);
+#pragma unroll
+    for (int k = 0; k < kCombineGroups; ++k)
+        ds_add_kahan(s.x, s.y, sh[k][c][lane].x, -sh[k][c][lane].y);
+    double *out = c == 0 ? ax : (c == 1 ? ay : az);
+    const double a = G * ((double)s.x + (double)s.y);
+    out[i] = a;
+    after_force(after, c, i, a);
 }
 
 // ---------------------------------------------------------------- mixed, unordered pairs
@@ -267,7 +281,7 @@ __global__ void __launch_bounds__(32 * kPairGroups)
 combine_mixed_pairs_kernel(const float2 *__restrict__ part, int n, int blocks, int p0, int np,
                            bool first, bool last, float *__restrict__ acc, double G,
                            double *__restrict__ ax, double *__restrict__ ay,
-                           double *__restrict__ az)
+                           double *__restrict__ az, const AfterForce after)
 {
     constexpr int H = kPairH, V = kPairV;
     __shared__ float2 sh[kPairGroups][3][32];
@@ -309,7 +323,9 @@ combine_mixed_pairs_kernel(const float2 *__restrict__ part, int n, int blocks, i
         return;
     }
     double *out = c == 0 ? ax : (c == 1 ? ay : az);
-    out[i] = G * ((double)s.x + (double)s.y);
+    const double a = G * ((double)s.x + (double)s.y);
+    out[i] = a;
+    after_force(after, c, i, a);
 }
 
 // ---------------------------------------------------------------- FP64
@@ -324,7 +340,7 @@ __global__ void __launch_bounds__(32)
 direct_fp64_row_kernel(const double *__restrict__ x, const double *__restrict__ y,
                        const double *__restrict__ z, const double *__restrict__ m, int n,
                        double eps2, double G, double *__restrict__ ax, double *__restrict__ ay,
-                       double *__restrict__ az)
+                       double *__restrict__ az, const AfterForce after)
 {
     const int i = blockIdx.x;
     const double xi = x[i], yi = y[i], zi = z[i];
@@ -341,10 +357,12 @@ direct_fp64_row_kernel(const double *__restrict__ x, const double *__restrict__ 
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
         for (int c = 0; c < 3; ++c) a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
-    if (threadIdx.x == 0) {
-        ax[i] = G * a[0];
-        ay[i] = G * a[1];
-        az[i] = G * a[2];
+    if (threadIdx.x < 3) {  // lane c finishes component c
+        const int c = threadIdx.x;
+        double *out = c == 0 ? ax : (c == 1 ? ay : az);
+        const double t = G * (c == 0 ? a[0] : (c == 1 ? a[1] : a[2]));
+        out[i] = t;
+        after_force(after, c, i, t);
     }
 }
 
@@ -492,7 +510,7 @@ direct_fp64_pairs_kernel(const double *__restrict__ x, const double *__restrict_
 __global__ void __launch_bounds__(256)
 combine_fp64_kernel(const double *__restrict__ part, int n, int blocks, int width, int p0, int np,
                     bool add, bool last, double G, double *__restrict__ ax,
-                    double *__restrict__ ay, double *__restrict__ az)
+                    double *__restrict__ ay, double *__restrict__ az, const AfterForce after)
 {
     __shared__ double sh[8][3][8];
     const int body = threadIdx.x & 7, g = threadIdx.x >> 3;
@@ -523,7 +541,9 @@ combine_fp64_kernel(const double *__restrict__ part, int n, int blocks, int widt
     double t = ((sh[0][c][body] + sh[1][c][body]) + (sh[2][c][body] + sh[3][c][body])) +
                ((sh[4][c][body] + sh[5][c][body]) + (sh[6][c][body] + sh[7][c][body]));
     if (add) t = out[i] + t;
-    out[i] = last ? G * t : t;
+    if (last) t = G * t;
+    out[i] = t;
+    if (last) after_force(after, c, i, t);
 }
 
 __global__ void split_kernel(const double *__restrict__ x, const double *__restrict__ y,
@@ -660,7 +680,8 @@ nb_status split_positions(const double *x, const double *y, const double *z, con
 
 static nb_status direct_mixed_pairs(const float4 *hi, const float4 *lo, int n, double G,
                                     double eps2, double *ax, double *ay, double *az,
-                                    DevBuf &partials, cudaStream_t st, const KernelTimer *timer)
+                                    DevBuf &partials, cudaStream_t st, const KernelTimer *timer,
+                                    const AfterForce &after)
 {
     const int blocks = (n + kPairBlock - 1) / kPairBlock, diagonals = blocks / 2 + 1;
     // planes of 3 n Kahan pairs, the diagonals in passes whose planes stay
@@ -685,7 +706,7 @@ static nb_status direct_mixed_pairs(const float4 *hi, const float4 *lo, int n, d
         const bool last = p0 + np == diagonals;
         if (last && timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
         combine_mixed_pairs_kernel<<<(n + 31) / 32, 32 * kPairGroups, 0, st>>>(
-            part, n, blocks, p0, np, p0 == 0, last, acc, G, ax, ay, az);
+            part, n, blocks, p0, np, p0 == 0, last, acc, G, ax, ay, az, after);
         NB_LAUNCH_CHECK();
     }
     return NB_OK;
@@ -693,11 +714,11 @@ static nb_status direct_mixed_pairs(const float4 *hi, const float4 *lo, int n, d
 
 nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, double eps2,
                        double *ax, double *ay, double *az, DevBuf &partials, cudaStream_t st,
-                       const KernelTimer *timer)
+                       const KernelTimer *timer, const AfterForce &after)
 {
     if (n <= 0) return NB_OK;
     if (n >= kMixedPairsMin)
-        return direct_mixed_pairs(hi, lo, n, G, eps2, ax, ay, az, partials, st, timer);
+        return direct_mixed_pairs(hi, lo, n, G, eps2, ax, ay, az, partials, st, timer, after);
     const DirectPlan p = direct_mixed_plan(n);
     NB_TRY(partials.reserve(sizeof(float) * 6 * (size_t)n * p.segments));
     float *psum = partials.as<float>();
@@ -707,8 +728,8 @@ nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, doub
         return fail(NB_ERR_UNSUPPORTED, "direct_mixed: unsupported tile shape");
     NB_LAUNCH_CHECK();
     if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
-    combine_mixed_kernel<<<(n + kCombineBlock - 1) / kCombineBlock, kCombineBlock, 0, st>>>(
-        psum, pcomp, n, p.segments, G, ax, ay, az);
+    combine_mixed_kernel<<<(n + 31) / 32, 32 * kCombineGroups, 0, st>>>(
+        psum, pcomp, n, p.segments, G, ax, ay, az, after);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
@@ -745,15 +766,18 @@ static void launch_fp64_pairs(const double *x, const double *y, const double *z,
 
 nb_status direct_fp64(const double *x, const double *y, const double *z, const double *m, int n,
                       double G, double eps2, double *ax, double *ay, double *az,
-                      DevBuf &partials, cudaStream_t st, const KernelTimer *timer)
+                      DevBuf &partials, cudaStream_t st, const KernelTimer *timer,
+                      const AfterForce &after)
 {
     if (n <= 0) return NB_OK;
     if (n <= kF64RowMax) {
         if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
         if (eps2 > 0.0)
-            direct_fp64_row_kernel<false><<<n, 32, 0, st>>>(x, y, z, m, n, eps2, G, ax, ay, az);
+            direct_fp64_row_kernel<false><<<n, 32, 0, st>>>(x, y, z, m, n, eps2, G, ax, ay, az,
+                                                             after);
         else
-            direct_fp64_row_kernel<true><<<n, 32, 0, st>>>(x, y, z, m, n, 0.0, G, ax, ay, az);
+            direct_fp64_row_kernel<true><<<n, 32, 0, st>>>(x, y, z, m, n, 0.0, G, ax, ay, az,
+                                                            after);
         NB_LAUNCH_CHECK();
         if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
         return NB_OK;
@@ -779,7 +803,7 @@ nb_status direct_fp64(const double *x, const double *y, const double *z, const d
         const bool last = p0 + np == diagonals;
         if (last && timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
         combine_fp64_kernel<<<(n + 7) / 8, 256, 0, st>>>(part, n, blocks, 32 * T, p0, np, p0 > 0,
-                                                         last, G, ax, ay, az);
+                                                         last, G, ax, ay, az, after);
         NB_LAUNCH_CHECK();
     }
     return NB_OK;
@@ -885,8 +909,8 @@ extern "C" nb_status nb_direct_mixed_forces_noalloc(size_t n, const double *x, c
     if (!launch_mixed(p, st, hi, lo, ni, eps2, psum, pcomp))
         return fail(NB_ERR_UNSUPPORTED, "nb_direct_mixed_forces_noalloc: tile shape");
     NB_LAUNCH_CHECK();
-    combine_mixed_kernel<<<(ni + kCombineBlock - 1) / kCombineBlock, kCombineBlock, 0, st>>>(
-        psum, pcomp, ni, p.segments, G, ax, ay, az);
+    combine_mixed_kernel<<<(ni + 31) / 32, 32 * kCombineGroups, 0, st>>>(
+        psum, pcomp, ni, p.segments, G, ax, ay, az, AfterForce{});
     NB_LAUNCH_CHECK();
     return NB_OK;
 }

@@ -12,6 +12,7 @@
 // These passes are HBM-bound (48-120 B per body); the force evaluation between
 // them dominates every step.
 #include "nb_internal.h"
+#include "nb_after.cuh"
 
 namespace nb {
 namespace {
@@ -29,7 +30,8 @@ __global__ void kick_drift_kernel(int n, double dt, double h, double *__restrict
                                   double *__restrict__ vz, const double *__restrict__ ax,
                                   const double *__restrict__ ay, const double *__restrict__ az,
                                   double *__restrict__ oax, double *__restrict__ oay,
-                                  double *__restrict__ oaz)
+                                  double *__restrict__ oaz, const double *__restrict__ m,
+                                  float4 *__restrict__ hi, float4 *__restrict__ lo)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -57,6 +59,9 @@ __global__ void kick_drift_kernel(int n, double dt, double h, double *__restrict
     } else {
         oax[i] = a[0]; oay[i] = a[1]; oaz[i] = a[2];
     }
+    if (hi)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) split_component(hi, lo, m, c, i, p[c]);
 }
 
 template <int KIND>
@@ -137,26 +142,29 @@ inline int blocks_for(int n) { return (n + 255) / 256; }
 
 nb_status kick_drift(int kind, int n, double dt, double *x, double *y, double *z, double *vx,
                      double *vy, double *vz, const double *ax, const double *ay,
-                     const double *az, double *oax, double *oay, double *oaz, cudaStream_t st)
+                     const double *az, double *oax, double *oay, double *oaz, cudaStream_t st,
+                     const double *m, float4 *hi, float4 *lo)
 {
     if (n <= 0) return NB_OK;
     const double h = dt / 2.0;
     switch (kind) {
     case kEuler:
         kick_drift_kernel<kEuler><<<blocks_for(n), 256, 0, st>>>(n, dt, h, x, y, z, vx, vy, vz,
-                                                                 ax, ay, az, oax, oay, oaz);
+                                                                 ax, ay, az, oax, oay, oaz, m,
+                                                                 hi, lo);
         break;
     case kEulerCromer:
         kick_drift_kernel<kEulerCromer><<<blocks_for(n), 256, 0, st>>>(
-            n, dt, h, x, y, z, vx, vy, vz, ax, ay, az, oax, oay, oaz);
+            n, dt, h, x, y, z, vx, vy, vz, ax, ay, az, oax, oay, oaz, m, hi, lo);
         break;
     case kLeapfrog:
         kick_drift_kernel<kLeapfrog><<<blocks_for(n), 256, 0, st>>>(
-            n, dt, h, x, y, z, vx, vy, vz, ax, ay, az, oax, oay, oaz);
+            n, dt, h, x, y, z, vx, vy, vz, ax, ay, az, oax, oay, oaz, m, hi, lo);
         break;
     case kVerlet:
         kick_drift_kernel<kVerlet><<<blocks_for(n), 256, 0, st>>>(n, dt, h, x, y, z, vx, vy, vz,
-                                                                  ax, ay, az, oax, oay, oaz);
+                                                                  ax, ay, az, oax, oay, oaz, m,
+                                                                  hi, lo);
         break;
     default:
         return fail(NB_ERR_INVALID_ARGUMENT, "kick_drift: bad integrator");
@@ -207,6 +215,34 @@ nb_status rk4_combine(int n, double dt, double *x, double *y, double *z, double 
     const size_t cap = (size_t)(k3 - k2) / 9;
     rk4_combine_kernel<<<blocks_for(n), 256, 0, st>>>(n, dt / 6.0, x, y, z, vx, vy, vz, ax, ay,
                                                       az, k2, k3, k4, cap);
+    NB_LAUNCH_CHECK();
+    return NB_OK;
+}
+
+nb_status apply_after(const AfterForce &t, int n, const double *ax, const double *ay,
+                      const double *az, cudaStream_t st)
+{
+    if (n <= 0 || t.kind == AfterForce::kNone) return NB_OK;
+    switch (t.kind) {
+    case AfterForce::kKick:
+        kick_kernel<kLeapfrog><<<blocks_for(n), 256, 0, st>>>(
+            n, t.h, t.v[0], t.v[1], t.v[2], ax, ay, az, nullptr, nullptr, nullptr);
+        break;
+    case AfterForce::kKickMean:
+        kick_kernel<kVerlet><<<blocks_for(n), 256, 0, st>>>(
+            n, t.h, t.v[0], t.v[1], t.v[2], ax, ay, az, t.a0[0], t.a0[1], t.a0[2]);
+        break;
+    case AfterForce::kStage:
+        rk4_stage_kernel<<<blocks_for(n), 256, 0, st>>>(
+            n, t.h, t.x0[0], t.x0[1], t.x0[2], t.v0[0], t.v0[1], t.v0[2], t.kv[0], t.kv[1],
+            t.kv[2], ax, ay, az, t.x[0], t.x[1], t.x[2], t.v[0], t.v[1], t.v[2]);
+        break;
+    default:  // kFinish; the last stage's planes begin three before its velocity
+        rk4_combine_kernel<<<blocks_for(n), 256, 0, st>>>(
+            n, t.h, t.x[0], t.x[1], t.x[2], t.v[0], t.v[1], t.v[2], t.a0[0], t.a0[1], t.a0[2],
+            t.k2, t.k3, t.kv[0] - 3 * t.ps, t.ps);
+        break;
+    }
     NB_LAUNCH_CHECK();
     return NB_OK;
 }

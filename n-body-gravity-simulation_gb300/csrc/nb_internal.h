@@ -86,6 +86,22 @@ struct KernelTimer {
     cudaEvent_t start = nullptr, stop = nullptr;
 };
 
+// The integrator's update of a body once its acceleration is known (nb_after.cuh):
+// the kernel that finishes the acceleration applies it.  Planes by component.
+struct AfterForce {
+    enum Kind { kNone, kKick, kKickMean, kStage, kFinish };
+    Kind kind = kNone;
+    double h = 0.0;                 // the update's step
+    double *x[3] = {}, *v[3] = {};  // written: velocities; positions too by kStage, kFinish
+    const double *a0[3] = {};       // kKickMean: a(t); kFinish: the first stage's
+    const double *x0[3] = {}, *v0[3] = {};  // kStage: the step's start
+    const double *kv[3] = {};       // kStage: the stage's velocity; kFinish: the last one's
+    const double *k2 = nullptr, *k3 = nullptr;  // kFinish: planes x y z vx vy vz ax ay az
+    size_t ps = 0;                              // and their stride
+    const double *m = nullptr;      // kStage, or null: the mirror split_positions
+    float4 *hi = nullptr, *lo = nullptr;        // would make of the new positions
+};
+
 // ---------------------------------------------------------------- direct sum
 struct DirectPlan {
     int block = 256;    // threads per CTA
@@ -98,7 +114,8 @@ struct DirectPlan {
 // (x_lo, y_lo, z_lo, 0) of every body.  Writes G * sum into ax/ay/az (FP64).
 nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, double eps2,
                        double *ax, double *ay, double *az, DevBuf &partials,
-                       cudaStream_t st, const KernelTimer *timer = nullptr);
+                       cudaStream_t st, const KernelTimer *timer = nullptr,
+                       const AfterForce &after = AfterForce{});
 
 // Thresholds of the sorted near/far kernels as (gap / D)^2, D the diameter of
 // a warp's i-box: a j-chunk at least D/8 away takes the plain FP32 term, one
@@ -152,20 +169,28 @@ bool direct_sorted_enabled(int n, int flags);
 // FP64 all-pairs kernel.
 nb_status direct_fp64(const double *x, const double *y, const double *z, const double *m,
                       int n, double G, double eps2, double *ax, double *ay, double *az,
-                      DevBuf &partials, cudaStream_t st, const KernelTimer *timer = nullptr);
+                      DevBuf &partials, cudaStream_t st, const KernelTimer *timer = nullptr,
+                      const AfterForce &after = AfterForce{});
 
 // Builds the float4 hi/lo mirror of FP64 positions + masses.
 nb_status split_positions(const double *x, const double *y, const double *z,
                           const double *m, int n, float4 *hi, float4 *lo, cudaStream_t st);
 
 // ---------------------------------------------------------------- integrators
+// hi, lo (or null): the mirror split_positions would make of the new positions.
 nb_status kick_drift(int kind, int n, double dt, double *x, double *y, double *z, double *vx,
                      double *vy, double *vz, const double *ax, const double *ay,
                      const double *az, double *oax, double *oay, double *oaz,
-                     cudaStream_t st);
+                     cudaStream_t st, const double *m = nullptr, float4 *hi = nullptr,
+                     float4 *lo = nullptr);
 nb_status kick(int kind, int n, double dt, double *vx, double *vy, double *vz,
                const double *ax, const double *ay, const double *az, const double *oax,
                const double *oay, const double *oaz, cudaStream_t st);
+
+// An AfterForce as a launch of its own, after a force evaluation that did not
+// apply it.
+nb_status apply_after(const AfterForce &after, int n, const double *ax, const double *ay,
+                      const double *az, cudaStream_t st);
 
 // RK4 stage kernels.  stage 2/3/4 positions/velocities from the base state.
 nb_status rk4_stage(int n, double h, const double *x, const double *y, const double *z,
@@ -362,9 +387,11 @@ struct nb_sim {
 };
 
 namespace nb {
-// Evaluates accelerations of positions (px,py,pz) with masses m into out*.
+// Evaluates accelerations of positions (px,py,pz) with masses m into out* and
+// applies `after`; split: the mixed kernels' mirror holds these positions already.
 nb_status eval_forces(nb_sim *s, const double *px, const double *py, const double *pz,
-                      double *oax, double *oay, double *oaz);
+                      double *oax, double *oay, double *oaz,
+                      const AfterForce &after = AfterForce{}, bool split = false);
 // Drops the captured step graph (the next steps run directly).
 void reset_step_graph(nb_sim *s);
 // Kernel launches made by a graph replay (the launch counter's evidence).

@@ -119,8 +119,22 @@ const DeviceProps &device_props()
 
 static size_t plane_stride(size_t capacity) { return (capacity + 31) / 32 * 32; }
 
+// Whether the force kernels apply an AfterForce themselves, and whether they read
+// the mixed kernels' mirror (which an update can then write with the positions).
+static bool fuses_updates(const nb_sim *s)
+{
+    return s->cfg.method == NB_DIRECT_FP64 ||
+           (s->cfg.method == NB_DIRECT_MIXED && !direct_sorted_enabled((int)s->n, s->cfg.flags));
+}
+
+static nb_status reserve_mirror(nb_sim *s)
+{
+    NB_TRY(s->split_hi.reserve(sizeof(float4) * s->capacity));
+    return s->split_lo.reserve(sizeof(float4) * s->capacity);
+}
+
 nb_status eval_forces(nb_sim *s, const double *px, const double *py, const double *pz,
-                      double *oax, double *oay, double *oaz)
+                      double *oax, double *oay, double *oaz, const AfterForce &after, bool split)
 {
     const int n = (int)s->n;
     const double eps2 = s->cfg.softening * s->cfg.softening;
@@ -128,25 +142,27 @@ nb_status eval_forces(nb_sim *s, const double *px, const double *py, const doubl
     switch (s->cfg.method) {
     case NB_DIRECT_FP64:
         return direct_fp64(px, py, pz, s->m(), n, s->cfg.G, eps2, oax, oay, oaz, s->partials,
-                           s->stream, timer);
+                           s->stream, timer, after);
     case NB_DIRECT_MIXED: {
-        if (direct_sorted_enabled(n, s->cfg.flags))
-            return direct_mixed_sorted(px, py, pz, s->m(), n, s->cfg.G, eps2, oax, oay, oaz,
-                                       s->sorted, s->stream, timer);
-        NB_TRY(s->split_hi.reserve(sizeof(float4) * s->capacity));
-        NB_TRY(s->split_lo.reserve(sizeof(float4) * s->capacity));
+        if (direct_sorted_enabled(n, s->cfg.flags)) {
+            NB_TRY(direct_mixed_sorted(px, py, pz, s->m(), n, s->cfg.G, eps2, oax, oay, oaz,
+                                       s->sorted, s->stream, timer));
+            return apply_after(after, n, oax, oay, oaz, s->stream);
+        }
+        NB_TRY(reserve_mirror(s));
         float4 *hi = s->split_hi.as<float4>(), *lo = s->split_lo.as<float4>();
-        NB_TRY(split_positions(px, py, pz, s->m(), n, hi, lo, s->stream));
+        if (!split) NB_TRY(split_positions(px, py, pz, s->m(), n, hi, lo, s->stream));
         return direct_mixed(hi, lo, n, s->cfg.G, eps2, oax, oay, oaz, s->partials, s->stream,
-                            timer);
+                            timer, after);
     }
     case NB_BARNES_HUT:
         if (!s->bh) s->bh = bh_create();
-        return bh_compute(s->bh, px, py, pz, s->m(), n, s->cfg.G, eps2, s->cfg.theta,
+        NB_TRY(bh_compute(s->bh, px, py, pz, s->m(), n, s->cfg.G, eps2, s->cfg.theta,
                           s->cfg.leaf_capacity, oax, oay, oaz, s->stream, timer,
                           NB_FLAG_BH_REUSE_OF(s->cfg.flags),
                           (s->cfg.flags & NB_FLAG_BH_QUADRUPOLE) != 0,
-                          (s->cfg.flags & NB_FLAG_BH_REFERENCE_OPENING) != 0);
+                          (s->cfg.flags & NB_FLAG_BH_REFERENCE_OPENING) != 0));
+        return apply_after(after, n, oax, oay, oaz, s->stream);
     default:
         return fail(NB_ERR_INVALID_ARGUMENT, "unknown force method");
     }
@@ -170,61 +186,77 @@ static nb_status step_once(nb_sim *s, int integ, double dt)
 {
     const int n = (int)s->n;
     cudaStream_t st = s->stream;
+    // the updates write the next evaluation's mirror where the kernels read one
+    const bool mirror = s->cfg.method == NB_DIRECT_MIXED && fuses_updates(s);
+    if (mirror) NB_TRY(reserve_mirror(s));
+    float4 *hi = mirror ? s->split_hi.as<float4>() : nullptr;
+    float4 *lo = mirror ? s->split_lo.as<float4>() : nullptr;
+    double *const x[3] = {s->x(), s->y(), s->z()}, *const v[3] = {s->vx(), s->vy(), s->vz()};
+    double *const a[3] = {s->ax(), s->ay(), s->az()};
+    AfterForce after;
+    for (int c = 0; c < 3; ++c) after.v[c] = v[c];
     switch (integ) {
     case NB_EULER:
     case NB_EULER_CROMER:
-        NB_TRY(eval_forces(s, s->x(), s->y(), s->z(), s->ax(), s->ay(), s->az()));
-        NB_TRY(kick_drift(integ, n, dt, s->x(), s->y(), s->z(), s->vx(), s->vy(), s->vz(),
-                          s->ax(), s->ay(), s->az(), nullptr, nullptr, nullptr, st));
+        NB_TRY(eval_forces(s, x[0], x[1], x[2], a[0], a[1], a[2]));
+        NB_TRY(kick_drift(integ, n, dt, x[0], x[1], x[2], v[0], v[1], v[2], a[0], a[1], a[2],
+                          nullptr, nullptr, nullptr, st));
         s->forces_valid = false;
         return NB_OK;
     case NB_LEAPFROG:
-        if (!s->forces_valid)
-            NB_TRY(eval_forces(s, s->x(), s->y(), s->z(), s->ax(), s->ay(), s->az()));
-        NB_TRY(kick_drift(integ, n, dt, s->x(), s->y(), s->z(), s->vx(), s->vy(), s->vz(),
-                          s->ax(), s->ay(), s->az(), nullptr, nullptr, nullptr, st));
+        if (!s->forces_valid) NB_TRY(eval_forces(s, x[0], x[1], x[2], a[0], a[1], a[2]));
+        NB_TRY(kick_drift(integ, n, dt, x[0], x[1], x[2], v[0], v[1], v[2], a[0], a[1], a[2],
+                          nullptr, nullptr, nullptr, st, s->m(), hi, lo));
         s->forces_valid = false;
-        NB_TRY(eval_forces(s, s->x(), s->y(), s->z(), s->ax(), s->ay(), s->az()));
-        NB_TRY(kick(integ, n, dt, s->vx(), s->vy(), s->vz(), s->ax(), s->ay(), s->az(), nullptr,
-                    nullptr, nullptr, st));
+        after.kind = AfterForce::kKick;
+        after.h = dt / 2.0;
+        NB_TRY(eval_forces(s, x[0], x[1], x[2], a[0], a[1], a[2], after, mirror));
         s->forces_valid = true;
         return NB_OK;
     case NB_VELOCITY_VERLET: {
         const size_t ps = plane_stride(s->capacity);
         NB_TRY(s->old_acc.reserve(sizeof(double) * 3 * ps));
         double *o = s->old_acc.as<double>();
-        if (!s->forces_valid)
-            NB_TRY(eval_forces(s, s->x(), s->y(), s->z(), s->ax(), s->ay(), s->az()));
-        NB_TRY(kick_drift(integ, n, dt, s->x(), s->y(), s->z(), s->vx(), s->vy(), s->vz(),
-                          s->ax(), s->ay(), s->az(), o, o + ps, o + 2 * ps, st));
+        if (!s->forces_valid) NB_TRY(eval_forces(s, x[0], x[1], x[2], a[0], a[1], a[2]));
+        NB_TRY(kick_drift(integ, n, dt, x[0], x[1], x[2], v[0], v[1], v[2], a[0], a[1], a[2], o,
+                          o + ps, o + 2 * ps, st, s->m(), hi, lo));
         s->forces_valid = false;
-        NB_TRY(eval_forces(s, s->x(), s->y(), s->z(), s->ax(), s->ay(), s->az()));
-        NB_TRY(kick(integ, n, dt, s->vx(), s->vy(), s->vz(), s->ax(), s->ay(), s->az(), o,
-                    o + ps, o + 2 * ps, st));
+        after.kind = AfterForce::kKickMean;
+        after.h = 0.5 * dt;
+        for (int c = 0; c < 3; ++c) after.a0[c] = o + c * ps;
+        NB_TRY(eval_forces(s, x[0], x[1], x[2], a[0], a[1], a[2], after, mirror));
         s->forces_valid = true;
         return NB_OK;
     }
     case NB_RK4: {
         const size_t ps = plane_stride(s->capacity);
         NB_TRY(s->rk4.reserve(sizeof(double) * 27 * ps));
-        double *k2 = s->rk4.as<double>(), *k3 = k2 + 9 * ps, *k4 = k3 + 9 * ps;
-        auto P = [ps](double *k, int c) { return k + c * ps; };
-        NB_TRY(eval_forces(s, s->x(), s->y(), s->z(), s->ax(), s->ay(), s->az()));
-        const double h = dt / 2.0;
-        NB_TRY(rk4_stage(n, h, s->x(), s->y(), s->z(), s->vx(), s->vy(), s->vz(), s->vx(),
-                         s->vy(), s->vz(), s->ax(), s->ay(), s->az(), P(k2, 0), P(k2, 1),
-                         P(k2, 2), P(k2, 3), P(k2, 4), P(k2, 5), st));
-        NB_TRY(eval_forces(s, P(k2, 0), P(k2, 1), P(k2, 2), P(k2, 6), P(k2, 7), P(k2, 8)));
-        NB_TRY(rk4_stage(n, h, s->x(), s->y(), s->z(), s->vx(), s->vy(), s->vz(), P(k2, 3),
-                         P(k2, 4), P(k2, 5), P(k2, 6), P(k2, 7), P(k2, 8), P(k3, 0), P(k3, 1),
-                         P(k3, 2), P(k3, 3), P(k3, 4), P(k3, 5), st));
-        NB_TRY(eval_forces(s, P(k3, 0), P(k3, 1), P(k3, 2), P(k3, 6), P(k3, 7), P(k3, 8)));
-        NB_TRY(rk4_stage(n, dt, s->x(), s->y(), s->z(), s->vx(), s->vy(), s->vz(), P(k3, 3),
-                         P(k3, 4), P(k3, 5), P(k3, 6), P(k3, 7), P(k3, 8), P(k4, 0), P(k4, 1),
-                         P(k4, 2), P(k4, 3), P(k4, 4), P(k4, 5), st));
-        NB_TRY(eval_forces(s, P(k4, 0), P(k4, 1), P(k4, 2), P(k4, 6), P(k4, 7), P(k4, 8)));
-        NB_TRY(rk4_combine(n, dt, s->x(), s->y(), s->z(), s->vx(), s->vy(), s->vz(), s->ax(),
-                           s->ay(), s->az(), k2, k3, k4, st));
+        // stage k's planes x y z vx vy vz ax ay az; the first stage is the state
+        double *const k[3] = {s->rk4.as<double>(), s->rk4.as<double>() + 9 * ps,
+                              s->rk4.as<double>() + 18 * ps};
+        after.m = s->m();
+        after.hi = hi;
+        after.lo = lo;
+        for (int stage = 0; stage < 4; ++stage) {
+            double *p[3], *acc[3];
+            for (int c = 0; c < 3; ++c) {
+                p[c] = stage == 0 ? x[c] : k[stage - 1] + c * ps;
+                after.kv[c] = stage == 0 ? v[c] : k[stage - 1] + (3 + c) * ps;
+                acc[c] = stage == 0 ? a[c] : k[stage - 1] + (6 + c) * ps;
+                after.x0[c] = x[c];
+                after.v0[c] = v[c];
+                after.a0[c] = a[c];
+                after.x[c] = stage < 3 ? k[stage] + c * ps : x[c];
+                after.v[c] = stage < 3 ? k[stage] + (3 + c) * ps : v[c];
+            }
+            after.kind = stage < 3 ? AfterForce::kStage : AfterForce::kFinish;
+            after.h = stage < 2 ? dt / 2.0 : (stage == 2 ? dt : dt / 6.0);
+            after.k2 = k[0];
+            after.k3 = k[1];
+            after.ps = ps;
+            NB_TRY(eval_forces(s, p[0], p[1], p[2], acc[0], acc[1], acc[2], after,
+                               mirror && stage > 0));
+        }
         s->forces_valid = false;
         return NB_OK;
     }
