@@ -1242,7 +1242,8 @@ group_kernel(const BHNode *__restrict__ nodes, const int *__restrict__ total,
              const int *__restrict__ parent, const unsigned char *__restrict__ octant,
              const float4 *__restrict__ pcen, const float4 *__restrict__ quad,
              BHGNode *__restrict__ gnodes, unsigned char *__restrict__ gnk,
-             float4 *__restrict__ gpcen, float4 *__restrict__ gquad)
+             float4 *__restrict__ gpcen, float4 *__restrict__ gquad,
+             const unsigned char *__restrict__ node_depth, unsigned *__restrict__ gkey)
 {
     const int num = *total;
     for (int k = blockIdx.x * 256 + threadIdx.x; k < num; k += gridDim.x * 256) {
@@ -1264,6 +1265,7 @@ group_kernel(const BHNode *__restrict__ nodes, const int *__restrict__ total,
         gnodes[pos] = g;
         gnk[pos] = (unsigned char)__popc(o);
         if (pcen) gpcen[pos] = pcen[k];
+        if (gkey) gkey[pos] = 1u + (unsigned)(num + node_depth[k] - nd.skip);
         if (quad) {
             gquad[2 * pos] = quad[2 * k];
             gquad[2 * pos + 1] = quad[2 * k + 1];
@@ -1294,7 +1296,7 @@ group_kernel(const BHNode *__restrict__ nodes, const int *__restrict__ total,
 // per group, took 2.32 ms at N = 2^20 (theta 0.5), 3.67 ms at N = 100,000 under
 // the reference's opening rule (ten warps per SM, each a serial walk, the longest
 // five times the mean); this takes 1.73 ms with one warp per walk and 0.55 ms with
-// sixteen.  Of the 1.73 ms, about 1.2 are the 15.5 dispatch cycles per interaction
+// sixteen (which the reference's rule takes only where the ordered walk below cannot).  Of the 1.73 ms, about 1.2 are the 15.5 dispatch cycles per interaction
 // of the evaluation, the rest the decisions (2,600 nodes per walk, a fifth of them
 // undecided).
 //
@@ -1425,19 +1427,6 @@ __device__ __forceinline__ int list_flush(WalkList &l, WalkQuads *quads, int cou
     return rest;
 }
 
-__device__ __forceinline__ float warp_min(float v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ float warp_max(float v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
 // The boxes of the CTA's 32-body chunks.
 template <int K>
 struct WalkBoxes {
@@ -1445,52 +1434,136 @@ struct WalkBoxes {
 };
 // Bounds of the squared distance from a point to the nearest body: the distance
 // to the nearest box, and that to the farthest point of the nearest face of a
-// box (on each face of a box lies one of its bodies).
-template <int K>
-__device__ __forceinline__ void box_distances(const WalkBoxes<K> &b, const float (&c)[3],
-                                              float &least, float &most)
+// box (on each face of a box lies one of its bodies).  The first box starts them.
+__device__ __forceinline__ void box_distances(const float (&mn)[3], const float (&mx)[3],
+                                              const float (&c)[3], bool starts, float &least,
+                                              float &most)
 {
+    float out[3], face[3], far[3];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        float out[3], face[3], far[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float lo = b.mn[k][d] - c[d], hi = c[d] - b.mx[k][d];
-            out[d] = fmaxf(0.f, fmaxf(lo, hi));
-            face[d] = fminf(fabsf(lo), fabsf(hi));
-            far[d] = fmaxf(fabsf(lo), fabsf(hi));
-        }
-        const float near2 = fmaf(out[2], out[2], fmaf(out[1], out[1], out[0] * out[0]));
-        const float xy = fmaf(far[1], far[1], far[0] * far[0]);
-        const float fx = fmaf(far[2], far[2], fmaf(far[1], far[1], face[0] * face[0]));
-        const float fy = fmaf(far[2], far[2], fmaf(face[1], face[1], far[0] * far[0]));
-        const float fz = fmaf(face[2], face[2], xy);
-        const float face2 = fminf(fx, fminf(fy, fz));
-        least = k == 0 ? near2 : fminf(least, near2);
-        most = k == 0 ? face2 : fminf(most, face2);
+    for (int d = 0; d < 3; ++d) {
+        const float lo = mn[d] - c[d], hi = c[d] - mx[d];
+        out[d] = fmaxf(0.f, fmaxf(lo, hi));
+        face[d] = fminf(fabsf(lo), fabsf(hi));
+        far[d] = fmaxf(fabsf(lo), fabsf(hi));
     }
+    const float near2 = fmaf(out[2], out[2], fmaf(out[1], out[1], out[0] * out[0]));
+    const float xy = fmaf(far[1], far[1], far[0] * far[0]);
+    const float fx = fmaf(far[2], far[2], fmaf(far[1], far[1], face[0] * face[0]));
+    const float fy = fmaf(far[2], far[2], fmaf(face[1], face[1], far[0] * far[0]));
+    const float fz = fmaf(face[2], face[2], xy);
+    const float face2 = fminf(fx, fminf(fy, fz));
+    least = starts ? near2 : fminf(least, near2);
+    most = starts ? face2 : fminf(most, face2);
 }
-// toward_body for the CTA's bodies by their boxes: whether some body may lie on
-// the node's side of its parent's centre, and whether all of a chunk's do.
-template <int K>
-__device__ __forceinline__ void toward_boxes(const WalkBoxes<K> &b, float4 pc, bool &some,
-                                             bool &all)
+// toward_body for a box's bodies: whether some body may lie on the node's side of
+// its parent's centre (some), and whether all of them do (all); or-ed.
+__device__ __forceinline__ void toward_box(const float (&mn)[3], const float (&mx)[3], float4 pc,
+                                           bool &some, bool &all)
 {
     const int oct = __float_as_int(pc.w);
     const float p[3] = {pc.x, pc.y, pc.z};
-    some = all = false;
+    bool may = oct < 8, must = oct < 8;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        bool may = oct < 8, must = oct < 8;
+    for (int d = 0; d < 3; ++d) {
+        const bool high = (oct >> d & 1) != 0;
+        may = may && (high ? mx[d] >= p[d] : mn[d] < p[d]);
+        must = must && (high ? mn[d] >= p[d] : mx[d] < p[d]);
+    }
+    some = some || may;
+    all = all || must;
+}
+
+// Chunk k's box.
+template <int K>
+__device__ __forceinline__ void load_box(const float (&p)[3], int k, WalkBoxes<K> &box)
+{
+    float mn[3] = {p[0], p[1], p[2]}, mx[3] = {p[0], p[1], p[2]};
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const bool high = (oct >> d & 1) != 0;
-            may = may && (high ? b.mx[k][d] >= p[d] : b.mn[k][d] < p[d]);
-            must = must && (high ? b.mn[k][d] >= p[d] : b.mx[k][d] < p[d]);
+            mn[d] = fminf(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
+            mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
         }
-        some = some || may;
-        all = all || must;
     }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        box.mn[k][d] = mn[d];
+        box.mx[k][d] = mx[d];
+    }
+}
+
+// Whether some body of the CTA opens the lane's node (have: it holds one); the
+// whole warp calls it.
+template <int K, bool DIR>
+__device__ __forceinline__ bool opened_nodes(const BHGNode &nd, bool have, float4 pc,
+                                             const WalkBoxes<K> &box, const float (&p)[K][3],
+                                             float theta2, int w0, int wend, float4 *test,
+                                             float4 *side)
+{
+    const int lane = threadIdx.x & 31;
+    const float c[3] = {nd.com_mass.x, nd.com_mass.y, nd.com_mass.z};
+    float least = 0.f, most = 0.f;
+    bool some = false, all = false;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        box_distances(box.mn[k], box.mx[k], c, k == 0, least, most);
+        if (DIR) toward_box(box.mn[k], box.mx[k], pc, some, all);
+    }
+    // a node that holds one of the CTA's bodies is opened (each body's own cell)
+    bool open = nd.first < wend && nd.first + nd.count > w0;
+    open = open || nd.size2 >= theta2 * most || all;
+    const bool by_distance = !(nd.size2 < theta2 * least), by_side = DIR && some;
+    unsigned left = __ballot_sync(0xffffffffu, have && !open && (by_distance || by_side));
+    if (!left) return open;
+    // where the boxes do not decide, every body, two nodes at a time: the distance first,
+    left = __ballot_sync(0xffffffffu, have && !open && by_distance);
+    test[lane] = make_float4(c[0], c[1], c[2], nd.size2);
+    if (DIR) side[lane] = pc;
+    __syncwarp();
+    while (left) {
+        const int q0 = __ffs(left) - 1;
+        left &= left - 1u;
+        const int q1 = left ? __ffs(left) - 1 : q0;
+        left &= left - 1u;
+        const float4 t0 = test[q0], t1 = test[q1];
+        bool any0 = false, any1 = false;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const float dx0 = t0.x - p[k][0], dx1 = t1.x - p[k][0];
+            const float dy0 = t0.y - p[k][1], dy1 = t1.y - p[k][1];
+            const float dz0 = t0.z - p[k][2], dz1 = t1.z - p[k][2];
+            any0 |= t0.w >= theta2 * fmaf(dz0, dz0, fmaf(dy0, dy0, dx0 * dx0));
+            any1 |= t1.w >= theta2 * fmaf(dz1, dz1, fmaf(dy1, dy1, dx1 * dx1));
+        }
+        any0 = __any_sync(0xffffffffu, any0);
+        any1 = __any_sync(0xffffffffu, any1);
+        if (lane == q0) open = any0;
+        if (lane == q1) open = any1;
+    }
+    if (DIR) {  // then the side
+        left = __ballot_sync(0xffffffffu, have && !open && by_side);
+        while (left) {
+            const int q0 = __ffs(left) - 1;
+            left &= left - 1u;
+            const int q1 = left ? __ffs(left) - 1 : q0;
+            left &= left - 1u;
+            const float4 c0 = side[q0], c1 = side[q1];
+            bool any0 = false, any1 = false;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                any0 |= toward_body(c0, p[k][0], p[k][1], p[k][2]);
+                any1 |= toward_body(c1, p[k][0], p[k][1], p[k][2]);
+            }
+            any0 = __any_sync(0xffffffffu, any0);
+            any1 = __any_sync(0xffffffffu, any1);
+            if (lane == q0) open = any0;
+            if (lane == q1) open = any1;
+        }
+    }
+    __syncwarp();
+    return open;
 }
 
 template <bool ZERO_SOFT, bool QUAD, int NP, bool DIR>
@@ -1500,17 +1573,19 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
                   const uint32_t *__restrict__ order, int n, float theta2, float eps2, double G,
                   double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
                   BHStats *__restrict__ stats, const float4 *__restrict__ gquad,
-                  const float4 *__restrict__ gpcen)
+                  const float4 *__restrict__ gpcen, const int2 *__restrict__ logged)
 {
+    // logged: the walks with a log (its count not negative) are done already
+    if (logged && logged[blockIdx.x].y >= 0) return;
     extern __shared__ __align__(16) unsigned char walk_shared[];
     using Shared = WalkShared<QUAD>;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
+    constexpr int K = 2 * NP;
     __shared__ int s_push[kWalkWarps];  // groups pushed in this round
     Shared &sh = reinterpret_cast<Shared *>(walk_shared)[w];
     int *s_first = reinterpret_cast<int *>(reinterpret_cast<Shared *>(walk_shared) + W);
     unsigned char *s_kids = reinterpret_cast<unsigned char *>(s_first + W * kWalkStack);
-    constexpr int K = 2 * NP;
-    const int num_nodes = *total;
+    [[maybe_unused]] const int num_nodes = *total;  // bounds checked builds only
     const int w0 = blockIdx.x * 32 * K;
     const int wend = min(n, w0 + 32 * K);  // the CTA's bodies: [w0, wend)
     const float2 e2 = dup2(eps2);
@@ -1526,11 +1601,7 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
         p[k][0] = q.x; p[k][1] = q.y; p[k][2] = q.z;
         wb.nx[k] = dup2(-q.x); wb.ny[k] = dup2(-q.y); wb.nz[k] = dup2(-q.z);
         wb.fx[k] = wb.fy[k] = wb.fz[k] = dup2(0.f);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            box.mn[k][d] = warp_min(p[k][d]);
-            box.mx[k][d] = warp_max(p[k][d]);
-        }
+        load_box(p[k], k, box);
     }
 
     unsigned m2p = 0, p2p = 0;
@@ -1542,6 +1613,13 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
     }
     while (sp > 0) {
         __syncthreads();
+        if (W > 1 && w >= sp) {  // a narrow round: no group for this warp
+            if (lane == 0) s_push[w] = 0;
+            __syncthreads();
+            sp = 0;
+            for (int v = 0; v < W; ++v) sp += s_push[v];
+            continue;
+        }
         // one node per lane: child lane & 7 of the warp's group lane >> 3
         const int e = sp - 1 - (w + W * (lane >> 3));
         const int kids = e >= 0 ? s_kids[e] : 0;
@@ -1549,57 +1627,9 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
         const int id = have ? s_first[e] + (lane & 7) : 0;
         sp = max(0, sp - 4 * W);
         const BHGNode nd = gnodes[NB_IN_RANGE(id, num_nodes) ? id : 0];
-        const float c[3] = {nd.com_mass.x, nd.com_mass.y, nd.com_mass.z};
-        float least, most;
-        box_distances(box, c, least, most);
-        // a node that holds one of the CTA's bodies is opened (each body's own cell)
-        bool open = nd.first < wend && nd.first + nd.count > w0;
-        open = open || nd.size2 >= theta2 * most;
-        bool closed = !open && nd.size2 < theta2 * least;
-        float4 pc = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (DIR) {
-            pc = gpcen[id];
-            bool some, all;
-            toward_boxes(box, pc, some, all);
-            open = open || all;
-            closed = closed && !some;
-        }
-        // the undecided ones by every body
-        unsigned undecided = __ballot_sync(0xffffffffu, have && !open && !closed);
-        if (undecided) {
-            sh.test[lane] = make_float4(c[0], c[1], c[2], nd.size2);
-            if (DIR) sh.side[lane] = pc;
-            __syncwarp();
-            while (undecided) {  // two at a time
-                const int q0 = __ffs(undecided) - 1;
-                undecided &= undecided - 1u;
-                const int q1 = undecided ? __ffs(undecided) - 1 : q0;
-                undecided &= undecided - 1u;
-                const float4 t0 = sh.test[q0], t1 = sh.test[q1];
-                bool any0 = false, any1 = false;
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    const float dx0 = t0.x - p[k][0], dx1 = t1.x - p[k][0];
-                    const float dy0 = t0.y - p[k][1], dy1 = t1.y - p[k][1];
-                    const float dz0 = t0.z - p[k][2], dz1 = t1.z - p[k][2];
-                    any0 |= t0.w >= theta2 * fmaf(dz0, dz0, fmaf(dy0, dy0, dx0 * dx0));
-                    any1 |= t1.w >= theta2 * fmaf(dz1, dz1, fmaf(dy1, dy1, dx1 * dx1));
-                }
-                if (DIR) {
-                    const float4 c0 = sh.side[q0], c1 = sh.side[q1];
-#pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        any0 |= toward_body(c0, p[k][0], p[k][1], p[k][2]);
-                        any1 |= toward_body(c1, p[k][0], p[k][1], p[k][2]);
-                    }
-                }
-                any0 = __any_sync(0xffffffffu, any0);
-                any1 = __any_sync(0xffffffffu, any1);
-                if (lane == q0) open = any0;
-                if (lane == q1) open = any1;
-            }
-            __syncwarp();
-        }
+        const float4 pc = DIR ? gpcen[id] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const bool open = opened_nodes<K, DIR>(nd, have, pc, box, p, theta2, w0, wend, sh.test,
+                                               sh.side);
 
         // push the groups of the opened internal nodes
         const bool inner = have && open && nd.kids >= 0;
@@ -1630,7 +1660,7 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
         const unsigned adds = __ballot_sync(0xffffffffu, add);
         if (add) {
             const int to = count + __popc(adds & below);
-            list_put(sh.list, to, c[0], c[1], c[2], nd.com_mass.w);
+            list_put(sh.list, to, nd.com_mass.x, nd.com_mass.y, nd.com_mass.z, nd.com_mass.w);
             if constexpr (QUAD) {
                 const float4 q0 = gquad[2 * id], q1 = gquad[2 * id + 1];
                 const float v[6] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
@@ -1741,6 +1771,311 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
     }
 }
 
+// ---------------------------------------------------------- ordered walk
+// The reference's opening rule makes walks of 20,000 interactions (n = 100,000,
+// theta 0.5, disk galaxy), and an FP32 sum of so many terms depends on their order in
+// the fifth digit.  This walk adds each body's terms one after the other in the
+// order of a serial walk over a stack of groups (last pushed, first visited; a
+// group's records in order), in two kernels:
+//   - decide_kernel finds the groups that the walk visits and which of their records
+//     are opened, in any order, by many warps (as group_walk_kernel), and sorts
+//     the groups by their place in the serial walk of the whole tree: the rank
+//     of the group's parent v in a preorder with children reversed, which is
+//     depth(v) - skip(v) but for a constant;
+//   - log_eval_kernel goes through a walk's groups in that order: four warps list the
+//     terms in shared memory, two add them up, a body per lane.
+// A walk that visits more than kLogGroups groups, or for whose log the pool has no
+// room, is left to group_walk_kernel.  A leapfrog step at n = 100,000: 3.87 ms with one
+// warp per walk, 1.06 in this way, 0.84 by group_walk_kernel, whose terms are in no
+// such order.
+constexpr int kLogGroups = 4096;  // at most 12 bits
+constexpr int kLogStack = 3072;
+constexpr int kLogPerBody = 16;   // pool entries per body (8 used at n = 100,000, theta 0.5)
+constexpr int kLogWarps = 16;     // of a decide_kernel CTA
+constexpr int kLogChunk = 256;    // terms per list
+constexpr int kLogListers = 128;  // threads of log_eval_kernel that list terms
+
+struct LogShared {
+    unsigned long long sorted[kLogGroups];  // key, slot (12 bits), records (4), opened ones (8)
+    int first[kLogGroups];                  // by slot: the group's first record
+    float4 test[kLogWarps][32], side[kLogWarps][32];
+    int s_first[kLogStack];  // the stack: as group_walk_kernel's, and the groups' keys
+    unsigned s_key[kLogStack];
+    unsigned char s_kids[kLogStack];
+};
+
+// Bound by dispatch: with 0.35 ms at n = 100,000 (theta 0.5, disk galaxy), by the
+// longest walk (1,939 groups in 35 rounds of up to 64, of 10,000 cycles each with
+// every node undecided by the boxes).  Tighter boxes (8 bodies each) and a pass over
+// the bodies per batch instead of one per node pair cost as much as they saved;
+// 8 warps took 0.12 ms longer, 4 warps for short walks with a second launch for the
+// rest 0.15.
+__global__ void __launch_bounds__(32 * kLogWarps, 2)
+decide_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restrict__ gnk,
+              const unsigned *__restrict__ gkey, const float4 *__restrict__ gpcen,
+              const int *__restrict__ total, const float4 *__restrict__ body, int n, float theta2,
+              BHStats *__restrict__ stats, int2 *__restrict__ walks, uint2 *__restrict__ pool,
+              int pool_size, unsigned long long *__restrict__ pool_next)
+{
+    constexpr int W = kLogWarps;
+    extern __shared__ __align__(16) unsigned char walk_shared[];
+    __shared__ int s_push[W];
+    __shared__ unsigned s_m2p, s_p2p;
+    __shared__ int s_at;
+    LogShared &sh = *reinterpret_cast<LogShared *>(walk_shared);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    [[maybe_unused]] const int num_nodes = *total;  // bounds checked builds only
+    const int w0 = blockIdx.x * 64, wend = min(n, w0 + 64);
+    WalkBoxes<2> box;
+    float p[2][3];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        // a slot past n walks with body w0: its tests repeat that body's
+        const int i = w0 + 32 * k + lane;
+        const float4 q = body[i < n ? i : w0];
+        p[k][0] = q.x; p[k][1] = q.y; p[k][2] = q.z;
+        load_box(p[k], k, box);
+    }
+    if (threadIdx.x == 0) {
+        sh.s_first[0] = 0;  // the root's group comes first: key 0
+        sh.s_kids[0] = 1;
+        sh.s_key[0] = 0;
+        s_m2p = s_p2p = 0;
+    }
+    unsigned m2p = 0, p2p = 0;  // per lane
+    int sp = 1, groups = 0;
+    bool fits = true;
+    while (sp > 0) {
+        __syncthreads();
+        const int take = min(sp, 4 * W);
+        fits = groups + take <= kLogGroups;
+        if (!fits) break;
+        // the first groups to the first warps: in a narrow round the others have none
+        const int j = 4 * w + (lane >> 3), e = sp - 1 - j;
+        const bool busy = 4 * w < take;
+        sp -= take;
+        bool inner = false;
+        unsigned push = 0;
+        int id = 0;
+        BHGNode nd;
+        if (busy) {
+            const int kids = e >= 0 ? sh.s_kids[e] : 0;
+            const bool have = (lane & 7) < kids;
+            id = have ? sh.s_first[e] + (lane & 7) : 0;
+            const unsigned key = e >= 0 ? sh.s_key[e] : 0;
+            nd = gnodes[NB_IN_RANGE(id, num_nodes) ? id : 0];
+            const bool open = opened_nodes<2, true>(nd, have, gpcen[id], box, p, theta2, w0, wend,
+                                                    sh.test[w], sh.side[w]);
+            const unsigned opened = __ballot_sync(0xffffffffu, have && open);
+            if (have) {
+                if (!open) ++m2p;
+                else if (nd.kids < 0) p2p += nd.count;
+            }
+            if (kids > 0 && (lane & 7) == 0) {
+                const int slot = groups + j;
+                sh.first[slot] = id;
+                sh.sorted[slot] = (unsigned long long)key << 24 | (unsigned)slot << 12 |
+                                  (unsigned)kids << 8 | ((opened >> lane) & 0xFFu);
+            }
+            inner = have && open && nd.kids >= 0;
+            push = __ballot_sync(0xffffffffu, inner);
+        }
+        groups += take;
+        if (lane == 0) s_push[w] = __popc(push);
+        __syncthreads();  // every warp has read its groups, too
+        int top = sp;
+        for (int v = 0; v < W; ++v) {
+            if (v < w) top += s_push[v];
+            sp += s_push[v];
+        }
+        fits = sp <= kLogStack;
+        if (!fits) break;
+        if (inner) {
+            const int to = top + __popc(push & ((1u << lane) - 1u));
+            sh.s_first[to] = nd.kids;
+            sh.s_kids[to] = gnk[id];
+            sh.s_key[to] = gkey[id];
+        }
+    }
+    if (!fits) {
+        if (threadIdx.x == 0) walks[blockIdx.x] = make_int2(0, -1);
+        return;
+    }
+    __syncthreads();
+    // bitonic sort of the groups, padded to a power of two
+    int size = 1;
+    while (size < groups) size <<= 1;
+    for (int k = groups + (int)threadIdx.x; k < size; k += blockDim.x) sh.sorted[k] = ~0ull;
+    for (int k = 2; k <= size; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            __syncthreads();
+            for (int t = threadIdx.x; t < size / 2; t += blockDim.x) {
+                const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo | j;
+                const unsigned long long a = sh.sorted[lo], b = sh.sorted[hi];
+                if ((a > b) == ((lo & k) == 0)) {
+                    sh.sorted[lo] = b;
+                    sh.sorted[hi] = a;
+                }
+            }
+        }
+    m2p = __reduce_add_sync(0xffffffffu, m2p);
+    p2p = __reduce_add_sync(0xffffffffu, p2p);
+    if (lane == 0) {
+        atomicAdd(&s_m2p, m2p);
+        atomicAdd(&s_p2p, p2p);
+    }
+    if (threadIdx.x == 0) {
+        const unsigned long long at = atomicAdd(pool_next, (unsigned long long)groups);
+        s_at = at + groups <= (unsigned long long)pool_size ? (int)at : -1;
+    }
+    __syncthreads();
+    const int at = s_at;
+    if (threadIdx.x == 0) {
+        walks[blockIdx.x] = make_int2(at, at < 0 ? -1 : groups);
+        if (at >= 0) {
+            const unsigned long long nv = wend - w0;
+            atomicAdd(&stats->m2p, s_m2p * nv);
+            atomicAdd(&stats->p2p, s_p2p * nv);
+            atomicAdd(&stats->total, (s_m2p + s_p2p) * nv);
+        }
+    }
+    if (at < 0) return;
+    for (int k = threadIdx.x; k < groups; k += blockDim.x) {
+        const unsigned low = (unsigned)sh.sorted[k];
+        pool[at + k] = make_uint2((unsigned)sh.first[(low >> 12) & 0xFFFu], low & 0xFFFu);
+    }
+}
+
+__device__ __forceinline__ void list_barrier()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(kLogListers) : "memory");
+}
+
+// Bound by dispatch: a term costs a warp 19 cycles (13 FP32 instructions, the
+// reciprocal root, two loads from shared memory), 0.2 ms in all at n = 100,000; with
+// the longest walk, whose terms are a chain, 0.46 ms.  A batch's records are loaded a
+// batch ahead (0.57 without), and a list is filled while the other is added up.
+template <bool ZERO_SOFT>
+__global__ void __launch_bounds__(64 + kLogListers)
+log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ body,
+                const uint32_t *__restrict__ order, int n, float eps2, double G,
+                double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
+                const int2 *__restrict__ walks, const uint2 *__restrict__ pool)
+{
+    __shared__ float4 s_term[2][kLogChunk];  // position, mass
+    __shared__ float2 s_soft[2][kLogChunk];  // eps^2, added before a body's r^2, after a node's
+    __shared__ int s_count[2];
+    // a batch of groups, a record per lister:
+    __shared__ float4 s_com[kLogListers];  // its term as a node
+    __shared__ int s_body[kLogListers];    // the first body of an opened leaf; -1: a node's term
+    __shared__ int s_incl[kLogListers];    // running count of terms
+    __shared__ int s_warp[kLogListers / 32];
+    const int2 walk = walks[blockIdx.x];
+    if (walk.y < 0) return;
+    const int w0 = blockIdx.x * 64;
+    if (threadIdx.x < 64) {
+        const int i = w0 + threadIdx.x;
+        const float4 q = body[i < n ? i : w0];
+        const float nx = -q.x, ny = -q.y, nz = -q.z;
+        float fx = 0.f, fy = 0.f, fz = 0.f;
+        for (int b = 0;; b ^= 1) {
+            __syncthreads();
+            const int count = s_count[b];
+            if (count == 0) break;
+#pragma unroll 8
+            for (int k = 0; k < count; ++k) {
+                const float4 t = s_term[b][k];
+                const float2 soft = s_soft[b][k];
+                const float dx = t.x + nx, dy = t.y + ny, dz = t.z + nz;
+                const float r2 =
+                    fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, soft.x))) + soft.y;
+                float inv = rsqrt_mufu(r2);
+                if (ZERO_SOFT) inv = r2 > 0.f ? inv : 0.f;
+                const float s = __fmul_rn(__fmul_rn(t.w, inv), __fmul_rn(inv, inv));
+                fx = fmaf(dx, s, fx);
+                fy = fmaf(dy, s, fy);
+                fz = fmaf(dz, s, fz);
+            }
+        }
+        if (i < n) {
+            const uint32_t o = order[i];
+            ax[o] = G * (double)fx;
+            ay[o] = G * (double)fy;
+            az[o] = G * (double)fz;
+        }
+        return;
+    }
+    // A lister's record of a batch, loaded a batch ahead, and the log entry of the
+    // batch after it: neither trip to memory waits for the other.
+    const int q = threadIdx.x - 64, lane = q & 31, wq = q >> 5;
+    const int child = q & 7;
+    auto load_log = [&](int g) {
+        return g < walk.y ? pool[walk.x + g] : make_uint2(0u, 0u);
+    };
+    auto load_node = [&](uint2 log) {
+        return gnodes[child < (int)(log.y >> 8) ? log.x + child : 0];
+    };
+    constexpr int kBatch = kLogListers / 8;
+    int next = 0;  // the next batch's first group
+    uint2 log = load_log(q >> 3), log_ahead = load_log(kBatch + (q >> 3));
+    BHGNode node_ahead = load_node(log);
+    int terms = 0, t0 = 0;  // of this batch: how many, how many listed
+    for (int b = 0;; b ^= 1) {
+        int filled = 0;
+        while (filled < kLogChunk) {
+            if (t0 == terms) {
+                if (next >= walk.y) break;
+                next += kBatch;
+                const BHGNode nd = node_ahead;
+                const bool have = child < (int)(log.y >> 8), open = (log.y >> child & 1u) != 0;
+                const int count = !have ? 0 : (!open ? 1 : (nd.kids < 0 ? nd.count : 0));
+                log = log_ahead;
+                node_ahead = load_node(log);
+                log_ahead = load_log(next + kBatch + (q >> 3));
+                int incl = count;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                list_barrier();  // the last batch's terms are read
+                if (lane == 31) s_warp[wq] = incl;
+                s_com[q] = nd.com_mass;
+                s_body[q] = open ? nd.first : -1;
+                list_barrier();
+#pragma unroll
+                for (int v = 0; v < kLogListers / 32 - 1; ++v)
+                    if (v < wq) incl += s_warp[v];
+                s_incl[q] = incl;
+                list_barrier();
+                terms = s_incl[kLogListers - 1];
+                t0 = 0;
+                continue;
+            }
+            const int take = min(kLogChunk - filled, terms - t0);
+            for (int k = q; k < take; k += kLogListers) {
+                const int t = t0 + k;
+                int node = 0;  // the number of running counts at most t
+#pragma unroll
+                for (int o = kLogListers / 2; o > 0; o >>= 1)
+                    if (s_incl[node + o - 1] <= t) node += o;
+                const int before = node > 0 ? s_incl[node - 1] : 0;
+                const int first = s_body[node];
+                float4 term;
+                if (first < 0) term = s_com[node];
+                else term = body[NB_IN_RANGE(first + t - before, n) ? first + t - before : 0];
+                s_term[b][filled + k] = term;
+                s_soft[b][filled + k] = first < 0 ? make_float2(0.f, eps2) : make_float2(eps2, 0.f);
+            }
+            filled += take;
+            t0 += take;
+        }
+        if (q == 0) s_count[b] = filled;
+        __syncthreads();
+        if (filled == 0) return;
+    }
+}
+
 int div_up(long a, long b) { return (int)((a + b - 1) / b); }
 
 template <class T>
@@ -1769,7 +2104,7 @@ struct BHTree {
     DevBuf part, root, keys0, keys1, vals0, vals1, hist, body, moments, prefix, chain_len,
         chain_depth, offsets, scan_tmp, nodes, node_depth, boxes, stats, moments2a, moments2b,
         prefix2a, prefix2b, quad, pcen, pstart, parent, octant, occ, kidflag, kbase, gnodes, gnk,
-        gpcen, gquad;
+        gpcen, gquad, gkey, walks, logs;
     bool with_quad = false;     // the nodes carry quadrupoles (quad, 2 float4 per node)
     bool ref_open = false;      // the reference's opening rule (the child toward the body too)
     bool pcen_valid = false;    // pcen holds the parent centres of the current topology
@@ -1800,7 +2135,7 @@ void bh_destroy(BHTree *t)
                       &t->boxes, &t->stats, &t->moments2a, &t->moments2b, &t->prefix2a,
                       &t->prefix2b, &t->quad, &t->pcen, &t->pstart, &t->parent, &t->octant,
                       &t->occ, &t->kidflag, &t->kbase, &t->gnodes,
-                      &t->gnk, &t->gpcen, &t->gquad};
+                      &t->gnk, &t->gpcen, &t->gquad, &t->gkey, &t->walks, &t->logs};
     for (DevBuf *b : bufs) b->release();
     if (t->h_total) cudaFreeHost(t->h_total);
     if (t->total_ready) cudaEventDestroy(t->total_ready);
@@ -1975,9 +2310,9 @@ nb_status bh_hilbert_order(BHTree *t, const double *x, const double *y, const do
 //   n =   262,144    999 /  928 /  881 /  913 / 1111
 //   n =   524,288   1380 / 1347 / 1364 / 1479 / 1887
 //   n = 1,048,576   2368 / 2395 / 2501 / 2725 / 3606
-// The reference's rule opens far more for some bodies than for others (the longest
-// walk at n = 100,000 has 20,270 interactions, the mean 3,891), so three times as
-// many, up to 16:
+// The reference's rule (its walks without a log) opens far more for some bodies than
+// for others (the longest walk at n = 100,000 has 20,270 interactions, the mean 3,891),
+// so three times as many, up to 16:
 //   n =   100,000   3141 / 1925 / 1196 /  922 /  830
 //   n =   400,000   7618 / 4921 / 3417 / 2928 / 3036
 // Quadrupoles hold more registers, so half as many:
@@ -2012,6 +2347,8 @@ bool group_walk()
     return !(e && std::strcmp(e, "preorder") == 0);
 }
 
+int log_pool_size(int n) { return (int)std::min((long)kLogPerBody * n + 64, (long)INT32_MAX); }
+
 template <bool ZS, bool Q, bool D>
 void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *ax, double *ay,
                  double *az, cudaStream_t st)
@@ -2023,13 +2360,31 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
         const unsigned char *gk = t->gnk.as<unsigned char>();
         const float4 *gq = t->gquad.as<float4>(), *gp = t->gpcen.as<float4>();
         const int ctas = div_up(n, 64 * np), warps = walk_warps<Q, D>(ctas);
+        const int2 *logged = nullptr;
+        if constexpr (D && !Q) {
+            if (np == 1) {
+                // logs: the pool's counter, then the pool
+                unsigned long long *next = t->logs.as<unsigned long long>();
+                uint2 *pool = reinterpret_cast<uint2 *>(next + 1);
+                int2 *walks = t->walks.as<int2>();
+                cudaMemsetAsync(next, 0, sizeof(*next), st);
+                cudaFuncSetAttribute(decide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(LogShared));
+                decide_kernel<<<ctas, 32 * kLogWarps, sizeof(LogShared), st>>>(
+                    gn, gk, t->gkey.as<unsigned>(), gp, d_total(t), t->body.as<float4>(), n,
+                    theta2, t->stats.as<BHStats>(), walks, pool, log_pool_size(n), next);
+                log_eval_kernel<ZS><<<ctas, 64 + kLogListers, 0, st>>>(gn, t->body.as<float4>(), t->order, n,
+                                                          eps2, G, ax, ay, az, walks, pool);
+                logged = walks;
+            }
+        }
         auto *kernel = np == 2 ? group_walk_kernel<ZS, Q, 2, D> : group_walk_kernel<ZS, Q, 1, D>;
         const size_t shared = walk_shared_bytes<Q>(warps);
         if (shared > 48 * 1024 - 256)
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
         kernel<<<ctas, 32 * warps, shared, st>>>(
             gn, gk, d_total(t), t->body.as<float4>(), t->order, n, theta2, eps2, G, ax, ay, az,
-            t->stats.as<BHStats>(), gq, gp);
+            t->stats.as<BHStats>(), gq, gp, logged);
     } else if (np == 2)
         walk2_kernel<ZS, Q, 2, D><<<div_up(n, 4 * kWalkBlock), kWalkBlock, 0, st>>>(
             t->nodes.as<BHNode>(), d_total(t), t->body.as<float4>(), t->order, n, theta2,
@@ -2057,6 +2412,10 @@ static nb_status launch_walk(BHTree *t, int n, double G, double eps2, double the
 {
     NvtxRange range("bh_walk");
     const float th2 = (float)(theta * theta), e2 = (float)eps2;
+    if (t->ref_open && !t->with_quad) {
+        NB_TRY(t->walks.reserve(sizeof(int2) * (size_t)div_up(n, 64)));
+        NB_TRY(t->logs.reserve(sizeof(uint2) * ((size_t)log_pool_size(n) + 1)));
+    }
     if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
     if (t->with_quad) {
         if (eps2 > 0.0) walk_launch_rule<false, true>(t, n, th2, e2, G, ax, ay, az, st);
@@ -2128,13 +2487,16 @@ static nb_status group_nodes(BHTree *t, cudaStream_t st, bool recount)
     NB_TRY(t->gnk.reserve((size_t)slots));
     if (t->ref_open) NB_TRY(t->gpcen.reserve(sizeof(float4) * (size_t)slots));
     if (t->with_quad) NB_TRY(t->gquad.reserve(sizeof(float4) * 2 * (size_t)slots));
+    const bool ordered = t->ref_open && !t->with_quad;  // walks with logs need the groups' ranks
+    if (ordered) NB_TRY(t->gkey.reserve(sizeof(unsigned) * (size_t)slots));
     group_kernel<<<grid, 256, 0, st>>>(
         t->nodes.as<BHNode>(), d_total(t), t->occ.as<unsigned>(), t->kbase.as<int>(),
         t->parent.as<int>(), t->octant.as<unsigned char>(),
         t->ref_open ? t->pcen.as<float4>() : nullptr,
         t->with_quad ? t->quad.as<float4>() : nullptr, t->gnodes.as<BHGNode>(),
         t->gnk.as<unsigned char>(), t->gpcen.as<float4>(),
-        t->with_quad ? t->gquad.as<float4>() : nullptr);
+        t->with_quad ? t->gquad.as<float4>() : nullptr, t->node_depth.as<unsigned char>(),
+        ordered ? t->gkey.as<unsigned>() : nullptr);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
