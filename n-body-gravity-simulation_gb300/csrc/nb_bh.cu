@@ -1772,11 +1772,11 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
 }
 
 // ---------------------------------------------------------- ordered walk
-// The reference's opening rule makes walks of 20,000 interactions (n = 100,000,
-// theta 0.5, disk galaxy), and an FP32 sum of so many terms depends on their order in
-// the fifth digit.  This walk adds each body's terms one after the other in the
-// order of a serial walk over a stack of groups (last pushed, first visited; a
-// group's records in order), in two kernels:
+// An FP32 sum of thousands of terms depends on their order in the fifth digit (walks
+// under the reference's opening rule have up to 20,000 at n = 100,000, theta 0.5,
+// disk galaxy), and a trajectory with it.  This walk adds each body's terms one after
+// the other in the order of a serial walk over a stack of groups (last pushed, first
+// visited; a group's records in order), in two kernels:
 //   - decide_kernel finds the groups that the walk visits and which of their records
 //     are opened, in any order, by many warps (as group_walk_kernel), and sorts
 //     the groups by their place in the serial walk of the whole tree: the rank
@@ -1784,45 +1784,60 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
 //     depth(v) - skip(v) but for a constant;
 //   - log_eval_kernel goes through a walk's groups in that order: four warps list the
 //     terms in shared memory, two add them up, a body per lane.
-// A walk that visits more than kLogGroups groups, or for whose log the pool has no
-// room, is left to group_walk_kernel.  A leapfrog step at n = 100,000: 3.87 ms with one
-// warp per walk, 1.06 in this way, 0.84 by group_walk_kernel, whose terms are in no
-// such order.
-constexpr int kLogGroups = 4096;  // at most 12 bits
-constexpr int kLogStack = 3072;
+// A walk that visits more groups than its log holds, or for whose log the pool has no
+// room, is left to group_walk_kernel.
+//
+// A force evaluation by one warp per walk (serial) / this walk / group_walk_kernel, in us:
+//   n =  16,384   712 /  315 /  281        reference's rule, n = 20,000:  1623 /  464 /  377
+//   n = 100,000   856 /  491 /  408        reference's rule, n = 100,000: 4242 / 1076 /  830
+//   n = 400,000  1484 / 1331 / 1095        quadrupoles, n = 100,000:      1001 /  750 /  619
+// Up to kOrderedBodies, and always under the reference's rule, this walk keeps the
+// serial walk's results bit for bit; beyond, where listing the terms apart from the
+// decisions eats what many warps gain (2^20 bodies: 2.88 ms serial, 2.28 by
+// group_walk_kernel), walks are of similar length and the order of summation shows in
+// velocities at 1e-8 of their scale after a step of 1e-3.
+constexpr int kOrderedBodies = 524288;
+// Up to this many walks 16 warps decide one, above it 4 (16 / 4 warps at 256, 512 and
+// 1024 walks: 314 / 332, 320 / 318, 406 / 380 us).  Under the reference's rule always 16,
+// with room for 4096 groups: its longest walks, not the number of walks, take the time.
+constexpr int kFewWalks = 400;
 constexpr int kLogPerBody = 16;   // pool entries per body (8 used at n = 100,000, theta 0.5)
-constexpr int kLogWarps = 16;     // of a decide_kernel CTA
 constexpr int kLogChunk = 256;    // terms per list
 constexpr int kLogListers = 128;  // threads of log_eval_kernel that list terms
 
+template <bool DIR, int WARPS, int GROUPS>
 struct LogShared {
-    unsigned long long sorted[kLogGroups];  // key, slot (12 bits), records (4), opened ones (8)
-    int first[kLogGroups];                  // by slot: the group's first record
-    float4 test[kLogWarps][32], side[kLogWarps][32];
-    int s_first[kLogStack];  // the stack: as group_walk_kernel's, and the groups' keys
-    unsigned s_key[kLogStack];
-    unsigned char s_kids[kLogStack];
+    static_assert(GROUPS <= 4096, "a slot has 12 bits");
+    static constexpr int kStack = 3 * GROUPS / 4;
+    unsigned long long sorted[GROUPS];  // key, slot (12 bits), records (4), opened ones (8)
+    int first[GROUPS];                  // by slot: the group's first record
+    float4 test[WARPS][32], side[DIR ? WARPS : 1][32];
+    int s_first[kStack];  // the stack: as group_walk_kernel's, and the groups' keys
+    unsigned s_key[kStack];
+    unsigned char s_kids[kStack];
 };
 
-// Bound by dispatch: with 0.35 ms at n = 100,000 (theta 0.5, disk galaxy), by the
-// longest walk (1,939 groups in 35 rounds of up to 64, of 10,000 cycles each with
+// Bound by dispatch; under the reference's rule, with 0.35 ms at n = 100,000 (theta
+// 0.5, disk galaxy), by that of the longest walk (1,939 groups in 35 rounds of up to 64, of 10,000 cycles each with
 // every node undecided by the boxes).  Tighter boxes (8 bodies each) and a pass over
 // the bodies per batch instead of one per node pair cost as much as they saved;
 // 8 warps took 0.12 ms longer, 4 warps for short walks with a second launch for the
 // rest 0.15.
-__global__ void __launch_bounds__(32 * kLogWarps, 2)
+template <bool DIR, int WARPS, int GROUPS>
+__global__ void __launch_bounds__(32 * WARPS, 32 / WARPS)
 decide_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restrict__ gnk,
               const unsigned *__restrict__ gkey, const float4 *__restrict__ gpcen,
               const int *__restrict__ total, const float4 *__restrict__ body, int n, float theta2,
               BHStats *__restrict__ stats, int2 *__restrict__ walks, uint2 *__restrict__ pool,
               int pool_size, unsigned long long *__restrict__ pool_next)
 {
-    constexpr int W = kLogWarps;
+    constexpr int W = WARPS;
     extern __shared__ __align__(16) unsigned char walk_shared[];
     __shared__ int s_push[W];
     __shared__ unsigned s_m2p, s_p2p;
     __shared__ int s_at;
-    LogShared &sh = *reinterpret_cast<LogShared *>(walk_shared);
+    using Shared = LogShared<DIR, WARPS, GROUPS>;
+    Shared &sh = *reinterpret_cast<Shared *>(walk_shared);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     [[maybe_unused]] const int num_nodes = *total;  // bounds checked builds only
     const int w0 = blockIdx.x * 64, wend = min(n, w0 + 64);
@@ -1848,7 +1863,7 @@ decide_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restric
     while (sp > 0) {
         __syncthreads();
         const int take = min(sp, 4 * W);
-        fits = groups + take <= kLogGroups;
+        fits = groups + take <= GROUPS;
         if (!fits) break;
         // the first groups to the first warps: in a narrow round the others have none
         const int j = 4 * w + (lane >> 3), e = sp - 1 - j;
@@ -1864,8 +1879,9 @@ decide_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restric
             id = have ? sh.s_first[e] + (lane & 7) : 0;
             const unsigned key = e >= 0 ? sh.s_key[e] : 0;
             nd = gnodes[NB_IN_RANGE(id, num_nodes) ? id : 0];
-            const bool open = opened_nodes<2, true>(nd, have, gpcen[id], box, p, theta2, w0, wend,
-                                                    sh.test[w], sh.side[w]);
+            const float4 pc = DIR ? gpcen[id] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const bool open = opened_nodes<2, DIR>(nd, have, pc, box, p, theta2, w0, wend,
+                                                   sh.test[w], sh.side[DIR ? w : 0]);
             const unsigned opened = __ballot_sync(0xffffffffu, have && open);
             if (have) {
                 if (!open) ++m2p;
@@ -1888,7 +1904,7 @@ decide_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restric
             if (v < w) top += s_push[v];
             sp += s_push[v];
         }
-        fits = sp <= kLogStack;
+        fits = sp <= Shared::kStack;
         if (!fits) break;
         if (inner) {
             const int to = top + __popc(push & ((1u << lane) - 1u));
@@ -1955,15 +1971,19 @@ __device__ __forceinline__ void list_barrier()
 // reciprocal root, two loads from shared memory), 0.2 ms in all at n = 100,000; with
 // the longest walk, whose terms are a chain, 0.46 ms.  A batch's records are loaded a
 // batch ahead (0.57 without), and a list is filled while the other is added up.
-template <bool ZERO_SOFT>
+template <bool ZERO_SOFT, bool QUAD>
 __global__ void __launch_bounds__(64 + kLogListers)
-log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ body,
+log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ gquad,
+                const float4 *__restrict__ body,
                 const uint32_t *__restrict__ order, int n, float eps2, double G,
                 double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
                 const int2 *__restrict__ walks, const uint2 *__restrict__ pool)
 {
     __shared__ float4 s_term[2][kLogChunk];  // position, mass
     __shared__ float2 s_soft[2][kLogChunk];  // eps^2, added before a body's r^2, after a node's
+    __shared__ float4 s_quad[2][QUAD ? kLogChunk : 1][2];
+    __shared__ unsigned char s_node[2][QUAD ? kLogChunk : 1];  // whether the term is a node's
+    __shared__ int s_id[QUAD ? kLogListers : 1];
     __shared__ int s_count[2];
     // a batch of groups, a record per lister:
     __shared__ float4 s_com[kLogListers];  // its term as a node
@@ -1995,6 +2015,19 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ b
                 fx = fmaf(dx, s, fx);
                 fy = fmaf(dy, s, fy);
                 fz = fmaf(dz, s, fz);
+                if (QUAD && s_node[b][k]) {
+                    const float4 q0 = s_quad[b][k][0], q1 = s_quad[b][k][1];
+                    const float qx = fmaf(q0.x, dx, fmaf(q0.w, dy, __fmul_rn(q1.x, dz)));
+                    const float qy = fmaf(q0.w, dx, fmaf(q0.y, dy, __fmul_rn(q1.y, dz)));
+                    const float qz = fmaf(q1.x, dx, fmaf(q1.y, dy, __fmul_rn(q0.z, dz)));
+                    const float rqr = fmaf(dx, qx, fmaf(dy, qy, __fmul_rn(dz, qz)));
+                    const float inv2 = __fmul_rn(inv, inv);
+                    const float inv5 = __fmul_rn(__fmul_rn(inv, inv2), inv2);
+                    const float f = __fmul_rn(__fmul_rn(2.5f, rqr), inv2);
+                    fx = fmaf(inv5, fmaf(f, dx, -qx), fx);
+                    fy = fmaf(inv5, fmaf(f, dy, -qy), fy);
+                    fz = fmaf(inv5, fmaf(f, dz, -qz), fz);
+                }
             }
         }
         if (i < n) {
@@ -2028,6 +2061,7 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ b
                 next += kBatch;
                 const BHGNode nd = node_ahead;
                 const bool have = child < (int)(log.y >> 8), open = (log.y >> child & 1u) != 0;
+                const int id = (int)log.x + child;
                 const int count = !have ? 0 : (!open ? 1 : (nd.kids < 0 ? nd.count : 0));
                 log = log_ahead;
                 node_ahead = load_node(log);
@@ -2041,6 +2075,7 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ b
                 list_barrier();  // the last batch's terms are read
                 if (lane == 31) s_warp[wq] = incl;
                 s_com[q] = nd.com_mass;
+                if (QUAD) s_id[q] = id;
                 s_body[q] = open ? nd.first : -1;
                 list_barrier();
 #pragma unroll
@@ -2062,8 +2097,15 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ b
                 const int before = node > 0 ? s_incl[node - 1] : 0;
                 const int first = s_body[node];
                 float4 term;
-                if (first < 0) term = s_com[node];
-                else term = body[NB_IN_RANGE(first + t - before, n) ? first + t - before : 0];
+                if (QUAD) s_node[b][filled + k] = first < 0;
+                if (first < 0) {
+                    term = s_com[node];
+                    if (QUAD) {
+                        const int id = s_id[node];
+                        s_quad[b][filled + k][0] = gquad[2 * id];
+                        s_quad[b][filled + k][1] = gquad[2 * id + 1];
+                    }
+                } else term = body[NB_IN_RANGE(first + t - before, n) ? first + t - before : 0];
                 s_term[b][filled + k] = term;
                 s_soft[b][filled + k] = first < 0 ? make_float2(0.f, eps2) : make_float2(eps2, 0.f);
             }
@@ -2107,6 +2149,7 @@ struct BHTree {
         gpcen, gquad, gkey, walks, logs;
     bool with_quad = false;     // the nodes carry quadrupoles (quad, 2 float4 per node)
     bool ref_open = false;      // the reference's opening rule (the child toward the body too)
+    bool ordered = false;       // walks add their terms in the serial walk's order (gkey is set)
     bool pcen_valid = false;    // pcen holds the parent centres of the current topology
     const uint64_t *sorted_codes = nullptr;
     const uint32_t *order = nullptr;
@@ -2361,22 +2404,27 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
         const float4 *gq = t->gquad.as<float4>(), *gp = t->gpcen.as<float4>();
         const int ctas = div_up(n, 64 * np), warps = walk_warps<Q, D>(ctas);
         const int2 *logged = nullptr;
-        if constexpr (D && !Q) {
-            if (np == 1) {
-                // logs: the pool's counter, then the pool
-                unsigned long long *next = t->logs.as<unsigned long long>();
-                uint2 *pool = reinterpret_cast<uint2 *>(next + 1);
-                int2 *walks = t->walks.as<int2>();
-                cudaMemsetAsync(next, 0, sizeof(*next), st);
-                cudaFuncSetAttribute(decide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(LogShared));
-                decide_kernel<<<ctas, 32 * kLogWarps, sizeof(LogShared), st>>>(
+        if (t->ordered && np == 1) {
+            // logs: the pool's counter, then the pool
+            unsigned long long *next = t->logs.as<unsigned long long>();
+            uint2 *pool = reinterpret_cast<uint2 *>(next + 1);
+            int2 *walks = t->walks.as<int2>();
+            cudaMemsetAsync(next, 0, sizeof(*next), st);
+            auto decide = [&](auto *kernel, int threads, size_t shared) {
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)shared);
+                kernel<<<ctas, threads, shared, st>>>(
                     gn, gk, t->gkey.as<unsigned>(), gp, d_total(t), t->body.as<float4>(), n,
                     theta2, t->stats.as<BHStats>(), walks, pool, log_pool_size(n), next);
-                log_eval_kernel<ZS><<<ctas, 64 + kLogListers, 0, st>>>(gn, t->body.as<float4>(), t->order, n,
-                                                          eps2, G, ax, ay, az, walks, pool);
-                logged = walks;
-            }
+            };
+            if (D || ctas <= kFewWalks)
+                decide(decide_kernel<D, 16, D ? 4096 : 1024>, 512,
+                       sizeof(LogShared<D, 16, D ? 4096 : 1024>));
+            else
+                decide(decide_kernel<D, 4, 1024>, 128, sizeof(LogShared<D, 4, 1024>));
+            log_eval_kernel<ZS, Q><<<ctas, 64 + kLogListers, 0, st>>>(
+                gn, gq, t->body.as<float4>(), t->order, n, eps2, G, ax, ay, az, walks, pool);
+            logged = walks;
         }
         auto *kernel = np == 2 ? group_walk_kernel<ZS, Q, 2, D> : group_walk_kernel<ZS, Q, 1, D>;
         const size_t shared = walk_shared_bytes<Q>(warps);
@@ -2412,7 +2460,7 @@ static nb_status launch_walk(BHTree *t, int n, double G, double eps2, double the
 {
     NvtxRange range("bh_walk");
     const float th2 = (float)(theta * theta), e2 = (float)eps2;
-    if (t->ref_open && !t->with_quad) {
+    if (t->ordered) {
         NB_TRY(t->walks.reserve(sizeof(int2) * (size_t)div_up(n, 64)));
         NB_TRY(t->logs.reserve(sizeof(uint2) * ((size_t)log_pool_size(n) + 1)));
     }
@@ -2487,8 +2535,8 @@ static nb_status group_nodes(BHTree *t, cudaStream_t st, bool recount)
     NB_TRY(t->gnk.reserve((size_t)slots));
     if (t->ref_open) NB_TRY(t->gpcen.reserve(sizeof(float4) * (size_t)slots));
     if (t->with_quad) NB_TRY(t->gquad.reserve(sizeof(float4) * 2 * (size_t)slots));
-    const bool ordered = t->ref_open && !t->with_quad;  // walks with logs need the groups' ranks
-    if (ordered) NB_TRY(t->gkey.reserve(sizeof(unsigned) * (size_t)slots));
+    t->ordered = t->ref_open || t->n <= kOrderedBodies;
+    if (t->ordered) NB_TRY(t->gkey.reserve(sizeof(unsigned) * (size_t)slots));
     group_kernel<<<grid, 256, 0, st>>>(
         t->nodes.as<BHNode>(), d_total(t), t->occ.as<unsigned>(), t->kbase.as<int>(),
         t->parent.as<int>(), t->octant.as<unsigned char>(),
@@ -2496,7 +2544,7 @@ static nb_status group_nodes(BHTree *t, cudaStream_t st, bool recount)
         t->with_quad ? t->quad.as<float4>() : nullptr, t->gnodes.as<BHGNode>(),
         t->gnk.as<unsigned char>(), t->gpcen.as<float4>(),
         t->with_quad ? t->gquad.as<float4>() : nullptr, t->node_depth.as<unsigned char>(),
-        ordered ? t->gkey.as<unsigned>() : nullptr);
+        t->ordered ? t->gkey.as<unsigned>() : nullptr);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
