@@ -1801,7 +1801,9 @@ constexpr int kOrderedBodies = 524288;
 // 1024 walks: 314 / 332, 320 / 318, 406 / 380 us).  Under the reference's rule always 16,
 // with room for 4096 groups: its longest walks, not the number of walks, take the time.
 constexpr int kFewWalks = 400;
-constexpr int kLogPerBody = 16;   // pool entries per body (8 used at n = 100,000, theta 0.5)
+// Pool entries per body, the second under the reference's rule (4 and 8 used at
+// n = 100,000, theta 0.5).
+constexpr int kLogPerBody[2] = {8, 16};
 constexpr int kLogChunk = 256;    // terms per list
 constexpr int kLogListers = 128;  // threads of log_eval_kernel that list terms
 
@@ -2169,6 +2171,13 @@ void bh_mark_count_stale(BHTree *t)
 
 BHTree *bh_create() { return new BHTree(); }
 
+nb_status bh_restart(BHTree *t, cudaStream_t st)
+{
+    t->tree_valid = false;
+    if (t->stats.ptr) NB_CUDA_TRY(cudaMemsetAsync(t->stats.ptr, 0, sizeof(BHStats), st));
+    return NB_OK;
+}
+
 void bh_destroy(BHTree *t)
 {
     if (!t) return;
@@ -2390,7 +2399,10 @@ bool group_walk()
     return !(e && std::strcmp(e, "preorder") == 0);
 }
 
-int log_pool_size(int n) { return (int)std::min((long)kLogPerBody * n + 64, (long)INT32_MAX); }
+int log_pool_size(const BHTree *t, int n)
+{
+    return (int)std::min((long)kLogPerBody[t->ref_open] * n + 64, (long)INT32_MAX);
+}
 
 template <bool ZS, bool Q, bool D>
 void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *ax, double *ay,
@@ -2415,7 +2427,7 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
                                      (int)shared);
                 kernel<<<ctas, threads, shared, st>>>(
                     gn, gk, t->gkey.as<unsigned>(), gp, d_total(t), t->body.as<float4>(), n,
-                    theta2, t->stats.as<BHStats>(), walks, pool, log_pool_size(n), next);
+                    theta2, t->stats.as<BHStats>(), walks, pool, log_pool_size(t, n), next);
             };
             if (D || ctas <= kFewWalks)
                 decide(decide_kernel<D, 16, D ? 4096 : 1024>, 512,
@@ -2462,7 +2474,7 @@ static nb_status launch_walk(BHTree *t, int n, double G, double eps2, double the
     const float th2 = (float)(theta * theta), e2 = (float)eps2;
     if (t->ordered) {
         NB_TRY(t->walks.reserve(sizeof(int2) * (size_t)div_up(n, 64)));
-        NB_TRY(t->logs.reserve(sizeof(uint2) * ((size_t)log_pool_size(n) + 1)));
+        NB_TRY(t->logs.reserve(sizeof(uint2) * ((size_t)log_pool_size(t, n) + 1)));
     }
     if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
     if (t->with_quad) {

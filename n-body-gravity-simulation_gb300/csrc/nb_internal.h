@@ -294,6 +294,8 @@ nb_status batch_sorted_forces(BatchSorted &b, const double *x, const double *y, 
 struct BHTree;  // opaque, defined in nb_bh.cu
 BHTree *bh_create();
 void bh_destroy(BHTree *t);
+// The tree object for other bodies: no topology, its counters at zero; its buffers stay.
+nb_status bh_restart(BHTree *t, cudaStream_t st);
 // Builds the tree of (x,y,z,m) and, when ax != nullptr, walks it writing
 // G * acceleration (FP64) in the original body order.  reuse > 1: the tree is
 // rebuilt every `reuse` walks; the walks in between keep its topology and

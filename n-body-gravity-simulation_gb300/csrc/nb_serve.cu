@@ -16,7 +16,8 @@
 //        that stream's later jobs), overlapping with the direct batch and
 //        with each other;
 //   3. retires jobs that reached their step count (state copied to the host,
-//      memory returned).
+//      pool slots returned, simulation objects kept for jobs to come within
+//      the budget).
 // A job's arithmetic does not depend on the other jobs of a tick (the batched
 // kernel sums each system alone, updates are per body, Barnes-Hut jobs are
 // separate objects), so its result is the same alone and in any mix.
@@ -46,6 +47,7 @@ using Clock = std::chrono::steady_clock;
 constexpr size_t kDirectBytesPerBody = 10 * 8 + 32;  // FP64 planes + hi/lo mirror
 constexpr size_t kBHBytesPerBody = 320;              // state + sort + tree buffers (upper bound)
 constexpr int kBHStreams = 16;
+constexpr size_t kIdleSims = 32;
 
 struct Job {
     int64_t id = 0;
@@ -57,6 +59,7 @@ struct Job {
     std::vector<double> result; // 10 n after retirement
     size_t first = 0;           // pool slot (direct)
     nb_sim *sim = nullptr;      // Barnes-Hut
+    size_t bytes = 0;           // its share of the budget
     int stream_index = 0;
     Clock::time_point submitted, admitted;
     bool finished = false;
@@ -220,6 +223,13 @@ struct nb_server {
     std::vector<std::unique_ptr<nb::Job>> running;
     std::map<int64_t, std::unique_ptr<nb::Job>> finished;
     size_t bh_bytes = 0;
+    // Simulations of jobs that have ended, oldest first, for jobs to come: making
+    // one costs about fifty device allocations and frees (half of the 20 ms that a burst
+    // of 16 jobs with seven trees, four steps, took to run; 10.2 ms now).  They count towards the budget and go
+    // when a job needs it, when there are more than kIdleSims, and with the server.
+    // Only the thread that ticks touches them, between ticks.
+    std::vector<nb_sim *> idle;
+    size_t idle_bytes = 0;
     size_t peak_bytes = 0;
     bool items_dirty = true;
     cudaEvent_t tick_start = nullptr, direct_done = nullptr;
@@ -260,6 +270,58 @@ nb_status upload_systems(nb_server *s, const std::vector<Job *> &jobs, nb_server
     return NB_OK;
 }
 
+size_t sim_bytes(const nb_sim *sim) { return kBHBytesPerBody * sim->capacity; }
+
+void drop_idle(nb_server *s, size_t k)
+{
+    s->idle_bytes -= sim_bytes(s->idle[k]);
+    nb_destroy(s->idle[k]);
+    s->idle.erase(s->idle.begin() + k);
+}
+
+// Keeps an ended job's simulation (none of its work is in flight).
+void keep_sim(nb_server *s, Job *j)
+{
+    s->bh_bytes -= j->bytes;
+    s->idle.push_back(j->sim);
+    s->idle_bytes += sim_bytes(j->sim);
+    j->sim = nullptr;
+    if (s->idle.size() > kIdleSims) drop_idle(s, 0);
+}
+
+// A simulation for n bodies on stream st: the smallest idle one that is not
+// over a quarter too large (and fits the budget at its size), or a new one.
+nb_status take_sim(nb_server *s, const nb_config &c, size_t n, cudaStream_t st, nb_sim **out)
+{
+    size_t best = s->idle.size();
+    for (size_t k = 0; k < s->idle.size(); ++k) {
+        const size_t cap = s->idle[k]->capacity;
+        if (cap >= n && cap <= n + n / 4 &&
+            pool_bytes(s) + s->bh_bytes + sim_bytes(s->idle[k]) <= s->cfg.hbm_budget_bytes &&
+            (best == s->idle.size() || cap < s->idle[best]->capacity))
+            best = k;
+    }
+    if (best < s->idle.size()) {
+        nb_sim *sim = s->idle[best];
+        sim->stream = st;  // its old stream is idle between ticks
+        if (!sim->bh || bh_restart(sim->bh, st) == NB_OK) {
+            s->idle_bytes -= sim_bytes(sim);
+            s->idle.erase(s->idle.begin() + best);
+            *out = sim;
+            return NB_OK;
+        }
+        drop_idle(s, best);
+    }
+    const size_t need = kBHBytesPerBody * n;
+    while (!s->idle.empty() &&
+           pool_bytes(s) + s->bh_bytes + need + s->idle_bytes > s->cfg.hbm_budget_bytes)
+        drop_idle(s, 0);
+    const nb_status r = nb_create(&c, n, st, out);
+    if (r == NB_OK || s->idle.empty()) return r;
+    while (!s->idle.empty()) drop_idle(s, 0);
+    return nb_create(&c, n, st, out);
+}
+
 // Frees a running job's device state (pool slot, or its simulation and its
 // share of the budget) and its event.  Only between ticks: nothing of the job
 // is in flight then.
@@ -268,9 +330,13 @@ void drop_resources(nb_server *s, Job *j)
     if (j->direct) {
         s->slots.give(j->first, j->n);
     } else if (j->sim) {
-        nb_destroy(j->sim);
-        j->sim = nullptr;
-        s->bh_bytes -= kBHBytesPerBody * j->n;
+        if (j->status == NB_ERR_CANCELLED) {
+            keep_sim(s, j);
+        } else {
+            nb_destroy(j->sim);
+            j->sim = nullptr;
+            s->bh_bytes -= j->bytes;
+        }
     }
     if (j->step_done) cudaEventDestroy(j->step_done);
     j->step_done = nullptr;
@@ -319,7 +385,7 @@ nb_status admit(nb_server *s, std::vector<Job *> &new_direct)
                 cudaStream_t st = s->bh_streams[j->stream_index];
                 const double *p = j->init.data();
                 const size_t n = j->n;
-                nb_status r = nb_create(&c, n, st, &j->sim);
+                nb_status r = take_sim(s, c, n, st, &j->sim);
                 if (r == NB_OK)
                     r = nb_load(j->sim, n, p, p + n, p + 2 * n, p + 3 * n, p + 4 * n,
                                 p + 5 * n, p + 6 * n);
@@ -337,7 +403,8 @@ nb_status admit(nb_server *s, std::vector<Job *> &new_direct)
                     it = s->queue.erase(it);
                     continue;
                 }
-                s->bh_bytes += need;
+                j->bytes = sim_bytes(j->sim);
+                s->bh_bytes += j->bytes;
                 ok = true;
             }
         }
@@ -354,7 +421,7 @@ nb_status admit(nb_server *s, std::vector<Job *> &new_direct)
             ++it;
         }
     }
-    s->peak_bytes = std::max(s->peak_bytes, pool_bytes(s) + s->bh_bytes);
+    s->peak_bytes = std::max(s->peak_bytes, pool_bytes(s) + s->bh_bytes + s->idle_bytes);
     return NB_OK;
 }
 
@@ -387,9 +454,7 @@ nb_status retire(nb_server *s)
             nb_bh_info info;
             if (nb_bh_get_info(j->sim, &info) == NB_OK)
                 s->interactions += (double)info.interactions_total;
-            nb_destroy(j->sim);
-            j->sim = nullptr;
-            s->bh_bytes -= kBHBytesPerBody * n;
+            keep_sim(s, j);
         }
         cudaEventDestroy(j->step_done);
         j->step_done = nullptr;
@@ -580,6 +645,7 @@ nb_status nb_server_destroy(nb_server *s)
     if (!s) return NB_OK;
     s->pool_threads.stop();
     if (s->stream) cudaStreamSynchronize(s->stream);
+    while (!s->idle.empty()) drop_idle(s, 0);
     for (auto &j : s->running) {
         if (j->sim) nb_destroy(j->sim);
         if (j->step_done) cudaEventDestroy(j->step_done);
