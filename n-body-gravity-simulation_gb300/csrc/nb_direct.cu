@@ -36,6 +36,8 @@
 #include "nb_after.cuh"
 #include "nb_tile.cuh"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -140,8 +142,7 @@ __global__ void __launch_bounds__(32 * kCombineGroups)
 combine_mixed_kernel(const float *__restrict__ psum,
                                      const float *__restrict__ pcomp, int n, int segments,
                                      double G, double *__restrict__ ax,
-                                     double *__restrict__ ay, double *__restrict__ az,
-                                     const AfterForce after)
+                                     double *__restrict__ ay, double *__restrict__ az)
 {
     __shared__ float2 sh[kCombineGroups][3][32];
     const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -175,9 +176,89 @@ combine_mixed_kernel(const float *__restrict__ psum,
     for (int k = 0; k < kCombineGroups; ++k)
         ds_add_kahan(s.x, s.y, sh[k][c][lane].x, -sh[k][c][lane].y);
     double *out = c == 0 ? ax : (c == 1 ? ay : az);
-    const double a = G * ((double)s.x + (double)s.y);
-    out[i] = a;
-    after_force(after, c, i, a);
+    out[i] = G * ((double)s.x + (double)s.y);
+}
+
+// ---------------------------------------------------------------- mixed, small systems
+// Below kMixedPairsMin bodies a cluster of 8 CTAs sums 32 i-bodies: each of its 32 warps
+// takes a share of the j-tiles (as direct_mixed_kernel does), a CTA combines its warps'
+// Kahan pairs, and the first the eight CTAs': no partial sums in memory, and no second
+// launch.
+// Bound by latency: launch, two trips to memory, the tiles' 16 steps each, the ordered
+// sums.  A velocity-Verlet step at n = 100 / 1000 / 2000 / 4000 takes 10.4 / 12.4 / 16.5 /
+// 26.8 us in a row of steps, with the sums in a second kernel 14.5 / 16.5 / 21.3 / 30.8;
+// 8 warps per CTA 10.4 / 14.5 / 16.5 / 25.2, two i-bodies per lane no less.
+constexpr int kSmallCtas = 8, kSmallWarps = 4;
+
+template <bool ZERO_SOFT>
+__global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(32 * kSmallWarps)
+direct_mixed_small_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo, int n,
+                          float eps2, int warp_tiles, double G, double *__restrict__ ax,
+                          double *__restrict__ ay, double *__restrict__ az,
+                          const AfterForce after)
+{
+    __shared__ PairTile tiles[kSmallWarps];
+    __shared__ float2 part[kSmallWarps][3][32];  // a warp's Kahan pairs (sum, comp)
+    __shared__ float2 sum[3][32];                // the CTA's, as double-singles
+    auto cluster = cooperative_groups::this_cluster();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int rank = blockIdx.x % kSmallCtas;
+    const int i = blockIdx.x / kSmallCtas * 32 + lane;
+
+    // the i-body negated and duplicated into f32x2 pairs
+    float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
+    if (i < n) {
+        h = hi[i];
+        l = lo[i];
+    }
+    const float2 nxh = dup2(-h.x), nyh = dup2(-h.y), nzh = dup2(-h.z);
+    const float2 nxl = dup2(-l.x), nyl = dup2(-l.y), nzl = dup2(-l.z);
+    const float2 e2 = dup2(eps2);
+    float s[3] = {0.f, 0.f, 0.f}, q[3] = {0.f, 0.f, 0.f};
+    const int j0 = (rank * kSmallWarps + w) * warp_tiles * 32;
+    const int j1 = min(n, j0 + warp_tiles * 32);
+    for (int t0 = j0; t0 < j1; t0 += 32) {
+        const int j = t0 + lane;
+        h = far_body();
+        l = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j < j1) {
+            h = hi[j];
+            l = lo[j];
+        }
+        __syncwarp();
+        pair_tile_put(tiles[w], lane, h.x, h.y, h.z, h.w, l.x, l.y, l.z);
+        __syncwarp();
+        float2 t[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
+#pragma unroll 2
+        for (int p = 0; p < 16; ++p)
+            pair_term2<ZERO_SOFT>(pair_tile_get(tiles[w], p), nxh, nyh, nzh, nxl, nyl, nzl, e2,
+                                  t[0], t[1], t[2]);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) kahan_add(s[c], q[c], t[c].x + t[c].y);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) part[w][c][lane] = make_float2(s[c], q[c]);
+    __syncthreads();
+    if (w < 3) {
+        float2 v = dup2(0.f);
+#pragma unroll
+        for (int u = 0; u < kSmallWarps; ++u)
+            ds_add_kahan(v.x, v.y, part[u][w][lane].x, part[u][w][lane].y);
+        sum[w][lane] = v;
+    }
+    cluster.sync();
+    if (rank == 0 && w < 3 && i < n) {  // warp c finishes component c
+        float2 t[kSmallCtas], v = dup2(0.f);
+#pragma unroll
+        for (int u = 0; u < kSmallCtas; ++u) t[u] = *cluster.map_shared_rank(&sum[w][lane], u);
+#pragma unroll
+        for (int u = 0; u < kSmallCtas; ++u) ds_add_kahan(v.x, v.y, t[u].x, -t[u].y);
+        double *out = w == 0 ? ax : (w == 1 ? ay : az);
+        const double a = G * ((double)v.x + (double)v.y);
+        out[i] = a;
+        after_force(after, w, i, a);
+    }
+    cluster.sync();  // no CTA leaves while its sums are read
 }
 
 // ---------------------------------------------------------------- mixed, unordered pairs
@@ -719,18 +800,14 @@ nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, doub
     if (n <= 0) return NB_OK;
     if (n >= kMixedPairsMin)
         return direct_mixed_pairs(hi, lo, n, G, eps2, ax, ay, az, partials, st, timer, after);
-    const DirectPlan p = direct_mixed_plan(n);
-    NB_TRY(partials.reserve(sizeof(float) * 6 * (size_t)n * p.segments));
-    float *psum = partials.as<float>();
-    float *pcomp = psum + 3 * (size_t)n * p.segments;
     if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
-    if (!launch_mixed(p, st, hi, lo, n, eps2, psum, pcomp))
-        return fail(NB_ERR_UNSUPPORTED, "direct_mixed: unsupported tile shape");
+    const int tiles = (n + 31) / 32, warps = kSmallCtas * kSmallWarps;
+    auto *kernel = eps2 > 0.0 ? direct_mixed_small_kernel<false> : direct_mixed_small_kernel<true>;
+    kernel<<<tiles * kSmallCtas, 32 * kSmallWarps, 0, st>>>(
+        hi, lo, n, eps2 > 0.0 ? (float)eps2 : 0.0f, (tiles + warps - 1) / warps, G, ax, ay, az,
+        after);
     NB_LAUNCH_CHECK();
     if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
-    combine_mixed_kernel<<<(n + 31) / 32, 32 * kCombineGroups, 0, st>>>(
-        psum, pcomp, n, p.segments, G, ax, ay, az, after);
-    NB_LAUNCH_CHECK();
     return NB_OK;
 }
 
@@ -910,7 +987,7 @@ extern "C" nb_status nb_direct_mixed_forces_noalloc(size_t n, const double *x, c
         return fail(NB_ERR_UNSUPPORTED, "nb_direct_mixed_forces_noalloc: tile shape");
     NB_LAUNCH_CHECK();
     combine_mixed_kernel<<<(ni + 31) / 32, 32 * kCombineGroups, 0, st>>>(
-        psum, pcomp, ni, p.segments, G, ax, ay, az, AfterForce{});
+        psum, pcomp, ni, p.segments, G, ax, ay, az);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
