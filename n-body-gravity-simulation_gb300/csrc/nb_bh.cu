@@ -74,7 +74,7 @@ struct BHRoot {
     int levels;                     // depths the root may split into (<= 21)
     float margin;                   // encode_kernel: distance from a grid line, in cells
     double scale;                   // 2^21 / size
-    double lo[3], lo_scaled[3];     // the cube's lower corner, and that times scale
+    double lo[3], grid_lo[3];       // the cube's lower corner; kGridBase - that times scale
 };
 
 // A leaf is the node whose skip pointer is the next node (no subtree).
@@ -92,6 +92,10 @@ struct BHStats {
     int leaves, max_depth;
     unsigned long long total;     // terms of every walk of this tree object (never reset)
 };
+
+// Added to a position in cells of the 2^21 grid (grid_index).
+constexpr double kGridBase = 402653184.0;  // 1.5 * 2^28
+constexpr unsigned long long kGridBits = 0x41B8000000000000ull;
 
 // ------------------------------------------------------------ bounding box
 __global__ void __launch_bounds__(256)
@@ -208,7 +212,7 @@ bbox_final_kernel(const long long *__restrict__ part, int nparts, BHRoot *root)
         if (lane == k) {
             (&root->cx)[k] = c;
             root->lo[k] = lo;
-            root->lo_scaled[k] = lo * scale;
+            root->grid_lo[k] = kGridBase - lo * scale;
         }
     }
     if (lane != 0) return;
@@ -228,17 +232,18 @@ bbox_final_kernel(const long long *__restrict__ part, int nparts, BHRoot *root)
 // cube and whether the position is far enough from every grid line that the
 // CPU tree's rounded running centres cannot compare differently.  f carries a
 // few roundings of ~2^-31 grid cells; the margin (>= 1e-6 cells) covers them.
-// Five FP64 operations (the FP64 pipe bounds this kernel): f, its floor as an
-// integer, back to FP64, the fraction, and the fraction in FP32 (an error of
-// ~2^-24, far below the margin) for the two comparisons.
-__device__ __forceinline__ bool grid_index(double p, double lo_scaled, double scale,
-                                           float margin, uint64_t *q)
+// One FP64 operation (the FP64 pipe bounds this kernel): the index f + kGridBase has
+// an ulp of 2^-24 cells, so its bits less kGridBase's are the index in fixed point,
+// 24 bits of it the fraction (two more roundings of 2^-25 cells, far below the
+// margin).  With f, its floor and its fraction in FP64 the kernel took 34 us at
+// N = 2^20, 14 now.
+__device__ __forceinline__ bool grid_index(double p, double lo, double scale, float margin,
+                                           uint64_t *q)
 {
-    const double f = fma(p, scale, -lo_scaled);
-    const long long fl = min(max(__double2ll_rd(f), 0ll), 2097151ll);
-    *q = (uint64_t)fl;
-    const float frac = __double2float_rn(f - (double)fl);  // in [0, 1) unless clamped
-    return frac > margin && frac < 1.0f - margin;
+    const unsigned long long f = (unsigned long long)bits_of(fma(p, scale, lo)) - kGridBits;
+    *q = f >> 24;
+    const float frac = (float)((unsigned)f & 0xFFFFFFu) * 5.9604644775390625e-8f;
+    return f < 1ull << 45 && frac > margin && frac < 1.0f - margin;
 }
 
 __global__ void __launch_bounds__(256)
@@ -253,9 +258,9 @@ encode_kernel(const double *__restrict__ x, const double *__restrict__ y,
     const int levels = root->levels;
     const double px = x[i], py = y[i], pz = z[i];
     uint64_t qx, qy, qz;
-    const bool okx = grid_index(px, root->lo_scaled[0], scale, margin, &qx);
-    const bool oky = grid_index(py, root->lo_scaled[1], scale, margin, &qy);
-    const bool okz = grid_index(pz, root->lo_scaled[2], scale, margin, &qz);
+    const bool okx = grid_index(px, root->grid_lo[0], scale, margin, &qx);
+    const bool oky = grid_index(py, root->grid_lo[1], scale, margin, &qy);
+    const bool okz = grid_index(pz, root->grid_lo[2], scale, margin, &qz);
     if (okx && oky && okz) {
         uint64_t code = (spread21(qx) << 2) | (spread21(qy) << 1) | spread21(qz);
         const int drop = 3 * (kMaxLevels - levels);  // digits below the split limit are 0
@@ -622,33 +627,51 @@ gather2_kernel(const uint32_t *__restrict__ order, const double *__restrict__ x,
     mb[i] = D4{mm * rx * rz, mm * ry * rz, 0.0, 0.0};
 }
 
-// One past the last body of the depth-d cell that contains bodies i .. from - 1.
-__device__ __forceinline__ int cell_end(const uint64_t *__restrict__ c, int n, int i, int d,
-                                        int from)
+// One past the last body of the depth-d cell of body i, its first: several probes per
+// round trip to memory, first the next eight bodies (which ends the search of a leaf),
+// then at distances 8^k, then within the bracket.
+__device__ __forceinline__ int cell_end(const uint64_t *__restrict__ c, int n, int i, int d)
 {
     if (d == 0) return n;
     const int sh = 63 - 3 * d;
     const uint64_t p = c[i] >> sh;
-    int lo = from - 1, hi, step = from - i;
-    while (true) {
-        hi = lo + step;
-        if (hi >= n) {
-            hi = n;
-            break;
+    const long limit = n - i;
+    auto inside = [&](long k) { return k < limit && (c[i + k] >> sh) == p; };
+    bool in[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) in[k] = inside(k + 1);
+    long lo = 0, hi;  // lo inside, hi not
+#pragma unroll
+    for (int k = 0; k < 8; ++k) lo += in[k];
+    if (lo < 8) return i + (int)lo + 1;
+#pragma unroll
+    for (int k = 2; k < 8; ++k) in[k] = inside(1l << 3 * k);
+    hi = 64;
+#pragma unroll
+    for (int k = 2; k < 8; ++k)
+        if (in[k]) {
+            lo = 1l << 3 * k;
+            hi = 8 * lo;
         }
-        if ((c[hi] >> sh) != p) break;
+    while (in[7] && inside(hi)) {  // beyond 8^7
         lo = hi;
-        step <<= 1;
+        hi = 8 * lo;
     }
+    hi = hi < limit ? hi : limit;
     while (hi - lo > 1) {
-        const int mid = lo + (hi - lo) / 2;
-        if ((c[mid] >> sh) == p) lo = mid;
-        else hi = mid;
+        const long step = (hi - lo + 7) / 8, from = lo;
+#pragma unroll
+        for (int k = 1; k < 8; ++k) in[k] = k * step < hi - from && inside(from + k * step);
+#pragma unroll
+        for (int k = 1; k < 8; ++k)
+            if (in[k]) lo = from + k * step;
+        hi = hi < lo + step ? hi : lo + step;
     }
-    return hi;
+    return i + (int)lo + 1;
 }
 
-// First index of the depth-d cell that contains body i.
+// First index of the depth-d cell that contains body i (galloping: most of the
+// searches are short).
 __device__ __forceinline__ int cell_start(const uint64_t *__restrict__ c, int i, int d)
 {
     if (d == 0) return 0;
@@ -756,50 +779,67 @@ __device__ __forceinline__ float4 parent_centre(uint64_t code, int d, const BHRo
                        (float)(((double)iz + 0.5) * side - h), __int_as_float(oct));
 }
 
+// The nodes' first bodies and depths, by the bodies their chains start at.
 __global__ void __launch_bounds__(256)
-node_kernel(const uint64_t *__restrict__ c, int n, int cap, const BHRoot *__restrict__ root,
-            const int *__restrict__ chain_len, const int *__restrict__ chain_depth,
+place_kernel(int n, const int *__restrict__ chain_len, const int *__restrict__ chain_depth,
+             const int *__restrict__ offsets, BHNode *__restrict__ nodes,
+             unsigned char *__restrict__ node_depth, int node_cap)
+{
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const int L = chain_len[i];
+    if (L == 0) return;
+    const int a = chain_depth[i], id0 = offsets[i];
+    for (int k = 0; k < L; ++k) {
+        if (!NB_IN_RANGE(id0 + k, node_cap)) break;
+        nodes[id0 + k].first = i;
+        node_depth[id0 + k] = (unsigned char)(a + k);
+    }
+}
+
+// The rest of every node, a thread per node.  By body, a thread writing its chain,
+// the longest chain was the critical path, and few lanes of a warp had the FP64 work:
+// 79 us at N = 2^20, 31 at 100,000; 43 and 20 now, with place_kernel.
+__global__ void __launch_bounds__(256)
+node_kernel(const uint64_t *__restrict__ c, int n, const BHRoot *__restrict__ root,
+            const int *__restrict__ total, const int *__restrict__ chain_depth,
             const int *__restrict__ offsets, const D4 *__restrict__ P,
-            BHNode *__restrict__ nodes, unsigned char *__restrict__ node_depth,
+            BHNode *__restrict__ nodes, const unsigned char *__restrict__ node_depth,
             const int *__restrict__ pstart, int *__restrict__ parent,
             unsigned char *__restrict__ octant, unsigned char *__restrict__ kidflag,
             BHStats *__restrict__ stats, int node_cap)
 {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    const int L = i < n ? chain_len[i] : 0;
-    const int a = L > 0 ? chain_depth[i] : 0;
-    const int id0 = L > 0 ? offsets[i] : 0;
-    const D4 before = L > 0 ? P[i] : D4{0.0, 0.0, 0.0, 0.0};
-    int end = i + 1;
-    for (int k = L - 1; k >= 0; --k) {  // deepest first: each cell holds the one before
-        const int d = a + k;
-        end = cell_end(c, n, i, d, end);
-        if (!NB_IN_RANGE(id0 + k, node_cap) || !NB_IN_RANGE(end, n + 1)) break;
+    const int num = *total;
+    int leaves = 0, deepest = 0;
+    for (int k = blockIdx.x * 256 + threadIdx.x; k < num; k += gridDim.x * 256) {
+        if (!NB_IN_RANGE(k, node_cap)) break;
         BHNode nd;
-        nd.com_mass = monopole(before, P[end]);
-        nd.first = i;
+        const int i = nd.first = nodes[k].first, d = node_depth[k];
+        const int end = cell_end(c, n, i, d);
+        if (!NB_IN_RANGE(i, n) || !NB_IN_RANGE(end, n + 1)) continue;
+        nd.com_mass = monopole(P[i], P[end]);
         nd.count = end - i;
         nd.skip = offsets[end];
         nd.size2 = root->size2[d];
-        nodes[id0 + k] = nd;
-        node_depth[id0 + k] = (unsigned char)d;
+        nodes[k] = nd;
         if (d > 0) {  // the parent: the previous node of the chain, or the one holding it
-            int par = id0 + k - 1;
-            if (k == 0) {
+            int par = k - 1;
+            if (k == offsets[i]) {
                 const int j = pstart[i];
                 par = offsets[j] + (d - 1 - chain_depth[j]);
             }
             const int oct = (int)((c[i] >> (63 - 3 * d)) & 7u);
-            parent[id0 + k] = par;
-            octant[id0 + k] = (unsigned char)oct;
+            parent[k] = par;
+            octant[k] = (unsigned char)oct;
             if (NB_IN_RANGE(par, node_cap)) kidflag[(size_t)par * 8 + oct] = 1;
         }
+        leaves += nd.skip == k + 1;
+        deepest = max(deepest, d);
     }
-    // every chain ends in a leaf
-    const unsigned leaves = __popc(__ballot_sync(0xffffffffu, L > 0));
-    const int deepest = __reduce_max_sync(0xffffffffu, L > 0 ? a + L - 1 : 0);
+    leaves = __reduce_add_sync(0xffffffffu, leaves);
+    deepest = __reduce_max_sync(0xffffffffu, deepest);
     if ((threadIdx.x & 31) == 0 && leaves > 0) {
-        atomicAdd(&stats->leaves, (int)leaves);
+        atomicAdd(&stats->leaves, leaves);
         atomicMax(&stats->max_depth, deepest);
     }
 }
@@ -2665,15 +2705,17 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
     t->n = n;
     NB_CUDA_TRY(cudaMemsetAsync(stats, 0, offsetof(BHStats, total), st));
     NB_CUDA_TRY(cudaMemsetAsync(t->kidflag.ptr, 0, 8 * cap, st));
-    node_kernel<<<div_up(n, 256), 256, 0, st>>>(kin, n, leaf_capacity, root,
-                                                t->chain_len.as<int>(), t->chain_depth.as<int>(),
-                                                t->offsets.as<int>(), t->prefix.as<D4>(),
-                                                t->nodes.as<BHNode>(),
-                                                t->node_depth.as<unsigned char>(),
-                                                t->pstart.as<int>(), t->parent.as<int>(),
-                                                t->octant.as<unsigned char>(),
-                                                t->kidflag.as<unsigned char>(), stats,
-                                                t->node_cap);
+    place_kernel<<<div_up(n, 256), 256, 0, st>>>(n, t->chain_len.as<int>(),
+                                                 t->chain_depth.as<int>(), t->offsets.as<int>(),
+                                                 t->nodes.as<BHNode>(),
+                                                 t->node_depth.as<unsigned char>(), t->node_cap);
+    NB_LAUNCH_CHECK();
+    const int node_grid = std::min(div_up(launch_nodes(t), 256), 8 * device_props().num_sms);
+    node_kernel<<<std::max(1, node_grid), 256, 0, st>>>(
+        kin, n, root, d_total(t), t->chain_depth.as<int>(), t->offsets.as<int>(),
+        t->prefix.as<D4>(), t->nodes.as<BHNode>(), t->node_depth.as<unsigned char>(),
+        t->pstart.as<int>(), t->parent.as<int>(), t->octant.as<unsigned char>(),
+        t->kidflag.as<unsigned char>(), stats, t->node_cap);
     NB_LAUNCH_CHECK();
     if (quad) NB_TRY(compute_quads(t, x, y, z, m, n, st));
     t->pcen_valid = false;
