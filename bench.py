@@ -717,7 +717,8 @@ def run_ours(a, rank, world, local_rank):
     peak = fp32_roofline_gint(props.multi_processor_count, peaks.get("sm_max_mhz", 2070.0))
     roofline = {
         "bound": "fp32",
-        "kernel": "direct_sorted_kernel" if n >= 16384 else "direct_mixed_kernel",
+        "kernel": ("direct_far_kernel" if n >= 16384 else "direct_mixed_pairs_kernel"
+                   if n >= 4096 else "direct_mixed_small_kernel"),
         "achieved": achieved,
         "peak": peak, "unit": "Ginteractions/s", "frac": achieved / peak,
         "peak_basis": (f"{props.multi_processor_count} SMs x {peaks.get('sm_max_mhz', 2070.0)}"
@@ -732,7 +733,7 @@ def run_ours(a, rank, world, local_rank):
     # the same fraction in FP32-pipe operations per second (12 per interaction)
     roofline["achieved_fp32_tops"] = achieved * 12.0 / 1e3
     roofline["peak_fp32_tops"] = peak * 12.0 / 1e3
-    roofline["traffic"] = profiled_traffic("direct_sorted_n65536.md") if n == N_BODIES else None
+    roofline["traffic"] = profiled_traffic("kernels_by_case.md") if n == N_BODIES else None
     roofline["algorithmic_bytes"] = 32 * n  # hi + lo mirror of every body, read once
     # the same kernel against a measured FP32-pipe rate (packed FMAs on every
     # SM, register-only probe), beside the lanes x clock peak above
@@ -783,7 +784,7 @@ def run_ours(a, rank, world, local_rank):
             "bodies_kappa_gt_10": int((~well).sum()),
             "note": ("kappa = sum_j |pair term| / |a|: a body whose force nearly cancels "
                      "(large kappa) carries a relative error ~kappa x that of its terms")}
-        extras["fp64_direct"] = {"gint_s": fp64_rate, "kernel": "direct_fp64_kernel",
+        extras["fp64_direct"] = {"gint_s": fp64_rate, "kernel": "direct_fp64_pairs_kernel",
                                  "mixed_speedup": achieved / fp64_rate}
         extras["gpu_baseline"] = reference_gpu_kernel_rate(st, n, inter, achieved, torch,
                                                            stream)

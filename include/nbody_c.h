@@ -253,9 +253,9 @@ nb_status nb_bh_read_nodes(nb_sim *sim, int max_nodes, int *depth, uint64_t *pre
 
 /* No counterpart in the reference (one system per process there).  Many
  * independent systems of uneven N, concatenated in system order, advanced
- * together: mixed-precision direct forces of all systems in one persistent
- * launch over a per-system work queue, per-body updates over the
- * concatenation, the step loop captured in a CUDA graph and replayed.  By
+ * together: mixed-precision direct forces of all systems in one launch
+ * over a table of work items (and one that combines the partial sums of
+ * systems from 1024 bodies), per-body updates over the concatenation, the step loop captured in a CUDA graph and replayed.  By
  * default every system is sorted along a Hilbert curve through its own cube
  * (at the start of each nb_ensemble_step call, every 25 steps within it, and
  * in nb_ensemble_compute_forces) and far 64-body tiles take the plain FP32
@@ -302,7 +302,7 @@ nb_status nb_ensemble_profile(nb_ensemble *e, int enable);
 /* No counterpart in the reference.  A continuous-batching server for
  * simulation jobs: each nb_server_tick admits queued jobs while their device
  * memory fits the HBM budget, advances every running job by one leapfrog
- * step (direct jobs together in one batched launch over a resident body
+ * step (direct jobs together in batched launches over a resident body
  * pool, Barnes-Hut jobs on their own streams, overlapping), and retires jobs
  * that reached their step count.  A job's result does not depend on the other
  * jobs it ran with. */
