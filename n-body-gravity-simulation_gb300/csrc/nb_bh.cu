@@ -42,6 +42,7 @@
 // same interactions (NB_BH_WALK=preorder).  Accelerations are scattered back
 // to the original order in FP64, multiplied by G.
 #include "nb_internal.h"
+#include "nb_after.cuh"
 #include "nb_check.cuh"
 #include "nb_curve.cuh"
 #include "nb_pair.cuh"
@@ -811,19 +812,26 @@ __device__ __forceinline__ float4 parent_centre(uint64_t code, int d, const BHRo
                        (float)(((double)iz + 0.5) * side - h), __int_as_float(oct));
 }
 
-// The nodes' first bodies and depths, by the bodies their chains start at.
+// The nodes' first bodies and depths, by the bodies their chains start at, and what
+// node_kernel adds to at zero (a memset each was a launch).
 __global__ void __launch_bounds__(256)
 place_kernel(int n, const int *__restrict__ chain_len, const int *__restrict__ chain_depth,
              const int *__restrict__ offsets, BHNode *__restrict__ nodes,
-             unsigned char *__restrict__ node_depth, int node_cap)
+             unsigned char *__restrict__ node_depth, unsigned long long *__restrict__ kidrows,
+             BHStats *__restrict__ stats, int node_cap)
 {
     const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i == 0) {
+        stats->m2p = stats->p2p = 0;
+        stats->leaves = stats->max_depth = 0;
+    }
     if (i >= n) return;
     const int L = chain_len[i];
     if (L == 0) return;
     const int a = chain_depth[i], id0 = offsets[i];
     for (int k = 0; k < L; ++k) {
         if (!NB_IN_RANGE(id0 + k, node_cap)) break;
+        kidrows[id0 + k] = 0;
         nodes[id0 + k].first = i;
         node_depth[id0 + k] = (unsigned char)(a + k);
     }
@@ -1315,8 +1323,10 @@ group_kernel(const BHNode *__restrict__ nodes, const int *__restrict__ total,
              const float4 *__restrict__ pcen, const float4 *__restrict__ quad,
              BHGNode *__restrict__ gnodes, unsigned char *__restrict__ gnk,
              float4 *__restrict__ gpcen, float4 *__restrict__ gquad,
-             const unsigned char *__restrict__ node_depth, unsigned *__restrict__ gkey)
+             const unsigned char *__restrict__ node_depth, unsigned *__restrict__ gkey,
+             unsigned long long *__restrict__ log_next)
 {
+    if (log_next && blockIdx.x == 0 && threadIdx.x == 0) *log_next = 0;  // a walk follows
     const int num = *total;
     for (int k = blockIdx.x * 256 + threadIdx.x; k < num; k += gridDim.x * 256) {
         int pos = 0;
@@ -1645,7 +1655,8 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
                   const uint32_t *__restrict__ order, int n, float theta2, float eps2, double G,
                   double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
                   BHStats *__restrict__ stats, const float4 *__restrict__ gquad,
-                  const float4 *__restrict__ gpcen, const int2 *__restrict__ logged)
+                  const float4 *__restrict__ gpcen, const int2 *__restrict__ logged,
+                  const AfterForce after)
 {
     // logged: the walks with a log (its count not negative) are done already
     if (logged && logged[blockIdx.x].y >= 0) return;
@@ -1837,9 +1848,13 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
         const int i = w0 + 32 * k + lane;
         if (i >= n) continue;
         const uint32_t o = order[i];
-        ax[o] = G * f[k][0];
-        ay[o] = G * f[k][1];
-        az[o] = G * f[k][2];
+        double *out[3] = {ax, ay, az};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double a = G * f[k][d];
+            out[d][o] = a;
+            after_force(after, d, (int)o, a);
+        }
     }
 }
 
@@ -2051,7 +2066,8 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ g
                 const float4 *__restrict__ body,
                 const uint32_t *__restrict__ order, int n, float eps2, double G,
                 double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
-                const int2 *__restrict__ walks, const uint2 *__restrict__ pool)
+                const int2 *__restrict__ walks, const uint2 *__restrict__ pool,
+                const AfterForce after)
 {
     __shared__ float4 s_term[2][kLogChunk];  // position, mass
     __shared__ float2 s_soft[2][kLogChunk];  // eps^2, added before a body's r^2, after a node's
@@ -2106,9 +2122,14 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ g
         }
         if (i < n) {
             const uint32_t o = order[i];
-            ax[o] = G * (double)fx;
-            ay[o] = G * (double)fy;
-            az[o] = G * (double)fz;
+            double *out[3] = {ax, ay, az};
+            const double f[3] = {(double)fx, (double)fy, (double)fz};
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double a = G * f[d];
+                out[d][o] = a;
+                after_force(after, d, (int)o, a);
+            }
         }
         return;
     }
@@ -2481,7 +2502,7 @@ int log_pool_size(const BHTree *t, int n)
 
 template <bool ZS, bool Q, bool D>
 void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *ax, double *ay,
-                 double *az, cudaStream_t st)
+                 double *az, cudaStream_t st, const AfterForce &after)
 {
     const int np = walk_pairs();
     const float4 *pc = t->pcen.as<float4>();
@@ -2489,14 +2510,14 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
         const BHGNode *gn = t->gnodes.as<BHGNode>();
         const unsigned char *gk = t->gnk.as<unsigned char>();
         const float4 *gq = t->gquad.as<float4>(), *gp = t->gpcen.as<float4>();
-        const int ctas = div_up(n, 64 * np), warps = walk_warps<Q, D>(ctas);
+        const int ctas = div_up(n, 64 * np);
+        int warps = walk_warps<Q, D>(ctas);
         const int2 *logged = nullptr;
         if (t->ordered && np == 1) {
             // logs: the pool's counter, then the pool
             unsigned long long *next = t->logs.as<unsigned long long>();
             uint2 *pool = reinterpret_cast<uint2 *>(next + 1);
             int2 *walks = t->walks.as<int2>();
-            cudaMemsetAsync(next, 0, sizeof(*next), st);
             auto decide = [&](auto *kernel, int threads, size_t shared) {
                 cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)shared);
@@ -2510,8 +2531,9 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
             else
                 decide(decide_kernel<D, 4, 1024>, 128, sizeof(LogShared<D, 4, 1024>));
             log_eval_kernel<ZS, Q><<<ctas, 64 + kLogListers, 0, st>>>(
-                gn, gq, t->body.as<float4>(), t->order, n, eps2, G, ax, ay, az, walks, pool);
+                gn, gq, t->body.as<float4>(), t->order, n, eps2, G, ax, ay, az, walks, pool, after);
             logged = walks;
+            if (!D) warps = std::min(warps, 2);  // mostly none are left: a launch that only looks
         }
         auto *kernel = np == 2 ? group_walk_kernel<ZS, Q, 2, D> : group_walk_kernel<ZS, Q, 1, D>;
         const size_t shared = walk_shared_bytes<Q>(warps);
@@ -2519,7 +2541,7 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
         kernel<<<ctas, 32 * warps, shared, st>>>(
             gn, gk, d_total(t), t->body.as<float4>(), t->order, n, theta2, eps2, G, ax, ay, az,
-            t->stats.as<BHStats>(), gq, gp, logged);
+            t->stats.as<BHStats>(), gq, gp, logged, after);
     } else if (np == 2)
         walk2_kernel<ZS, Q, 2, D><<<div_up(n, 4 * kWalkBlock), kWalkBlock, 0, st>>>(
             t->nodes.as<BHNode>(), d_total(t), t->body.as<float4>(), t->order, n, theta2,
@@ -2536,31 +2558,30 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
 
 template <bool ZS, bool Q>
 void walk_launch_rule(BHTree *t, int n, float theta2, float eps2, double G, double *ax,
-                      double *ay, double *az, cudaStream_t st)
+                      double *ay, double *az, cudaStream_t st, const AfterForce &after)
 {
-    if (t->ref_open) walk_launch<ZS, Q, true>(t, n, theta2, eps2, G, ax, ay, az, st);
-    else walk_launch<ZS, Q, false>(t, n, theta2, eps2, G, ax, ay, az, st);
+    if (t->ref_open) walk_launch<ZS, Q, true>(t, n, theta2, eps2, G, ax, ay, az, st, after);
+    else walk_launch<ZS, Q, false>(t, n, theta2, eps2, G, ax, ay, az, st, after);
 }
 
 static nb_status launch_walk(BHTree *t, int n, double G, double eps2, double theta, double *ax,
-                             double *ay, double *az, cudaStream_t st, const KernelTimer *timer)
+                             double *ay, double *az, cudaStream_t st, const KernelTimer *timer,
+                             const AfterForce &after)
 {
     NvtxRange range("bh_walk");
     const float th2 = (float)(theta * theta), e2 = (float)eps2;
-    if (t->ordered) {
-        NB_TRY(t->walks.reserve(sizeof(int2) * (size_t)div_up(n, 64)));
-        NB_TRY(t->logs.reserve(sizeof(uint2) * ((size_t)log_pool_size(t, n) + 1)));
-    }
     if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
     if (t->with_quad) {
-        if (eps2 > 0.0) walk_launch_rule<false, true>(t, n, th2, e2, G, ax, ay, az, st);
-        else walk_launch_rule<true, true>(t, n, th2, 0.0f, G, ax, ay, az, st);
+        if (eps2 > 0.0) walk_launch_rule<false, true>(t, n, th2, e2, G, ax, ay, az, st, after);
+        else walk_launch_rule<true, true>(t, n, th2, 0.0f, G, ax, ay, az, st, after);
     } else {
-        if (eps2 > 0.0) walk_launch_rule<false, false>(t, n, th2, e2, G, ax, ay, az, st);
-        else walk_launch_rule<true, false>(t, n, th2, 0.0f, G, ax, ay, az, st);
+        if (eps2 > 0.0) walk_launch_rule<false, false>(t, n, th2, e2, G, ax, ay, az, st, after);
+        else walk_launch_rule<true, false>(t, n, th2, 0.0f, G, ax, ay, az, st, after);
     }
     NB_LAUNCH_CHECK();
     if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
+    // the child-group walks apply the update, the preorder walks do not
+    if (!group_walk() || walk_pairs() < 1) return apply_after(after, n, ax, ay, az, st);
     return NB_OK;
 }
 
@@ -2623,7 +2644,11 @@ static nb_status group_nodes(BHTree *t, cudaStream_t st, bool recount)
     if (t->ref_open) NB_TRY(t->gpcen.reserve(sizeof(float4) * (size_t)slots));
     if (t->with_quad) NB_TRY(t->gquad.reserve(sizeof(float4) * 2 * (size_t)slots));
     t->ordered = t->ref_open || t->n <= kOrderedBodies;
-    if (t->ordered) NB_TRY(t->gkey.reserve(sizeof(unsigned) * (size_t)slots));
+    if (t->ordered) {
+        NB_TRY(t->gkey.reserve(sizeof(unsigned) * (size_t)slots));
+        NB_TRY(t->walks.reserve(sizeof(int2) * (size_t)div_up(t->n, 64)));
+        NB_TRY(t->logs.reserve(sizeof(uint2) * ((size_t)log_pool_size(t, t->n) + 1)));
+    }
     group_kernel<<<grid, 256, 0, st>>>(
         t->nodes.as<BHNode>(), d_total(t), t->occ.as<unsigned>(), t->kbase.as<int>(),
         t->parent.as<int>(), t->octant.as<unsigned char>(),
@@ -2631,7 +2656,8 @@ static nb_status group_nodes(BHTree *t, cudaStream_t st, bool recount)
         t->with_quad ? t->quad.as<float4>() : nullptr, t->gnodes.as<BHGNode>(),
         t->gnk.as<unsigned char>(), t->gpcen.as<float4>(),
         t->with_quad ? t->gquad.as<float4>() : nullptr, t->node_depth.as<unsigned char>(),
-        t->ordered ? t->gkey.as<unsigned>() : nullptr);
+        t->ordered ? t->gkey.as<unsigned>() : nullptr,
+        t->ordered ? t->logs.as<unsigned long long>() : nullptr);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
@@ -2669,7 +2695,8 @@ static nb_status refit(BHTree *t, const double *x, const double *y, const double
 nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *z,
                      const double *m, int n, double G, double eps2, double theta,
                      int leaf_capacity, double *ax, double *ay, double *az, cudaStream_t st,
-                     const KernelTimer *timer, int reuse, bool quad, bool ref_open)
+                     const KernelTimer *timer, int reuse, bool quad, bool ref_open,
+                     const AfterForce &after)
 {
     if (n <= 0) return NB_OK;
     t->with_quad = quad;
@@ -2680,7 +2707,7 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
         NB_TRY(ensure_pcen(t, st));
         NB_TRY(group_nodes(t, st, false));
         ++t->evals_since_build;
-        return launch_walk(t, n, G, eps2, theta, ax, ay, az, st, timer);
+        return launch_walk(t, n, G, eps2, theta, ax, ay, az, st, timer, after);
     }
     t->tree_valid = false;
     NvtxRange range("bh_build");
@@ -2738,12 +2765,12 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
     t->node_cap = (int)std::min(cap, (size_t)INT32_MAX);
     t->num_nodes = -1;
     t->n = n;
-    NB_CUDA_TRY(cudaMemsetAsync(stats, 0, offsetof(BHStats, total), st));
-    NB_CUDA_TRY(cudaMemsetAsync(t->kidflag.ptr, 0, 8 * cap, st));
     place_kernel<<<div_up(n, 256), 256, 0, st>>>(n, t->chain_len.as<int>(),
                                                  t->chain_depth.as<int>(), t->offsets.as<int>(),
                                                  t->nodes.as<BHNode>(),
-                                                 t->node_depth.as<unsigned char>(), t->node_cap);
+                                                 t->node_depth.as<unsigned char>(),
+                                                 t->kidflag.as<unsigned long long>(), stats,
+                                                 t->node_cap);
     NB_LAUNCH_CHECK();
     const int node_grid = std::min(div_up(launch_nodes(t), 256), 8 * device_props().num_sms);
     node_kernel<<<std::max(1, node_grid), 256, 0, st>>>(
@@ -2760,7 +2787,7 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
     t->evals_since_build = 0;
     if (!ax) return NB_OK;
     t->evals_since_build = 1;
-    return launch_walk(t, n, G, eps2, theta, ax, ay, az, st, timer);
+    return launch_walk(t, n, G, eps2, theta, ax, ay, az, st, timer, after);
 }
 
 nb_status bh_info(BHTree *t, cudaStream_t st, nb_bh_info *info)

@@ -306,7 +306,7 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
                      const double *m, int n, double G, double eps2, double theta,
                      int leaf_capacity, double *ax, double *ay, double *az, cudaStream_t st,
                      const KernelTimer *timer = nullptr, int reuse = 1, bool quad = false,
-                     bool ref_open = false);
+                     bool ref_open = false, const AfterForce &after = AfterForce{});
 // The next bh_compute rebuilds (the bodies were replaced).
 void bh_invalidate(BHTree *t);
 // A replayed build changed the node count behind the host's back.

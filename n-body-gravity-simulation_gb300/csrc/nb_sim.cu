@@ -119,12 +119,11 @@ const DeviceProps &device_props()
 
 static size_t plane_stride(size_t capacity) { return (capacity + 31) / 32 * 32; }
 
-// Whether the force kernels apply an AfterForce themselves, and whether they read
-// the mixed kernels' mirror (which an update can then write with the positions).
-static bool fuses_updates(const nb_sim *s)
+// Whether the force kernels read the mixed kernels' mirror in the caller's order (which
+// an update can then write with the positions).
+static bool reads_mirror(const nb_sim *s)
 {
-    return s->cfg.method == NB_DIRECT_FP64 ||
-           (s->cfg.method == NB_DIRECT_MIXED && !direct_sorted_enabled((int)s->n, s->cfg.flags));
+    return s->cfg.method == NB_DIRECT_MIXED && !direct_sorted_enabled((int)s->n, s->cfg.flags);
 }
 
 static nb_status reserve_mirror(nb_sim *s)
@@ -157,12 +156,11 @@ nb_status eval_forces(nb_sim *s, const double *px, const double *py, const doubl
     }
     case NB_BARNES_HUT:
         if (!s->bh) s->bh = bh_create();
-        NB_TRY(bh_compute(s->bh, px, py, pz, s->m(), n, s->cfg.G, eps2, s->cfg.theta,
+        return bh_compute(s->bh, px, py, pz, s->m(), n, s->cfg.G, eps2, s->cfg.theta,
                           s->cfg.leaf_capacity, oax, oay, oaz, s->stream, timer,
                           NB_FLAG_BH_REUSE_OF(s->cfg.flags),
                           (s->cfg.flags & NB_FLAG_BH_QUADRUPOLE) != 0,
-                          (s->cfg.flags & NB_FLAG_BH_REFERENCE_OPENING) != 0));
-        return apply_after(after, n, oax, oay, oaz, s->stream);
+                          (s->cfg.flags & NB_FLAG_BH_REFERENCE_OPENING) != 0, after);
     default:
         return fail(NB_ERR_INVALID_ARGUMENT, "unknown force method");
     }
@@ -187,7 +185,7 @@ static nb_status step_once(nb_sim *s, int integ, double dt)
     const int n = (int)s->n;
     cudaStream_t st = s->stream;
     // the updates write the next evaluation's mirror where the kernels read one
-    const bool mirror = s->cfg.method == NB_DIRECT_MIXED && fuses_updates(s);
+    const bool mirror = reads_mirror(s);
     if (mirror) NB_TRY(reserve_mirror(s));
     float4 *hi = mirror ? s->split_hi.as<float4>() : nullptr;
     float4 *lo = mirror ? s->split_lo.as<float4>() : nullptr;
