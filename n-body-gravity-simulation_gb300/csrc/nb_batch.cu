@@ -498,12 +498,12 @@ int bucket_of(int n)
     return b;  // floor(log2(n))
 }
 
-size_t batch_layout(std::vector<SysDesc> &sys, int *tiles)
+size_t batch_layout(std::vector<SysDesc> &sys, int pairs_min, int *tiles)
 {
     int t = 0;
     long long pairs = 0;
     for (SysDesc &s : sys) {
-        s.blocks = s.n < kBatchPairsMin ? 0 : (s.n + kBatchBlockBodies - 1) / kBatchBlockBodies;
+        s.blocks = s.n < pairs_min ? 0 : (s.n + kBatchBlockBodies - 1) / kBatchBlockBodies;
         s.tile0 = t;
         s.part0 = pairs;
         t += (s.n + kTile - 1) / kTile;
@@ -520,7 +520,7 @@ void build_work_items(const std::vector<SysDesc> &sys, std::vector<PairItem> &it
     // cost, largest first, in units of a 64 x 64 tile pair (a stable counting
     // sort: all full items of all systems cost the same; a row item is two
     // tiles against half its system's, both directions apart)
-    constexpr int kMost = kBatchPairsMin / 16;
+    constexpr int kMost = 64;
     std::vector<PairItem> by_cost[kMost + 1];
     items.clear();
     for (int s = 0; s < (int)sys.size(); ++s) {

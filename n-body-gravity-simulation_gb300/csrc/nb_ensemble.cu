@@ -60,7 +60,7 @@ constexpr int kGraphChunk = 25;
 nb_status upload_items(nb_ensemble *e)
 {
     BatchQueue &q = e->queue;
-    const size_t bytes = batch_layout(e->sys, &q.num_tiles);
+    const size_t bytes = batch_layout(e->sys, kBatchPairsMin, &q.num_tiles);
     std::vector<PairItem> items;
     build_work_items(e->sys, items, &q.num_blocks);
     q.num_items = (int)items.size();

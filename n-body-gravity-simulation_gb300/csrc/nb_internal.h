@@ -232,6 +232,11 @@ constexpr int kBatchBlockBodies = 256;  // four tiles of 64
 // pair can carry a body's whole force, and the row sum is the order of rounding
 // that its trajectory has had.
 constexpr int kBatchPairsMin = 1024;
+// The server's jobs run many steps and may be dense disks, in which a close pair carries
+// a force of 100 (1.4e-7 of the velocities' scale after four steps of 1e-3 at n = 2705 by
+// unordered pairs, against the row sum); up to 4095 bodies their work is a few percent
+// of the direct jobs' (a burst of 16 jobs: 15.7 ms, 15.5 by pairs from 1024).
+constexpr int kServePairsMin = 4096;
 // A system of a batch: bodies [first, first + n) of the batch's pool.
 struct SysDesc {
     int first;
@@ -258,7 +263,7 @@ struct BatchQueue {
 int bucket_of(int n);  // floor(log2(n))
 // Sets every system's blocks, tile0 and part0; returns the bytes of the
 // partial planes and the tile count.
-size_t batch_layout(std::vector<SysDesc> &sys, int *tiles);
+size_t batch_layout(std::vector<SysDesc> &sys, int pairs_min, int *tiles);
 // The combine's blocks, then the items of every system, largest cost first.
 void build_work_items(const std::vector<SysDesc> &sys, std::vector<PairItem> &items,
                       int *num_blocks);

@@ -251,7 +251,7 @@ nb_status upload_systems(nb_server *s, const std::vector<Job *> &jobs, nb_server
 {
     std::vector<SysDesc> sys;
     for (Job *j : jobs) sys.push_back(SysDesc{(int)j->first, (int)j->n, 0, 0, 0});
-    const size_t bytes = batch_layout(sys, &to.q.num_tiles);
+    const size_t bytes = batch_layout(sys, kServePairsMin, &to.q.num_tiles);
     std::vector<PairItem> items;
     build_work_items(sys, items, &to.q.num_blocks);
     to.q.num_items = (int)items.size();
