@@ -255,7 +255,8 @@ nb_status nb_bh_read_nodes(nb_sim *sim, int max_nodes, int *depth, uint64_t *pre
  * independent systems of uneven N, concatenated in system order, advanced
  * together: mixed-precision direct forces of all systems in one launch
  * over a table of work items (and one that combines the partial sums of
- * systems from 1024 bodies), per-body updates over the concatenation, the step loop captured in a CUDA graph and replayed.  By
+ * systems from 2048 bodies), per-body updates over the concatenation, the
+ * step loop captured in a CUDA graph and replayed.  By
  * default every system is sorted along a Hilbert curve through its own cube
  * (at the start of each nb_ensemble_step call, every 25 steps within it, and
  * in nb_ensemble_compute_forces) and far 64-body tiles take the plain FP32

@@ -228,10 +228,12 @@ constexpr int kBatchBlockBodies = 256;  // four tiles of 64
 // Smallest system summed over unordered pairs; smaller ones by rows (ordered
 // pairs).  On the 1024-system ensemble (n log-uniform in [32, 4096], two RK4 steps)
 // a line at 512 / 1024 / 2048 / beyond every system measured 7.58 / 7.69 / 8.12 /
-// 9.15 ms (one i-tile at a time).  It lies at 1024, not 512: in a system of a few hundred bodies one close
-// pair can carry a body's whole force, and the row sum is the order of rounding
-// that its trajectory has had.
-constexpr int kBatchPairsMin = 1024;
+// 9.15 ms (one i-tile at a time; at 1024 / 2048 7.04 / 7.51 ms with four i-bodies per
+// lane).  It lies at 2048: in a smaller system one close pair can carry a body's whole
+// force, and the row sum is the order of rounding that its trajectory has had (of 30
+// ensembles, the largest difference of a velocity after two steps was 4.4e-8 of their
+// scale with the line at 1024, 2.5e-8 at 2048).
+constexpr int kBatchPairsMin = 2048;
 // The server's jobs run many steps and may be dense disks, in which a close pair carries
 // a force of 100 (1.4e-7 of the velocities' scale after four steps of 1e-3 at n = 2705 by
 // unordered pairs, against the row sum); up to 4095 bodies their work is a few percent

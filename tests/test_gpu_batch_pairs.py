@@ -10,7 +10,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 33, 1023, 1024, 1025, 1088, 1280, 1281, 1311, 1536, 1793, 2049, 3841]
+SIZES = [1, 33, 1025, 1311, 2047, 2048, 2049, 2112, 2304, 2305, 2335, 2560, 2817, 3841]
 TOL = 1e-6
 
 
