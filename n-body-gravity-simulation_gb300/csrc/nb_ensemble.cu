@@ -66,7 +66,7 @@ nb_status upload_items(nb_ensemble *e)
     q.num_items = (int)items.size();
     NB_TRY(e->d_sys.reserve(sizeof(SysDesc) * e->sys.size()));
     NB_TRY(e->d_items.reserve(sizeof(PairItem) * items.size()));
-    NB_TRY(e->part.reserve(bytes));
+    if (bytes) NB_TRY(e->part.reserve(bytes));  // 0: every system by rows
     q.d_sys = e->d_sys.as<SysDesc>();
     q.d_items = e->d_items.as<PairItem>();
     q.part = e->part.as<float2>();

@@ -258,7 +258,7 @@ nb_status upload_systems(nb_server *s, const std::vector<Job *> &jobs, nb_server
     if (sys.empty()) return NB_OK;
     NB_TRY(to.d_sys.reserve(sizeof(SysDesc) * sys.size()));
     NB_TRY(to.d_items.reserve(sizeof(PairItem) * items.size()));
-    NB_TRY(to.part.reserve(bytes));
+    if (bytes) NB_TRY(to.part.reserve(bytes));  // 0: every job by rows
     to.q.d_sys = to.d_sys.as<SysDesc>();
     to.q.d_items = to.d_items.as<PairItem>();
     to.q.part = to.part.as<float2>();
