@@ -188,6 +188,8 @@ combine_mixed_kernel(const float *__restrict__ psum,
 // sums.  A velocity-Verlet step at n = 100 / 1000 / 2000 / 4000 takes 10.4 / 12.4 / 16.5 /
 // 26.8 us in a row of steps, with the sums in a second kernel 14.5 / 16.5 / 21.3 / 30.8;
 // 8 warps per CTA 10.4 / 14.5 / 16.5 / 25.2, two i-bodies per lane no less.
+// A cluster writes its bodies' next split positions (after) while others still read the
+// present ones: those are two arrays.
 constexpr int kSmallCtas = 8, kSmallWarps = 4;
 
 template <bool ZERO_SOFT>
@@ -674,9 +676,6 @@ int resident_ctas(const void *fn)
 
 constexpr int kMixBlock = 256;
 constexpr int kMixIpt = 4;
-// Smallest system the mixed path sums over unordered pairs: an evaluation takes
-// 24.8 us there and 28.9 with ordered pairs at n = 4,000, 24.7 and 22.7 at 3,000.
-constexpr int kMixedPairsMin = 4096;
 constexpr size_t kPairPlaneBytes = (size_t)512 << 20;  // partial planes per pass
 constexpr int kF64RowMax = 512;  // largest N of the one-warp-per-body FP64 kernel
 constexpr size_t kF64PlaneBytes = (size_t)512 << 20;  // FP64 partial planes per pass

@@ -112,6 +112,12 @@ struct DirectPlan {
 
 // Mixed FP32/double-single all-pairs kernel.  hi/lo: float4 (x, y, z, m) and
 // (x_lo, y_lo, z_lo, 0) of every body.  Writes G * sum into ax/ay/az (FP64).
+// after.hi, after.lo: below kMixedPairsMin other arrays than hi, lo, since one launch
+// reads every body's entry and writes the new ones.
+// kMixedPairsMin: smallest system summed over unordered pairs, by several launches.  An
+// evaluation takes 24.8 us there and 28.9 with ordered pairs at n = 4,000, 24.7 and
+// 22.7 at 3,000.
+constexpr int kMixedPairsMin = 4096;
 nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, double eps2,
                        double *ax, double *ay, double *az, DevBuf &partials,
                        cudaStream_t st, const KernelTimer *timer = nullptr,
@@ -357,7 +363,10 @@ struct nb_sim {
     double *f[10] = {};
     bool forces_valid = false;
 
-    nb::DevBuf split_hi, split_lo;   // float4 mirrors for the mixed kernel
+    // Float4 mirrors for the mixed kernel.  An RK4 step below kMixedPairsMin bodies
+    // alternates between two: a stage's launch reads one and writes the next stage's
+    // positions to the other.
+    nb::DevBuf split_hi[2], split_lo[2];
     nb::SortedBuffers sorted;        // Hilbert-sorted near/far variant of the mixed kernel
     nb::DevBuf partials;             // j-split partial sums
     nb::DevBuf old_acc;              // velocity-Verlet a(t)
@@ -397,10 +406,12 @@ struct nb_sim {
 
 namespace nb {
 // Evaluates accelerations of positions (px,py,pz) with masses m into out* and
-// applies `after`; split: the mixed kernels' mirror holds these positions already.
+// applies `after`.  mirror: the one the mixed kernels read; split: it holds these
+// positions already.
 nb_status eval_forces(nb_sim *s, const double *px, const double *py, const double *pz,
                       double *oax, double *oay, double *oaz,
-                      const AfterForce &after = AfterForce{}, bool split = false);
+                      const AfterForce &after = AfterForce{}, bool split = false,
+                      int mirror = 0);
 // Drops the captured step graph (the next steps run directly).
 void reset_step_graph(nb_sim *s);
 // Kernel launches made by a graph replay (the launch counter's evidence).

@@ -126,14 +126,15 @@ static bool reads_mirror(const nb_sim *s)
     return s->cfg.method == NB_DIRECT_MIXED && !direct_sorted_enabled((int)s->n, s->cfg.flags);
 }
 
-static nb_status reserve_mirror(nb_sim *s)
+static nb_status reserve_mirror(nb_sim *s, int mirror)
 {
-    NB_TRY(s->split_hi.reserve(sizeof(float4) * s->capacity));
-    return s->split_lo.reserve(sizeof(float4) * s->capacity);
+    NB_TRY(s->split_hi[mirror].reserve(sizeof(float4) * s->capacity));
+    return s->split_lo[mirror].reserve(sizeof(float4) * s->capacity);
 }
 
 nb_status eval_forces(nb_sim *s, const double *px, const double *py, const double *pz,
-                      double *oax, double *oay, double *oaz, const AfterForce &after, bool split)
+                      double *oax, double *oay, double *oaz, const AfterForce &after, bool split,
+                      int mirror)
 {
     const int n = (int)s->n;
     const double eps2 = s->cfg.softening * s->cfg.softening;
@@ -148,8 +149,8 @@ nb_status eval_forces(nb_sim *s, const double *px, const double *py, const doubl
                                        s->sorted, s->stream, timer));
             return apply_after(after, n, oax, oay, oaz, s->stream);
         }
-        NB_TRY(reserve_mirror(s));
-        float4 *hi = s->split_hi.as<float4>(), *lo = s->split_lo.as<float4>();
+        NB_TRY(reserve_mirror(s, mirror));
+        float4 *hi = s->split_hi[mirror].as<float4>(), *lo = s->split_lo[mirror].as<float4>();
         if (!split) NB_TRY(split_positions(px, py, pz, s->m(), n, hi, lo, s->stream));
         return direct_mixed(hi, lo, n, s->cfg.G, eps2, oax, oay, oaz, s->partials, s->stream,
                             timer, after);
@@ -186,9 +187,9 @@ static nb_status step_once(nb_sim *s, int integ, double dt)
     cudaStream_t st = s->stream;
     // the updates write the next evaluation's mirror where the kernels read one
     const bool mirror = reads_mirror(s);
-    if (mirror) NB_TRY(reserve_mirror(s));
-    float4 *hi = mirror ? s->split_hi.as<float4>() : nullptr;
-    float4 *lo = mirror ? s->split_lo.as<float4>() : nullptr;
+    if (mirror) NB_TRY(reserve_mirror(s, 0));
+    float4 *hi = mirror ? s->split_hi[0].as<float4>() : nullptr;
+    float4 *lo = mirror ? s->split_lo[0].as<float4>() : nullptr;
     double *const x[3] = {s->x(), s->y(), s->z()}, *const v[3] = {s->vx(), s->vy(), s->vz()};
     double *const a[3] = {s->ax(), s->ay(), s->az()};
     AfterForce after;
@@ -233,10 +234,14 @@ static nb_status step_once(nb_sim *s, int integ, double dt)
         double *const k[3] = {s->rk4.as<double>(), s->rk4.as<double>() + 9 * ps,
                               s->rk4.as<double>() + 18 * ps};
         after.m = s->m();
-        after.hi = hi;
-        after.lo = lo;
+        const int other = mirror && n < kMixedPairsMin ? 1 : 0;
+        if (other) NB_TRY(reserve_mirror(s, 1));
         for (int stage = 0; stage < 4; ++stage) {
             double *p[3], *acc[3];
+            if (mirror) {  // the next stage's
+                after.hi = s->split_hi[other & (stage + 1)].as<float4>();
+                after.lo = s->split_lo[other & (stage + 1)].as<float4>();
+            }
             for (int c = 0; c < 3; ++c) {
                 p[c] = stage == 0 ? x[c] : k[stage - 1] + c * ps;
                 after.kv[c] = stage == 0 ? v[c] : k[stage - 1] + (3 + c) * ps;
@@ -253,7 +258,7 @@ static nb_status step_once(nb_sim *s, int integ, double dt)
             after.k3 = k[1];
             after.ps = ps;
             NB_TRY(eval_forces(s, p[0], p[1], p[2], acc[0], acc[1], acc[2], after,
-                               mirror && stage > 0));
+                               mirror && stage > 0, other & stage));
         }
         s->forces_valid = false;
         return NB_OK;
@@ -410,8 +415,10 @@ nb_status nb_destroy(nb_sim *s)
     }
     if (s->bh) bh_destroy(s->bh);
     s->state.release();
-    s->split_hi.release();
-    s->split_lo.release();
+    for (int k = 0; k < 2; ++k) {
+        s->split_hi[k].release();
+        s->split_lo[k].release();
+    }
     s->sorted.release();
     s->partials.release();
     s->old_acc.release();
