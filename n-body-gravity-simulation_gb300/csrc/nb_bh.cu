@@ -48,6 +48,7 @@
 #include "nb_pair.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
@@ -1378,7 +1379,7 @@ group_kernel(const BHNode *__restrict__ nodes, const int *__restrict__ total,
 // per group, took 2.32 ms at N = 2^20 (theta 0.5), 3.67 ms at N = 100,000 under
 // the reference's opening rule (ten warps per SM, each a serial walk, the longest
 // five times the mean); this takes 1.73 ms with one warp per walk and 0.55 ms with
-// sixteen (which the reference's rule takes only where the ordered walk below cannot).  Of the 1.73 ms, about 1.2 are the 15.5 dispatch cycles per interaction
+// sixteen.  Of the 1.73 ms, about 1.2 are the 15.5 dispatch cycles per interaction
 // of the evaluation, the rest the decisions (2,600 nodes per walk, a fifth of them
 // undecided).
 //
@@ -1655,11 +1656,8 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
                   const uint32_t *__restrict__ order, int n, float theta2, float eps2, double G,
                   double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
                   BHStats *__restrict__ stats, const float4 *__restrict__ gquad,
-                  const float4 *__restrict__ gpcen, const int2 *__restrict__ logged,
-                  const AfterForce after)
+                  const float4 *__restrict__ gpcen, const AfterForce after)
 {
-    // logged: the walks with a log (its count not negative) are done already
-    if (logged && logged[blockIdx.x].y >= 0) return;
     extern __shared__ __align__(16) unsigned char walk_shared[];
     using Shared = WalkShared<QUAD>;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
@@ -1858,12 +1856,162 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
     }
 }
 
+// ------------------------------------------------------------ serial walk
+// One warp walks for 64 consecutive sorted bodies, two per lane (a packed pair):
+// one round trip to memory brings a group's records into shared memory, and the
+// warp tests the children one after the other, adding the monopoles of the children
+// that no body opens and opened leaves' bodies in that order, and pushing the groups of
+// opened internal children onto its stack.  The interactions are those of
+// walk2_kernel; only their order differs.
+// Bound by dispatch when the walks fill the chip (it spends least on a walk: no list, no
+// sort), by each walk's chain of trips to memory when they do not.  The ordered walk
+// below adds the same terms in the same order, so the two give the same bits and any
+// walk may go by either.
+//
+// A depth-first walk over groups keeps, per level of its current path, at most
+// 7 groups of unvisited siblings, plus the at most 8 groups the last group
+// pushed; groups lie at levels 0 .. kMaxLevels.
+constexpr int kSerialStack = 8 * (kMaxLevels + 1);
+
+template <bool ZERO_SOFT, bool QUAD, bool DIR>
+__global__ void __launch_bounds__(32)
+serial_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restrict__ gnk,
+                   const int *__restrict__ total, const float4 *__restrict__ body,
+                   const uint32_t *__restrict__ order, int n, float theta2, float eps2, double G,
+                   double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
+                   BHStats *__restrict__ stats, const float4 *__restrict__ gquad,
+                   const float4 *__restrict__ gpcen, const int2 *__restrict__ logged,
+                   const AfterForce after)
+{
+    // logged: the walks with a log (its count not negative) are done already
+    if (logged && logged[blockIdx.x].y >= 0) return;
+    __shared__ BHGNode s_rec[8];
+    __shared__ float4 s_quad[QUAD ? 16 : 1];
+    __shared__ float4 s_pc[DIR ? 8 : 1];
+    __shared__ int2 s_stack[kSerialStack];
+    [[maybe_unused]] const int num_nodes = *total;  // bounds checked builds only
+    const int lane = threadIdx.x;
+    const int w0 = blockIdx.x * 64, wend = min(n, w0 + 64);  // the warp's bodies: [w0, wend)
+    const int ia = w0 + lane, ib = ia + 32;
+    // a slot past n walks with body w0: its tests repeat that body's
+    const float4 pa = body[ia < n ? ia : w0], pb = body[ib < n ? ib : w0];
+    const float2 npx = make_float2(-pa.x, -pb.x), npy = make_float2(-pa.y, -pb.y),
+                 npz = make_float2(-pa.z, -pb.z);
+    float2 fx = dup2(0.f), fy = dup2(0.f), fz = dup2(0.f);
+    const float2 e2 = dup2(eps2), t2 = dup2(theta2);
+    unsigned m2p = 0, p2p = 0;
+    int sp = 1;
+    if (lane == 0) s_stack[0] = make_int2(0, 1);
+    while (sp > 0) {
+        __syncwarp();
+        const int2 g = s_stack[--sp];
+        if (!NB_IN_RANGE(g.x + g.y - 1, num_nodes)) break;
+        int mynk = 0;
+        if (lane < g.y) {
+            s_rec[lane] = gnodes[g.x + lane];
+            mynk = gnk[g.x + lane];
+            if (DIR) s_pc[lane] = gpcen[g.x + lane];
+        }
+        if (QUAD && lane < 2 * g.y) s_quad[lane] = gquad[2 * g.x + lane];
+        __syncwarp();
+        for (int c = 0; c < g.y; ++c) {
+            const BHGNode nd = s_rec[c];
+            const float2 dx = add2(dup2(nd.com_mass.x), npx), dy = add2(dup2(nd.com_mass.y), npy),
+                         dz = add2(dup2(nd.com_mass.z), npz);
+            const float2 d2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+            const float2 td2 = mul2(t2, d2);
+            // a node that holds one of the warp's bodies is opened (each body's
+            // own cell); the others by the opening test of any body
+            bool open = nd.first < wend && nd.first + nd.count > w0;
+            open = open | (nd.size2 >= td2.x) | (nd.size2 >= td2.y);
+            if (DIR) {
+                const float4 pc = s_pc[c];
+                open = open | toward_body(pc, -npx.x, -npy.x, -npz.x) |
+                       toward_body(pc, -npx.y, -npy.y, -npz.y);
+            }
+            if (__any_sync(0xffffffffu, open)) {
+                if (nd.kids >= 0) {  // internal: its children's group, later
+                    const int nk = __shfl_sync(0xffffffffu, mynk, c);
+                    if (NB_IN_RANGE(sp, kSerialStack)) {
+                        if (lane == 0) s_stack[sp] = make_int2(nd.kids, nk);
+                        ++sp;
+                    }
+                    continue;
+                }
+                const int e = NB_IN_RANGE(nd.first, n) && NB_IN_RANGE(nd.first + nd.count - 1, n)
+                                  ? nd.first + nd.count
+                                  : nd.first;
+#pragma unroll 2
+                for (int b = nd.first; b < e; ++b) {
+                    const float4 q = body[b];
+                    const float2 rx = add2(dup2(q.x), npx), ry = add2(dup2(q.y), npy),
+                                 rz = add2(dup2(q.z), npz);
+                    const float2 r2 = fma2(rz, rz, fma2(ry, ry, fma2(rx, rx, e2)));
+                    float2 inv = make_float2(rsqrt_mufu(r2.x), rsqrt_mufu(r2.y));
+                    if (ZERO_SOFT) {
+                        inv.x = r2.x > 0.f ? inv.x : 0.f;
+                        inv.y = r2.y > 0.f ? inv.y : 0.f;
+                    }
+                    const float2 s = mul2(mul2(dup2(q.w), inv), mul2(inv, inv));
+                    fx = fma2(rx, s, fx);
+                    fy = fma2(ry, s, fy);
+                    fz = fma2(rz, s, fz);
+                }
+                p2p += nd.count;
+            } else {
+                const float2 r2 = add2(d2, e2);
+                const float2 inv = make_float2(rsqrt_mufu(r2.x), rsqrt_mufu(r2.y));
+                const float2 inv2 = mul2(inv, inv);
+                const float2 s = mul2(mul2(dup2(nd.com_mass.w), inv), inv2);
+                fx = fma2(dx, s, fx);
+                fy = fma2(dy, s, fy);
+                fz = fma2(dz, s, fz);
+                if (QUAD) {
+                    const float4 q0 = s_quad[2 * c], q1 = s_quad[2 * c + 1];
+                    const float2 qx =
+                        fma2(dup2(q0.x), dx, fma2(dup2(q0.w), dy, mul2(dup2(q1.x), dz)));
+                    const float2 qy =
+                        fma2(dup2(q0.w), dx, fma2(dup2(q0.y), dy, mul2(dup2(q1.y), dz)));
+                    const float2 qz =
+                        fma2(dup2(q1.x), dx, fma2(dup2(q1.y), dy, mul2(dup2(q0.z), dz)));
+                    const float2 rqr = fma2(dx, qx, fma2(dy, qy, mul2(dz, qz)));
+                    const float2 inv5 = mul2(mul2(inv, inv2), inv2);
+                    const float2 f = mul2(mul2(dup2(2.5f), rqr), inv2);
+                    fx = fma2(inv5, fma2(f, dx, make_float2(-qx.x, -qx.y)), fx);
+                    fy = fma2(inv5, fma2(f, dy, make_float2(-qy.x, -qy.y)), fy);
+                    fz = fma2(inv5, fma2(f, dz, make_float2(-qz.x, -qz.y)), fz);
+                }
+                ++m2p;
+            }
+        }
+    }
+    double *const out[3] = {ax, ay, az};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int i = w0 + 32 * k + lane;
+        if (i >= n) continue;
+        const uint32_t o = order[i];
+        const float f[3] = {k ? fx.y : fx.x, k ? fy.y : fy.x, k ? fz.y : fz.x};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double a = G * (double)f[d];
+            out[d][o] = a;
+            after_force(after, d, (int)o, a);
+        }
+    }
+    if (lane == 0) {
+        const unsigned long long nv = wend - w0;
+        atomicAdd(&stats->m2p, m2p * nv);
+        atomicAdd(&stats->p2p, p2p * nv);
+        atomicAdd(&stats->total, (m2p + p2p) * nv);
+    }
+}
+
 // ---------------------------------------------------------- ordered walk
 // An FP32 sum of thousands of terms depends on their order in the fifth digit (walks
 // under the reference's opening rule have up to 20,000 at n = 100,000, theta 0.5,
 // disk galaxy), and a trajectory with it.  This walk adds each body's terms one after
-// the other in the order of a serial walk over a stack of groups (last pushed, first
-// visited; a group's records in order), in two kernels:
+// the other in the order of the serial walk, in two kernels:
 //   - decide_kernel finds the groups that the walk visits and which of their records
 //     are opened, in any order, by many warps (as group_walk_kernel), and sorts
 //     the groups by their place in the serial walk of the whole tree: the rank
@@ -1871,15 +2019,22 @@ group_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__res
 //     depth(v) - skip(v) but for a constant;
 //   - log_eval_kernel goes through a walk's groups in that order: four warps list the
 //     terms in shared memory, two add them up, a body per lane.
-// A walk that visits more groups than its log holds, or for whose log the pool has no
-// room, is left to group_walk_kernel.
+// The stack is kept in the serial walk's order, so whatever sorts before its top is
+// complete: a CTA that has no room for more groups moves those to the pool and goes on
+// (a walk under the reference's rule visits up to 4,900 at n = 400,000, theta 0.5, and
+// 18,000 with one body per leaf).  A walk that the pool has no room for (which ones
+// depends on scheduling), or whose stack is full, is left to serial_walk_kernel, which
+// gives the same bits but takes 9 ms for that one.
 //
-// A force evaluation by one warp per walk (serial) / this walk / group_walk_kernel, in us:
-//   n =  16,384   712 /  315 /  281        reference's rule, n = 20,000:  1623 /  464 /  377
-//   n = 100,000   856 /  491 /  408        reference's rule, n = 100,000: 4242 / 1076 /  830
-//   n = 400,000  1484 / 1331 / 1095        quadrupoles, n = 100,000:      1001 /  750 /  619
-// Up to kOrderedBodies, and always under the reference's rule, this walk keeps the
-// serial walk's results bit for bit; beyond, where listing the terms apart from the
+// A force evaluation by serial_walk_kernel / this walk, disk galaxy, in us:
+//                        theta 0.5        0.3             0.5, reference's rule
+//   n =  16,384        564 /  272     892 /  315        1817 /  426
+//   n = 100,000       1001 /  503    1921 /  782        3910 / 1048
+//   n = 400,000       1342 / 1227    3091 / 2410       11208 / 3598
+// (group_walk_kernel, in another order, took 0.83 times as long at n = 100,000, theta 0.5,
+// 0.82 at 400,000 and 0.77 under the reference's rule at 100,000.)
+// Up to kOrderedBodies, and always under the reference's rule, results are the serial
+// walk's bit for bit; beyond, where listing the terms apart from the
 // decisions eats what many warps gain (2^20 bodies: 2.88 ms serial, 2.28 by
 // group_walk_kernel), walks are of similar length and the order of summation shows in
 // velocities at 1e-8 of their scale after a step of 1e-3.
@@ -1888,23 +2043,97 @@ constexpr int kOrderedBodies = 524288;
 // 1024 walks: 314 / 332, 320 / 318, 406 / 380 us).  Under the reference's rule always 16,
 // with room for 4096 groups: its longest walks, not the number of walks, take the time.
 constexpr int kFewWalks = 400;
-// Pool entries per body, the second under the reference's rule (4 and 8 used at
-// n = 100,000, theta 0.5).
-constexpr int kLogPerBody[2] = {8, 16};
+constexpr int kLogSegments = 16;  // times a walk's groups may move to the pool
+// Beyond this many pool entries per body the serial walk is taken (log_per_body).
+constexpr double kMostLogPerBody = 64.0;
 constexpr int kLogChunk = 256;    // terms per list
 constexpr int kLogListers = 128;  // threads of log_eval_kernel that list terms
 
 template <bool DIR, int WARPS, int GROUPS>
 struct LogShared {
     static_assert(GROUPS <= 4096, "a slot has 12 bits");
+    static_assert(GROUPS % (32 * WARPS) == 0 && (GROUPS & (GROUPS - 1)) == 0, "log_flush");
     static constexpr int kStack = 3 * GROUPS / 4;
     unsigned long long sorted[GROUPS];  // key, slot (12 bits), records (4), opened ones (8)
     int first[GROUPS];                  // by slot: the group's first record
+    static constexpr int kKeep = GROUPS / (32 * WARPS);
     float4 test[WARPS][32], side[DIR ? WARPS : 1][32];
     int s_first[kStack];  // the stack: as group_walk_kernel's, and the groups' keys
     unsigned s_key[kStack];
     unsigned char s_kids[kStack];
 };
+
+// Sorts the CTA's groups and moves the complete ones, those before `key` in the serial
+// order (all: every one), to the pool, as segment `seg` of the walk; the rest take the
+// first slots.  Returns how many stay, or -1 where there is no room.
+template <class Shared>
+__device__ __forceinline__ int log_flush(Shared &sh, int groups, bool all, unsigned key, int seg,
+                                         int2 *__restrict__ segs, uint2 *__restrict__ pool,
+                                         int pool_size, unsigned long long *__restrict__ pool_next,
+                                         int before, int *s_at)
+{
+    __syncthreads();
+    // bitonic sort, padded to a power of two
+    int size = 1;
+    while (size < groups) size <<= 1;
+    for (int k = groups + (int)threadIdx.x; k < size; k += blockDim.x) sh.sorted[k] = ~0ull;
+    for (int k = 2; k <= size; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            __syncthreads();
+            for (int t = threadIdx.x; t < size / 2; t += blockDim.x) {
+                const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo | j;
+                const unsigned long long a = sh.sorted[lo], b = sh.sorted[hi];
+                if ((a > b) == ((lo & k) == 0)) {
+                    sh.sorted[lo] = b;
+                    sh.sorted[hi] = a;
+                }
+            }
+        }
+    __syncthreads();
+    int done = groups;
+    if (!all) {  // the number of groups before key
+        int lo = -1;
+        while (done - lo > 1) {
+            const int mid = (lo + done) / 2;
+            if ((unsigned)(sh.sorted[mid] >> 24) < key) lo = mid;
+            else done = mid;
+        }
+    }
+    if (threadIdx.x == 0) {
+        const unsigned long long at = atomicAdd(pool_next, (unsigned long long)done);
+        const bool room = seg < kLogSegments &&
+                          at + done <= (unsigned long long)pool_size;
+        *s_at = room ? (int)at : -1;
+        if (room) segs[seg] = make_int2((int)at, before + done);
+    }
+    __syncthreads();
+    const int at = *s_at;
+    if (at < 0) return -1;
+    for (int k = threadIdx.x; k < done; k += blockDim.x) {
+        const unsigned low = (unsigned)sh.sorted[k];
+        pool[at + k] = make_uint2((unsigned)sh.first[(low >> 12) & 0xFFFu], low & 0xFFFu);
+    }
+    if (all) return 0;
+    unsigned long long kept[Shared::kKeep];
+    int first[Shared::kKeep];
+#pragma unroll
+    for (int u = 0; u < Shared::kKeep; ++u) {
+        const int k = done + (int)threadIdx.x + u * (int)blockDim.x;
+        kept[u] = k < groups ? sh.sorted[k] : 0ull;
+        first[u] = k < groups ? sh.first[(unsigned)(kept[u] >> 12) & 0xFFFu] : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < Shared::kKeep; ++u) {
+        const int to = (int)threadIdx.x + u * (int)blockDim.x;
+        if (done + to < groups) {
+            sh.sorted[to] = (kept[u] & ~0xFFF000ull) | (unsigned)to << 12;
+            sh.first[to] = first[u];
+        }
+    }
+    __syncthreads();
+    return groups - done;
+}
 
 // Bound by dispatch; under the reference's rule, with 0.35 ms at n = 100,000 (theta
 // 0.5, disk galaxy), by that of the longest walk (1,939 groups in 35 rounds of up to 64, of 10,000 cycles each with
@@ -1917,8 +2146,9 @@ __global__ void __launch_bounds__(32 * WARPS, 32 / WARPS)
 decide_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restrict__ gnk,
               const unsigned *__restrict__ gkey, const float4 *__restrict__ gpcen,
               const int *__restrict__ total, const float4 *__restrict__ body, int n, float theta2,
-              BHStats *__restrict__ stats, int2 *__restrict__ walks, uint2 *__restrict__ pool,
-              int pool_size, unsigned long long *__restrict__ pool_next)
+              BHStats *__restrict__ stats, int2 *__restrict__ walks, int2 *__restrict__ segs,
+              uint2 *__restrict__ pool, int pool_size,
+              unsigned long long *__restrict__ pool_next)
 {
     constexpr int W = WARPS;
     extern __shared__ __align__(16) unsigned char walk_shared[];
@@ -1946,14 +2176,21 @@ decide_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restric
         sh.s_key[0] = 0;
         s_m2p = s_p2p = 0;
     }
+    segs += (size_t)blockIdx.x * kLogSegments;
     unsigned m2p = 0, p2p = 0;  // per lane
-    int sp = 1, groups = 0;
+    int sp = 1, groups = 0, moved = 0, seg = 0;  // moved: groups in the pool
     bool fits = true;
     while (sp > 0) {
         __syncthreads();
         const int take = min(sp, 4 * W);
-        fits = groups + take <= GROUPS;
-        if (!fits) break;
+        if (groups + take > GROUPS) {
+            const int stay = log_flush(sh, groups, false, sh.s_key[sp - 1], seg++, segs, pool,
+                                       pool_size, pool_next, moved, &s_at);
+            moved += groups - stay;
+            groups = stay;
+            fits = stay >= 0 && stay + take <= GROUPS;
+            if (!fits) break;
+        }
         // the first groups to the first warps: in a narrow round the others have none
         const int j = 4 * w + (lane >> 3), e = sp - 1 - j;
         const bool busy = 4 * w < take;
@@ -1988,66 +2225,39 @@ decide_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__restric
         groups += take;
         if (lane == 0) s_push[w] = __popc(push);
         __syncthreads();  // every warp has read its groups, too
+        // in the serial order: the first group's children on top, the last child first
         int top = sp;
         for (int v = 0; v < W; ++v) {
-            if (v < w) top += s_push[v];
+            if (v > w) top += s_push[v];
             sp += s_push[v];
         }
         fits = sp <= Shared::kStack;
         if (!fits) break;
         if (inner) {
-            const int to = top + __popc(push & ((1u << lane) - 1u));
+            const unsigned mine = 0xFFu << (lane & 24), later = ~(mine | (mine - 1u));
+            const int to = top + __popc(push & (later | (mine & ((1u << lane) - 1u))));
             sh.s_first[to] = nd.kids;
             sh.s_kids[to] = gnk[id];
             sh.s_key[to] = gkey[id];
         }
     }
-    if (!fits) {
-        if (threadIdx.x == 0) walks[blockIdx.x] = make_int2(0, -1);
-        return;
-    }
-    __syncthreads();
-    // bitonic sort of the groups, padded to a power of two
-    int size = 1;
-    while (size < groups) size <<= 1;
-    for (int k = groups + (int)threadIdx.x; k < size; k += blockDim.x) sh.sorted[k] = ~0ull;
-    for (int k = 2; k <= size; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            __syncthreads();
-            for (int t = threadIdx.x; t < size / 2; t += blockDim.x) {
-                const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo | j;
-                const unsigned long long a = sh.sorted[lo], b = sh.sorted[hi];
-                if ((a > b) == ((lo & k) == 0)) {
-                    sh.sorted[lo] = b;
-                    sh.sorted[hi] = a;
-                }
-            }
-        }
+    if (fits)
+        fits = log_flush(sh, groups, true, 0u, seg++, segs, pool, pool_size, pool_next, moved,
+                         &s_at) == 0;
+    if (threadIdx.x == 0) walks[blockIdx.x] = make_int2(seg, fits ? moved + groups : -1);
+    if (!fits) return;
     m2p = __reduce_add_sync(0xffffffffu, m2p);
     p2p = __reduce_add_sync(0xffffffffu, p2p);
     if (lane == 0) {
         atomicAdd(&s_m2p, m2p);
         atomicAdd(&s_p2p, p2p);
     }
-    if (threadIdx.x == 0) {
-        const unsigned long long at = atomicAdd(pool_next, (unsigned long long)groups);
-        s_at = at + groups <= (unsigned long long)pool_size ? (int)at : -1;
-    }
     __syncthreads();
-    const int at = s_at;
     if (threadIdx.x == 0) {
-        walks[blockIdx.x] = make_int2(at, at < 0 ? -1 : groups);
-        if (at >= 0) {
-            const unsigned long long nv = wend - w0;
-            atomicAdd(&stats->m2p, s_m2p * nv);
-            atomicAdd(&stats->p2p, s_p2p * nv);
-            atomicAdd(&stats->total, (s_m2p + s_p2p) * nv);
-        }
-    }
-    if (at < 0) return;
-    for (int k = threadIdx.x; k < groups; k += blockDim.x) {
-        const unsigned low = (unsigned)sh.sorted[k];
-        pool[at + k] = make_uint2((unsigned)sh.first[(low >> 12) & 0xFFFu], low & 0xFFFu);
+        const unsigned long long nv = wend - w0;
+        atomicAdd(&stats->m2p, s_m2p * nv);
+        atomicAdd(&stats->p2p, s_p2p * nv);
+        atomicAdd(&stats->total, (s_m2p + s_p2p) * nv);
     }
 }
 
@@ -2066,8 +2276,8 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ g
                 const float4 *__restrict__ body,
                 const uint32_t *__restrict__ order, int n, float eps2, double G,
                 double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
-                const int2 *__restrict__ walks, const uint2 *__restrict__ pool,
-                const AfterForce after)
+                const int2 *__restrict__ walks, const int2 *__restrict__ segs,
+                const uint2 *__restrict__ pool, const AfterForce after)
 {
     __shared__ float4 s_term[2][kLogChunk];  // position, mass
     __shared__ float2 s_soft[2][kLogChunk];  // eps^2, added before a body's r^2, after a node's
@@ -2080,7 +2290,7 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ g
     __shared__ int s_body[kLogListers];    // the first body of an opened leaf; -1: a node's term
     __shared__ int s_incl[kLogListers];    // running count of terms
     __shared__ int s_warp[kLogListers / 32];
-    const int2 walk = walks[blockIdx.x];
+    const int2 walk = walks[blockIdx.x];  // segments, groups
     if (walk.y < 0) return;
     const int w0 = blockIdx.x * 64;
     if (threadIdx.x < 64) {
@@ -2137,8 +2347,17 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ g
     // batch after it: neither trip to memory waits for the other.
     const int q = threadIdx.x - 64, lane = q & 31, wq = q >> 5;
     const int child = q & 7;
+    // the segment of the lister's next group (they only go up): its place in the pool, the
+    // group after its last, and its first
+    const int2 *seg = segs + (size_t)blockIdx.x * kLogSegments, *const last = seg + walk.x - 1;
+    int2 in_seg = *seg;
+    int seg0 = 0;
     auto load_log = [&](int g) {
-        return g < walk.y ? pool[walk.x + g] : make_uint2(0u, 0u);
+        while (g >= in_seg.y && seg < last) {
+            seg0 = in_seg.y;
+            in_seg = *++seg;
+        }
+        return g < walk.y ? pool[in_seg.x + g - seg0] : make_uint2(0u, 0u);
     };
     auto load_node = [&](uint2 log) {
         return gnodes[child < (int)(log.y >> 8) ? log.x + child : 0];
@@ -2213,6 +2432,53 @@ log_eval_kernel(const BHGNode *__restrict__ gnodes, const float4 *__restrict__ g
     }
 }
 
+// How a walk is computed.  The serial and the ordered walk give the same bits.
+enum class Walk { kPreorder, kGroup, kSerial, kOrdered };
+
+// Body pairs per lane of the walk (0: the one-body-per-lane preorder walk);
+// NB_BH_WALK_PAIRS overrides the default.
+int walk_pairs()
+{
+    static const int np = [] {
+        const char *e = std::getenv("NB_BH_WALK_PAIRS");
+        const int v = e ? std::atoi(e) : 1;
+        return v < 0 ? 0 : (v > 2 ? 2 : v);
+    }();
+    return np;
+}
+
+// Pool entries per body that an ordered walk is given, above the mean of the groups that
+// walks visit divided by their 64 bodies.  Means of Plummer spheres (disks have half),
+// per body, at theta 0.5 / 0.4 / 0.3 / 0.2:
+//   n =    16,384    4.3 /  5.7 /  8.2 / 11.6    the reference's rule   6.1 /  7.6 /  9.6 / 12.5
+//   n =   100,000    6.3 /  9.3 / 16.3 / 32.1                          10.9 / 15.1 / 23.0 / 39.7
+//   n =   500,000    7.3 / 11.4 / 22.1 / 53.0                          15.6 / 22.7 / 38.4 / 78.9
+//   n = 1,000,000                                                      17.5 / 25.7 / 45.4 / 98.5
+// With one body per leaf 1.5 times as many, twice under the reference's rule.  Where
+// that is more than kMostLogPerBody (512 bytes per body) the serial walk is taken: its
+// walks fill the chip then, and what the ordered walk lists and sorts costs more.
+double log_per_body(int n, double theta, int leaf_capacity, bool ref_open)
+{
+    const double base = ref_open ? 18.0 : 8.0, angle = 0.5 / std::max(theta, 1e-3);
+    const double small = ref_open ? std::pow(n / 1e6, 0.30) : std::pow(n / 5e5, 0.35);
+    const double more = std::max(0.0, std::pow(angle, ref_open ? 1.9 : 2.3) - 1.0);
+    const double leaves = 1.0 + std::max(0, 8 - leaf_capacity) / (ref_open ? 7.0 : 14.0);
+    return base * leaves * (1.0 + more * std::min(1.0, small));
+}
+
+// The walk of n bodies: over child groups, or the stackless preorder walk
+// (NB_BH_WALK=preorder, read at every walk; both find the same interactions).
+// NB_BH_WALK=serial takes the serial walk where the ordered one is the default.
+Walk choose_walk(int n, double theta, int leaf_capacity, bool ref_open)
+{
+    const char *e = std::getenv("NB_BH_WALK");
+    if (walk_pairs() < 1 || (e && std::strcmp(e, "preorder") == 0)) return Walk::kPreorder;
+    if (walk_pairs() > 1 || (!ref_open && n > kOrderedBodies)) return Walk::kGroup;
+    if (e && std::strcmp(e, "serial") == 0) return Walk::kSerial;
+    return log_per_body(n, theta, leaf_capacity, ref_open) <= kMostLogPerBody ? Walk::kOrdered
+                                                                              : Walk::kSerial;
+}
+
 int div_up(long a, long b) { return (int)((a + b - 1) / b); }
 
 template <class T>
@@ -2244,7 +2510,8 @@ struct BHTree {
         gpcen, gquad, gkey, walks, logs;
     bool with_quad = false;     // the nodes carry quadrupoles (quad, 2 float4 per node)
     bool ref_open = false;      // the reference's opening rule (the child toward the body too)
-    bool ordered = false;       // walks add their terms in the serial walk's order (gkey is set)
+    Walk walk = Walk::kGroup;   // the next walk's kernels (ordered: gkey and logs are set)
+    int log_pool = 0;           // entries of the pool in logs
     bool pcen_valid = false;    // pcen holds the parent centres of the current topology
     const uint64_t *sorted_codes = nullptr;
     const uint32_t *order = nullptr;
@@ -2448,7 +2715,7 @@ nb_status bh_hilbert_order(BHTree *t, const double *x, const double *y, const do
     return NB_OK;
 }
 
-// Warps that share the walk of one CTA's bodies: doubled while there are no more
+// Warps that share the group walk of one CTA's bodies: doubled while there are no more
 // than 110 per SM, up to 8.  Fewer CTAs than fill the chip leave it to the longest
 // walks, which more warps shorten; with enough CTAs the rounds' barriers and the
 // shorter lists only cost.  A whole force evaluation took, with 1 / 2 / 4 / 8 / 16
@@ -2458,7 +2725,7 @@ nb_status bh_hilbert_order(BHTree *t, const double *x, const double *y, const do
 //   n =   262,144    999 /  928 /  881 /  913 / 1111
 //   n =   524,288   1380 / 1347 / 1364 / 1479 / 1887
 //   n = 1,048,576   2368 / 2395 / 2501 / 2725 / 3606
-// The reference's rule (its walks without a log) opens far more for some bodies than
+// The reference's rule opens far more for some bodies than
 // for others (the longest walk at n = 100,000 has 20,270 interactions, the mean 3,891),
 // so three times as many, up to 16:
 //   n =   100,000   3141 / 1925 / 1196 /  922 /  830
@@ -2475,55 +2742,29 @@ int walk_warps(int ctas)
     return w;
 }
 
-// Body pairs per lane of the walk (0: the one-body-per-lane preorder walk);
-// NB_BH_WALK_PAIRS overrides the default.
-int walk_pairs()
-{
-    static const int np = [] {
-        const char *e = std::getenv("NB_BH_WALK_PAIRS");
-        const int v = e ? std::atoi(e) : 1;
-        return v < 0 ? 0 : (v > 2 ? 2 : v);
-    }();
-    return np;
-}
-
-// The walk over child groups (default) or the stackless preorder walk
-// (NB_BH_WALK=preorder, read at every walk; both find the same interactions).
-bool group_walk()
-{
-    const char *e = std::getenv("NB_BH_WALK");
-    return !(e && std::strcmp(e, "preorder") == 0);
-}
-
-int log_pool_size(const BHTree *t, int n)
-{
-    return (int)std::min((long)kLogPerBody[t->ref_open] * n + 64, (long)INT32_MAX);
-}
-
 template <bool ZS, bool Q, bool D>
 void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *ax, double *ay,
                  double *az, cudaStream_t st, const AfterForce &after)
 {
     const int np = walk_pairs();
     const float4 *pc = t->pcen.as<float4>();
-    if (group_walk() && np >= 1) {
-        const BHGNode *gn = t->gnodes.as<BHGNode>();
-        const unsigned char *gk = t->gnk.as<unsigned char>();
-        const float4 *gq = t->gquad.as<float4>(), *gp = t->gpcen.as<float4>();
-        const int ctas = div_up(n, 64 * np);
-        int warps = walk_warps<Q, D>(ctas);
+    const BHGNode *gn = t->gnodes.as<BHGNode>();
+    const unsigned char *gk = t->gnk.as<unsigned char>();
+    const float4 *gq = t->gquad.as<float4>(), *gp = t->gpcen.as<float4>();
+    if (t->walk == Walk::kOrdered || t->walk == Walk::kSerial) {
+        const int ctas = div_up(n, 64);
         const int2 *logged = nullptr;
-        if (t->ordered && np == 1) {
+        if (t->walk == Walk::kOrdered) {
             // logs: the pool's counter, then the pool
             unsigned long long *next = t->logs.as<unsigned long long>();
             uint2 *pool = reinterpret_cast<uint2 *>(next + 1);
-            int2 *walks = t->walks.as<int2>();
+            int2 *walks = t->walks.as<int2>(), *segs = walks + ctas;
             auto decide = [&](auto *kernel, int threads, size_t shared) {
                 cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)shared);
                 kernel<<<ctas, threads, shared, st>>>(
                     gn, gk, t->gkey.as<unsigned>(), gp, d_total(t), t->body.as<float4>(), n,
-                    theta2, t->stats.as<BHStats>(), walks, pool, log_pool_size(t, n), next);
+                    theta2, t->stats.as<BHStats>(), walks, segs, pool, t->log_pool, next);
             };
             if (D || ctas <= kFewWalks)
                 decide(decide_kernel<D, 16, D ? 4096 : 1024>, 512,
@@ -2531,17 +2772,23 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
             else
                 decide(decide_kernel<D, 4, 1024>, 128, sizeof(LogShared<D, 4, 1024>));
             log_eval_kernel<ZS, Q><<<ctas, 64 + kLogListers, 0, st>>>(
-                gn, gq, t->body.as<float4>(), t->order, n, eps2, G, ax, ay, az, walks, pool, after);
-            logged = walks;
-            if (!D) warps = std::min(warps, 2);  // mostly none are left: a launch that only looks
+                gn, gq, t->body.as<float4>(), t->order, n, eps2, G, ax, ay, az, walks, segs, pool,
+                after);
+            logged = walks;  // mostly none are left: a launch that only looks
         }
-        auto *kernel = np == 2 ? group_walk_kernel<ZS, Q, 2, D> : group_walk_kernel<ZS, Q, 1, D>;
+        serial_walk_kernel<ZS, Q, D><<<ctas, 32, 0, st>>>(
+            gn, gk, d_total(t), t->body.as<float4>(), t->order, n, theta2, eps2, G, ax, ay, az,
+            t->stats.as<BHStats>(), gq, gp, logged, after);
+    } else if (t->walk == Walk::kGroup) {
+        const int ctas = div_up(n, 64 * np), warps = walk_warps<Q, D>(ctas);
+        // one pair per lane: never under the reference's rule (choose_walk)
+        auto *kernel = np == 2 ? group_walk_kernel<ZS, Q, 2, D> : group_walk_kernel<ZS, Q, 1, false>;
         const size_t shared = walk_shared_bytes<Q>(warps);
         if (shared > 48 * 1024 - 256)
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
         kernel<<<ctas, 32 * warps, shared, st>>>(
             gn, gk, d_total(t), t->body.as<float4>(), t->order, n, theta2, eps2, G, ax, ay, az,
-            t->stats.as<BHStats>(), gq, gp, logged, after);
+            t->stats.as<BHStats>(), gq, gp, after);
     } else if (np == 2)
         walk2_kernel<ZS, Q, 2, D><<<div_up(n, 4 * kWalkBlock), kWalkBlock, 0, st>>>(
             t->nodes.as<BHNode>(), d_total(t), t->body.as<float4>(), t->order, n, theta2,
@@ -2581,7 +2828,7 @@ static nb_status launch_walk(BHTree *t, int n, double G, double eps2, double the
     NB_LAUNCH_CHECK();
     if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
     // the child-group walks apply the update, the preorder walks do not
-    if (!group_walk() || walk_pairs() < 1) return apply_after(after, n, ax, ay, az, st);
+    if (t->walk == Walk::kPreorder) return apply_after(after, n, ax, ay, az, st);
     return NB_OK;
 }
 
@@ -2643,11 +2890,10 @@ static nb_status group_nodes(BHTree *t, cudaStream_t st, bool recount)
     NB_TRY(t->gnk.reserve((size_t)slots));
     if (t->ref_open) NB_TRY(t->gpcen.reserve(sizeof(float4) * (size_t)slots));
     if (t->with_quad) NB_TRY(t->gquad.reserve(sizeof(float4) * 2 * (size_t)slots));
-    t->ordered = t->ref_open || t->n <= kOrderedBodies;
-    if (t->ordered) {
+    if (t->walk == Walk::kOrdered) {
         NB_TRY(t->gkey.reserve(sizeof(unsigned) * (size_t)slots));
-        NB_TRY(t->walks.reserve(sizeof(int2) * (size_t)div_up(t->n, 64)));
-        NB_TRY(t->logs.reserve(sizeof(uint2) * ((size_t)log_pool_size(t, t->n) + 1)));
+        NB_TRY(t->walks.reserve(sizeof(int2) * (1 + kLogSegments) * (size_t)div_up(t->n, 64)));
+        NB_TRY(t->logs.reserve(sizeof(uint2) * ((size_t)t->log_pool + 1)));
     }
     group_kernel<<<grid, 256, 0, st>>>(
         t->nodes.as<BHNode>(), d_total(t), t->occ.as<unsigned>(), t->kbase.as<int>(),
@@ -2656,8 +2902,8 @@ static nb_status group_nodes(BHTree *t, cudaStream_t st, bool recount)
         t->with_quad ? t->quad.as<float4>() : nullptr, t->gnodes.as<BHGNode>(),
         t->gnk.as<unsigned char>(), t->gpcen.as<float4>(),
         t->with_quad ? t->gquad.as<float4>() : nullptr, t->node_depth.as<unsigned char>(),
-        t->ordered ? t->gkey.as<unsigned>() : nullptr,
-        t->ordered ? t->logs.as<unsigned long long>() : nullptr);
+        t->walk == Walk::kOrdered ? t->gkey.as<unsigned>() : nullptr,
+        t->walk == Walk::kOrdered ? t->logs.as<unsigned long long>() : nullptr);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
@@ -2701,6 +2947,8 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
     if (n <= 0) return NB_OK;
     t->with_quad = quad;
     t->ref_open = ref_open;
+    t->walk = choose_walk(n, theta, leaf_capacity, ref_open);
+    t->log_pool = (int)std::min(log_per_body(n, theta, leaf_capacity, ref_open) * n + 64.0, 2e9);
     if (ax && reuse > 1 && t->tree_valid && t->n == n && t->evals_since_build < reuse) {
         NB_TRY(refit(t, x, y, z, m, n, st));
         if (quad) NB_TRY(compute_quads(t, x, y, z, m, n, st));
