@@ -2733,12 +2733,17 @@ nb_status bh_hilbert_order(BHTree *t, const double *x, const double *y, const do
 // Quadrupoles hold more registers, so half as many:
 //   n =   100,000    766 /  726 /  665 /  685 /  806
 //   n =   500,000   2132 / 2169 / 2324 / 2666 / 3400
+template <bool D>
+constexpr int most_walk_warps()
+{
+    return D ? kWalkWarps : kWalkWarps / 2;
+}
 template <bool Q, bool D>
 int walk_warps(int ctas)
 {
     const long sought = (Q ? 55L : 110L) * (D ? 3 : 1) * device_props().num_sms;
     int w = 1;
-    while (w < (D ? kWalkWarps : kWalkWarps / 2) && 2L * w * ctas <= sought) w *= 2;
+    while (w < most_walk_warps<D>() && 2L * w * ctas <= sought) w *= 2;
     return w;
 }
 
@@ -2784,8 +2789,10 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
         // one pair per lane: never under the reference's rule (choose_walk)
         auto *kernel = np == 2 ? group_walk_kernel<ZS, Q, 2, D> : group_walk_kernel<ZS, Q, 1, false>;
         const size_t shared = walk_shared_bytes<Q>(warps);
-        if (shared > 48 * 1024 - 256)
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        // what the most warps need, not these: the attribute is the function's, and
+        // another thread's launch may come between this call and the launch below
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)walk_shared_bytes<Q>(most_walk_warps<D>()));
         kernel<<<ctas, 32 * warps, shared, st>>>(
             gn, gk, d_total(t), t->body.as<float4>(), t->order, n, theta2, eps2, G, ax, ay, az,
             t->stats.as<BHStats>(), gq, gp, after);
