@@ -2747,9 +2747,11 @@ int walk_warps(int ctas)
     return w;
 }
 
+// Every launch is checked before the next: a kernel that did not run leaves walks and
+// logs of an earlier evaluation, which the next would follow.
 template <bool ZS, bool Q, bool D>
-void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *ax, double *ay,
-                 double *az, cudaStream_t st, const AfterForce &after)
+nb_status walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *ax,
+                      double *ay, double *az, cudaStream_t st, const AfterForce &after)
 {
     const int np = walk_pairs();
     const float4 *pc = t->pcen.as<float4>();
@@ -2764,21 +2766,24 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
             unsigned long long *next = t->logs.as<unsigned long long>();
             uint2 *pool = reinterpret_cast<uint2 *>(next + 1);
             int2 *walks = t->walks.as<int2>(), *segs = walks + ctas;
-            auto decide = [&](auto *kernel, int threads, size_t shared) {
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)shared);
+            auto decide = [&](auto *kernel, int threads, size_t shared) -> nb_status {
+                NB_CUDA_TRY(cudaFuncSetAttribute(
+                    kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
                 kernel<<<ctas, threads, shared, st>>>(
                     gn, gk, t->gkey.as<unsigned>(), gp, d_total(t), t->body.as<float4>(), n,
                     theta2, t->stats.as<BHStats>(), walks, segs, pool, t->log_pool, next);
+                NB_LAUNCH_CHECK();
+                return NB_OK;
             };
             if (D || ctas <= kFewWalks)
-                decide(decide_kernel<D, 16, D ? 4096 : 1024>, 512,
-                       sizeof(LogShared<D, 16, D ? 4096 : 1024>));
+                NB_TRY(decide(decide_kernel<D, 16, D ? 4096 : 1024>, 512,
+                              sizeof(LogShared<D, 16, D ? 4096 : 1024>)));
             else
-                decide(decide_kernel<D, 4, 1024>, 128, sizeof(LogShared<D, 4, 1024>));
+                NB_TRY(decide(decide_kernel<D, 4, 1024>, 128, sizeof(LogShared<D, 4, 1024>)));
             log_eval_kernel<ZS, Q><<<ctas, 64 + kLogListers, 0, st>>>(
                 gn, gq, t->body.as<float4>(), t->order, n, eps2, G, ax, ay, az, walks, segs, pool,
                 after);
+            NB_LAUNCH_CHECK();
             logged = walks;  // mostly none are left: a launch that only looks
         }
         serial_walk_kernel<ZS, Q, D><<<ctas, 32, 0, st>>>(
@@ -2791,8 +2796,8 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
         const size_t shared = walk_shared_bytes<Q>(warps);
         // what the most warps need, not these: the attribute is the function's, and
         // another thread's launch may come between this call and the launch below
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)walk_shared_bytes<Q>(most_walk_warps<D>()));
+        NB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)walk_shared_bytes<Q>(most_walk_warps<D>())));
         kernel<<<ctas, 32 * warps, shared, st>>>(
             gn, gk, d_total(t), t->body.as<float4>(), t->order, n, theta2, eps2, G, ax, ay, az,
             t->stats.as<BHStats>(), gq, gp, after);
@@ -2808,14 +2813,16 @@ void walk_launch(BHTree *t, int n, float theta2, float eps2, double G, double *a
         walk_kernel<ZS, Q, D><<<div_up(n, kWalkBlock), kWalkBlock, 0, st>>>(
             t->nodes.as<BHNode>(), d_total(t), t->body.as<float4>(), t->order, n, theta2,
             eps2, G, ax, ay, az, t->stats.as<BHStats>(), t->quad.as<float4>(), pc);
+    NB_LAUNCH_CHECK();
+    return NB_OK;
 }
 
 template <bool ZS, bool Q>
-void walk_launch_rule(BHTree *t, int n, float theta2, float eps2, double G, double *ax,
-                      double *ay, double *az, cudaStream_t st, const AfterForce &after)
+nb_status walk_launch_rule(BHTree *t, int n, float theta2, float eps2, double G, double *ax,
+                           double *ay, double *az, cudaStream_t st, const AfterForce &after)
 {
-    if (t->ref_open) walk_launch<ZS, Q, true>(t, n, theta2, eps2, G, ax, ay, az, st, after);
-    else walk_launch<ZS, Q, false>(t, n, theta2, eps2, G, ax, ay, az, st, after);
+    return t->ref_open ? walk_launch<ZS, Q, true>(t, n, theta2, eps2, G, ax, ay, az, st, after)
+                       : walk_launch<ZS, Q, false>(t, n, theta2, eps2, G, ax, ay, az, st, after);
 }
 
 static nb_status launch_walk(BHTree *t, int n, double G, double eps2, double theta, double *ax,
@@ -2825,14 +2832,11 @@ static nb_status launch_walk(BHTree *t, int n, double G, double eps2, double the
     NvtxRange range("bh_walk");
     const float th2 = (float)(theta * theta), e2 = (float)eps2;
     if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
-    if (t->with_quad) {
-        if (eps2 > 0.0) walk_launch_rule<false, true>(t, n, th2, e2, G, ax, ay, az, st, after);
-        else walk_launch_rule<true, true>(t, n, th2, 0.0f, G, ax, ay, az, st, after);
-    } else {
-        if (eps2 > 0.0) walk_launch_rule<false, false>(t, n, th2, e2, G, ax, ay, az, st, after);
-        else walk_launch_rule<true, false>(t, n, th2, 0.0f, G, ax, ay, az, st, after);
-    }
-    NB_LAUNCH_CHECK();
+    const bool zero = !(eps2 > 0.0);
+    auto *launch = t->with_quad
+                       ? (zero ? walk_launch_rule<true, true> : walk_launch_rule<false, true>)
+                       : (zero ? walk_launch_rule<true, false> : walk_launch_rule<false, false>);
+    NB_TRY(launch(t, n, th2, zero ? 0.0f : e2, G, ax, ay, az, st, after));
     if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
     // the child-group walks apply the update, the preorder walks do not
     if (t->walk == Walk::kPreorder) return apply_after(after, n, ax, ay, az, st);
