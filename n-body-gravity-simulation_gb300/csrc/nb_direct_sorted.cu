@@ -319,12 +319,11 @@ __device__ __forceinline__ void far_tile_pair(const float4 *__restrict__ hi,
 // tile pairs are met one by one, relative to the smaller tile's centre and with
 // the Newton step.
 // part: plane p - p0 holds the first side's sums of diagonal p, plane np + p - p0
-// the second's (one rounding of a Kahan pair: with 64 planes and more it adds
-// 2e-9 to an error of 3e-8).
+// the second's, as Kahan pairs (sum, negated compensation).
 __global__ void __launch_bounds__(32, kFarCtas)
 direct_far_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                   const float4 *__restrict__ tile, int n, int tiles, float eps2, int blocks,
-                  int p0, int np, float *__restrict__ part)
+                  int p0, int np, float2 *__restrict__ part)
 {
     static_assert(kFarTiles == 4, "the lanes' tile-pair tests");
     __shared__ TileJ stage;
@@ -374,7 +373,7 @@ direct_far_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     const float2 e2 = dup2(eps2);
     for (int v = 0; v < kFarTiles; ++v) tile_sums_zero(jsum[v], lane);
     const size_t plane = (size_t)n;
-    float *pa = part + 3 * plane * dp, *pb = part + 3 * plane * (np + dp);
+    float2 *pa = part + 3 * plane * dp, *pb = part + 3 * plane * (np + dp);
     for (int h = 0; 2 * h < ta; ++h) {
         tile_sums_zero(isum[0], lane);
         tile_sums_zero(isum[1], lane);
@@ -428,8 +427,8 @@ direct_far_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                     two_sum(t.y, js.y, t.y, r.y);
                     e = make_float2(r.x + (e.x + jc.x), r.y + (e.y + jc.y));
                 }
-                if (i < n) pa[d * plane + i] = t.x + e.x;
-                if (i + 32 < n) pa[d * plane + i + 32] = t.y + e.y;
+                if (i < n) pa[d * plane + i] = make_float2(t.x, e.x);
+                if (i + 32 < n) pa[d * plane + i + 32] = make_float2(t.y, e.y);
             }
         }
     }
@@ -439,8 +438,8 @@ direct_far_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const float2 js = jsum[v].s[d][lane], jc = jsum[v].c[d][lane];
-            if (j < n) pb[d * plane + j] = js.x + jc.x;
-            if (j + 32 < n) pb[d * plane + j + 32] = js.y + jc.y;
+            if (j < n) pb[d * plane + j] = make_float2(js.x, jc.x);
+            if (j + 32 < n) pb[d * plane + j + 32] = make_float2(js.y, jc.y);
         }
     }
 }
@@ -911,7 +910,7 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
 // thread per body had too few loads in flight (66 us at n = 65,536, 205 MB).
 constexpr int kCombineGroups = 8;
 __global__ void __launch_bounds__(32 * kCombineGroups)
-combine_sorted_kernel(const float *__restrict__ part, int blocks, int p0, int np, bool first,
+combine_sorted_kernel(const float2 *__restrict__ part, int blocks, int p0, int np, bool first,
                       bool last, float *__restrict__ acc, const float *__restrict__ psum,
                       const float *__restrict__ pcomp, int n, int segments, double G,
                       const uint32_t *__restrict__ order, const double *__restrict__ ex,
@@ -926,7 +925,7 @@ combine_sorted_kernel(const float *__restrict__ part, int blocks, int p0, int np
     float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
     if (i < n) {
         for (int k0 = g; k0 < 2 * np; k0 += 8 * kCombineGroups) {
-            float t[8][3];
+            float2 t[8][3];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int k = k0 + u * kCombineGroups;
@@ -934,12 +933,12 @@ combine_sorted_kernel(const float *__restrict__ part, int blocks, int p0, int np
                                         : k < 2 * np && pair_second(p0 + k - np, blk, blocks);
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
-                    t[u][c] = use ? part[((size_t)k * 3 + c) * plane + i] : 0.f;
+                    t[u][c] = use ? part[((size_t)k * 3 + c) * plane + i] : dup2(0.f);
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u)
 #pragma unroll
-                for (int c = 0; c < 3; ++c) ds_add_kahan(hi[c], lo[c], t[u][c], 0.f);
+                for (int c = 0; c < 3; ++c) ds_add_kahan(hi[c], lo[c], t[u][c].x, -t[u][c].y);
         }
         for (int s = g; last && s < segments; s += kCombineGroups)
 #pragma unroll
@@ -1095,7 +1094,7 @@ nb_status direct_mixed_sorted(const double *x, const double *y, const double *z,
     const int segments = near_segments(tiles);
     const int blocks = (tiles + kFarTiles - 1) / kFarTiles, diagonals = blocks / 2 + 1;
     // the diagonals in passes whose planes stay within kFarPlaneBytes
-    const size_t per_diagonal = sizeof(float) * 6 * (size_t)n;
+    const size_t per_diagonal = sizeof(float2) * 6 * (size_t)n;
     const int pass = (int)std::min<size_t>(diagonals,
                                            std::max<size_t>(1, kFarPlaneBytes / per_diagonal));
     NB_TRY(b.far.reserve(per_diagonal * pass));
@@ -1107,7 +1106,7 @@ nb_status direct_mixed_sorted(const double *x, const double *y, const double *z,
         const int np = std::min(pass, diagonals - p0);
         direct_far_kernel<<<(unsigned)blocks * (unsigned)np, 32, 0, st>>>(
             hi, lo, b.tiles.as<float4>(), n, tiles, eps2 > 0.0 ? (float)eps2 : 0.0f, blocks, p0, np,
-            b.far.as<float>());
+            b.far.as<float2>());
         NB_LAUNCH_CHECK();
         const bool last = p0 + np == diagonals;
         if (last) {
@@ -1115,7 +1114,7 @@ nb_status direct_mixed_sorted(const double *x, const double *y, const double *z,
             if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
         }
         combine_sorted_kernel<<<(n + 31) / 32, 32 * kCombineGroups, 0, st>>>(
-            b.far.as<float>(), blocks, p0, np, p0 == 0, last, b.acc.as<float>(), psum, pcomp, n,
+            b.far.as<float2>(), blocks, p0, np, p0 == 0, last, b.acc.as<float>(), psum, pcomp, n,
             segments, G, order, b.exact.as<double>(), exact_shares(tiles), ax, ay, az);
         NB_LAUNCH_CHECK();
     }
