@@ -12,9 +12,10 @@
 // keeping the second block's sums in shared memory, and writes one partial sum
 // (a Kahan pair) per body of either block to that body's plane of the (diagonal,
 // side); a
-// second launch adds each body's planes in order as a double-single.  A system's
-// partial sums depend on that system alone: it gives the same bits alone and in
-// any mix.
+// second launch adds each body's planes in order as a double-single.  Systems whose
+// planes exceed a buffer of fixed size take turns in it, one of them diagonals by
+// diagonals if need be.  A system's partial sums depend on that system alone: it gives
+// the same bits alone and in any mix.
 #include "nb_internal.h"
 #include "nb_check.cuh"
 #include "nb_curve.cuh"
@@ -171,7 +172,7 @@ __device__ __forceinline__ void batch_row(const float4 *__restrict__ hi,
 // ensemble (8.4e8 unordered pairs an evaluation) take 7.17 ms, with one i-tile at
 // a time and the masses in the loop 7.78, with a row of 32 or 64 bodies per warp
 // over ordered pairs 9.92.
-template <bool SORTED, bool ZERO_SOFT>
+template <bool SORTED, bool ZERO_SOFT, bool PARTS>
 __global__ void __launch_bounds__(32, kBatchCtas)
 batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                    const float4 *__restrict__ boxes, const SysDesc *__restrict__ sys,
@@ -210,8 +211,9 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     const float2 e2 = dup2(eps2);
     const bool soft = eps2 >= 1e-22f;  // equal_range's nearest pair
     const size_t plane = (size_t)sd.n;
-    float2 *pa = part + sd.part0 + 3 * plane * it.p;
-    float2 *pb = part + sd.part0 + 3 * plane * (sd.blocks / 2 + it.p);
+    float2 *pa = part + sd.part0 + 3 * plane * (PARTS ? it.p - sd.p0 : it.p);
+    float2 *pb = part + sd.part0 +
+                 3 * plane * (PARTS ? sd.np - (sd.p0 == 0) + it.p - sd.p0 : sd.blocks / 2 + it.p);
     for (int v = 0; v < kBatchTiles; ++v) tile_sums_zero(sums[v], lane);
 
     for (int u0 = 0; u0 < ta; u0 += 2) {
@@ -312,10 +314,13 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
 }
 
 // a = G * the sum of a body's planes in order (diagonal 0, 1, ... of the first
-// side, then 1, 2, ... of the second), as a double-single: one block per block
-// of bodies; order (sorted batches): the pool slot of a sorted body.
+// side, then 1, 2, ... of the second; those of earlier passes, acc, before them), as a
+// double-single: one block per block of bodies; order (sorted batches): the pool slot of
+// a sorted body.
+template <bool PARTS>
 __global__ void __launch_bounds__(kBatchBlockBodies)
-batch_combine_kernel(const float2 *__restrict__ part, const SysDesc *__restrict__ sys,
+batch_combine_kernel(const float2 *__restrict__ part, float2 *__restrict__ acc,
+                     const SysDesc *__restrict__ sys,
                      const PairItem *__restrict__ items, const uint32_t *__restrict__ order,
                      double G, double *__restrict__ ax, double *__restrict__ ay,
                      double *__restrict__ az, int total)
@@ -326,15 +331,26 @@ batch_combine_kernel(const float2 *__restrict__ part, const SysDesc *__restrict_
     if (i >= sd.n || !NB_IN_RANGE(sd.first + i, total)) return;
     const size_t plane = (size_t)sd.n;
     const float2 *src = part + sd.part0 + i;
-    const int half = sd.blocks / 2, planes = 2 * half + 1;
+    // the planes of the first side, then of the second, which diagonal 0 has not
+    const int p0 = PARTS ? sd.p0 : 0, from = p0 == 0;
+    const int np = PARTS ? sd.np : sd.blocks / 2 + 1, planes = 2 * np - from;
     float s[3] = {0.f, 0.f, 0.f}, r[3] = {0.f, 0.f, 0.f};
+    if (PARTS && p0 > 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 a = acc[sd.acc0 + c * plane + i];
+            s[c] = a.x;
+            r[c] = a.y;
+        }
     for (int k0 = 0; k0 < planes; k0 += 4) {
         float2 t[4][3];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int k = k0 + u;
-            const bool use = k < planes && (k <= half ? pair_first(k, it.a, sd.blocks)
-                                                      : pair_second(k - half, it.a, sd.blocks));
+            const bool first = k < np;
+            const int p = p0 + (first ? k : k - np + from);
+            const bool use = k < planes && (first ? pair_first(p, it.a, sd.blocks)
+                                                  : pair_second(p, it.a, sd.blocks));
 #pragma unroll
             for (int c = 0; c < 3; ++c)
                 t[u][c] = use ? src[(3 * (size_t)k + c) * plane] : dup2(0.f);
@@ -343,6 +359,11 @@ batch_combine_kernel(const float2 *__restrict__ part, const SysDesc *__restrict_
         for (int u = 0; u < 4; ++u)
 #pragma unroll
             for (int c = 0; c < 3; ++c) ds_add_kahan(s[c], r[c], t[u][c].x, -t[u][c].y);
+    }
+    if (PARTS && p0 + np <= sd.blocks / 2) {  // a later pass has more
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[sd.acc0 + c * plane + i] = make_float2(s[c], r[c]);
+        return;
     }
     const int o = order ? (int)order[sd.first + i] : sd.first + i;
     if (!NB_IN_RANGE(o, total)) return;
@@ -491,54 +512,124 @@ batch_split_sorted_kernel(const uint32_t *__restrict__ order, const double *__re
 
 } // namespace
 
-int bucket_of(int n)
+void build_batch(BatchWork &w, int pairs_min, size_t plane_bytes)
 {
-    int b = 0;
-    while ((2 << b) <= n && b < 30) ++b;
-    return b;  // floor(log2(n))
-}
-
-size_t batch_layout(std::vector<SysDesc> &sys, int pairs_min, int *tiles)
-{
-    int t = 0;
-    long long pairs = 0;
-    for (SysDesc &s : sys) {
-        s.blocks = s.n < pairs_min ? 0 : (s.n + kBatchBlockBodies - 1) / kBatchBlockBodies;
-        s.tile0 = t;
-        s.part0 = pairs;
-        t += (s.n + kTile - 1) / kTile;
-        if (s.blocks) pairs += 3ll * s.n * (2 * (s.blocks / 2) + 1);
+    const long long limit = (long long)(plane_bytes / sizeof(float2));
+    const int systems = (int)w.sys.size();
+    w.num_tiles = 0;
+    std::vector<std::vector<int>> passes(1);  // the descriptors of each
+    std::vector<int> parts;                   // systems that do not fit one
+    long long used = 0, most = 0;
+    for (int k = 0; k < systems; ++k) {
+        SysDesc &s = w.sys[k];
+        s.tile0 = w.num_tiles;
+        w.num_tiles += (s.n + kTile - 1) / kTile;
+        const bool pairs = s.n >= pairs_min && s.n <= kBatchPairsMax;
+        s.blocks = pairs ? (s.n + kBatchBlockBodies - 1) / kBatchBlockBodies : 0;
+        s.np = s.blocks / 2 + 1;
+        if (!pairs) {
+            passes[0].push_back(k);
+            continue;
+        }
+        const long long need = 3ll * s.n * (2 * s.np - 1);
+        if (need > limit) {
+            parts.push_back(k);
+            continue;
+        }
+        if (used + need > limit) {
+            passes.emplace_back();
+            used = 0;
+        }
+        s.part0 = used;
+        used += need;
+        most = std::max(most, used);
+        passes.back().push_back(k);
     }
-    *tiles = t;
-    return sizeof(float2) * (size_t)pairs;
-}
-
-void build_work_items(const std::vector<SysDesc> &sys, std::vector<PairItem> &items,
-                      int *num_blocks)
-{
-    // first the (system, block, 0) list of the combine, then every item by
-    // cost, largest first, in units of a 64 x 64 tile pair (a stable counting
-    // sort: all full items of all systems cost the same; a row item is two
-    // tiles against half its system's, both directions apart)
+    if (passes[0].empty()) passes.erase(passes.begin());
+    for (int k : parts) {
+        // the sums between passes, then two planes a diagonal
+        const long long plane = 3ll * w.sys[k].n;
+        const int diagonals = w.sys[k].np;
+        const int np = (int)std::min<long long>(
+            diagonals, std::max<long long>(1, (limit - plane) / (2 * plane)));
+        for (int p0 = 0; p0 < diagonals; p0 += np) {
+            SysDesc d = w.sys[k];
+            d.p0 = p0;
+            d.np = std::min(np, diagonals - p0);
+            d.part0 = plane;  // behind the sums, at 0
+            passes.push_back({(int)w.sys.size()});
+            w.sys.push_back(d);
+        }
+        most = std::max(most, plane * (1 + 2 * np));
+    }
+    w.part_bytes = sizeof(float2) * (size_t)most;
+    // items by cost in units of a 64 x 64 tile pair (a stable counting sort: all full
+    // items of all systems cost the same; a row item is two tiles against half its
+    // system's, both directions apart)
     constexpr int kMost = 64;
-    std::vector<PairItem> by_cost[kMost + 1];
-    items.clear();
-    for (int s = 0; s < (int)sys.size(); ++s) {
-        const int M = sys[s].blocks, tiles = (sys[s].n + kTile - 1) / kTile;
-        for (int r = 0; M == 0 && r * 32 < sys[s].n; ++r)
-            by_cost[std::min(kMost, (tiles + 1) / 2)].push_back(PairItem{s, r, -1});
-        if (M == 0) continue;
-        auto width = [&](int b) { return std::min(kBatchTiles, tiles - b * kBatchTiles); };
-        for (int p = 0; p <= M / 2; ++p)
-            for (int a = 0; a < M; ++a) {
-                if (p == 0) items.push_back(PairItem{s, a, 0});
-                if (!pair_first(p, a, M)) continue;
-                const int ta = width(a), tb = width((a + p) % M);
-                by_cost[p == 0 ? ta * (ta + 1) / 2 : ta * tb].push_back(PairItem{s, a, p});
-            }
+    for (const std::vector<int> &pass : passes) {
+        std::vector<PairItem> by_cost[kMost + 1];
+        BatchPass at;
+        at.block0 = (int)w.blocks.size();
+        at.item0 = (int)w.items.size();
+        for (int s : pass) {
+            const SysDesc &sd = w.sys[s];
+            const int M = sd.blocks, tiles = (sd.n + kTile - 1) / kTile;
+            for (int r = 0; M == 0 && r * 32 < sd.n; ++r)
+                by_cost[std::min(kMost, (tiles + 1) / 2)].push_back(PairItem{s, r, -1});
+            if (M == 0) continue;
+            for (int a = 0; a < M; ++a) w.blocks.push_back(PairItem{s, a, 0});
+            auto width = [&](int b) { return std::min(kBatchTiles, tiles - b * kBatchTiles); };
+            for (int p = sd.p0; p < sd.p0 + sd.np; ++p)
+                for (int a = 0; a < M; ++a) {
+                    if (!pair_first(p, a, M)) continue;
+                    const int ta = width(a), tb = width((a + p) % M);
+                    by_cost[p == 0 ? ta * (ta + 1) / 2 : ta * tb].push_back(PairItem{s, a, p});
+                }
+        }
+        for (int c = kMost; c >= 0; --c)
+            w.items.insert(w.items.end(), by_cost[c].begin(), by_cost[c].end());
+        at.parts = pass[0] >= systems;
+        at.blocks = (int)w.blocks.size() - at.block0;
+        at.items = (int)w.items.size() - at.item0;
+        w.passes.push_back(at);
     }
-    *num_blocks = (int)items.size();
-    for (int c = kMost; c >= 0; --c) items.insert(items.end(), by_cost[c].begin(), by_cost[c].end());
+}
+
+void BatchQueue::release()
+{
+    d_sys.release();
+    d_blocks.release();
+    d_items.release();
+}
+
+nb_status upload_batch(BatchQueue &q, const BatchWork &w, cudaStream_t st)
+{
+    q.passes.clear();
+    q.num_tiles = w.num_tiles;
+    q.num_items = (long long)w.items.size();
+    auto put = [&](DevBuf &to, const void *from, size_t bytes) -> nb_status {
+        if (bytes == 0) return NB_OK;
+        NB_TRY(to.reserve(bytes));
+        NB_CUDA_TRY(cudaMemcpyAsync(to.ptr, from, bytes, cudaMemcpyHostToDevice, st));
+        return NB_OK;
+    };
+    NB_TRY(put(q.d_sys, w.sys.data(), sizeof(SysDesc) * w.sys.size()));
+    NB_TRY(put(q.d_blocks, w.blocks.data(), sizeof(PairItem) * w.blocks.size()));
+    NB_TRY(put(q.d_items, w.items.data(), sizeof(PairItem) * w.items.size()));
+    NB_CUDA_TRY(cudaStreamSynchronize(st));  // the host vectors may go
+    q.passes = w.passes;
+    return NB_OK;
+}
+
+template <bool PARTS>
+static auto batch_kernel(bool sorted, double eps2)
+{
+    if (sorted)
+        return eps2 > 0.0 ? batch_pairs_kernel<true, false, PARTS>
+                          : batch_pairs_kernel<true, true, PARTS>;
+    return eps2 > 0.0 ? batch_pairs_kernel<false, false, PARTS>
+                      : batch_pairs_kernel<false, true, PARTS>;
 }
 
 static nb_status launch_batch(const float4 *hi, const float4 *lo, const float4 *boxes,
@@ -546,27 +637,22 @@ static nb_status launch_batch(const float4 *hi, const float4 *lo, const float4 *
                               double *ax, double *ay, double *az, int total, int num_tiles,
                               cudaStream_t st, const KernelTimer *timer)
 {
-    const PairItem *pairs = q.d_items + q.num_blocks;
-    const int num_pairs = q.num_items - q.num_blocks;
+    const SysDesc *sys = q.d_sys.as<SysDesc>();
     if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
-    if (boxes && eps2 > 0.0)
-        batch_pairs_kernel<true, false><<<num_pairs, 32, 0, st>>>(
-            hi, lo, boxes, q.d_sys, pairs, (float)eps2, q.part, G, order, ax, ay, az, total, num_tiles);
-    else if (boxes)
-        batch_pairs_kernel<true, true><<<num_pairs, 32, 0, st>>>(
-            hi, lo, boxes, q.d_sys, pairs, 0.0f, q.part, G, order, ax, ay, az, total, num_tiles);
-    else if (eps2 > 0.0)
-        batch_pairs_kernel<false, false><<<num_pairs, 32, 0, st>>>(
-            hi, lo, boxes, q.d_sys, pairs, (float)eps2, q.part, G, order, ax, ay, az, total, num_tiles);
-    else
-        batch_pairs_kernel<false, true><<<num_pairs, 32, 0, st>>>(
-            hi, lo, boxes, q.d_sys, pairs, 0.0f, q.part, G, order, ax, ay, az, total, num_tiles);
-    NB_LAUNCH_CHECK();
-    if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
-    if (q.num_blocks == 0) return NB_OK;  // small systems only: no partial sums
-    batch_combine_kernel<<<q.num_blocks, kBatchBlockBodies, 0, st>>>(
-        q.part, q.d_sys, q.d_items, order, G, ax, ay, az, total);
-    NB_LAUNCH_CHECK();
+    for (const BatchPass &p : q.passes) {
+        auto *kernel = p.parts ? batch_kernel<true>(boxes, eps2) : batch_kernel<false>(boxes, eps2);
+        kernel<<<p.items, 32, 0, st>>>(hi, lo, boxes, sys, q.d_items.as<PairItem>() + p.item0,
+                                       eps2 > 0.0 ? (float)eps2 : 0.0f, q.part, G, order, ax, ay,
+                                       az, total, num_tiles);
+        NB_LAUNCH_CHECK();
+        if (timer && timer->stop && &p == &q.passes.back())
+            NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
+        if (p.blocks == 0) continue;  // rows only: no partial sums
+        auto *combine = p.parts ? batch_combine_kernel<true> : batch_combine_kernel<false>;
+        combine<<<p.blocks, kBatchBlockBodies, 0, st>>>(
+            q.part, q.part, sys, q.d_blocks.as<PairItem>() + p.block0, order, G, ax, ay, az, total);
+        NB_LAUNCH_CHECK();
+    }
     return NB_OK;
 }
 
@@ -574,7 +660,6 @@ nb_status batch_forces(const float4 *hi, const float4 *lo, const BatchQueue &q, 
                        double eps2, double *ax, double *ay, double *az, int total,
                        cudaStream_t st, const KernelTimer *timer)
 {
-    if (q.num_items <= 0) return NB_OK;
     return launch_batch(hi, lo, nullptr, q, G, eps2, nullptr, ax, ay, az, total, q.num_tiles, st,
                         timer);
 }
@@ -629,7 +714,6 @@ nb_status batch_sorted_forces(BatchSorted &b, const double *x, const double *y, 
                               float4 *hi, float4 *lo, double *ax, double *ay, double *az,
                               cudaStream_t st, const KernelTimer *timer)
 {
-    if (q.num_items <= 0) return NB_OK;
     if (!b.order) return fail(NB_ERR_NOT_LOADED, "sorted batch: no order (sort first)");
     batch_split_sorted_kernel<<<(2 * b.num_tiles + 7) / 8, 256, 0, st>>>(
         b.order, x, y, z, m, b.tiles.as<int4>(), b.num_tiles, b.geom.as<double4>(), b.total, hi,

@@ -29,7 +29,7 @@ struct nb_ensemble {
     bool own_stream = false;
     bool loaded = false;
 
-    nb::DevBuf state, hi, lo, old_acc, rk4, d_sys, d_items, part;
+    nb::DevBuf state, hi, lo, old_acc, rk4, part;
     double *f[10] = {};
     std::vector<nb::SysDesc> sys;
     nb::BatchQueue queue;
@@ -59,24 +59,12 @@ constexpr int kGraphChunk = 25;
 
 nb_status upload_items(nb_ensemble *e)
 {
-    BatchQueue &q = e->queue;
-    const size_t bytes = batch_layout(e->sys, kBatchPairsMin, &q.num_tiles);
-    std::vector<PairItem> items;
-    build_work_items(e->sys, items, &q.num_blocks);
-    q.num_items = (int)items.size();
-    NB_TRY(e->d_sys.reserve(sizeof(SysDesc) * e->sys.size()));
-    NB_TRY(e->d_items.reserve(sizeof(PairItem) * items.size()));
-    if (bytes) NB_TRY(e->part.reserve(bytes));  // 0: every system by rows
-    q.d_sys = e->d_sys.as<SysDesc>();
-    q.d_items = e->d_items.as<PairItem>();
-    q.part = e->part.as<float2>();
-    NB_CUDA_TRY(cudaMemcpyAsync(e->d_sys.ptr, e->sys.data(), sizeof(SysDesc) * e->sys.size(),
-                                cudaMemcpyHostToDevice, e->stream));
-    NB_CUDA_TRY(cudaMemcpyAsync(e->d_items.ptr, items.data(), sizeof(PairItem) * items.size(),
-                                cudaMemcpyHostToDevice, e->stream));
-    // the host vectors go out of scope: wait for the copies
-    NB_CUDA_TRY(cudaStreamSynchronize(e->stream));
-    return NB_OK;
+    BatchWork w;
+    w.sys = e->sys;
+    build_batch(w, kBatchPairsMin, kBatchPlaneBytes);
+    if (w.part_bytes) NB_TRY(e->part.reserve(w.part_bytes));  // 0: every system by rows
+    e->queue.part = e->part.as<float2>();
+    return upload_batch(e->queue, w, e->stream);
 }
 
 const KernelTimer *ens_timer(nb_ensemble *e, bool capturing)
@@ -123,7 +111,7 @@ nb_status setup(nb_ensemble *e)
 {
     NB_TRY(upload_items(e));
     if (e->sorted)
-        NB_TRY(batch_sorted_setup(e->sb, e->queue.d_sys, e->num_sys, e->queue.num_tiles,
+        NB_TRY(batch_sorted_setup(e->sb, e->queue.d_sys.as<SysDesc>(), e->num_sys, e->queue.num_tiles,
                                   (int)e->total, e->stream));
     e->ready = true;
     return NB_OK;
@@ -133,7 +121,7 @@ nb_status setup(nb_ensemble *e)
 nb_status sort_systems(nb_ensemble *e)
 {
     if (!e->sorted) return NB_OK;
-    return batch_sorted_sort(e->sb, e->queue.d_sys, e->f[0], e->f[1], e->f[2],
+    return batch_sorted_sort(e->sb, e->queue.d_sys.as<SysDesc>(), e->f[0], e->f[1], e->f[2],
                              e->stream);
 }
 
@@ -196,7 +184,7 @@ nb_status nb_ensemble_create(const nb_config *cfg, int num_systems, const int *s
     size_t first = 0;
     e->sys.resize(num_systems);
     for (int s = 0; s < num_systems; ++s) {
-        e->sys[s] = SysDesc{(int)first, sizes[s], 0, 0, 0};
+        e->sys[s] = SysDesc{(int)first, sizes[s]};
         first += sizes[s];
     }
     e->sorted = (cfg->flags & NB_FLAG_MIXED_UNSORTED) == 0;
@@ -213,9 +201,9 @@ nb_status nb_ensemble_destroy(nb_ensemble *e)
         cudaEventDestroy(t.start);
         cudaEventDestroy(t.stop);
     }
-    nb::DevBuf *bufs[] = {&e->state, &e->hi, &e->lo, &e->old_acc, &e->rk4, &e->d_sys,
-                          &e->d_items, &e->part};
+    nb::DevBuf *bufs[] = {&e->state, &e->hi, &e->lo, &e->old_acc, &e->rk4, &e->part};
     for (nb::DevBuf *b : bufs) b->release();
+    e->queue.release();
     e->sb.release();
     if (e->own_stream) cudaStreamDestroy(e->stream);
     delete e;
@@ -365,7 +353,7 @@ nb_status nb_ensemble_info(nb_ensemble *e, nb_ensemble_info_t *info)
     double inter = 0.0;
     for (int n : e->sizes) inter += (double)n * (double)(n - 1);
     info->interactions_per_eval = inter;
-    info->work_items = e->queue.num_items - e->queue.num_blocks;
+    info->work_items = (int)std::min<long long>(e->queue.num_items, INT32_MAX);
     for (int b = 0; b < 32; ++b) info->ipt_by_bucket[b] = e->ipt_bucket[b];
     info->graph_launches = e->graph_launches;
     info->graph_steps = e->graph_steps;

@@ -245,36 +245,64 @@ constexpr int kBatchPairsMin = 2048;
 // unordered pairs, against the row sum); up to 4095 bodies their work is a few percent
 // of the direct jobs' (a burst of 16 jobs: 15.7 ms, 15.5 by pairs from 1024).
 constexpr int kServePairsMin = 4096;
-// A system of a batch: bodies [first, first + n) of the batch's pool.
+// Largest system summed over unordered pairs: the table of its items grows as n^2 (8
+// million at 2^20 bodies, 100 MB); larger ones go by rows, n / 32 items.
+constexpr int kBatchPairsMax = 1 << 20;
+// Partial planes of a pass over an ensemble's systems (a system needs 24 B a body and
+// diagonal and side, 400 B a body at 4096 bodies; 4096 systems of 32 to 4096 bodies
+// 0.55 GB, one pass).
+constexpr size_t kBatchPlaneBytes = (size_t)1 << 30;
+// A system of a batch: bodies [first, first + n) of the batch's pool; or, of one whose
+// planes do not fit a pass, the diagonals [p0, p0 + np) alone.
 struct SysDesc {
     int first;
     int n;
-    int blocks;       // blocks of kBatchBlockBodies; 0: a small system, summed by rows
-    int tile0;        // first 64-body tile of the system
-    long long part0;  // its first entry of the partial planes
+    int blocks = 0;       // blocks of kBatchBlockBodies; 0: summed by rows
+    int tile0 = 0;        // first 64-body tile of the system
+    // the place of its partial planes, 3 n entries each: the first sides of its diagonals,
+    // then the second (which diagonal 0 has not)
+    long long part0 = 0;
+    int p0 = 0, np = 0;   // diagonals of its block pairs
+    long long acc0 = 0;   // not all diagonals: its sums between passes
 };
 // One queue item: blocks a and (a + p) mod blocks of system `sys`; p < 0: the
-// rows of its 128 bodies from 128 a.
+// 32 rows from body 32 a.
 struct PairItem {
     int sys;
     int a;
     int p;
 };
-// The uploaded work of a set of systems: num_blocks (system, block, 0) entries
-// for the combine, then the items of the pair kernel; part: the partial planes.
-struct BatchQueue {
-    const SysDesc *d_sys = nullptr;
-    const PairItem *d_items = nullptr;
-    int num_blocks = 0, num_items = 0, num_tiles = 0;
-    float2 *part = nullptr;
+// The systems are summed in passes, whose partial planes take turns in one buffer: a
+// pass is a range of items of the pair kernel and one of (system, block, 0) entries for
+// the combine.
+struct BatchPass {
+    int item0 = 0, items = 0;
+    int block0 = 0, blocks = 0;
+    bool parts = false;  // some diagonals of one system
 };
-int bucket_of(int n);  // floor(log2(n))
-// Sets every system's blocks, tile0 and part0; returns the bytes of the
-// partial planes and the tile count.
-size_t batch_layout(std::vector<SysDesc> &sys, int pairs_min, int *tiles);
-// The combine's blocks, then the items of every system, largest cost first.
-void build_work_items(const std::vector<SysDesc> &sys, std::vector<PairItem> &items,
-                      int *num_blocks);
+// The work of a set of systems.  In: sys, first and n of each.
+struct BatchWork {
+    std::vector<SysDesc> sys;      // the systems, then descriptors of parts of them
+    std::vector<PairItem> blocks;  // the combine's entries, pass by pass
+    std::vector<PairItem> items;   // the pair kernel's, each pass by cost, largest first
+    std::vector<BatchPass> passes;
+    size_t part_bytes = 0;         // of the buffer of partial planes
+    int num_tiles = 0;
+};
+// A system's result depends on it, pairs_min and plane_bytes alone.
+void build_batch(BatchWork &w, int pairs_min, size_t plane_bytes);
+// The work on the device.
+struct BatchQueue {
+    DevBuf d_sys, d_blocks, d_items;
+    std::vector<BatchPass> passes;
+    int num_tiles = 0;
+    long long num_items = 0;
+    float2 *part = nullptr;
+    size_t bytes() const { return d_sys.bytes + d_blocks.bytes + d_items.bytes; }
+    void release();
+};
+// Uploads w (and waits for the copies); q.part is the caller's to set.
+nb_status upload_batch(BatchQueue &q, const BatchWork &w, cudaStream_t st);
 // Mixed-precision forces of all systems of the queue.
 nb_status batch_forces(const float4 *hi, const float4 *lo, const BatchQueue &q, double G,
                        double eps2, double *ax, double *ay, double *az, int total,

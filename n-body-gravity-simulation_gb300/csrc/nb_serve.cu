@@ -213,7 +213,7 @@ struct nb_server {
     nb::DevBuf pool, hi, lo;
     // the direct jobs' work queue, and that of the jobs admitted this tick
     struct Queue {
-        nb::DevBuf d_sys, d_items, part;
+        nb::DevBuf part;
         nb::BatchQueue q;
     } queue_all, queue_new;
     double *f[10] = {};
@@ -249,25 +249,12 @@ size_t pool_bytes(const nb_server *s) { return s->pool.bytes + s->hi.bytes + s->
 
 nb_status upload_systems(nb_server *s, const std::vector<Job *> &jobs, nb_server::Queue &to)
 {
-    std::vector<SysDesc> sys;
-    for (Job *j : jobs) sys.push_back(SysDesc{(int)j->first, (int)j->n, 0, 0, 0});
-    const size_t bytes = batch_layout(sys, kServePairsMin, &to.q.num_tiles);
-    std::vector<PairItem> items;
-    build_work_items(sys, items, &to.q.num_blocks);
-    to.q.num_items = (int)items.size();
-    if (sys.empty()) return NB_OK;
-    NB_TRY(to.d_sys.reserve(sizeof(SysDesc) * sys.size()));
-    NB_TRY(to.d_items.reserve(sizeof(PairItem) * items.size()));
-    if (bytes) NB_TRY(to.part.reserve(bytes));  // 0: every job by rows
-    to.q.d_sys = to.d_sys.as<SysDesc>();
-    to.q.d_items = to.d_items.as<PairItem>();
+    BatchWork w;
+    for (Job *j : jobs) w.sys.push_back(SysDesc{(int)j->first, (int)j->n});
+    build_batch(w, kServePairsMin, kBatchPlaneBytes);
+    if (w.part_bytes) NB_TRY(to.part.reserve(w.part_bytes));  // 0: every job by rows
     to.q.part = to.part.as<float2>();
-    NB_CUDA_TRY(cudaMemcpyAsync(to.d_sys.ptr, sys.data(), sizeof(SysDesc) * sys.size(),
-                                cudaMemcpyHostToDevice, s->stream));
-    NB_CUDA_TRY(cudaMemcpyAsync(to.d_items.ptr, items.data(), sizeof(PairItem) * items.size(),
-                                cudaMemcpyHostToDevice, s->stream));
-    NB_CUDA_TRY(cudaStreamSynchronize(s->stream));
-    return NB_OK;
+    return upload_batch(to.q, w, s->stream);
 }
 
 size_t sim_bytes(const nb_sim *sim) { return kBHBytesPerBody * sim->capacity; }
@@ -650,10 +637,10 @@ nb_status nb_server_destroy(nb_server *s)
         if (j->sim) nb_destroy(j->sim);
         if (j->step_done) cudaEventDestroy(j->step_done);
     }
-    DevBuf *bufs[] = {&s->pool, &s->hi, &s->lo, &s->queue_all.d_sys, &s->queue_all.d_items,
-                      &s->queue_all.part, &s->queue_new.d_sys, &s->queue_new.d_items,
-                      &s->queue_new.part};
+    DevBuf *bufs[] = {&s->pool, &s->hi, &s->lo, &s->queue_all.part, &s->queue_new.part};
     for (DevBuf *b : bufs) b->release();
+    s->queue_all.q.release();
+    s->queue_new.q.release();
     if (s->tick_start) cudaEventDestroy(s->tick_start);
     if (s->direct_done) cudaEventDestroy(s->direct_done);
     for (int k = 0; k < kBHStreams; ++k)
