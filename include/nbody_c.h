@@ -306,7 +306,14 @@ nb_status nb_ensemble_profile(nb_ensemble *e, int enable);
  * step (direct jobs together in batched launches over a resident body
  * pool, Barnes-Hut jobs on their own streams, overlapping), and retires jobs
  * that reached their step count.  A job's result does not depend on the other
- * jobs it ran with. */
+ * jobs it ran with.
+ * The budget covers the body pool (112 bytes a body), the partial sums of direct
+ * jobs (at most 256 MiB, and a sixteenth of what the pool leaves; allocated with
+ * the server) and the Barnes-Hut jobs' simulations (470 bytes a body at leaf
+ * capacity 8), running ones and those kept for jobs to come.  Submission asks
+ * for 320 bytes a body; a job that was accepted so and needs more than there is
+ * runs once no other tree is resident, the one case in which the budget is
+ * exceeded. */
 typedef struct nb_server nb_server;
 
 typedef struct nb_server_config {

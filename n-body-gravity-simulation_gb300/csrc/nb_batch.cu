@@ -524,7 +524,7 @@ void build_batch(BatchWork &w, int pairs_min, size_t plane_bytes)
         SysDesc &s = w.sys[k];
         s.tile0 = w.num_tiles;
         w.num_tiles += (s.n + kTile - 1) / kTile;
-        const bool pairs = s.n >= pairs_min && s.n <= kBatchPairsMax;
+        const bool pairs = s.n >= pairs_min && s.n <= kBatchPairsMax && 9ll * s.n <= limit;
         s.blocks = pairs ? (s.n + kBatchBlockBodies - 1) / kBatchBlockBodies : 0;
         s.np = s.blocks / 2 + 1;
         if (!pairs) {

@@ -2466,6 +2466,14 @@ double log_per_body(int n, double theta, int leaf_capacity, bool ref_open)
     return base * leaves * (1.0 + more * std::min(1.0, small));
 }
 
+// Entries of an ordered walk's log pool; 0: no such walk.
+int log_pool_entries(int n, double theta, int leaf_capacity, bool ref_open)
+{
+    const double per_body = log_per_body(n, theta, leaf_capacity, ref_open);
+    if ((!ref_open && n > kOrderedBodies) || per_body > kMostLogPerBody) return 0;
+    return (int)std::min(per_body * n + 64.0, 2e9);
+}
+
 // The walk of n bodies: over child groups, or the stackless preorder walk
 // (NB_BH_WALK=preorder, read at every walk; both find the same interactions).
 // NB_BH_WALK=serial takes the serial walk where the ordered one is the default.
@@ -2475,8 +2483,8 @@ Walk choose_walk(int n, double theta, int leaf_capacity, bool ref_open)
     if (walk_pairs() < 1 || (e && std::strcmp(e, "preorder") == 0)) return Walk::kPreorder;
     if (walk_pairs() > 1 || (!ref_open && n > kOrderedBodies)) return Walk::kGroup;
     if (e && std::strcmp(e, "serial") == 0) return Walk::kSerial;
-    return log_per_body(n, theta, leaf_capacity, ref_open) <= kMostLogPerBody ? Walk::kOrdered
-                                                                              : Walk::kSerial;
+    return log_pool_entries(n, theta, leaf_capacity, ref_open) > 0 ? Walk::kOrdered
+                                                                   : Walk::kSerial;
 }
 
 int div_up(long a, long b) { return (int)((a + b - 1) / b); }
@@ -2504,14 +2512,14 @@ struct BHTree {
     int node_cap = 0;           // node slots reserved (an upper bound of the count)
     int *h_total = nullptr;     // pinned host copy of the count, filled asynchronously
     cudaEvent_t total_ready = nullptr;
-    DevBuf part, root, keys0, keys1, vals0, vals1, hist, body, moments, prefix, chain_len,
+    DevBuf part, root, keys0, keys1, vals0, vals1, hist, body, moments, chain_len,
         chain_depth, offsets, scan_tmp, nodes, node_depth, boxes, stats, moments2a, moments2b,
         prefix2a, prefix2b, quad, pcen, pstart, parent, octant, occ, kidflag, kbase, gnodes, gnk,
-        gpcen, gquad, gkey, walks, logs;
+        gpcen, gquad, gkey, walks;
     bool with_quad = false;     // the nodes carry quadrupoles (quad, 2 float4 per node)
     bool ref_open = false;      // the reference's opening rule (the child toward the body too)
-    Walk walk = Walk::kGroup;   // the next walk's kernels (ordered: gkey and logs are set)
-    int log_pool = 0;           // entries of the pool in logs
+    Walk walk = Walk::kGroup;   // the next walk's kernels (ordered: gkey is set)
+    int log_pool = 0;           // entries of the log pool
     bool pcen_valid = false;    // pcen holds the parent centres of the current topology
     const uint64_t *sorted_codes = nullptr;
     const uint32_t *order = nullptr;
@@ -2542,16 +2550,25 @@ void bh_destroy(BHTree *t)
 {
     if (!t) return;
     DevBuf *bufs[] = {&t->part, &t->root, &t->keys0, &t->keys1, &t->vals0, &t->vals1,
-                      &t->hist, &t->body, &t->moments, &t->prefix, &t->chain_len,
+                      &t->hist, &t->body, &t->moments, &t->chain_len,
                       &t->chain_depth, &t->offsets, &t->scan_tmp, &t->nodes, &t->node_depth,
                       &t->boxes, &t->stats, &t->moments2a, &t->moments2b, &t->prefix2a,
                       &t->prefix2b, &t->quad, &t->pcen, &t->pstart, &t->parent, &t->octant,
                       &t->occ, &t->kidflag, &t->kbase, &t->gnodes,
-                      &t->gnk, &t->gpcen, &t->gquad, &t->gkey, &t->walks, &t->logs};
+                      &t->gnk, &t->gpcen, &t->gquad, &t->gkey, &t->walks};
     for (DevBuf *b : bufs) b->release();
     if (t->h_total) cudaFreeHost(t->h_total);
     if (t->total_ready) cudaEventDestroy(t->total_ready);
     delete t;
+}
+
+// The moments buffer: the bodies' moments, then their prefix sums, which nothing reads
+// once the nodes and their quadrupoles are made; the walk's log pool takes their place
+// (its counter first), until the next evaluation.
+static D4 *prefix_sums(const BHTree *t, int n) { return t->moments.as<D4>() + n; }
+static size_t moments_bytes(int n, int log_pool)
+{
+    return std::max(sizeof(D4) * (2 * (size_t)n + 1), sizeof(uint2) * ((size_t)log_pool + 1));
 }
 
 // The device copy of the node count of the last build (scan total).
@@ -2588,6 +2605,22 @@ static size_t node_bound(int n, int leaf_capacity)
 // Root cube, 63-bit codes and the stable LSD sort of the code bits
 // [first_shift, 64) (first_shift 0: the full code).  Leaves the sorted codes
 // and the permutation (sorted index -> original index) in t.
+size_t bh_bytes(int n, double theta, int leaf_capacity)
+{
+    const size_t N = (size_t)n, cap = node_bound(n, leaf_capacity);
+    const size_t sort = 2 * (sizeof(uint64_t) + sizeof(uint32_t)) * N +
+                        sizeof(int) * (3 * (256 * (size_t)div_up(n, kSortTile) + 1) + 256);
+    const size_t bodies =
+        sizeof(float4) * N + moments_bytes(n, log_pool_entries(n, theta, leaf_capacity, false)) +
+        sizeof(int) * (4 * N + 1) + sizeof(D4) * (N / 1024 + 1);
+    // nodes and node_depth, parent, octant, occ, kidflag, kbase, gnodes and gnk, gkey
+    const size_t nodes = (sizeof(BHNode) + 1 + 4 + 1 + 4 + 8 + 4 + sizeof(BHGNode) + 1 + 4) * cap;
+    const size_t walks = sizeof(int2) * (1 + kLogSegments) * (size_t)div_up(n, 64);
+    const size_t rest = sizeof(long long) * 6 * 4 * (size_t)device_props().num_sms +
+                        sizeof(BHRoot) + sizeof(BHStats) + 64;
+    return sort + bodies + nodes + walks + rest;
+}
+
 // Key/value ping-pong buffers and digit histograms for n entries.
 static nb_status reserve_sort(BHTree *t, int n)
 {
@@ -2763,7 +2796,7 @@ nb_status walk_launch(BHTree *t, int n, float theta2, float eps2, double G, doub
         const int2 *logged = nullptr;
         if (t->walk == Walk::kOrdered) {
             // logs: the pool's counter, then the pool
-            unsigned long long *next = t->logs.as<unsigned long long>();
+            unsigned long long *next = t->moments.as<unsigned long long>();
             uint2 *pool = reinterpret_cast<uint2 *>(next + 1);
             int2 *walks = t->walks.as<int2>(), *segs = walks + ctas;
             auto decide = [&](auto *kernel, int threads, size_t shared) -> nb_status {
@@ -2860,7 +2893,7 @@ static nb_status compute_quads(BHTree *t, const double *x, const double *y, cons
     NB_LAUNCH_CHECK();
     NB_TRY(scan_exclusive<D4>(t->moments2a.as<D4>(), n, t->prefix2a.as<D4>(), t->scan_tmp, st));
     NB_TRY(scan_exclusive<D4>(t->moments2b.as<D4>(), n, t->prefix2b.as<D4>(), t->scan_tmp, st));
-    quad_kernel<<<div_up(nn, 256), 256, 0, st>>>(t->nodes.as<BHNode>(), d_total(t), t->prefix.as<D4>(),
+    quad_kernel<<<div_up(nn, 256), 256, 0, st>>>(t->nodes.as<BHNode>(), d_total(t), prefix_sums(t, n),
                                                  t->prefix2a.as<D4>(), t->prefix2b.as<D4>(),
                                                  t->quad.as<float4>());
     NB_LAUNCH_CHECK();
@@ -2904,7 +2937,7 @@ static nb_status group_nodes(BHTree *t, cudaStream_t st, bool recount)
     if (t->walk == Walk::kOrdered) {
         NB_TRY(t->gkey.reserve(sizeof(unsigned) * (size_t)slots));
         NB_TRY(t->walks.reserve(sizeof(int2) * (1 + kLogSegments) * (size_t)div_up(t->n, 64)));
-        NB_TRY(t->logs.reserve(sizeof(uint2) * ((size_t)t->log_pool + 1)));
+        NB_TRY(t->moments.reserve(moments_bytes(t->n, t->log_pool)));  // done with, now
     }
     group_kernel<<<grid, 256, 0, st>>>(
         t->nodes.as<BHNode>(), d_total(t), t->occ.as<unsigned>(), t->kbase.as<int>(),
@@ -2914,7 +2947,7 @@ static nb_status group_nodes(BHTree *t, cudaStream_t st, bool recount)
         t->gnk.as<unsigned char>(), t->gpcen.as<float4>(),
         t->with_quad ? t->gquad.as<float4>() : nullptr, t->node_depth.as<unsigned char>(),
         t->walk == Walk::kOrdered ? t->gkey.as<unsigned>() : nullptr,
-        t->walk == Walk::kOrdered ? t->logs.as<unsigned long long>() : nullptr);
+        t->walk == Walk::kOrdered ? t->moments.as<unsigned long long>() : nullptr);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }
@@ -2930,10 +2963,10 @@ static nb_status refit(BHTree *t, const double *x, const double *y, const double
     gather_kernel<<<div_up(n, 256), 256, 0, st>>>(t->order, x, y, z, m, n, root,
                                                   t->body.as<float4>(), t->moments.as<D4>());
     NB_LAUNCH_CHECK();
-    NB_TRY(scan_exclusive<D4>(t->moments.as<D4>(), n, t->prefix.as<D4>(), t->scan_tmp, st));
+    NB_TRY(scan_exclusive<D4>(t->moments.as<D4>(), n, prefix_sums(t, n), t->scan_tmp, st));
     refit_kernel<<<div_up(nn, 256), 256, 0, st>>>(t->nodes.as<BHNode>(), d_total(t),
                                                   t->node_depth.as<unsigned char>(),
-                                                  t->prefix.as<D4>(), root, t->body.as<float4>(),
+                                                  prefix_sums(t, n), root, t->body.as<float4>(),
                                                   t->boxes.as<float4>());
     NB_LAUNCH_CHECK();
     // internal nodes, deepest first (an internal node is shallower than the
@@ -2959,7 +2992,7 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
     t->with_quad = quad;
     t->ref_open = ref_open;
     t->walk = choose_walk(n, theta, leaf_capacity, ref_open);
-    t->log_pool = (int)std::min(log_per_body(n, theta, leaf_capacity, ref_open) * n + 64.0, 2e9);
+    t->log_pool = log_pool_entries(n, theta, leaf_capacity, ref_open);
     if (ax && reuse > 1 && t->tree_valid && t->n == n && t->evals_since_build < reuse) {
         NB_TRY(refit(t, x, y, z, m, n, st));
         if (quad) NB_TRY(compute_quads(t, x, y, z, m, n, st));
@@ -2972,8 +3005,7 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
     NvtxRange range("bh_build");
     const size_t N = (size_t)n;
     NB_TRY(t->body.reserve(sizeof(float4) * N));
-    NB_TRY(t->moments.reserve(sizeof(D4) * N));
-    NB_TRY(t->prefix.reserve(sizeof(D4) * (N + 1)));
+    NB_TRY(t->moments.reserve(moments_bytes(n, t->log_pool)));
     NB_TRY(t->chain_len.reserve(sizeof(int) * N));
     NB_TRY(t->chain_depth.reserve(sizeof(int) * N));
     NB_TRY(t->offsets.reserve(sizeof(int) * (N + 1)));
@@ -2991,7 +3023,7 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
     gather_kernel<<<div_up(n, 256), 256, 0, st>>>(vin, x, y, z, m, n, root,
                                                   t->body.as<float4>(), t->moments.as<D4>());
     NB_LAUNCH_CHECK();
-    NB_TRY(scan_exclusive<D4>(t->moments.as<D4>(), n, t->prefix.as<D4>(), t->scan_tmp, st));
+    NB_TRY(scan_exclusive<D4>(t->moments.as<D4>(), n, prefix_sums(t, n), t->scan_tmp, st));
     chain_kernel<<<div_up(n, 256), 256, 0, st>>>(kin, n, leaf_capacity, root,
                                                  t->chain_len.as<int>(),
                                                  t->chain_depth.as<int>(), t->pstart.as<int>());
@@ -3034,7 +3066,7 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
     const int node_grid = std::min(div_up(launch_nodes(t), 256), 8 * device_props().num_sms);
     node_kernel<<<std::max(1, node_grid), 256, 0, st>>>(
         kin, n, root, d_total(t), t->chain_depth.as<int>(), t->offsets.as<int>(),
-        t->prefix.as<D4>(), t->nodes.as<BHNode>(), t->node_depth.as<unsigned char>(),
+        prefix_sums(t, n), t->nodes.as<BHNode>(), t->node_depth.as<unsigned char>(),
         t->pstart.as<int>(), t->parent.as<int>(), t->octant.as<unsigned char>(),
         t->kidflag.as<unsigned char>(), stats, t->node_cap);
     NB_LAUNCH_CHECK();

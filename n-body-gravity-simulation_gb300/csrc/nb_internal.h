@@ -289,7 +289,8 @@ struct BatchWork {
     size_t part_bytes = 0;         // of the buffer of partial planes
     int num_tiles = 0;
 };
-// A system's result depends on it, pairs_min and plane_bytes alone.
+// Systems by pairs: pairs_min to kBatchPairsMax bodies, one diagonal of which fits
+// plane_bytes.  A system's result depends on it, pairs_min and plane_bytes alone.
 void build_batch(BatchWork &w, int pairs_min, size_t plane_bytes);
 // The work on the device.
 struct BatchQueue {
@@ -348,6 +349,9 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
                      int leaf_capacity, double *ax, double *ay, double *az, cudaStream_t st,
                      const KernelTimer *timer = nullptr, int reuse = 1, bool quad = false,
                      bool ref_open = false, const AfterForce &after = AfterForce{});
+// The device memory that bh_compute reserves at most for n bodies (every evaluation a
+// build, no quadrupoles, the default opening rule).
+size_t bh_bytes(int n, double theta, int leaf_capacity);
 // The next bh_compute rebuilds (the bodies were replaced).
 void bh_invalidate(BHTree *t);
 // A replayed build changed the node count behind the host's back.

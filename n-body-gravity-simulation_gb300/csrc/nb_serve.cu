@@ -45,7 +45,16 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 constexpr size_t kDirectBytesPerBody = 10 * 8 + 32;  // FP64 planes + hi/lo mirror
-constexpr size_t kBHBytesPerBody = 320;              // state + sort + tree buffers (upper bound)
+// What a Barnes-Hut job is asked for at submission.  At leaf capacity 8 it takes up to 1.5
+// times as much (sim_bytes), which is what it is admitted by; one that does not fit so
+// waits until no other tree is resident (it was accepted, so it runs).
+constexpr size_t kBHBytesPerBody = 320;
+// Partial planes of the direct jobs, one buffer for both work queues: at most this, and a
+// sixteenth of what the budget leaves beside the pool.  A tick of a full pool of 2 Mi
+// bodies goes through it in about five passes, of 22,000 CTAs each.
+constexpr size_t kServePlaneBytes = (size_t)256 << 20;
+// Below this every direct job goes by rows, which need no planes.
+constexpr size_t kServePlanesLeast = (size_t)16 << 20;
 constexpr int kBHStreams = 16;
 constexpr size_t kIdleSims = 32;
 
@@ -212,10 +221,8 @@ struct nb_server {
     size_t ps = 0;
     nb::DevBuf pool, hi, lo;
     // the direct jobs' work queue, and that of the jobs admitted this tick
-    struct Queue {
-        nb::DevBuf part;
-        nb::BatchQueue q;
-    } queue_all, queue_new;
+    nb::BatchQueue queue_all, queue_new;
+    nb::DevBuf part;  // their partial planes, one after the other
     double *f[10] = {};
     nb::SlotAllocator slots;
     int64_t next_id = 1;
@@ -246,22 +253,31 @@ namespace nb {
 namespace {
 
 size_t pool_bytes(const nb_server *s) { return s->pool.bytes + s->hi.bytes + s->lo.bytes; }
+// The device memory that is not a tree's.
+size_t fixed_bytes(const nb_server *s)
+{
+    return pool_bytes(s) + s->part.bytes + s->queue_all.bytes() + s->queue_new.bytes();
+}
 
-nb_status upload_systems(nb_server *s, const std::vector<Job *> &jobs, nb_server::Queue &to)
+nb_status upload_systems(nb_server *s, const std::vector<Job *> &jobs, BatchQueue &to)
 {
     BatchWork w;
     for (Job *j : jobs) w.sys.push_back(SysDesc{(int)j->first, (int)j->n});
-    build_batch(w, kServePairsMin, kBatchPlaneBytes);
-    if (w.part_bytes) NB_TRY(to.part.reserve(w.part_bytes));  // 0: every job by rows
-    to.q.part = to.part.as<float2>();
-    return upload_batch(to.q, w, s->stream);
+    build_batch(w, kServePairsMin, s->part.bytes);
+    to.part = s->part.as<float2>();
+    return upload_batch(to, w, s->stream);
 }
 
-size_t sim_bytes(const nb_sim *sim) { return kBHBytesPerBody * sim->capacity; }
+// The device memory of a Barnes-Hut job's simulation.
+size_t sim_bytes(const nb_server *s, size_t capacity)
+{
+    return sizeof(double) * 10 * ((capacity + 31) / 32 * 32) +
+           bh_bytes((int)capacity, s->cfg.theta, s->cfg.leaf_capacity);
+}
 
 void drop_idle(nb_server *s, size_t k)
 {
-    s->idle_bytes -= sim_bytes(s->idle[k]);
+    s->idle_bytes -= sim_bytes(s, s->idle[k]->capacity);
     nb_destroy(s->idle[k]);
     s->idle.erase(s->idle.begin() + k);
 }
@@ -271,7 +287,7 @@ void keep_sim(nb_server *s, Job *j)
 {
     s->bh_bytes -= j->bytes;
     s->idle.push_back(j->sim);
-    s->idle_bytes += sim_bytes(j->sim);
+    s->idle_bytes += sim_bytes(s, j->sim->capacity);
     j->sim = nullptr;
     if (s->idle.size() > kIdleSims) drop_idle(s, 0);
 }
@@ -284,7 +300,7 @@ nb_status take_sim(nb_server *s, const nb_config &c, size_t n, cudaStream_t st, 
     for (size_t k = 0; k < s->idle.size(); ++k) {
         const size_t cap = s->idle[k]->capacity;
         if (cap >= n && cap <= n + n / 4 &&
-            pool_bytes(s) + s->bh_bytes + sim_bytes(s->idle[k]) <= s->cfg.hbm_budget_bytes &&
+            fixed_bytes(s) + s->bh_bytes + sim_bytes(s, cap) <= s->cfg.hbm_budget_bytes &&
             (best == s->idle.size() || cap < s->idle[best]->capacity))
             best = k;
     }
@@ -292,16 +308,16 @@ nb_status take_sim(nb_server *s, const nb_config &c, size_t n, cudaStream_t st, 
         nb_sim *sim = s->idle[best];
         sim->stream = st;  // its old stream is idle between ticks
         if (!sim->bh || bh_restart(sim->bh, st) == NB_OK) {
-            s->idle_bytes -= sim_bytes(sim);
+            s->idle_bytes -= sim_bytes(s, sim->capacity);
             s->idle.erase(s->idle.begin() + best);
             *out = sim;
             return NB_OK;
         }
         drop_idle(s, best);
     }
-    const size_t need = kBHBytesPerBody * n;
+    const size_t need = sim_bytes(s, n);
     while (!s->idle.empty() &&
-           pool_bytes(s) + s->bh_bytes + need + s->idle_bytes > s->cfg.hbm_budget_bytes)
+           fixed_bytes(s) + s->bh_bytes + need + s->idle_bytes > s->cfg.hbm_budget_bytes)
         drop_idle(s, 0);
     const nb_status r = nb_create(&c, n, st, out);
     if (r == NB_OK || s->idle.empty()) return r;
@@ -359,8 +375,9 @@ nb_status admit(nb_server *s, std::vector<Job *> &new_direct)
                 ok = true;
             }
         } else {
-            const size_t need = kBHBytesPerBody * j->n;
-            if (pool_bytes(s) + s->bh_bytes + need <= s->cfg.hbm_budget_bytes) {
+            const size_t need = sim_bytes(s, j->n);
+            if (s->bh_bytes == 0 ||
+                fixed_bytes(s) + s->bh_bytes + need <= s->cfg.hbm_budget_bytes) {
                 nb_config c;
                 nb_config_default(&c);
                 c.method = NB_BARNES_HUT;
@@ -390,7 +407,7 @@ nb_status admit(nb_server *s, std::vector<Job *> &new_direct)
                     it = s->queue.erase(it);
                     continue;
                 }
-                j->bytes = sim_bytes(j->sim);
+                j->bytes = sim_bytes(s, j->sim->capacity);
                 s->bh_bytes += j->bytes;
                 ok = true;
             }
@@ -408,7 +425,7 @@ nb_status admit(nb_server *s, std::vector<Job *> &new_direct)
             ++it;
         }
     }
-    s->peak_bytes = std::max(s->peak_bytes, pool_bytes(s) + s->bh_bytes + s->idle_bytes);
+    s->peak_bytes = std::max(s->peak_bytes, fixed_bytes(s) + s->bh_bytes + s->idle_bytes);
     return NB_OK;
 }
 
@@ -515,14 +532,14 @@ nb_status tick(nb_server *s)
             // start-of-step force of the jobs admitted this tick
             NB_TRY(upload_systems(s, new_direct, s->queue_new));
             NB_TRY(split_positions(s->f[0], s->f[1], s->f[2], s->f[9], hw, hi, lo, s->stream));
-            NB_TRY(batch_forces(hi, lo, s->queue_new.q, s->cfg.G, eps2, s->f[6], s->f[7],
+            NB_TRY(batch_forces(hi, lo, s->queue_new, s->cfg.G, eps2, s->f[6], s->f[7],
                                 s->f[8], hw, s->stream));
         }
         NB_TRY(kick_drift(NB_LEAPFROG, hw, dt, s->f[0], s->f[1], s->f[2], s->f[3], s->f[4],
                           s->f[5], s->f[6], s->f[7], s->f[8], nullptr, nullptr, nullptr,
                           s->stream));
         NB_TRY(split_positions(s->f[0], s->f[1], s->f[2], s->f[9], hw, hi, lo, s->stream));
-        NB_TRY(batch_forces(hi, lo, s->queue_all.q, s->cfg.G, eps2, s->f[6], s->f[7], s->f[8], hw,
+        NB_TRY(batch_forces(hi, lo, s->queue_all, s->cfg.G, eps2, s->f[6], s->f[7], s->f[8], hw,
                             s->stream));
         NB_TRY(kick(NB_LEAPFROG, hw, dt, s->f[3], s->f[4], s->f[5], s->f[6], s->f[7], s->f[8],
                     nullptr, nullptr, nullptr, s->stream));
@@ -606,6 +623,11 @@ nb_status nb_server_create(const nb_server_config *cfg, nb_server **out)
     if (st == NB_OK) st = s->pool.reserve(sizeof(double) * 10 * s->ps);
     if (st == NB_OK) st = s->hi.reserve(sizeof(float4) * s->ps);
     if (st == NB_OK) st = s->lo.reserve(sizeof(float4) * s->ps);
+    // here, not when a job needs them: a server that has started has its planes
+    const size_t left = cfg->hbm_budget_bytes - std::min(cfg->hbm_budget_bytes, pool_bytes(s));
+    const size_t planes = std::min(kServePlaneBytes, left / 16);
+    if (st == NB_OK && cfg->direct_max_n > kServePairsMin && planes >= kServePlanesLeast)
+        st = s->part.reserve(planes);
     if (st == NB_OK) {
         e = cudaMemsetAsync(s->pool.ptr, 0, s->pool.bytes, s->stream);
         if (e != cudaSuccess) st = cuda_fail(e, "cudaMemsetAsync");
@@ -637,10 +659,10 @@ nb_status nb_server_destroy(nb_server *s)
         if (j->sim) nb_destroy(j->sim);
         if (j->step_done) cudaEventDestroy(j->step_done);
     }
-    DevBuf *bufs[] = {&s->pool, &s->hi, &s->lo, &s->queue_all.part, &s->queue_new.part};
+    DevBuf *bufs[] = {&s->pool, &s->hi, &s->lo, &s->part};
     for (DevBuf *b : bufs) b->release();
-    s->queue_all.q.release();
-    s->queue_new.q.release();
+    s->queue_all.release();
+    s->queue_new.release();
     if (s->tick_start) cudaEventDestroy(s->tick_start);
     if (s->direct_done) cudaEventDestroy(s->direct_done);
     for (int k = 0; k < kBHStreams; ++k)
