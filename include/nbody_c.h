@@ -308,7 +308,7 @@ nb_status nb_ensemble_profile(nb_ensemble *e, int enable);
  * that reached their step count.  A job's result does not depend on the other
  * jobs it ran with.
  * The budget covers the body pool (112 bytes a body), the partial sums of direct
- * jobs (at most 256 MiB, and a sixteenth of what the pool leaves; allocated with
+ * jobs (at most 1 GiB, and a sixteenth of what the pool leaves; allocated with
  * the server) and the Barnes-Hut jobs' simulations (470 bytes a body at leaf
  * capacity 8), running ones and those kept for jobs to come.  Submission asks
  * for 320 bytes a body; a job that was accepted so and needs more than there is

@@ -2518,6 +2518,7 @@ struct BHTree {
         gpcen, gquad, gkey, walks;
     bool with_quad = false;     // the nodes carry quadrupoles (quad, 2 float4 per node)
     bool ref_open = false;      // the reference's opening rule (the child toward the body too)
+    bool prefer_serial = false; // the serial walk where the ordered one would be taken
     Walk walk = Walk::kGroup;   // the next walk's kernels (ordered: gkey is set)
     int log_pool = 0;           // entries of the log pool
     bool pcen_valid = false;    // pcen holds the parent centres of the current topology
@@ -2536,6 +2537,8 @@ void bh_mark_count_stale(BHTree *t)
 {
     if (t) t->num_nodes = -1;
 }
+
+void bh_prefer_serial(BHTree *t, bool serial) { t->prefer_serial = serial; }
 
 BHTree *bh_create() { return new BHTree(); }
 
@@ -2992,6 +2995,7 @@ nb_status bh_compute(BHTree *t, const double *x, const double *y, const double *
     t->with_quad = quad;
     t->ref_open = ref_open;
     t->walk = choose_walk(n, theta, leaf_capacity, ref_open);
+    if (t->walk == Walk::kOrdered && t->prefer_serial) t->walk = Walk::kSerial;
     t->log_pool = log_pool_entries(n, theta, leaf_capacity, ref_open);
     if (ax && reuse > 1 && t->tree_valid && t->n == n && t->evals_since_build < reuse) {
         NB_TRY(refit(t, x, y, z, m, n, st));

@@ -336,6 +336,9 @@ nb_status batch_sorted_forces(BatchSorted &b, const double *x, const double *y, 
 struct BHTree;  // opaque, defined in nb_bh.cu
 BHTree *bh_create();
 void bh_destroy(BHTree *t);
+// Whether walks that would be ordered go one warp each (the same bits): less work, for a
+// GPU that other trees fill, and a longer wait for a lone one.
+void bh_prefer_serial(BHTree *t, bool serial);
 // The tree object for other bodies: no topology, its counters at zero; its buffers stay.
 nb_status bh_restart(BHTree *t, cudaStream_t st);
 // Builds the tree of (x,y,z,m) and, when ax != nullptr, walks it writing
@@ -405,6 +408,7 @@ struct nb_sim {
     nb::DevBuf rk4;                  // RK4 stage states and accelerations
     nb::DevBuf diag_scratch;
     nb::BHTree *bh = nullptr;
+    bool bh_serial = false;          // bh_prefer_serial; a captured step keeps its walk
 
     // One step as a CUDA graph (nb_step): captured on the second of two
     // consecutive eligible steps with the same integrator and dt, replayed

@@ -50,12 +50,21 @@ constexpr size_t kDirectBytesPerBody = 10 * 8 + 32;  // FP64 planes + hi/lo mirr
 // waits until no other tree is resident (it was accepted, so it runs).
 constexpr size_t kBHBytesPerBody = 320;
 // Partial planes of the direct jobs, one buffer for both work queues: at most this, and a
-// sixteenth of what the budget leaves beside the pool.  A tick of a full pool of 2 Mi
-// bodies goes through it in about five passes, of 22,000 CTAs each.
-constexpr size_t kServePlaneBytes = (size_t)256 << 20;
+// sixteenth of what the budget leaves beside the pool.  At saturation with a pool of 2 Mi
+// bodies the median step takes 9.2 ms with 1 GiB, 11.0 with 256 MiB (five passes a tick).
+constexpr size_t kServePlaneBytes = (size_t)1 << 30;
 // Below this every direct job goes by rows, which need no planes.
 constexpr size_t kServePlanesLeast = (size_t)16 << 20;
 constexpr int kBHStreams = 16;
+// From this many bodies in resident trees on, their walks go one warp each, which costs
+// the least in all; below the second number again by the ordered walk, which finishes
+// each soonest.  The bits are the same.  A tick of K trees of n bodies, ordered / serial,
+// in ms:
+//   60,000 x 1, 4, 8, 16, 32    0.45 / 0.72   0.70 / 0.88   1.10 / 1.20   1.89 / 1.80   3.64 / 3.36
+//   20,000 x 8, 16, 32, 64      0.63 / 0.71   0.99 / 0.89   1.83 / 1.57   3.47 / 2.88
+//   250,000 x 1, 2, 4, 8        0.92 / 0.96   1.30 / 1.34   2.23 / 2.07   4.10 / 3.55
+// At saturation (200 jobs/s offered for 10 s) 940 / 1070 Gint/s, p99 step 119 / 89 ms.
+constexpr size_t kSerialFrom = 640000, kSerialBelow = 400000;
 constexpr size_t kIdleSims = 32;
 
 struct Job {
@@ -239,6 +248,7 @@ struct nb_server {
     size_t idle_bytes = 0;
     size_t peak_bytes = 0;
     bool items_dirty = true;
+    bool serial_walks = false;
     cudaEvent_t tick_start = nullptr, direct_done = nullptr;
     // statistics
     std::vector<double> step_ms, queue_ms;
@@ -487,6 +497,15 @@ nb_status tick(nb_server *s)
     s->max_running = std::max(s->max_running, (int)s->running.size());
     std::vector<Job *> direct, bh;
     for (auto &j : s->running) (j->direct ? direct : bh).push_back(j.get());
+    size_t tree_bodies = 0;
+    for (Job *j : bh) tree_bodies += j->n;
+    if (tree_bodies >= kSerialFrom) s->serial_walks = true;
+    if (tree_bodies < kSerialBelow) s->serial_walks = false;
+    for (Job *j : bh)
+        if (j->sim->bh_serial != s->serial_walks) {
+            j->sim->bh_serial = s->serial_walks;
+            reset_step_graph(j->sim);  // nothing of it is in flight between ticks
+        }
     const double eps2 = s->cfg.softening * s->cfg.softening;
     const double dt = s->cfg.dt;
     const int hw = (int)s->slots.high_water;

@@ -157,6 +157,7 @@ nb_status eval_forces(nb_sim *s, const double *px, const double *py, const doubl
     }
     case NB_BARNES_HUT:
         if (!s->bh) s->bh = bh_create();
+        bh_prefer_serial(s->bh, s->bh_serial);
         return bh_compute(s->bh, px, py, pz, s->m(), n, s->cfg.G, eps2, s->cfg.theta,
                           s->cfg.leaf_capacity, oax, oay, oaz, s->stream, timer,
                           NB_FLAG_BH_REUSE_OF(s->cfg.flags),
