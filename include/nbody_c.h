@@ -451,7 +451,7 @@ nb_status nb_checkpoint_load(nb_sim *sim, const char *path);
  * its own pool allocator, a plugin with a fixed device-memory budget, a loop
  * that cannot take the implicit synchronisation of cudaMalloc/cudaFree).
  * Computes G-scaled accelerations of n bodies with the all-pairs mixed kernels
- * (split, all-pairs sum, combine) from caller-owned DEVICE arrays x, y, z, m
+ * from caller-owned DEVICE arrays x, y, z, m
  * into caller-owned DEVICE arrays ax, ay, az, on `stream` (NULL = legacy
  * default stream), asynchronously.  It never runs the Hilbert-sorted kernel
  * that NB_DIRECT_MIXED uses from 16,384 bodies nor the unordered-pairs one it uses

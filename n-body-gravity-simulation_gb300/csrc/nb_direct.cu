@@ -3,8 +3,8 @@
 // Replaces computeAccelerationNaiveKernel (CUDA/src/force_calculator_naive.cu:4-59,
 // one FP64 thread per body, 256-body tiles, ceil(N/256) CTAs).  Two kernels:
 //
-//  * direct_mixed_kernel -- the mixed path of small systems and of the no-allocation
-//    entry point.  Each body is held as a float4
+//  * direct_mixed_kernel -- the mixed term over ordered pairs: the no-allocation entry
+//    point from 4096 bodies.  Each body is held as a float4
 //    "hi" (x, y, z, m) plus a float4 "lo" (x - hi, ...): a double-single copy of
 //    its FP64 position.  The pair displacement is formed as
 //    (xj_hi - xi_hi) + (xj_lo - xi_lo), which is exact to FP32 rounding for close
@@ -21,6 +21,8 @@
 //    as FP32 (sum, comp) and the segments are combined as a double-single,
 //    scaled by G in FP64.
 //    The tensor cores stay idle: a softened 1/r^3 sum is not a contraction.
+//
+//  * direct_mixed_small_kernel -- the same term below 4096 bodies, in one launch.
 //
 //  * direct_mixed_pairs_kernel -- the same term over unordered pairs from 4096
 //    bodies (below 16,384, where the Hilbert-sorted path takes over).
@@ -666,88 +668,38 @@ int pick_segments(int iblocks, int tiles, int slots)
     return best;
 }
 
-template <int BLOCK, int IPT>
-int resident_ctas(const void *fn)
-{
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, BLOCK, 0);
-    return std::max(1, per_sm) * device_props().num_sms;
-}
-
 constexpr int kMixBlock = 256;
 constexpr int kMixIpt = 4;
 constexpr size_t kPairPlaneBytes = (size_t)512 << 20;  // partial planes per pass
 constexpr int kF64RowMax = 512;  // largest N of the one-warp-per-body FP64 kernel
 constexpr size_t kF64PlaneBytes = (size_t)512 << 20;  // FP64 partial planes per pass
 
-template <int B, int I>
 int mix_slots()
 {
-    static const int slots = resident_ctas<B, I>((const void *)direct_mixed_kernel<B, I, false>);
+    static const int slots = [] {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, (const void *)direct_mixed_kernel<kMixBlock, kMixIpt, false>, kMixBlock, 0);
+        return std::max(1, per_sm) * device_props().num_sms;
+    }();
     return slots;
 }
 
-int mix_slots_for(int block, int ipt)
+// Launches the small systems' kernel.
+nb_status launch_small(const float4 *hi, const float4 *lo, int n, double G, double eps2,
+                       double *ax, double *ay, double *az, cudaStream_t st,
+                       const AfterForce &after)
 {
-    if (block == kMixBlock && ipt == kMixIpt) return mix_slots<kMixBlock, kMixIpt>();
-    if (block == 32 && ipt == 1) return mix_slots<32, 1>();
-    if (block == 32 && ipt == 2) return mix_slots<32, 2>();
-    return 0;
-}
-
-template <int B, int I>
-void launch_mixed_shape(dim3 grid, cudaStream_t st, const float4 *hi, const float4 *lo, int n,
-                        double eps2, int seg_len, float *psum, float *pcomp)
-{
-    if (eps2 > 0.0)
-        direct_mixed_kernel<B, I, false>
-            <<<grid, B, 0, st>>>(hi, lo, n, (float)eps2, seg_len, psum, pcomp);
-    else
-        direct_mixed_kernel<B, I, true><<<grid, B, 0, st>>>(hi, lo, n, 0.0f, seg_len, psum, pcomp);
-}
-
-// Launches the all-pairs kernel of plan p (partials psum/pcomp sized for
-// p.segments); returns false for a shape that is not compiled in.
-bool launch_mixed(const DirectPlan &p, cudaStream_t st, const float4 *hi, const float4 *lo,
-                  int n, double eps2, float *psum, float *pcomp)
-{
-    const int per_cta = p.block * p.ipt;
-    dim3 grid((n + per_cta - 1) / per_cta, p.segments);
-    const int seg_len = p.seg_tiles * p.block;
-    if (p.block == kMixBlock && p.ipt == kMixIpt)
-        launch_mixed_shape<kMixBlock, kMixIpt>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
-    else if (p.block == 32 && p.ipt == 1)
-        launch_mixed_shape<32, 1>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
-    else if (p.block == 32 && p.ipt == 2)
-        launch_mixed_shape<32, 2>(grid, st, hi, lo, n, eps2, seg_len, psum, pcomp);
-    else
-        return false;
-    return true;
-}
-
-DirectPlan plan_for_shape(int n, int block, int ipt)
-{
-    DirectPlan p;
-    p.block = block;
-    p.ipt = ipt;
-    const int per_cta = block * ipt;
-    const int iblocks = (n + per_cta - 1) / per_cta;
-    const int tiles = (n + block - 1) / block;
-    p.segments = pick_segments(iblocks, tiles, mix_slots_for(block, ipt));
-    p.seg_tiles = (tiles + p.segments - 1) / p.segments;
-    p.segments = (tiles + p.seg_tiles - 1) / p.seg_tiles;
-    return p;
+    const int tiles = (n + 31) / 32, warps = kSmallCtas * kSmallWarps;
+    auto *kernel = eps2 > 0.0 ? direct_mixed_small_kernel<false> : direct_mixed_small_kernel<true>;
+    kernel<<<tiles * kSmallCtas, 32 * kSmallWarps, 0, st>>>(
+        hi, lo, n, eps2 > 0.0 ? (float)eps2 : 0.0f, (tiles + warps - 1) / warps, G, ax, ay, az,
+        after);
+    NB_LAUNCH_CHECK();
+    return NB_OK;
 }
 
 } // namespace
-
-// The ordered-pairs kernel's shape: one-warp CTAs, as many as the j-split allows,
-// for small systems; kMixBlock x kMixIpt above (the no-allocation entry point).
-DirectPlan direct_mixed_plan(int n)
-{
-    if (n < 4096) return plan_for_shape(n, 32, n < 2048 ? 1 : 2);
-    return plan_for_shape(n, kMixBlock, kMixIpt);
-}
 
 nb_status split_positions(const double *x, const double *y, const double *z, const double *m,
                           int n, float4 *hi, float4 *lo, cudaStream_t st)
@@ -800,12 +752,7 @@ nb_status direct_mixed(const float4 *hi, const float4 *lo, int n, double G, doub
     if (n >= kMixedPairsMin)
         return direct_mixed_pairs(hi, lo, n, G, eps2, ax, ay, az, partials, st, timer, after);
     if (timer && timer->start) NB_CUDA_TRY(cudaEventRecord(timer->start, st));
-    const int tiles = (n + 31) / 32, warps = kSmallCtas * kSmallWarps;
-    auto *kernel = eps2 > 0.0 ? direct_mixed_small_kernel<false> : direct_mixed_small_kernel<true>;
-    kernel<<<tiles * kSmallCtas, 32 * kSmallWarps, 0, st>>>(
-        hi, lo, n, eps2 > 0.0 ? (float)eps2 : 0.0f, (tiles + warps - 1) / warps, G, ax, ay, az,
-        after);
-    NB_LAUNCH_CHECK();
+    NB_TRY(launch_small(hi, lo, n, G, eps2, ax, ay, az, st, after));
     if (timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));
     return NB_OK;
 }
@@ -895,10 +842,10 @@ nb_status direct_fp64(const double *x, const double *y, const double *z, const d
 // pool allocator, a plugin that is given a fixed device-memory budget at
 // start-up, or a real-time loop that cannot afford the implicit device-wide
 // synchronisation an allocation or free can cause.  For them,
-// nb_direct_mixed_forces_noalloc runs the same split / all-pairs / combine
-// kernels as the NB_DIRECT_MIXED method, but keeps its scratch (the float4
-// hi/lo mirror of the bodies and the per-segment Kahan partial sums) in the
-// file-scope device array below instead of memory it allocates.
+// nb_direct_mixed_forces_noalloc keeps its scratch in the file-scope device array
+// below instead of memory it allocates: the float4 hi/lo mirror of the bodies and, from
+// kMixedPairsMin bodies, the per-segment Kahan partial sums of the ordered pairs.  Below,
+// it launches the kernel of the NB_DIRECT_MIXED method, which needs the mirror alone.
 //
 // The array is kNoAllocScratchBytes (16 MiB) on every device that loads this
 // library, held until the process exits, and limits n to kNoAllocMaxBodies.
@@ -966,27 +913,33 @@ extern "C" nb_status nb_direct_mixed_forces_noalloc(size_t n, const double *x, c
     float4 *lo = reinterpret_cast<float4 *>(static_cast<unsigned char *>(base) + mirror);
     float *psum = reinterpret_cast<float *>(static_cast<unsigned char *>(base) + 2 * mirror);
 
-    // Same plan as the allocating path, with the j-split capped so that the
-    // partial sums fit the remaining scratch.
-    DirectPlan p = direct_mixed_plan(ni);
-    const int tiles = (ni + p.block - 1) / p.block;
-    const size_t per_segment = sizeof(float) * 6 * n;
-    const int max_segments = (int)std::max<size_t>(1, (kNoAllocScratchBytes - 2 * mirror) /
-                                                          per_segment);
-    if (p.segments > max_segments) {
-        p.seg_tiles = (tiles + max_segments - 1) / max_segments;
-        p.segments = (tiles + p.seg_tiles - 1) / p.seg_tiles;
-    }
-    float *pcomp = psum + 3 * n * (size_t)p.segments;
-
     split_kernel<<<(ni + 255) / 256, 256, 0, st>>>(x, y, z, m, ni, hi, lo);
     NB_LAUNCH_CHECK();
     const double eps2 = softening * softening;
-    if (!launch_mixed(p, st, hi, lo, ni, eps2, psum, pcomp))
-        return fail(NB_ERR_UNSUPPORTED, "nb_direct_mixed_forces_noalloc: tile shape");
+    if (ni < kMixedPairsMin)
+        return launch_small(hi, lo, ni, G, eps2, ax, ay, az, st, AfterForce{});
+
+    // i-blocks by j-segments in whole waves, the segments few enough for their partial
+    // sums to fit the remaining scratch
+    const int iblocks = (ni + kMixBlock * kMixIpt - 1) / (kMixBlock * kMixIpt);
+    const int tiles = (ni + kMixBlock - 1) / kMixBlock;
+    const size_t per_segment = sizeof(float) * 6 * n;
+    const int max_segments = (int)std::max<size_t>(1, (kNoAllocScratchBytes - 2 * mirror) /
+                                                          per_segment);
+    int segments = std::min(pick_segments(iblocks, tiles, mix_slots()), max_segments);
+    const int seg_tiles = (tiles + segments - 1) / segments;
+    segments = (tiles + seg_tiles - 1) / seg_tiles;
+    float *pcomp = psum + 3 * n * (size_t)segments;
+    const dim3 grid(iblocks, segments);
+    if (eps2 > 0.0)
+        direct_mixed_kernel<kMixBlock, kMixIpt, false><<<grid, kMixBlock, 0, st>>>(
+            hi, lo, ni, (float)eps2, seg_tiles * kMixBlock, psum, pcomp);
+    else
+        direct_mixed_kernel<kMixBlock, kMixIpt, true><<<grid, kMixBlock, 0, st>>>(
+            hi, lo, ni, 0.0f, seg_tiles * kMixBlock, psum, pcomp);
     NB_LAUNCH_CHECK();
     combine_mixed_kernel<<<(ni + 31) / 32, 32 * kCombineGroups, 0, st>>>(
-        psum, pcomp, ni, p.segments, G, ax, ay, az);
+        psum, pcomp, ni, segments, G, ax, ay, az);
     NB_LAUNCH_CHECK();
     return NB_OK;
 }

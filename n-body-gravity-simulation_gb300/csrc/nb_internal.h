@@ -103,13 +103,6 @@ struct AfterForce {
 };
 
 // ---------------------------------------------------------------- direct sum
-struct DirectPlan {
-    int block = 256;    // threads per CTA
-    int ipt = 4;        // i-bodies per thread
-    int segments = 1;   // j-split factor (CTAs along y)
-    int seg_tiles = 1;  // j-tiles per segment
-};
-
 // Mixed FP32/double-single all-pairs kernel.  hi/lo: float4 (x, y, z, m) and
 // (x_lo, y_lo, z_lo, 0) of every body.  Writes G * sum into ax/ay/az (FP64).
 // after.hi, after.lo: below kMixedPairsMin other arrays than hi, lo, since one launch
