@@ -209,7 +209,7 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     const int ta = min(kBatchTiles, tiles - ti0), tb = min(kBatchTiles, tiles - tj0);
     const float4 *bhi = hi + sd.first, *blo = lo + sd.first;
     const float2 e2 = dup2(eps2);
-    const bool soft = eps2 >= 1e-22f;  // equal_range's nearest pair
+    const bool soft = equal_soft(eps2);
     const size_t plane = (size_t)sd.n;
     float2 *pa = part + sd.part0 + 3 * plane * (PARTS ? it.p - sd.p0 : it.p);
     float2 *pb = part + sd.part0 +

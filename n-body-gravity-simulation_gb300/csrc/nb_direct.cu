@@ -299,7 +299,7 @@ direct_mixed_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restric
     const bool two = u + 1 < ta;
     const float2 e2 = dup2(eps2);
     const float c[3] = {0.f, 0.f, 0.f};
-    const bool soft = eps2 >= 1e-22f;  // equal_range's nearest pair
+    const bool soft = equal_soft(eps2);
     tile_sums_zero(jsum, lane);
     tile_sums_zero(isum[0], lane);
     tile_sums_zero(isum[1], lane);

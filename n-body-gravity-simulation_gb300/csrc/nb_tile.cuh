@@ -266,6 +266,11 @@ __device__ __forceinline__ void tile_relative(const float4 h, const float4 l, co
     }
     m = h.w;
 }
+// The same for any pair of bodies that are tile_in_span, by the softening alone.
+__device__ __forceinline__ bool equal_soft(float eps2)
+{
+    return equal_range(0.f, 7.5e21f, eps2);
+}
 // Coordinates whose differences stay within equal_range's farthest pair.
 __device__ __forceinline__ bool tile_in_span(const float (&S)[3])
 {
