@@ -516,6 +516,8 @@ nb_status nb_bind_device(nb_sim *s, size_t n, double *const *arrays10)
         for (int k = 0; k < 10; ++k) s->f[k] = s->state.as<double>() + k * ps;
         s->n = std::min(s->n, s->capacity);
         s->forces_valid = false;
+        bh_invalidate(s->bh);
+        reset_step_graph(s);  // it holds the bound arrays
         return NB_OK;
     }
     if (n > s->capacity) return fail(NB_ERR_CAPACITY, "n exceeds the capacity of the simulation");
