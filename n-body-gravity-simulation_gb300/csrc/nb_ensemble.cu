@@ -33,7 +33,6 @@ struct nb_ensemble {
     double *f[10] = {};
     std::vector<nb::SysDesc> sys;
     nb::BatchQueue queue;
-    int ipt_bucket[32];
     bool ready = false;  // the work queue is uploaded
     bool forces_valid = false;
 
@@ -56,6 +55,14 @@ namespace nb {
 namespace {
 
 constexpr int kGraphChunk = 25;
+
+// i-bodies per lane of the kernels that sum a system of 2^bucket bodies: rows, or block
+// pairs (two i-tiles at a time).
+int bodies_per_lane(int bucket)
+{
+    const long long n = 1ll << bucket;
+    return n >= kBatchPairsMin && n < kBatchPairsMax ? 4 : 1;
+}
 
 nb_status upload_items(nb_ensemble *e)
 {
@@ -160,7 +167,6 @@ nb_status nb_ensemble_create(const nb_config *cfg, int num_systems, const int *s
     e->sizes.assign(sizes, sizes + num_systems);
     e->total = total;
     e->ps = (total + 31) / 32 * 32;
-    for (int b = 0; b < 32; ++b) e->ipt_bucket[b] = 2;
     if (stream) {
         e->stream = static_cast<cudaStream_t>(stream);
     } else {
@@ -254,7 +260,7 @@ nb_status nb_ensemble_tune(nb_ensemble *e, int *ipt_by_bucket)
     }
     NB_TRY(setup(e));
     if (ipt_by_bucket)
-        for (int b = 0; b < 32; ++b) ipt_by_bucket[b] = e->ipt_bucket[b];
+        for (int b = 0; b < 32; ++b) ipt_by_bucket[b] = bodies_per_lane(b);
     return NB_OK;
 }
 
@@ -354,7 +360,7 @@ nb_status nb_ensemble_info(nb_ensemble *e, nb_ensemble_info_t *info)
     for (int n : e->sizes) inter += (double)n * (double)(n - 1);
     info->interactions_per_eval = inter;
     info->work_items = (int)std::min<long long>(e->queue.num_items, INT32_MAX);
-    for (int b = 0; b < 32; ++b) info->ipt_by_bucket[b] = e->ipt_bucket[b];
+    for (int b = 0; b < 32; ++b) info->ipt_by_bucket[b] = bodies_per_lane(b);
     info->graph_launches = e->graph_launches;
     info->graph_steps = e->graph_steps;
     double total_ms = 0.0;
