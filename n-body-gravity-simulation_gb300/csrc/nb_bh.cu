@@ -2724,22 +2724,6 @@ nb_status bh_sort_keys(BHTree *t, int n, int first_shift, cudaStream_t st,
     return NB_OK;
 }
 
-nb_status bh_morton_order(BHTree *t, const double *x, const double *y, const double *z, int n,
-                          int levels, cudaStream_t st, const uint32_t **order,
-                          const double **root_centre)
-{
-    if (n <= 0) return NB_OK;
-    levels = std::max(1, std::min(levels, kMaxLevels));
-    // LSD passes over the top 3*levels bits: start at the lowest of them,
-    // rounded down to a digit boundary.
-    const int first_shift = std::max(0, (63 - 3 * levels) / 8 * 8);
-    NB_TRY(morton_sort(t, x, y, z, n, first_shift, st));
-    *order = t->order;
-    *root_centre = &t->root.as<BHRoot>()->cx;
-    t->tree_valid = false;  // the sort replaced the tree's codes
-    return NB_OK;
-}
-
 nb_status bh_hilbert_order(BHTree *t, const double *x, const double *y, const double *z, int n,
                            cudaStream_t st, const uint32_t **order, const double **root_centre)
 {

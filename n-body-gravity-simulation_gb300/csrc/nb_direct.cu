@@ -41,9 +41,6 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <cmath>
-#include <cstdlib>
-#include <cstring>
 #include <mutex>
 #include <string>
 

@@ -71,7 +71,6 @@ constexpr size_t kFarPlaneBytes = (size_t)1 << 30;  // its partial planes per pa
 constexpr int kExactWarps = 8;         // warps of exact_pairs_kernel per tile
 constexpr int kExactRound = 64;        // left-out pairs evaluated per round and warp
 constexpr int kResortEvals = 8;        // force evaluations per re-sort
-constexpr bool kHilbertOrder = true;   // sort along the Hilbert curve (else Morton)
 
 // The mass of a tile whose bodies do not all have one (compares false).
 #define kNoMass __int_as_float(0x7fffffff)
@@ -1070,10 +1069,7 @@ nb_status direct_mixed_sorted(const double *x, const double *y, const double *z,
     if (!b.sorter) b.sorter = bh_create();
     if (b.order_n != n || b.evals_since_sort >= kResortEvals) {
         // 2^30 cells: far smaller than a 32-body chunk
-        if (kHilbertOrder)
-            NB_TRY(bh_hilbert_order(b.sorter, x, y, z, n, st, &b.order, &b.centre));
-        else
-            NB_TRY(bh_morton_order(b.sorter, x, y, z, n, 10, st, &b.order, &b.centre));
+        NB_TRY(bh_hilbert_order(b.sorter, x, y, z, n, st, &b.order, &b.centre));
         b.order_n = n;
         b.evals_since_sort = 0;
     }

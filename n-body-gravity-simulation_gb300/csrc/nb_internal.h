@@ -353,15 +353,11 @@ void bh_invalidate(BHTree *t);
 // A replayed build changed the node count behind the host's back.
 void bh_mark_count_stale(BHTree *t);
 nb_status bh_info(BHTree *t, cudaStream_t st, nb_bh_info *info);
-// Morton order of the bodies by the top 3*levels code bits: *order maps a
-// sorted index to the original one; *root_centre points at the device copy of
-// the root cube centre (3 doubles), followed by the cube's side (a 4th
-// double).  Both stay valid until the next call on t.
-nb_status bh_morton_order(BHTree *t, const double *x, const double *y, const double *z, int n,
-                          int levels, cudaStream_t st, const uint32_t **order,
-                          const double **root_centre);
-// The same for the order along the Hilbert curve through the 2^10-cell grid of
-// the root cube (runs of sorted bodies fill compact regions).
+// Order of the bodies along the Hilbert curve through the 2^10-cell grid of the root cube
+// (runs of sorted bodies fill compact regions): *order maps a sorted index to the
+// original one; *root_centre points at the device copy of the root cube centre (3
+// doubles), followed by the cube's side (a 4th double).  Both stay valid until the next
+// call on t.
 nb_status bh_hilbert_order(BHTree *t, const double *x, const double *y, const double *z, int n,
                            cudaStream_t st, const uint32_t **order, const double **root_centre);
 // A stable sort of caller-made keys: bh_sort_buffers returns the key and

@@ -73,30 +73,6 @@ __device__ __forceinline__ float rel_s(float h, float l, float c)
     return s + (e + l);
 }
 
-// a += m_j (r_j - r_i) / (|r_j - r_i|^2 + eps2)^(3/2) for one (i, j) pair.
-// ZERO_SOFT: eps2 == 0, where the j == i term (r2 == 0) must give 0.
-template <bool ZERO_SOFT>
-__device__ __forceinline__ void pair_term(const float4 &H, const float4 &L, float xh, float yh,
-                                          float zh, float xl, float yl, float zl, float eps2,
-                                          float &ax, float &ay, float &az)
-{
-    const float dx = (H.x - xh) + (L.x - xl);
-    const float dy = (H.y - yh) + (L.y - yl);
-    const float dz = (H.z - zh) + (L.z - zl);
-    const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-    float inv = rsqrt_mufu(r2);
-    if (ZERO_SOFT) inv = (r2 > 0.f) ? inv : 0.f;
-    const float inv2 = inv * inv;
-    // MUFU rsqrt is good to ~1.3e-7; y^3 with y = y0 (1 + d) is y0^3 (1 - 3d)
-    // to first order and r2 y0^2 = 1 + 2d, so y^3 ~= y0^3 (2.5 - 1.5 r2 y0^2):
-    // one Newton step folded into the cube leaves an O(d^2) error.
-    const float corr = fmaf(-1.5f, r2 * inv2, 2.5f);
-    const float s = ((H.w * inv) * inv2) * corr;
-    ax = fmaf(dx, s, ax);
-    ay = fmaf(dy, s, ay);
-    az = fmaf(dz, s, az);
-}
-
 // ---------------------------------------------------------------- packed f32x2
 // sm_100-class SMs run FP32 add, multiply and FMA on register pairs at the
 // FP32 pipe's lane rate for half the issue slots; each lane rounds exactly
@@ -108,8 +84,10 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
-// m r^-3 of a j-pair with the folded Newton step of pair_term; ZERO_SOFT
-// zeroes the r2 == 0 (j == i) lane.
+// m r^-3 of a j-pair; ZERO_SOFT: eps2 == 0, where the j == i lane (r2 == 0) gives 0.
+// MUFU rsqrt is good to ~1.3e-7; y^3 with y = y0 (1 + d) is y0^3 (1 - 3d)
+// to first order and r2 y0^2 = 1 + 2d, so y^3 ~= y0^3 (2.5 - 1.5 r2 y0^2):
+// one Newton step folded into the cube leaves an O(d^2) error.
 template <bool ZERO_SOFT>
 __device__ __forceinline__ float2 pair_scale(float2 r2, float2 m)
 {
@@ -205,7 +183,7 @@ __device__ __forceinline__ PairGeom pair_geom(const JPair &j, float2 nxh, float2
     return g;
 }
 
-// The double-single pair term of pair_term for a j-pair against one i-body.
+// a += m_j (r_j - r_i) / (|r_j - r_i|^2 + eps2)^(3/2) for a j-pair against one i-body.
 template <bool ZERO_SOFT>
 __device__ __forceinline__ void pair_term2(const JPair &j, float2 nxh, float2 nyh, float2 nzh,
                                            float2 nxl, float2 nyl, float2 nzl, float2 e2,
