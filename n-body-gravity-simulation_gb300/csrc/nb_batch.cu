@@ -176,8 +176,8 @@ template <bool SORTED, bool ZERO_SOFT, bool PARTS>
 __global__ void __launch_bounds__(32, kBatchCtas)
 batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
                    const float4 *__restrict__ boxes, const SysDesc *__restrict__ sys,
-                   const PairItem *__restrict__ items, float eps2, float2 *__restrict__ part,
-                   double G, const uint32_t *__restrict__ order, double *__restrict__ ax,
+                   const PairItem *__restrict__ items, float eps2, bool soft,
+                   float2 *__restrict__ part, double G, const uint32_t *__restrict__ order, double *__restrict__ ax,
                    double *__restrict__ ay, double *__restrict__ az, int total, int num_tiles)
 {
     __shared__ union {
@@ -209,7 +209,6 @@ batch_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
     const int ta = min(kBatchTiles, tiles - ti0), tb = min(kBatchTiles, tiles - tj0);
     const float4 *bhi = hi + sd.first, *blo = lo + sd.first;
     const float2 e2 = dup2(eps2);
-    const bool soft = equal_soft(eps2);
     const size_t plane = (size_t)sd.n;
     float2 *pa = part + sd.part0 + 3 * plane * (PARTS ? it.p - sd.p0 : it.p);
     float2 *pb = part + sd.part0 +
@@ -642,8 +641,8 @@ static nb_status launch_batch(const float4 *hi, const float4 *lo, const float4 *
     for (const BatchPass &p : q.passes) {
         auto *kernel = p.parts ? batch_kernel<true>(boxes, eps2) : batch_kernel<false>(boxes, eps2);
         kernel<<<p.items, 32, 0, st>>>(hi, lo, boxes, sys, q.d_items.as<PairItem>() + p.item0,
-                                       eps2 > 0.0 ? (float)eps2 : 0.0f, q.part, G, order, ax, ay,
-                                       az, total, num_tiles);
+                                       eps2 > 0.0 ? (float)eps2 : 0.0f, equal_soft(eps2), q.part, G,
+                                       order, ax, ay, az, total, num_tiles);
         NB_LAUNCH_CHECK();
         if (timer && timer->stop && &p == &q.passes.back())
             NB_CUDA_TRY(cudaEventRecord(timer->stop, st));

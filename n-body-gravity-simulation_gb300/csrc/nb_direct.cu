@@ -280,7 +280,8 @@ constexpr int kPairH = kPairTiles / 2, kPairV = kPairTiles;
 template <bool ZERO_SOFT>
 __global__ void __launch_bounds__(32, 16)
 direct_mixed_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo, int n,
-                          float eps2, int blocks, int p0, int np, float2 *__restrict__ part)
+                          float eps2, bool soft, int blocks, int p0, int np,
+                          float2 *__restrict__ part)
 {
     __shared__ TileJ stage;
     __shared__ TileJLow low;
@@ -296,7 +297,6 @@ direct_mixed_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restric
     const bool two = u + 1 < ta;
     const float2 e2 = dup2(eps2);
     const float c[3] = {0.f, 0.f, 0.f};
-    const bool soft = equal_soft(eps2);
     tile_sums_zero(jsum, lane);
     tile_sums_zero(isum[0], lane);
     tile_sums_zero(isum[1], lane);
@@ -726,11 +726,11 @@ static nb_status direct_mixed_pairs(const float4 *hi, const float4 *lo, int n, d
         const int np = std::min(pass, diagonals - p0);
         const unsigned grid = (unsigned)blocks * (unsigned)np * (kPairH * kPairV);
         if (eps2 > 0.0)
-            direct_mixed_pairs_kernel<false><<<grid, 32, 0, st>>>(hi, lo, n, (float)eps2, blocks,
-                                                                  p0, np, part);
+            direct_mixed_pairs_kernel<false><<<grid, 32, 0, st>>>(
+                hi, lo, n, (float)eps2, equal_soft(eps2), blocks, p0, np, part);
         else
-            direct_mixed_pairs_kernel<true><<<grid, 32, 0, st>>>(hi, lo, n, 0.0f, blocks, p0, np,
-                                                                 part);
+            direct_mixed_pairs_kernel<true><<<grid, 32, 0, st>>>(hi, lo, n, 0.0f, false, blocks,
+                                                                 p0, np, part);
         NB_LAUNCH_CHECK();
         const bool last = p0 + np == diagonals;
         if (last && timer && timer->stop) NB_CUDA_TRY(cudaEventRecord(timer->stop, st));

@@ -246,7 +246,7 @@ __device__ __forceinline__ void tile_self(const TileJ &t, const TileJLow *low, i
 
 // Whether r^-3 of pairs at least sqrt(gap2 + eps2) and at most sqrt(span2 + eps2)
 // apart is well inside FP32's normal range (r in [1e-11, 1e11]).
-__device__ __forceinline__ bool equal_range(float gap2, float span2, float eps2)
+__host__ __device__ __forceinline__ bool equal_range(float gap2, float span2, float eps2)
 {
     return gap2 + eps2 >= 1e-22f && span2 + eps2 <= 1e22f;
 }
@@ -266,11 +266,9 @@ __device__ __forceinline__ void tile_relative(const float4 h, const float4 l, co
     }
     m = h.w;
 }
-// The same for any pair of bodies that are tile_in_span, by the softening alone.
-__device__ __forceinline__ bool equal_soft(float eps2)
-{
-    return equal_range(0.f, 7.5e21f, eps2);
-}
+// The same for any pair of bodies that are tile_in_span, by the softening alone: decided
+// on the host, once per launch.
+inline bool equal_soft(double eps2) { return equal_range(0.f, 7.5e21f, (float)eps2); }
 // Coordinates whose differences stay within equal_range's farthest pair.
 __device__ __forceinline__ bool tile_in_span(const float (&S)[3])
 {
