@@ -2031,13 +2031,19 @@ serial_walk_kernel(const BHGNode *__restrict__ gnodes, const unsigned char *__re
 //   n =  16,384        564 /  272     892 /  315        1817 /  426
 //   n = 100,000       1001 /  503    1921 /  782        3910 / 1048
 //   n = 400,000       1342 / 1227    3091 / 2410       11208 / 3598
-// (group_walk_kernel, in another order, took 0.83 times as long at n = 100,000, theta 0.5,
-// 0.82 at 400,000 and 0.77 under the reference's rule at 100,000.)
 // Up to kOrderedBodies, and always under the reference's rule, results are the serial
-// walk's bit for bit; beyond, where listing the terms apart from the
-// decisions eats what many warps gain (2^20 bodies: 2.88 ms serial, 2.28 by
-// group_walk_kernel), walks are of similar length and the order of summation shows in
-// velocities at 1e-8 of their scale after a step of 1e-3.
+// walk's bit for bit.  That has its price: by group_walk_kernel, in another order, an
+// evaluation takes about 0.8 times as long at every size (serial / ordered / group, disk,
+// theta 0.5):
+//   n =   200,000     936 /  722 /  602      with quadrupoles  1305 / 1140 /  991
+//   n =   400,000    1350 / 1227 /  993                        1917 / 2035 / 1697
+//   n =   524,288    1591 / 1570 / 1263                        2379 / 2657 / 2084
+//   n =   800,000    2087 / 2253 / 1689                        3236 / 3866 / 2923
+//   n = 1,048,576    2900 / 3083 / 2296                        4518 / 5424 / 4100
+// Summed in another order, velocities after a few steps of 1e-3 moved by up to 9e-8 of
+// their scale for trees of 16,000 to 200,000 bodies.  The line lies where the ordered walk
+// is no faster than the serial one; beyond, walks are of similar length and the order shows
+// at 1e-8.
 constexpr int kOrderedBodies = 524288;
 // Up to this many walks 16 warps decide one, above it 4 (16 / 4 warps at 256, 512 and
 // 1024 walks: 314 / 332, 320 / 318, 406 / 380 us).  Under the reference's rule always 16,
