@@ -181,12 +181,18 @@ def profiled_traffic(name: str):
     return None
 
 
-def fp32_roofline_gint(num_sms: int, mhz: float) -> float:
-    """All-pairs roofline: 12 FP32-pipe operations per interaction (3 FADD for
-    the displacement, 3 FFMA for r^2, 3 FMUL for m r^-3, 3 FFMA to accumulate)
-    on 128 FP32 lanes per SM per clock; the one MUFU rsqrt per interaction
-    (16/clk/SM) does not bind."""
-    return num_sms * mhz * 1e6 * 128.0 / 12.0 / 1e9
+def pair_ops(n: int) -> float:
+    """FP32-pipe operations an interaction cannot do without, in the kernel that n
+    bodies take: 12 where every ordered pair is evaluated (displacement 3, r^2 3,
+    m r^-3 3, accumulation 3; the MUFU rsqrt beside them does not bind), 8 where one r^-3 serves both bodies of a pair (16 a
+    pair: displacement 3, r^2 3, r^-3 2, two masses, two accumulations of 3)."""
+    return 8.0 if n >= 4096 else 12.0
+
+
+def fp32_roofline_gint(num_sms: int, mhz: float, ops: float) -> float:
+    """All-pairs roofline of `ops` FP32-pipe operations per interaction at 128 lanes
+    per SM and clock."""
+    return num_sms * mhz * 1e6 * 128.0 / ops / 1e9
 
 
 def load_oracle():
@@ -465,7 +471,7 @@ def run_bh(a, nb, torch, dev, stream, flush, np):
     if "rebuild" in variants:
         out.update(timed(0))
         out["timing"] = ("CUDA events per leapfrog step, L2 flushed before each; a build "
-                         "reads the node count on the host once per step")
+                         "makes no host read before its walk")
     keys = ("ms_per_step", "steps_per_s", "walk_ms", "interactions_per_body",
             "force_error_vs_direct")
     if "reuse4" in variants:
@@ -714,7 +720,8 @@ def run_ours(a, rank, world, local_rank):
     kernel_ms = prof["force_kernel_ms"] / max(1, prof["force_launches"])
     achieved = inter / (kernel_ms / 1e3) / 1e9
     clk = clocks.summary(t_wall0, t_wall1)
-    peak = fp32_roofline_gint(props.multi_processor_count, peaks.get("sm_max_mhz", 2070.0))
+    ops = pair_ops(n)
+    peak = fp32_roofline_gint(props.multi_processor_count, peaks.get("sm_max_mhz", 2070.0), ops)
     roofline = {
         "bound": "fp32",
         "kernel": ("direct_far_kernel" if n >= 16384 else "direct_mixed_pairs_kernel"
@@ -722,26 +729,26 @@ def run_ours(a, rank, world, local_rank):
         "achieved": achieved,
         "peak": peak, "unit": "Ginteractions/s", "frac": achieved / peak,
         "peak_basis": (f"{props.multi_processor_count} SMs x {peaks.get('sm_max_mhz', 2070.0)}"
-                       f" MHz ({peak_kind} sm_max_mhz) x 128 FP32 lanes / 12 FP32 ops per "
+                       f" MHz ({peak_kind} sm_max_mhz) x 128 FP32 lanes / {ops:g} FP32 ops per "
                        "interaction"),
         "traffic": None,
         "kernel_ms": kernel_ms,
     }
     if clk.get("sm_mhz"):
         roofline["frac_at_measured_clock"] = achieved / fp32_roofline_gint(
-            props.multi_processor_count, clk["sm_mhz"])
-    # the same fraction in FP32-pipe operations per second (12 per interaction)
-    roofline["achieved_fp32_tops"] = achieved * 12.0 / 1e3
-    roofline["peak_fp32_tops"] = peak * 12.0 / 1e3
+            props.multi_processor_count, clk["sm_mhz"], ops)
+    # the same fraction in FP32-pipe operations per second
+    roofline["achieved_fp32_tops"] = achieved * ops / 1e3
+    roofline["peak_fp32_tops"] = peak * ops / 1e3
     roofline["traffic"] = profiled_traffic("kernels_by_case.md") if n == N_BODIES else None
     roofline["algorithmic_bytes"] = 32 * n  # hi + lo mirror of every body, read once
     # the same kernel against a measured FP32-pipe rate (packed FMAs on every
     # SM, register-only probe), beside the lanes x clock peak above
     fma_rate = nb.debug_fp32_rate()
     roofline["peak_measured_fp32"] = {
-        "value": fma_rate / 12.0 / 1e9, "unit": "Ginteractions/s",
-        "frac": achieved / (fma_rate / 12.0 / 1e9), "fma_lane_tops": fma_rate / 1e12,
-        "basis": "nb_debug_fp32_rate (independent packed FMAs, best of 3 launches) / 12"}
+        "value": fma_rate / ops / 1e9, "unit": "Ginteractions/s",
+        "frac": achieved / (fma_rate / ops / 1e9), "fma_lane_tops": fma_rate / 1e12,
+        "basis": f"nb_debug_fp32_rate (independent packed FMAs, best of 3 launches) / {ops:g}"}
 
     extras = {}
     if not a.skip_extras and rank == 0:

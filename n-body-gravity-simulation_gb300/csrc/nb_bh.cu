@@ -22,24 +22,26 @@
 // Build.  After the sort, body i starts a node at depth d exactly when its
 // depth-d cell begins at i and that cell's parent holds more than
 // leaf_capacity bodies.  The nodes starting at i form a chain of consecutive
-// depths that ends at the first leaf; one thread per body finds its chain by
-// galloping over the sorted codes, an exclusive scan of the chain lengths
+// depths that ends at the first leaf; one thread per body finds its chain from
+// the depths that its code shares with its neighbours', an exclusive scan of the chain lengths
 // numbers every node in preorder (depth-first, children in Morton order), and
 // the node after a cell's subtree -- its skip pointer -- is simply the first
 // node of the body that follows the cell.  Masses and centres of mass come
 // from FP64 prefix sums of (m, m x, m y, m z) over the sorted bodies (positions
 // relative to the root centre), so no level-by-level pass is needed.
 //
-// Walk.  One CTA walks for 64 consecutive sorted bodies, two per lane of each of
-// its warps.  At each node every body applies the reference's opening test (open
+// Walk.  A walk serves 64 consecutive sorted bodies, two per lane of each warp that
+// shares it.  At each node every body applies the reference's opening test (open
 // when size^2 >= theta^2 d^2 to the COM, or when the node holds the body); the
 // node is opened if any body does (so each body gets a refinement of its own walk,
 // never a coarser one).  The children of every node are stored together (a
 // group): a warp decides the nodes of four groups at once, lists the monopoles of
 // the nodes no body opens and the bodies of opened leaves for evaluation, and
 // pushes the groups of opened internal nodes on the CTA's stack, which holds the
-// deepest tree's groups.  The stackless preorder walk over skip pointers finds the
-// same interactions (NB_BH_WALK=preorder).  Accelerations are scattered back
+// deepest tree's groups (group_walk_kernel).  Up to 524,288 bodies, and always under the
+// reference's opening rule, every body's terms are added in the order of a serial walk,
+// by serial_walk_kernel or by the ordered walk, which many warps share.  The stackless
+// preorder walk over skip pointers finds the same interactions (NB_BH_WALK=preorder).  Accelerations are scattered back
 // to the original order in FP64, multiplied by G.
 #include "nb_internal.h"
 #include "nb_after.cuh"

@@ -24,7 +24,7 @@
 // its own shared memory: no CTA-wide barrier.
 //
 // Measured at N = 65,536 (a velocity-Verlet step) and N = 400,003 (an
-// evaluation): 1.48 and 46.3 ms, where the row kernel over every j-chunk, each
+// evaluation): 1.51 and 47.7 ms, where the row kernel over every j-chunk, each
 // pair evaluated twice, took 1.98 and 67 ms.
 //
 // Packed arithmetic.  sm_100-class SMs execute FP32 add, multiply and FMA on
@@ -67,7 +67,9 @@ constexpr int kIpt = kTile / kChunk;   // 32-body i-chunks per warp
 constexpr int kFarTiles = 4;           // tiles per block of the far kernel
 // Its one-warp CTAs per SM: 12 / 14 / 16 measured 1.53 / 1.47 / 1.47 ms a step.
 constexpr int kFarCtas = 16;
-constexpr size_t kFarPlaneBytes = (size_t)1 << 30;  // its partial planes per pass
+// Its partial planes per pass.  Each pass ends with a thinly filled last wave: with 256
+// MiB an evaluation takes 3.3 % longer at N = 65,536 and 8.4 % at 400,003.
+constexpr size_t kFarPlaneBytes = (size_t)1 << 30;
 constexpr int kExactWarps = 8;         // warps of exact_pairs_kernel per tile
 constexpr int kExactRound = 64;        // left-out pairs evaluated per round and warp
 constexpr int kResortEvals = 8;        // force evaluations per re-sort
@@ -907,7 +909,7 @@ exact_pairs_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
 // passes (first: none yet), written back unless this is the last pass, which
 // adds the near segments (sum - comp; in strides too) and the left-out pairs:
 // a[order[i]] = G * (far + near + ex_i), scaled in FP64.  Bound by memory: one
-// thread per body had too few loads in flight (66 us at n = 65,536, 205 MB).
+// thread per body had too few loads in flight (66 us at n = 65,536 and half of the present 410 MB).
 constexpr int kCombineGroups = 8;
 __global__ void __launch_bounds__(32 * kCombineGroups)
 combine_sorted_kernel(const float2 *__restrict__ part, int blocks, int p0, int np, bool first,

@@ -228,15 +228,20 @@ constexpr int kBatchBlockBodies = 256;  // four tiles of 64
 // pairs).  On the 1024-system ensemble (n log-uniform in [32, 4096], two RK4 steps)
 // a line at 512 / 1024 / 2048 / beyond every system measured 7.58 / 7.69 / 8.12 /
 // 9.15 ms (one i-tile at a time; at 1024 / 2048 7.04 / 7.51 ms with four i-bodies per
-// lane).  It lies at 2048: in a smaller system one close pair can carry a body's whole
-// force, and the row sum is the order of rounding that its trajectory has had (of 30
-// ensembles, the largest difference of a velocity after two steps was 4.4e-8 of their
-// scale with the line at 1024, 2.5e-8 at 2048).
+// lane).  Against 64 bits neither sum is better: over 12 systems each of 600 to 2,047
+// bodies, Plummer and disk, the pairs' RMS error was 0.79 to 1.02 of the rows', the largest
+// of a body 1.6e-7 to 3.6e-7 and 1.9e-7 to 3.9e-7 of its terms' magnitudes.  The line lies
+// at 2048 so that smaller systems, in which one close pair can carry a body's whole
+// force, keep the sums and so the trajectories they have had (of 30 ensembles, the
+// largest difference of a velocity after two steps was 4.4e-8 of their scale with the line
+// at 1024, 2.5e-8 at 2048).
 constexpr int kBatchPairsMin = 2048;
 // The server's jobs run many steps and may be dense disks, in which a close pair carries
-// a force of 100 (1.4e-7 of the velocities' scale after four steps of 1e-3 at n = 2705 by
-// unordered pairs, against the row sum); up to 4095 bodies their work is a few percent
-// of the direct jobs' (a burst of 16 jobs: 15.7 ms, 15.5 by pairs from 1024).
+// a force of 100: the two sums of the same terms are apart by 1.4e-7 of the velocities'
+// scale after four steps of 1e-3 at n = 2705 (and as close to 64 bits: RMS errors of an
+// acceleration 6.4e-8 by pairs, 6.6e-8 by rows for disks of 3,000).  Up to 4095 bodies
+// their work is a few percent of the direct jobs' (a burst of 16 jobs: 15.7 ms, 15.5 by
+// pairs from 1024), so they keep the rows that their trajectories have had.
 constexpr int kServePairsMin = 4096;
 // Largest system summed over unordered pairs: the table of its items grows as n^2 (8
 // million at 2^20 bodies, 100 MB); larger ones go by rows, n / 32 items.

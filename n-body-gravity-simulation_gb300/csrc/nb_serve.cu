@@ -6,15 +6,14 @@
 //      that does not fit) while their device memory fits the HBM budget;
 //   2. advances every running job by one leapfrog step:
 //      - direct jobs (n < direct_max_n) live in one body pool and advance
-//        together: one per-body kick-drift and kick over the pool and one
-//        batched force launch over all of them (nb_batch.cu);
+//        together: one per-body kick-drift and kick over the pool and
+//        batched force launches over all of them (nb_batch.cu);
 //      - Barnes-Hut jobs each own a simulation object and run on one of
 //        kBHStreams streams (the process should allow that many hardware
 //        queues: CUDA_DEVICE_MAX_CONNECTIONS >= 16), each stream's jobs issued
 //        by that stream's thread of a pool kept for the server's lifetime (a
-//        tree build reads its node count on the host, which then blocks only
-//        that stream's later jobs), overlapping with the direct batch and
-//        with each other;
+//        full launch queue then blocks only that stream's later jobs),
+//        overlapping with the direct batch and with each other;
 //   3. retires jobs that reached their step count (state copied to the host,
 //      pool slots returned, simulation objects kept for jobs to come within
 //      the budget).
