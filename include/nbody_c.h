@@ -147,7 +147,14 @@ nb_status nb_config_default(nb_config *cfg);
 
 /* Creates a simulation able to hold up to `capacity` bodies on the current
  * CUDA device.  Replaces allocateParticles (CUDA/src/particle_data.cu:6-43)
- * together with the calculator constructors. */
+ * together with the calculator constructors.
+ * Beside the 80 bytes a body of the state, a simulation keeps work buffers from
+ * the first call that needs them until nb_destroy: partial sums of at most 1 GiB
+ * (mixed from 16,384 bodies) or 512 MiB (FP64 from 513; mixed from 4096) or one
+ * diagonal's (48 to 144 bytes a body), whichever is more; 32 or 64 bytes a body
+ * for the mixed method; about 390 for Barnes-Hut at leaf capacity 8 (more at
+ * theta below 0.5, with quadrupoles and under the reference's rule); 24 for
+ * velocity Verlet, 216 for RK4. */
 nb_status nb_create(const nb_config *cfg, size_t capacity, void *stream, nb_sim **out);
 
 /* Replaces freeParticles (CUDA/src/particle_data.cu:46-92) and the calculator

@@ -602,15 +602,24 @@ void BatchQueue::release()
     d_items.release();
 }
 
-nb_status upload_batch(BatchQueue &q, const BatchWork &w, cudaStream_t st)
+nb_status reserve_batch(BatchQueue &q, const BatchWork &w)
 {
     q.passes.clear();
+    if (w.sys.empty()) return NB_OK;
+    NB_TRY(q.d_sys.reserve(sizeof(SysDesc) * w.sys.size()));
+    NB_TRY(q.d_items.reserve(sizeof(PairItem) * w.items.size()));
+    if (w.blocks.empty()) return NB_OK;
+    return q.d_blocks.reserve(sizeof(PairItem) * w.blocks.size());
+}
+
+nb_status upload_batch(BatchQueue &q, const BatchWork &w, cudaStream_t st)
+{
+    NB_TRY(reserve_batch(q, w));
     q.num_tiles = w.num_tiles;
     q.num_items = (long long)w.items.size();
     auto put = [&](DevBuf &to, const void *from, size_t bytes) -> nb_status {
-        if (bytes == 0) return NB_OK;
-        NB_TRY(to.reserve(bytes));
-        NB_CUDA_TRY(cudaMemcpyAsync(to.ptr, from, bytes, cudaMemcpyHostToDevice, st));
+        if (bytes > 0)
+            NB_CUDA_TRY(cudaMemcpyAsync(to.ptr, from, bytes, cudaMemcpyHostToDevice, st));
         return NB_OK;
     };
     NB_TRY(put(q.d_sys, w.sys.data(), sizeof(SysDesc) * w.sys.size()));

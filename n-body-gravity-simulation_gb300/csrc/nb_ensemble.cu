@@ -116,6 +116,7 @@ nb_status step_direct(nb_ensemble *e, int integ, double dt, bool capturing)
 // Uploads the work queue and, for the sorted path, its tables.
 nb_status setup(nb_ensemble *e)
 {
+    e->ready = false;  // until all of it is there
     NB_TRY(upload_items(e));
     if (e->sorted)
         NB_TRY(batch_sorted_setup(e->sb, e->queue.d_sys.as<SysDesc>(), e->num_sys, e->queue.num_tiles,

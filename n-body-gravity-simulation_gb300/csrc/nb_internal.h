@@ -300,6 +300,8 @@ struct BatchQueue {
     size_t bytes() const { return d_sys.bytes + d_blocks.bytes + d_items.bytes; }
     void release();
 };
+// Room for w in q, whose contents then are void.
+nb_status reserve_batch(BatchQueue &q, const BatchWork &w);
 // Uploads w (and waits for the copies); q.part is the caller's to set.
 nb_status upload_batch(BatchQueue &q, const BatchWork &w, cudaStream_t st);
 // Mixed-precision forces of all systems of the queue.

@@ -72,6 +72,7 @@ struct Job {
     int steps = 0;
     int done = 0;
     bool direct = true;
+    bool fresh = true;          // its start-of-step force is still to come (direct)
     std::vector<double> init;   // 7 n: x y z vx vy vz m (until admitted)
     std::vector<double> result; // 10 n after retirement
     size_t first = 0;           // pool slot (direct)
@@ -268,13 +269,12 @@ size_t fixed_bytes(const nb_server *s)
     return pool_bytes(s) + s->part.bytes + s->queue_all.bytes() + s->queue_new.bytes();
 }
 
-nb_status upload_systems(nb_server *s, const std::vector<Job *> &jobs, BatchQueue &to)
+BatchWork systems_of(const nb_server *s, const std::vector<Job *> &jobs)
 {
     BatchWork w;
     for (Job *j : jobs) w.sys.push_back(SysDesc{(int)j->first, (int)j->n});
     build_batch(w, kServePairsMin, s->part.bytes);
-    to.part = s->part.as<float2>();
-    return upload_batch(to, w, s->stream);
+    return w;
 }
 
 // The device memory of a Barnes-Hut job's simulation.
@@ -366,7 +366,7 @@ void end_job(nb_server *s, std::unique_ptr<Job> j)
     s->finished[id] = std::move(j);
 }
 
-nb_status admit(nb_server *s, std::vector<Job *> &new_direct)
+nb_status admit(nb_server *s)
 {
     for (auto it = s->queue.begin(); it != s->queue.end();) {
         Job *j = it->get();
@@ -380,7 +380,6 @@ nb_status admit(nb_server *s, std::vector<Job *> &new_direct)
                     NB_CUDA_TRY(cudaMemcpyAsync(s->f[plane[k]] + first, j->init.data() + k * j->n,
                                                 j->n * sizeof(double), cudaMemcpyHostToDevice,
                                                 s->stream));
-                new_direct.push_back(j);
                 ok = true;
             }
         } else {
@@ -487,15 +486,17 @@ double ms_since(Clock::time_point t0)
 nb_status tick(nb_server *s)
 {
     NvtxRange range("server_tick");
-    std::vector<Job *> new_direct;
     auto t_phase = Clock::now();
-    NB_TRY(admit(s, new_direct));
+    NB_TRY(admit(s));
     s->admit_ms += ms_since(t_phase);
     t_phase = Clock::now();
     if (s->running.empty()) return NB_OK;
     s->max_running = std::max(s->max_running, (int)s->running.size());
-    std::vector<Job *> direct, bh;
-    for (auto &j : s->running) (j->direct ? direct : bh).push_back(j.get());
+    std::vector<Job *> direct, bh, new_direct;
+    for (auto &j : s->running) {
+        (j->direct ? direct : bh).push_back(j.get());
+        if (j->direct && j->fresh) new_direct.push_back(j.get());
+    }
     size_t tree_bodies = 0;
     for (Job *j : bh) tree_bodies += j->n;
     if (tree_bodies >= kSerialFrom) s->serial_walks = true;
@@ -510,10 +511,15 @@ nb_status tick(nb_server *s)
     const int hw = (int)s->slots.high_water;
     if (s->items_dirty) {
         const auto t_up = Clock::now();
-        NB_TRY(upload_systems(s, direct, s->queue_all));
+        NB_TRY(upload_batch(s->queue_all, systems_of(s, direct), s->stream));
         s->items_dirty = false;
         s->upload_ms += ms_since(t_up);
     }
+    // every allocation of the direct batch comes before anything is stepped: a tick that
+    // fails for one can be repeated
+    const BatchWork new_work = systems_of(s, new_direct);
+    NB_TRY(reserve_batch(s->queue_new, new_work));
+    s->queue_all.part = s->queue_new.part = s->part.as<float2>();
     NB_CUDA_TRY(cudaEventRecord(s->tick_start, s->stream));
     // BH streams wait for the tick start so that latencies share one origin
     for (int k = 0; k < kBHStreams; ++k)
@@ -547,11 +553,12 @@ nb_status tick(nb_server *s)
     if (!direct.empty()) {
         float4 *hi = s->hi.as<float4>(), *lo = s->lo.as<float4>();
         if (!new_direct.empty()) {
-            // start-of-step force of the jobs admitted this tick
-            NB_TRY(upload_systems(s, new_direct, s->queue_new));
+            // start-of-step force of the jobs admitted since the last one
+            NB_TRY(upload_batch(s->queue_new, new_work, s->stream));
             NB_TRY(split_positions(s->f[0], s->f[1], s->f[2], s->f[9], hw, hi, lo, s->stream));
             NB_TRY(batch_forces(hi, lo, s->queue_new, s->cfg.G, eps2, s->f[6], s->f[7],
                                 s->f[8], hw, s->stream));
+            for (Job *j : new_direct) j->fresh = false;
         }
         NB_TRY(kick_drift(NB_LEAPFROG, hw, dt, s->f[0], s->f[1], s->f[2], s->f[3], s->f[4],
                           s->f[5], s->f[6], s->f[7], s->f[8], nullptr, nullptr, nullptr,
