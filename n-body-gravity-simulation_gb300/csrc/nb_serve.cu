@@ -520,6 +520,7 @@ nb_status tick(nb_server *s)
     const BatchWork new_work = systems_of(s, new_direct);
     NB_TRY(reserve_batch(s->queue_new, new_work));
     s->queue_all.part = s->queue_new.part = s->part.as<float2>();
+    s->peak_bytes = std::max(s->peak_bytes, fixed_bytes(s) + s->bh_bytes + s->idle_bytes);
     NB_CUDA_TRY(cudaEventRecord(s->tick_start, s->stream));
     // BH streams wait for the tick start so that latencies share one origin
     for (int k = 0; k < kBHStreams; ++k)
