@@ -159,9 +159,12 @@ nb_status direct_mixed_sorted(const double *x, const double *y, const double *z,
                               double *ay, double *az, SortedBuffers &b, cudaStream_t st,
                               const KernelTimer *timer = nullptr);
 // Whether an evaluation of n bodies takes the sorted variant: flags
-// NB_FLAG_MIXED_SORTED / NB_FLAG_MIXED_UNSORTED decide, else n >= kSortedMinBodies
-// (measured on GB300 per evaluation of a Plummer sphere, unsorted vs sorted:
-// 12,288 bodies 0.120 vs 0.136 ms, 16,384 bodies 0.201 vs 0.194 ms).
+// NB_FLAG_MIXED_SORTED / NB_FLAG_MIXED_UNSORTED decide, else n >= kSortedMinBodies.
+// Per evaluation of a Plummer sphere, unsorted / sorted, in us: 8,192 bodies 46 / 143,
+// 16,384 134 / 221, 24,576 291 / 323, 32,768 500 / 501, 49,152 1103 / 919.  By time alone
+// the line would lie at 32,768; it lies where it did when the unsorted sum took ordered
+// pairs (201 / 194 us), since from there on results promise 1e-6 of every body's force,
+// which the sorted kernel alone gives.
 constexpr int kSortedMinBodies = 16384;
 bool direct_sorted_enabled(int n, int flags);
 
