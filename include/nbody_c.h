@@ -370,7 +370,8 @@ nb_status nb_server_submit(nb_server *s, size_t n, const double *x, const double
  * jobs.  A failure that belongs to one Barnes-Hut job (its allocation, load or
  * step returned an error) ends that job alone -- its result then reports the
  * error -- and the tick still returns NB_OK; a failure of the shared direct
- * batch or of the device fails the tick. */
+ * batch or of the device fails the tick.  A tick that failed for an allocation
+ * has stepped nothing and can be repeated. */
 nb_status nb_server_tick(nb_server *s, int *running, int *queued);
 /* State of a finished job (NB_ERR_NOT_LOADED until it finished; a job that
  * failed returns the status it failed with, its message in nb_last_error();
